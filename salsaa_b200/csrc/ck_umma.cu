@@ -2,6 +2,8 @@
 // products, and a self-test of the int8 tensor-core building block.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "../../include/salsaa_gpu.h"
 #include "kernels.cuh"
 #include "ntt.cuh"
@@ -1264,6 +1266,18 @@ int launch_nc_gram_sums(const u64* gram, u32 rows, const ModQ& M, const DevState
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "nc_gram_sums launch");
+}
+
+u32* tc_error_word() {
+  static std::atomic<u32*> word[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  u32* p = word[dev].load(std::memory_order_acquire);
+  if (p) return p;
+  void* v = nullptr;
+  if (cudaGetSymbolAddress(&v, g_tc_error) != cudaSuccess) return nullptr;
+  word[dev].store((u32*)v, std::memory_order_release);
+  return (u32*)v;
 }
 
 int tc_error_check() {

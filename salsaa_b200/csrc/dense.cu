@@ -12,6 +12,7 @@
 
 #include "../../include/salsaa_gpu.h"
 #include "kernels.cuh"
+#include "ntt_img.cuh"
 #include "ntt.cuh"
 
 using namespace salsaa;
@@ -150,14 +151,29 @@ extern "C" int salsaa_dense_commit(salsaa_dense_key* k, const uint64_t* d_w, uin
       if (p) cudaFreeAsync(p, s);
     }
   } free_tmp{tmp, st};
-  int rc = ntt_launch(d_w, d_w_slot, r * m, *k->T, true, false, st);
-  if (rc) return rc;
+  // columns as a byte image (never larger than their words) when the shapes
+  // allow, else in slot form
+  const bool img = k->tk8 && (uintptr_t)d_w % 16 == 0 && (uintptr_t)d_w_slot % 16 == 0 &&
+                   cki_ok(1, m, k->n, (u32)m, k->q);
+  int rc = 0;
+  if (!img && (rc = ntt_launch(d_w, d_w_slot, r * m, *k->T, true, false, st))) return rc;
   u64* acc = k->scratch;
   u64* cout = k->scratch + (u64)nr * DENSE_GROUP * d;
   for (u64 g0 = 0; g0 < r; g0 += DENSE_GROUP) {
     const u32 G = (u32)((r - g0) < DENSE_GROUP ? (r - g0) : DENSE_GROUP);
     CommitArgs a{};
     for (u32 c = 0; c < G; c++) a.w.p[c] = d_w_slot + (g0 + c) * m * d;
+    CkImage im{};
+    if (img) {
+      im = cki_shape(G, m, k->n, (u32)m);
+      im.p = (uint8_t*)(d_w_slot + g0 * m * d);
+      ImgRows rows{};
+      for (u32 c = 0; c < G; c++) rows.src[c] = d_w + (g0 + c) * m * d;
+      rows.rows = G;
+      rows.width = m;
+      if ((rc = ntt_img_launch(rows, im, *k->T, st))) return rc;
+      a.img = &im;
+    }
     a.rows = G;
     a.width = m;
     a.nck = nr;

@@ -10,6 +10,7 @@
 //   structured dot products  src/arithmetic.rs:459-536
 #include <vector>
 #include "kernels.cuh"
+#include "ntt_img.cuh"
 
 namespace salsaa {
 
@@ -934,7 +935,7 @@ __global__ void sc_finalize_kernel(const u64* sums, u32 rows, u32 nr, u64 q, u64
 template <bool LAZY>
 static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
                            SumcheckBufs B, u32 nr, bool plain, cudaStream_t st) {
-  const u64 sa = nlen / 2, sb = nlen / 4;  // strides of the two ping-pong buffers
+  const u64 sa = nlen >> SC_T, sb = nlen >> (2 * SC_T);  // strides: a pass divides the length by 16
   u64 L = nlen;
   u32 j = 0;
   const u64* in = nullptr;
@@ -2345,7 +2346,12 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ss, a.ev_fork, 0);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "commit: fork");
   }
-  if (a.nck && ck_umma_ok(a, n)) {
+  if (a.nck && a.img) {
+    const CkImgArgs ca{a.tk8, a.thi, a.nck, a.ck_bt, a.ck_nhi, a.acc};
+    if (a.img->R != a.rows || a.img->width != a.width) return salsaa_set_error(-2, "commit: image of other rows");
+    int rc = launch_ck_img(ca, *a.img, M, T.zeta, st);
+    if (rc) return rc;
+  } else if (a.nck && ck_umma_ok(a, n)) {
     u32 Bk, G;
     ck_umma_shape(a.width, a.rows, n, a.ck_bt, &Bk, &G);
     int rc = launch_ck_umma(a, n, Bk, G, M, T.zeta, plain, st);

@@ -113,6 +113,8 @@ int launch_nc_gram_sums(const u64* gram, u32 rows, const ModQ& M, const DevState
                         bool plain, cudaStream_t st);
 // Nonzero (and the last error set) when a tensor-core kernel's bounded wait gave up.
 int tc_error_check();
+// The current device's error word of the tensor-core kernels (null if unavailable).
+u32* tc_error_word();
 int launch_gen_witness(u64* w, u32 rows, u64 width, u32 d, u64 q, const DevState* ds, cudaStream_t st);
 int launch_expand_i8(const int8_t* in, u64 n, u64 q, u64* out, cudaStream_t st);
 int launch_fill(u64* p, u64 n, u64 v, cudaStream_t st);
@@ -122,8 +124,8 @@ int launch_pointwise_mul(u64* r, const u64* b, u64 n, u64 q, cudaStream_t st);
 // sumcheck of `rows` witness rows (coefficient form, length nlen each), both
 // amplification repetitions at once; see sumcheck implementation for buffers.
 struct SumcheckBufs {
-  u64* a;     // 2 * rows * nlen/2
-  u64* b;     // 2 * rows * nlen/4
+  u64* a;     // 2 * rows * nlen/16
+  u64* b;     // 2 * rows * nlen/256
   u64* sums;  // 2 * nr * rows * 3 (zeroed by the launcher)
   u64* cap;   // 2 * rows * d: vector after log2(width) rounds
   u64* gram;  // rows * 256 + 1 (Gram matrices and a flag word) or null: first pass on tcgen05
@@ -177,8 +179,10 @@ int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ&
 
 // <statement rows, witness rows> in slot form.  acc: (nck + nsc) x rows x d
 // scratch; out_slot: results in statement order given by `order`.
+struct CkImage;
 struct CommitArgs {
-  RowSet w;          // slot-form witness rows
+  RowSet w;          // slot-form witness rows (unused when img is set and coef_sc or nsc = 0)
+  const CkImage* img;  // byte image of the same rows for the key rows (ntt_img.cuh), or null
   RowSet wc;         // the same rows in coefficient form (used when coef_sc)
   bool coef_sc;      // scalar rows over wc, their sums moved to slot form after
   u32 rows;

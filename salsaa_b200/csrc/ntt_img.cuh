@@ -1,0 +1,81 @@
+// ntt_img.cuh — byte images of slot-form witnesses: the operand layout the
+// tensor-core key-row product (ck_img.cu) copies straight into shared memory,
+// and the forward transforms (ntt_img.cu) that write it.
+#pragma once
+#include "kernels.cuh"
+
+namespace salsaa {
+
+// Byte image of R witness rows of `width` ring elements in slot form.  With
+// bt = min(width, key-table block), element i = hi bt + lo.  G key blocks
+// (hi = hg G + g) are stacked as virtual rows v = g R + k, so one tile shares
+// its key bytes among them.  Row (v, half h, byte y) of a tile is
+// 14 v + 7 h + y; rows are padded to VP (a multiple of 8).  The 16 bytes of
+// elements 16 j .. 16 j + 15 of one row are one unit:
+//   unit(hg, chunk c = lo / 64, slot s, j = (lo / 16) % 4, row)
+//     = (((hg nlc + c) n + s) 4 + j) VP + row,
+// i.e. a (chunk, slot) tile is 64 VP contiguous bytes in the K-major operand
+// layout (16-byte K slices of VP rows each), one bulk copy.
+struct CkImage {
+  uint8_t* p;
+  u32 R, G, VP, n, btlog, nlc, nhg;
+  u64 width;
+};
+constexpr u32 CKI_CHUNK = 64;
+// Most virtual rows of a tile: 9 x 14 = 126 of the MMA's 128 rows.
+constexpr u32 CKI_MAX_V = 9;
+
+inline u32 cki_vp(u32 V) { return (V * 14 + 7) / 8 * 8; }
+// Shape of the image of R rows x width under a key table of ck_bt elements per block.
+CkImage cki_shape(u32 R, u64 width, u32 n, u32 ck_bt);
+u64 cki_bytes(const CkImage& im);
+// n, q and the key table fit the image path: FP64 transforms (q < 2^50) of
+// n = 64, 128 or 256 slots, a power-of-two width of at least 64 elements.
+bool cki_ok(u32 R, u64 width, u32 n, u32 ck_bt, u64 q);
+
+// 16-byte unit index of (image row k, element i, slot 0, byte row 0); i a multiple of 16.
+__device__ __forceinline__ u64 cki_unit(const CkImage& im, u32 k, u64 i) {
+  const u64 hi = i >> im.btlog;
+  const u32 lo = (u32)(i & ((1ull << im.btlog) - 1));
+  const u32 g = (u32)(hi & (im.G - 1));  // G is a power of two
+  const u64 hg = hi / im.G;
+  return (((hg * im.nlc + (lo >> 6)) * im.n) * 4 + ((lo >> 4) & 3)) * im.VP + (g * im.R + k) * 14;
+}
+
+// Forward incomplete transform of coefficient-form rows (canonical words)
+// into the image.  Row r of the source (rows x width) becomes image row
+// k0 + r; with split != 0 its two halves become the image rows k0 + r and
+// k0 + rows + r of width / 2.
+struct ImgRows {
+  const u64* src[MAX_WROWS];
+  u32 rows, k0, split;
+  u64 width;
+  u64* slots;        // slot-form words too (rows x width), or null
+  u64* mag_or;       // OR of the centred magnitudes of the source, or null
+};
+int ntt_img_launch(const ImgRows& a, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// The same for the two decomposition digits of each source row: digit c of
+// row r is row 2 r + c of the digit space (2 rows x width), whose halves
+// become image rows as above.  bw_or, rlog_out, radix_out as in
+// ntt_digits_launch; coef: the digits as centred int32.
+struct ImgDigits {
+  ImgRows rows;
+  const u64* bw_or;
+  u64* rlog_out;
+  u64* radix_out;
+  int* coef;
+};
+int ntt_img_digits_launch(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// Key rows x image (q < 2^50): the sums of key row r and witness row k are
+// added to acc row r * R + k (slot form, zeroed by the caller).
+struct CkImgArgs {
+  const uint8_t* tk8;
+  const u64* thi;
+  u32 nck, ck_bt, ck_nhi;
+  u64* acc;
+};
+int launch_ck_img(const CkImgArgs& a, const CkImage& im, const ModQ& M, const u64* zeta, cudaStream_t st);
+
+}  // namespace salsaa

@@ -16,6 +16,7 @@
 #include "../../include/salsaa_gpu.h"
 #include "host_math.h"
 #include "kernels.cuh"
+#include "ntt_img.cuh"
 
 using namespace salsaa;
 
@@ -169,6 +170,8 @@ struct Shapes {
   u32 max_rows = 0;          // witness rows in any call
   u32 max_stmt = 0;          // statement rows
   u32 nsc_total = 0;         // scalar rows pushed by the whole proof
+  bool use_img = false;      // every key-row product of the proof goes through a byte image
+  u64 max_img = 0;           // its largest image, bytes
 };
 
 static Shapes walk(const salsaa_params* p) {
@@ -201,6 +204,15 @@ static Shapes walk(const salsaa_params* p) {
     return S;
   }
   S.basic_ok = true;
+  const u32 ck_bt = (u32)(L < CK_KEY_BLOCK ? L : CK_KEY_BLOCK);
+  S.use_img = p->module_size <= CKU_MAX_KEYS && ck_bt >= 128;
+  auto image = [&](u64 R, u64 wd) {  // key rows x R rows of width wd
+    S.use_img = S.use_img && cki_ok((u32)R, wd, (u32)(d / 2), ck_bt, q);
+    if (!S.use_img) return;
+    const u64 b = cki_bytes(cki_shape((u32)R, wd, (u32)(d / 2), ck_bt));
+    S.max_img = b > S.max_img ? b : S.max_img;
+  };
+  if (p->folding || !p->nof_rounds) image(p->init_wit_rep, L);
   u64 w = 8, Sn = p->module_size, K = p->init_wit_rep, width = L;
   S.max_d_rows_width = K * width;
   S.max_rows = (u32)K;
@@ -214,6 +226,7 @@ static Shapes walk(const salsaa_params* p) {
       }
       w += 1 + Sn * K * parts * d;
       K *= parts;
+      S.use_img = S.use_img && parts == 2;
       if (K * width > S.max_d_rows_width) S.max_d_rows_width = K * width;
     } else if (!p->folding && i > 0 && K * width > S.max_d_rows_width) {
       S.max_d_rows_width = K * width;  // the joined witness moves to the decomposition buffers
@@ -255,6 +268,7 @@ static Shapes walk(const salsaa_params* p) {
       return S;
     }
     if (width > S.max_fp_width) S.max_fp_width = width;
+    image(p->folding ? 1 : K + 1, width);
     w += Sn * d;
     w += (K + 1) * d;
     Sn += 1;
@@ -266,6 +280,7 @@ static Shapes walk(const salsaa_params* p) {
       w += 1 + Sn * K * 2 * d;
       K *= 2;
       if (K * width > S.max_d_rows_width) S.max_d_rows_width = K * width;
+      image(K, width);
       break;
     }
     if (Sn > S.max_stmt) S.max_stmt = (u32)Sn;
@@ -274,6 +289,7 @@ static Shapes walk(const salsaa_params* p) {
   if (K > S.max_rows) S.max_rows = (u32)K;
   if (!p->folding) w += K * width * d;
   S.proof_words = w;
+  if (!S.use_img) S.max_img = 0;
   S.ok = true;
   return S;
 }
@@ -341,6 +357,7 @@ static int ctx_build(salsaa_ctx* c, DevBuf& mem) {
       TRY(launch_ck_tk8(c->tlo, ms, n, c->ck_bt, c->P.q < (1ULL << 50), c->tk8, 0));
     }
   }
+  if (!tc_error_word()) return salsaa_set_error(-1, "ctx: tensor-core error word");
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ctx: build");
   return 0;
@@ -402,7 +419,9 @@ struct salsaa_prover {
   bool overlap = false;        // use the side stream (salsaa_prover_set_overlap)
   DevBuf mem;
   DevState* ds = nullptr;
-  u64 *Dc = nullptr, *Ds = nullptr, *Fc = nullptr, *Fs = nullptr, *Pc = nullptr, *Ps = nullptr;
+  u64 *Dc = nullptr, *Ds = nullptr, *Fc = nullptr, *Fs = nullptr, *Pc = nullptr;
+  u64* Ps = nullptr;       // slot form of the projected row; null with an image (only the key rows read it)
+  uint8_t* img = nullptr;  // byte image of the key rows' witness (ntt_img.cuh), or null
   SumcheckBufs sc{};
   u64* row_base = nullptr;  // TENSOR row bases, nsc_total x d
   u64* row_cj = nullptr;    // PERIODIC row scalars, rounds x CK_BLOCK
@@ -459,9 +478,10 @@ extern "C" uint64_t salsaa_workspace_bytes(const salsaa_params* p) {
   const u64 d = p->d, L = p->wit_len;
   u64 words = 0;
   words += 2 * S.max_d_rows_width * d;        // Dc, Ds
-  words += 4 * S.max_fp_width * d;            // Fc, Fs, Pc, Ps
-  words += S.max_nc_rows_width * d;           // sumcheck a
-  words += S.max_nc_rows_width * d / 2;       // sumcheck b
+  words += (S.use_img ? 3 : 4) * S.max_fp_width * d;  // Fc, Fs, Pc, and Ps without an image
+  words += S.max_img / 8;                     // byte image of the key rows' witness
+  words += S.max_nc_rows_width * d / 8;       // sumcheck a
+  words += S.max_nc_rows_width * d / 128;     // sumcheck b
   words += (u64)MAX_WROWS * 256 + 1;          // sumcheck Gram matrices
   words += (u64)S.nsc_total * d + p->nof_rounds * CK_BLOCK;
   const u64 stmt = S.max_stmt + 2;
@@ -509,9 +529,10 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
   if ((rc = m.alloc(&pr->ds, 1, "ds")) || (rc = m.alloc(&pr->Dc, S.max_d_rows_width * d, "Dc")) ||
       (rc = m.alloc(&pr->Ds, S.max_d_rows_width * d, "Ds")) || (rc = m.alloc(&pr->Fc, S.max_fp_width * d, "Fc")) ||
       (rc = m.alloc(&pr->Fs, S.max_fp_width * d, "Fs")) || (rc = m.alloc(&pr->Pc, S.max_fp_width * d, "Pc")) ||
-      (rc = m.alloc(&pr->Ps, S.max_fp_width * d, "Ps")) ||
-      (rc = m.alloc(&pr->sc.a, S.max_nc_rows_width * d, "sumcheck a")) ||
-      (rc = m.alloc(&pr->sc.b, S.max_nc_rows_width * d / 2 + 1, "sumcheck b")) ||
+      (!S.use_img && (rc = m.alloc(&pr->Ps, S.max_fp_width * d, "Ps"))) ||
+      (S.use_img && (rc = m.alloc(&pr->img, S.max_img, "key-row image"))) ||
+      (rc = m.alloc(&pr->sc.a, S.max_nc_rows_width * d / 8 + 1, "sumcheck a")) ||
+      (rc = m.alloc(&pr->sc.b, S.max_nc_rows_width * d / 128 + 1, "sumcheck b")) ||
       (rc = m.alloc(&pr->sc.sums, 2ULL * 64 * MAX_WROWS * 3, "sumcheck sums")) ||
       (rc = m.alloc(&pr->sc.cap, 2ULL * MAX_WROWS * d, "sumcheck cap")) ||
       (rc = m.alloc(&pr->sc.gram, (u64)MAX_WROWS * 256 + 1, "sumcheck gram")) ||
@@ -629,13 +650,15 @@ __global__ void set_seed_kernel(DevState* ds, u64 seed) { ds->seed = seed; }
 // <statement rows [0, nck) ++ scalar rows [sc_first, sc_first + nsc), witness rows>
 // -> slot-form ring elements in pr->cout, row-major (statement, witness).
 // wc: the same witness rows in coefficient form (scalar rows are summed there), or null.
+// img: their byte image for the key rows (ws is then not read), or null.
 static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* wc, u32 rows, u64 width, u32 nck,
-                            u32 sc_first, u32 nsc) {
+                            u32 sc_first, u32 nsc, const CkImage* img = nullptr) {
   salsaa_ctx* c = pr->ctx;
   if ((u64)sc_first + nsc > c->S.nsc_total || nck > c->P.module_size)
     return salsaa_set_error(-9, "commit: statement row range outside the proof's rows");
   CommitArgs a{};
   a.w = ws;
+  a.img = img;
   if (wc && nsc) {
     a.wc = *wc;
     a.coef_sc = true;
@@ -674,8 +697,8 @@ static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* w
 
 // Same, in coefficient form at proof_out.
 static int commit_rows(salsaa_prover* pr, const RowSet& ws, const RowSet* wc, u32 rows, u64 width, u32 nck,
-                       u32 sc_first, u32 nsc, u64* proof_out) {
-  TRY(commit_rows_slot(pr, ws, wc, rows, width, nck, sc_first, nsc));
+                       u32 sc_first, u32 nsc, u64* proof_out, const CkImage* img = nullptr) {
+  TRY(commit_rows_slot(pr, ws, wc, rows, width, nck, sc_first, nsc, img));
   return ntt_launch(pr->cout, proof_out, (u64)(nck + nsc) * rows, *pr->ctx->T, true, true, pr->st);
 }
 
@@ -690,6 +713,23 @@ static RowSet rows_of_narrow(const u64* base, u32 rows, u64 width, u32 d) {
   for (u32 k = 0; k < rows; k++) r.p[k] = (const u64*)((const int*)base + (u64)k * width * d);
   r.narrow = rows >= 32 ? ~0u : ((1u << rows) - 1);
   return r;
+}
+
+// decomp_ell into two digits, as centred int32 coefficients (Dc), the image
+// rows and, with slots, slot-form words.
+static int decompose_image(salsaa_prover* pr, const RowSet& src, u32 rows, u64 width, u32 didx, bool split, u64* slots,
+                           u64* proof_radix, const CkImage& im) {
+  ImgDigits a{};
+  for (u32 k = 0; k < rows; k++) a.rows.src[k] = src.p[k];
+  a.rows.rows = rows;
+  a.rows.split = split ? 1 : 0;
+  a.rows.width = width;
+  a.rows.slots = slots;
+  a.bw_or = &pr->ds->bw_or[didx];
+  a.rlog_out = &pr->ds->rlog[didx];
+  a.radix_out = proof_radix;
+  a.coef = (int*)pr->Dc;
+  return ntt_img_digits_launch(a, im, *pr->ctx->T, pr->st);
 }
 
 static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* proof) {
@@ -717,7 +757,34 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     wbase = pr->Dc;
   }
   Wc = rows_of(wbase, K, width, d);
-  TRY(ntt_launch(wbase, pr->Ds, (u64)K * width, T, true, false, st));
+  // With use_img the key rows read the witness as a byte image, written by the
+  // transforms themselves: rows L_0.., R_0.., P of the split witness in the
+  // SNARK, each commitment's own rows in the folding scheme.
+  CkImage im{};
+  const CkImage* imp = c->S.use_img ? &im : nullptr;
+  auto image = [&](u32 R, u64 w) {
+    im = cki_shape(R, w, c->n, c->ck_bt);
+    im.p = pr->img;
+  };
+  auto image_rows = [&](const RowSet& src, u32 rows, u64 w, u32 k0, bool split, u64* slots, u64* mag,
+                        cudaStream_t s) {
+    ImgRows r{};
+    for (u32 k = 0; k < rows; k++) r.src[k] = src.p[k];
+    r.rows = rows;
+    r.k0 = k0;
+    r.split = split ? 1 : 0;
+    r.width = w;
+    r.slots = slots;
+    r.mag_or = mag;
+    return ntt_img_launch(r, im, T, s);
+  };
+  if (imp) {
+    const bool split = !P.folding && P.nof_rounds > 0;
+    image(split ? 2 * K + 1 : K, split ? width / 2 : width);
+    TRY(image_rows(Wc, K, width, 0, split, pr->Ds, nullptr, st));
+  } else {
+    TRY(ntt_launch(wbase, pr->Ds, (u64)K * width, T, true, false, st));
+  }
   Ws = rows_of(pr->Ds, K, width, d);
   // commitment: parallel_dot_series_matrix(crs.ck, witness), src/protocol.rs:138.
   // In the SNARK it is derived from round 0's split commitment through the
@@ -725,7 +792,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
   u64 pend_off = cur;             // pending derived commitment: proof offset,
   u32 pend_rows = ms, pend_K = K; // statement rows and witness rows
   bool pending = !P.folding && P.nof_rounds > 0;
-  if (!pending) TRY(commit_rows(pr, Ws, &Wc, K, width, ms, 0, 0, proof + cur));
+  if (!pending) TRY(commit_rows(pr, Ws, &Wc, K, width, ms, 0, 0, proof + cur, imp));
   cur += (u64)ms * K * d;
   u32 nsc = 0, didx = 0;
   bool mag_ready = false;  // bw_or[didx] filled by the transforms of the joined witness
@@ -735,8 +802,15 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       // decomp_ell (src/subroutines/decomp.rs:32-67)
       TRY(mark(pr, PH_DECOMP));
       bool narrow = false;
-      TRY(launch_decompose_ntt(Wc, K, width, d, q, parts, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
-                               mag_ready, &narrow));
+      if (imp) {
+        if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
+        image(2 * parts * K + 1, width / 2);
+        TRY(decompose_image(pr, Wc, K, width, didx++, true, pr->Ds, proof + cur, im));
+        narrow = true;
+      } else {
+        TRY(launch_decompose_ntt(Wc, K, width, d, q, parts, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
+                                 mag_ready, &narrow));
+      }
       mag_ready = false;
       cur += 1;
       K *= parts;
@@ -755,12 +829,16 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       for (u32 k = 0; k < K; k++) {
         e = cudaMemcpyAsync(pr->Dc + (u64)k * width * d, Wc.p[k], width * d * sizeof(u64), cudaMemcpyDeviceToDevice,
                             st);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && !imp)
           e = cudaMemcpyAsync(pr->Ds + (u64)k * width * d, Ws.p[k], width * d * sizeof(u64),
                               cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: joined witness");
       }
       Wc = rows_of(pr->Dc, K, width, d);
+      if (imp) {
+        image(2 * K + 1, width / 2);
+        TRY(image_rows(Wc, K, width, 0, true, pr->Ds, nullptr, st));
+      }
       Ws = rows_of(pr->Ds, K, width, d);
     }
     // split (src/subroutines/split.rs:45-76): rows L_0..L_{K-1}, R_0..R_{K-1},
@@ -801,12 +879,18 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     const bool next_decomp =
         P.folding || (rd + 1 < P.nof_rounds && P.decomp_parts[rd + 1 < 12 ? rd + 1 : 11] > 1);
     u64* mag = nullptr;
-    if (next_decomp && didx < 16 && ntt_mag_ok(pr->Pc, pr->Ps, T, true) && ntt_mag_ok(pr->Fs, pr->Fc, T, true)) {
+    if (next_decomp && didx < 16 && (imp || ntt_mag_ok(pr->Pc, pr->Ps, T, true)) &&
+        ntt_mag_ok(pr->Fs, pr->Fc, T, true)) {
       mag = &pr->ds->bw_or[didx];
       e = cudaMemsetAsync(mag, 0, sizeof(u64), ps);
       if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: magnitude OR");
     }
-    TRY(ntt_launch(pr->Pc, pr->Ps, width2, T, true, false, ps, mag));
+    if (imp) {
+      if (P.folding) image(1, width2);
+      TRY(image_rows(rows_of(pr->Pc, 1, width2, d), 1, width2, P.folding ? 0 : K2, false, nullptr, mag, ps));
+    } else {
+      TRY(ntt_launch(pr->Pc, pr->Ps, width2, T, true, false, ps, mag));
+    }
     if (pr->overlap && (e = cudaEventRecord(pr->ev_join, ps)) != cudaSuccess)
       return salsaa_set_cuda_error(e, "enqueue: join");
 
@@ -847,7 +931,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       RowSet both = Ws, bothc = Wc;
       both.p[K] = pr->Ps;
       bothc.p[K] = pr->Pc;
-      TRY(commit_rows_slot(pr, both, &bothc, K + 1, width, ms, 0, nsc + 2));
+      TRY(commit_rows_slot(pr, both, &bothc, K + 1, width, ms, 0, nsc + 2, imp));
       TRY(ntt_launch(pr->cout, pr->cout2, (u64)(S + 2) * (K + 1), T, true, true, st));
       const size_t row_bytes = (size_t)(K + 1) * d * sizeof(u64);
       e = cudaMemcpy2DAsync(proof + cur, (size_t)K * d * sizeof(u64), pr->cout2, row_bytes,
@@ -880,7 +964,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
         pending = false;
       }
     } else {
-      TRY(commit_rows(pr, Pr, &Prc, 1, width, ms, 0, nsc, proof + cur));
+      TRY(commit_rows(pr, Pr, &Prc, 1, width, ms, 0, nsc, proof + cur, imp));
       cur += (u64)S * d;
     }
     // batch_projections (src/subroutines/project.rs:131-203): witness_rhs, projection_rhs
@@ -930,14 +1014,21 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     if (P.folding) {
       TRY(mark(pr, PH_DECOMP));
       bool narrow = false;
-      TRY(launch_decompose_ntt(Wc, K, width, d, q, 2, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
-                               mag_ready, &narrow));
+      if (imp) {
+        if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
+        image(2 * K, width);
+        TRY(decompose_image(pr, Wc, K, width, didx++, false, nullptr, proof + cur, im));
+        narrow = true;
+      } else {
+        TRY(launch_decompose_ntt(Wc, K, width, d, q, 2, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
+                                 mag_ready, &narrow));
+      }
       mag_ready = false;
       cur += 1;
       K *= 2;
       Ws = rows_of(pr->Ds, K, width, d);
       const RowSet Dcr = narrow ? rows_of_narrow(pr->Dc, K, width, d) : rows_of(pr->Dc, K, width, d);
-      TRY(commit_rows(pr, Ws, &Dcr, K, width, ms, 0, nsc, proof + cur));
+      TRY(commit_rows(pr, Ws, &Dcr, K, width, ms, 0, nsc, proof + cur, imp));
       cur += (u64)(ms + nsc) * K * d;
       break;
     }
@@ -1693,14 +1784,26 @@ extern "C" int salsaa_commit(salsaa_ctx* c, const uint64_t* d_w, uint64_t rows, 
   cudaStream_t st = (cudaStream_t)stream;
   const u32 d = c->d, ms = (u32)c->P.module_size;
   Tmp t(st);
-  u64 *ws, *acc, *cout;
+  u64 *ws = nullptr, *acc, *cout;
   DevState* ds;
-  TRY(t.get(&ws, rows * width * d));
   TRY(t.get(&acc, (u64)ms * rows * d));
   TRY(t.get(&cout, (u64)ms * rows * d));
   TRY(t.get(&ds, 1));
-  TRY(ntt_launch(d_w, ws, rows * width, *c->T, true, false, st));
   CommitArgs a{};
+  CkImage im{};
+  if (c->tk8 && (uintptr_t)d_w % 16 == 0 && cki_ok((u32)rows, width, c->n, c->ck_bt, c->P.q)) {
+    im = cki_shape((u32)rows, width, c->n, c->ck_bt);
+    TRY(t.get(&im.p, cki_bytes(im)));
+    ImgRows r{};
+    for (u32 k = 0; k < rows; k++) r.src[k] = d_w + (u64)k * width * d;
+    r.rows = (u32)rows;
+    r.width = width;
+    TRY(ntt_img_launch(r, im, *c->T, st));
+    a.img = &im;
+  } else {
+    TRY(t.get(&ws, rows * width * d));
+    TRY(ntt_launch(d_w, ws, rows * width, *c->T, true, false, st));
+  }
   a.tl8 = c->tl8;
   a.tk8 = c->tk8;
   a.w = rows_of(ws, (u32)rows, width, d);
@@ -1791,8 +1894,8 @@ extern "C" int salsaa_sumcheck(const uint64_t* d_w, uint64_t rows, uint64_t n, u
   Tmp t(st);
   SumcheckBufs B{};
   DevState* ds;
-  TRY(t.get(&B.a, rows * n));
-  TRY(t.get(&B.b, rows * n / 2));
+  TRY(t.get(&B.a, rows * n / 8));
+  TRY(t.get(&B.b, rows * n / 128));
   TRY(t.get(&B.sums, 2ULL * 64 * rows * 3));
   TRY(t.get(&B.cap, 2ULL * rows * d));
   TRY(t.get(&B.gram, rows * 256 + 1));

@@ -56,6 +56,35 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t
       : "memory");
 }
 
+// The same from warp-uniform code under elect_one(), without the disable-lane
+// mask: with the loop around it uniform and the descriptors advanced by
+// constants the issue keeps up with the tensor core (measured, M = 128,
+// K = 32: 48 / 64 / 88 clocks per MMA at N = 64 / 128 / 176, against
+// 113 .. 124 at any N up to 224 from a one-lane branch that rebuilds its descriptors).
+__device__ __forceinline__ void mma_i8_u(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// One lane of a fully active warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 // Arrive on an mbarrier once every MMA issued so far by this thread completes.
 __device__ __forceinline__ void commit(uint64_t* mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
