@@ -150,6 +150,14 @@ __host__ __device__ __forceinline__ u64 domain_id(u64 kind, u64 a, u64 b) { retu
 
 int salsaa_set_cuda_error(cudaError_t e, const char* what);
 int salsaa_set_error(int code, const char* msg);
+// Stream-ordered scratch of one call, from the library's own memory pool (see
+// prover.cu); freed on the same stream.
+cudaError_t salsaa_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+// Gives the pool's unused memory on the current device back to the system.
+void salsaa_scratch_trim();
+// A context or dense key came (+1) or went (-1); after the last one went the
+// pool's unused memory goes back.
+void salsaa_scratch_users(int delta);
 // Counts kernel launches issued by this library (reported by the benchmark).
 void salsaa_count_launch();
 // Optional device-time trace of named kernels (off unless enabled through the

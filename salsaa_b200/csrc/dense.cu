@@ -70,6 +70,7 @@ extern "C" int salsaa_dense_key_create(const uint64_t* d_a, uint64_t nrows, uint
   if (!T) return salsaa_set_error(-1, "dense_key_create: no incomplete NTT for (d, q)");
   cudaStream_t st = (cudaStream_t)stream;
   salsaa_dense_key* k = new salsaa_dense_key;
+  salsaa_scratch_users(1);  // undone by salsaa_dense_key_destroy, on the failure paths too
   k->nrows = (u32)nrows;
   k->d = (u32)d;
   k->n = (u32)(d / 2);
@@ -128,6 +129,7 @@ extern "C" void salsaa_dense_key_destroy(salsaa_dense_key* k) {
   cudaFree(k->tk8);
   cudaFree(k->scratch);
   cudaFree(k->ds);
+  salsaa_scratch_users(-1);
   delete k;
 }
 
@@ -140,7 +142,7 @@ extern "C" int salsaa_dense_commit(salsaa_dense_key* k, const uint64_t* d_w, uin
   const u64 m = k->m;
   u64* tmp = nullptr;
   if (!d_w_slot) {
-    cudaError_t e = cudaMallocAsync(&tmp, r * m * d * sizeof(u64), st);
+    cudaError_t e = salsaa_scratch_alloc((void**)&tmp, r * m * d * sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "dense_commit: workspace");
     d_w_slot = tmp;
   }

@@ -804,33 +804,31 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   // device scratch: sums, two ping-pong areas, descriptors, nrs / offs
   const u32 maxlev = 8;  // 16^8 > 2^30
   const u64 desc_bytes = (u64)(maxlev + 1) * SB_MAX_INST * sizeof(SbInst);
-  u64 *sums = nullptr, *bufa = nullptr, *bufb = nullptr, *doffs = nullptr;
-  SbInst* ddesc = nullptr;
-  u32* dnrs = nullptr;
-  auto alloc = [&](void** p, u64 bytes) {
-    cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, st);
-    return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sumcheck_batch: workspace");
-  };
+  int rc = 0;
   struct Guard {
-    std::vector<void*> v;
+    void* p;
     cudaStream_t s;
     ~Guard() {
-      for (void* p : v) cudaFreeAsync(p, s);
+      if (p) cudaFreeAsync(p, s);
     }
-  } guard{{}, st};
-  int rc = 0;
-  if ((rc = alloc((void**)&sums, (u64)count * nrmax * 3 * 8))) return rc;
-  guard.v.push_back(sums);
-  if ((rc = alloc((void**)&bufa, tot_a * 8))) return rc;
-  guard.v.push_back(bufa);
-  if ((rc = alloc((void**)&bufb, tot_b * 8))) return rc;
-  guard.v.push_back(bufb);
-  if ((rc = alloc((void**)&ddesc, desc_bytes))) return rc;
-  guard.v.push_back(ddesc);
-  if ((rc = alloc((void**)&dnrs, count * 4))) return rc;
-  guard.v.push_back(dnrs);
-  if ((rc = alloc((void**)&doffs, count * 8))) return rc;
-  guard.v.push_back(doffs);
+  } guard{nullptr, st};
+  // one allocation: sums | descriptors | nrs | offs | the two areas
+  auto up = [](u64 b) { return (b + 255) / 256 * 256; };
+  const u64 sum_b = up((u64)count * nrmax * 3 * 8), desc_b = up(desc_bytes), nr_b = up(count * 4), off_b = up(count * 8);
+  {
+    cudaError_t ea = salsaa_scratch_alloc(&guard.p, sum_b + desc_b + nr_b + off_b + up(tot_a * 8) + tot_b * 8 + 256, st);
+    if (ea != cudaSuccess) {
+      guard.p = nullptr;
+      return salsaa_set_cuda_error(ea, "sumcheck_batch: workspace");
+    }
+  }
+  char* base = (char*)guard.p;
+  u64* sums = (u64*)base;
+  SbInst* ddesc = (SbInst*)(base + sum_b);
+  u32* dnrs = (u32*)(base + sum_b + desc_b);
+  u64* doffs = (u64*)(base + sum_b + desc_b + nr_b);
+  u64* bufa = (u64*)(base + sum_b + desc_b + nr_b + off_b);
+  u64* bufb = (u64*)((char*)bufa + up(tot_a * 8));
   cudaError_t e = cudaMemsetAsync(sums, 0, (u64)count * nrmax * 3 * 8, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: memset");
   // host plan: per level, the instances still longer than SC_TAIL, then the tail

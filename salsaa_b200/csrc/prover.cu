@@ -327,6 +327,11 @@ struct DevBuf {
   int alloc(T** p, u64 count, const char* what) {
     void* v = nullptr;
     cudaError_t e = cudaMalloc(&v, (count ? count : 1) * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {  // once more with the scratch pool's unused memory given back
+      cudaGetLastError();
+      salsaa_scratch_trim();
+      e = cudaMalloc(&v, (count ? count : 1) * sizeof(T));
+    }
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, what);
     ptrs.push_back(v);
     *p = (T*)v;
@@ -401,6 +406,7 @@ extern "C" int salsaa_ctx_create(const salsaa_params* p, uint64_t crs_seed, int 
     std::lock_guard<std::mutex> lk(g_ctx_bufs_mu);
     g_ctx_bufs.push_back({c, mem});
   }
+  salsaa_scratch_users(1);
   *out = c;
   return 0;
 }
@@ -1672,28 +1678,95 @@ extern "C" void salsaa_ctx_destroy(salsaa_ctx* c) {
       g_ctx_bufs.erase(g_ctx_bufs.begin() + i);
       break;
     }
+  salsaa_scratch_users(-1);
   delete c;
 }
 
 // ---------------------------------------------------------------------------
 // subroutine-level entry points (stream-ordered temporary allocations)
 // ---------------------------------------------------------------------------
+// The device's default pool gives freed memory back to the system at every
+// synchronisation, so a caller that waits for each result paid for mapping
+// the workspace again on every call (a commitment of 4 x 2^17 ring elements:
+// 8.4 ms alone against 0.55 ms back to back).  The library's own pool per
+// device keeps at most SCRATCH_KEEP bytes between calls: the largest
+// workspace of a call over an A0-sized witness (2^26 coefficients, 512 MiB)
+// with room for a second stream.  What exceeds it goes back at the next
+// synchronisation as before, and all of it when the last context or dense key
+// is destroyed or one of the library's own allocations fails.
+static constexpr uint64_t SCRATCH_KEEP = 1ULL << 30;
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64];
+static bool g_pool_tried[64];
+
+static cudaMemPool_t scratch_pool(cudaStream_t st) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool_tried[dev]) return g_pool[dev];
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;  // not created inside a capture: the default pool serves this call
+  }
+  g_pool_tried[dev] = true;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  uint64_t keep = SCRATCH_KEEP;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  g_pool[dev] = pool;
+  return pool;
+}
+
+cudaError_t salsaa_scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = scratch_pool(st);
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+
+void salsaa_scratch_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
+
+static std::atomic<int> g_scratch_users{0};
+void salsaa_scratch_users(int delta) {
+  if (g_scratch_users.fetch_add(delta) + delta == 0 && delta < 0) salsaa_scratch_trim();
+}
+
 namespace {
+// The scratch buffers of one call, carved from one allocation: want() each,
+// then alloc().
 struct Tmp {
   cudaStream_t st;
-  std::vector<void*> v;
+  void* base = nullptr;
+  size_t bytes = 0;
+  std::vector<std::pair<void**, size_t>> parts;
   explicit Tmp(cudaStream_t s) : st(s) {}
   template <class T>
-  int get(T** p, u64 count) {
-    void* x = nullptr;
-    cudaError_t e = cudaMallocAsync(&x, (count ? count : 1) * sizeof(T), st);
-    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "temporary allocation");
-    v.push_back(x);
-    *p = (T*)x;
+  void want(T** p, u64 count) {
+    parts.push_back({(void**)p, bytes});
+    bytes += ((count ? count : 1) * sizeof(T) + 255) / 256 * 256;
+  }
+  int alloc() {
+    cudaError_t e = salsaa_scratch_alloc(&base, bytes, st);
+    if (e != cudaSuccess) {
+      base = nullptr;
+      return salsaa_set_cuda_error(e, "temporary allocation");
+    }
+    for (auto& p : parts) *p.first = (char*)base + p.second;
     return 0;
   }
   ~Tmp() {
-    for (void* x : v) cudaFreeAsync(x, st);
+    if (base) cudaFreeAsync(base, st);
   }
 };
 }  // namespace
@@ -1729,7 +1802,8 @@ extern "C" int salsaa_poly_mul(const uint64_t* d_a, const uint64_t* d_b, uint64_
   // three passes: NTT(a) -> r, NTT(b) -> tmp, r *= tmp, INTT(r)
   Tmp t(st);
   u64* tb;
-  TRY(t.get(&tb, count * n));
+  t.want(&tb, count * n);
+  TRY(t.alloc());
   TRY(ntt_launch(d_b, tb, count, *T, false, false, st));
   TRY(ntt_launch(d_a, d_r, count, *T, false, false, st));
   TRY(launch_pointwise_mul(d_r, tb, count * n, q, st));
@@ -1762,7 +1836,8 @@ extern "C" int salsaa_sumcheck_fq2_batch(const uint64_t* const* d_vecs, const ui
   cudaStream_t st = (cudaStream_t)stream;
   Tmp t(st);
   u64* scratch;
-  TRY(t.get(&scratch, words + (u64)count * nrmax * 6));
+  t.want(&scratch, words + (u64)count * nrmax * 6);
+  TRY(t.alloc());
   return launch_sumcheck_fq2_batch(d_vecs, lens, count, make_modq(q), shift, seed, (u32)round, d_claims, d_polys,
                                    scratch, st);
 }
@@ -1786,14 +1861,20 @@ extern "C" int salsaa_commit(salsaa_ctx* c, const uint64_t* d_w, uint64_t rows, 
   Tmp t(st);
   u64 *ws = nullptr, *acc, *cout;
   DevState* ds;
-  TRY(t.get(&acc, (u64)ms * rows * d));
-  TRY(t.get(&cout, (u64)ms * rows * d));
-  TRY(t.get(&ds, 1));
+  t.want(&acc, (u64)ms * rows * d);
+  t.want(&cout, (u64)ms * rows * d);
+  t.want(&ds, 1);
   CommitArgs a{};
   CkImage im{};
-  if (c->tk8 && (uintptr_t)d_w % 16 == 0 && cki_ok((u32)rows, width, c->n, c->ck_bt, c->P.q)) {
+  const bool img = c->tk8 && (uintptr_t)d_w % 16 == 0 && cki_ok((u32)rows, width, c->n, c->ck_bt, c->P.q);
+  if (img) {
     im = cki_shape((u32)rows, width, c->n, c->ck_bt);
-    TRY(t.get(&im.p, cki_bytes(im)));
+    t.want(&im.p, cki_bytes(im));
+  } else {
+    t.want(&ws, rows * width * d);
+  }
+  TRY(t.alloc());
+  if (img) {
     ImgRows r{};
     for (u32 k = 0; k < rows; k++) r.src[k] = d_w + (u64)k * width * d;
     r.rows = (u32)rows;
@@ -1801,7 +1882,6 @@ extern "C" int salsaa_commit(salsaa_ctx* c, const uint64_t* d_w, uint64_t rows, 
     TRY(ntt_img_launch(r, im, *c->T, st));
     a.img = &im;
   } else {
-    TRY(t.get(&ws, rows * width * d));
     TRY(ntt_launch(d_w, ws, rows * width, *c->T, true, false, st));
   }
   a.tl8 = c->tl8;
@@ -1837,9 +1917,10 @@ extern "C" int salsaa_commit_multi(salsaa_ctx* c, const uint64_t* const* d_w, co
   }
   Tmp t(st);
   u64 *ws, *acc, *cout;
-  TRY(t.get(&ws, wtot));
-  TRY(t.get(&acc, etot));
-  TRY(t.get(&cout, etot));
+  t.want(&ws, wtot);
+  t.want(&acc, etot);
+  t.want(&cout, etot);
+  TRY(t.alloc());
   // every witness to slot form in one launch
   const u64* ins[CKU_MULTI_MAX];
   u64* outs[CKU_MULTI_MAX];
@@ -1894,12 +1975,13 @@ extern "C" int salsaa_sumcheck(const uint64_t* d_w, uint64_t rows, uint64_t n, u
   Tmp t(st);
   SumcheckBufs B{};
   DevState* ds;
-  TRY(t.get(&B.a, rows * n / 8));
-  TRY(t.get(&B.b, rows * n / 128));
-  TRY(t.get(&B.sums, 2ULL * 64 * rows * 3));
-  TRY(t.get(&B.cap, 2ULL * rows * d));
-  TRY(t.get(&B.gram, rows * 256 + 1));
-  TRY(t.get(&ds, 1));
+  t.want(&B.a, rows * n / 8);
+  t.want(&B.b, rows * n / 128);
+  t.want(&B.sums, 2ULL * 64 * rows * 3);
+  t.want(&B.cap, 2ULL * rows * d);
+  t.want(&B.gram, rows * 256 + 1);
+  t.want(&ds, 1);
+  TRY(t.alloc());
   set_seed_kernel<<<1, 1, 0, st>>>(ds, seed);
   const u64 nr = ilog2u(n);
   RowSet w = rows_of(d_w, (u32)rows, n / d, (u32)d);
@@ -1914,7 +1996,8 @@ extern "C" int salsaa_decompose(const uint64_t* d_w, uint64_t rows, uint64_t wid
   cudaStream_t st = (cudaStream_t)stream;
   Tmp t(st);
   DevState* ds;
-  TRY(t.get(&ds, 1));
+  t.want(&ds, 1);
+  TRY(t.alloc());
   RowSet w = rows_of(d_w, (u32)rows, width, (u32)d);
   return launch_decompose(w, (u32)rows, width, (u32)d, q, (u32)parts, 0, ds, d_out, d_radix, st);
 }
@@ -1930,10 +2013,11 @@ extern "C" int salsaa_project(const uint64_t* d_w, uint64_t rows, uint64_t width
   DevState* ds;
   u32 *pm, *nm;
   int8_t* J;
-  TRY(t.get(&ds, 1));
-  TRY(t.get(&pm, 256 * cw / 32));
-  TRY(t.get(&nm, 256 * cw / 32));
-  TRY(t.get(&J, 256 * cw));
+  t.want(&ds, 1);
+  t.want(&pm, 256 * cw / 32);
+  t.want(&nm, 256 * cw / 32);
+  t.want(&J, 256 * cw);
+  TRY(t.alloc());
   set_seed_kernel<<<1, 1, 0, st>>>(ds, seed);
   TRY(launch_proj_tables(ds, (u32)round, (u32)cw, pm, nm, J, nullptr, q, st));
   RowSet w = rows_of(d_w, (u32)rows, width, (u32)d);
@@ -1949,10 +2033,11 @@ extern "C" int salsaa_fold(const uint64_t* d_w, uint64_t rows, uint64_t width, u
   cudaStream_t st = (cudaStream_t)stream;
   Tmp t(st);
   u64 *ws, *cs, *fs, *pre;
-  TRY(t.get(&ws, rows * width * d));
-  TRY(t.get(&cs, rows * d));
-  TRY(t.get(&fs, width * d));
-  TRY(t.get(&pre, rows * (d / 2) * 6));
+  t.want(&ws, rows * width * d);
+  t.want(&cs, rows * d);
+  t.want(&fs, width * d);
+  t.want(&pre, rows * (d / 2) * 6);
+  TRY(t.alloc());
   TRY(ntt_launch(d_w, ws, rows * width, *T, true, false, st));
   TRY(ntt_launch(d_c, cs, rows, *T, true, false, st));
   TRY(launch_fold(rows_of(ws, (u32)rows, width, (u32)d), (u32)rows, width, *T, make_modq(q), cs, pre, fs, st));
