@@ -327,7 +327,10 @@ CkImage cki_shape(u32 R, u64 width, u32 n, u32 ck_bt) {
   const u64 nhi = width / bt;
   // few rows: stack key blocks while they fit the MMA's 128 rows
   im.G = 1;
-  while (2 * im.G * R <= CKI_MAX_V && nhi % (2 * im.G) == 0) im.G *= 2;
+  while (2 * im.G * R <= CKI_MAX_V && nhi % (2 * im.G) == 0) {
+    im.G *= 2;
+    im.glog++;
+  }
   im.nhg = (u32)(nhi / im.G);
   im.VP = cki_vp(R * im.G);
   return im;

@@ -173,7 +173,7 @@ extern "C" int salsaa_dense_commit(salsaa_dense_key* k, const uint64_t* d_w, uin
       for (u32 c = 0; c < G; c++) rows.src[c] = d_w + (g0 + c) * m * d;
       rows.rows = G;
       rows.width = m;
-      if ((rc = ntt_img_launch(rows, im, *k->T, st))) return rc;
+      if ((rc = ntt_short_img_launch(rows, &k->ds->tc_flag, im, *k->T, st))) return rc;
       a.img = &im;
     }
     a.rows = G;

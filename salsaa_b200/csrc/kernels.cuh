@@ -55,6 +55,7 @@ struct DevState {
   u64 bw_or[16];   // decomposition: OR of centred magnitudes, per decomposition index
   u64 rlog[16];    // decomposition: radix log2, per decomposition index
   u64 proj_flag;   // projection: set when a witness value does not fit int8
+  u32 tc_flag;     // tensor-core transform of a single call: set when a value does not fit int8
 };
 
 // Indices of the scalar rows one commitment pass covers (passed by value).

@@ -95,7 +95,37 @@ const NttDev* ntt_tables(u32 n, u64 q) {
     cudaFree(dd);
     return nullptr;
   }
+  // Byte planes of the transform matrix W[s][k] = psi^((2 bitrev(s) + 1) k),
+  // plane y as a 128 x 128 K-major operand tile (16-byte K slices of 128
+  // rows).  n = 128: row s, column k.  n = 64: both halves of an interleaved
+  // ring element at once, row 64 h + s, column 2 k + h, zero elsewhere.
+  uint8_t* dw = nullptr;
+  if ((n == 64 || n == 128) && q < (1ULL << 50)) {
+    std::vector<u64> pw(2 * (size_t)n);
+    u64 x = 1;
+    for (u64 i = 0; i < 2 * n; i++) {
+      pw[i] = x;
+      x = host::mulmod(x, psi, q);
+    }
+    std::vector<uint8_t> w(TCW_BYTES, 0);
+    for (u32 s = 0; s < n; s++)
+      for (u32 k = 0; k < n; k++) {
+        const u64 v = pw[((2 * (u64)host::bitrev(s, logn) + 1) * k) % (2 * n)];
+        for (u32 h = 0; h < (n == 64 ? 2u : 1u); h++) {
+          const u32 m = n == 64 ? 64 * h + s : s, kk = n == 64 ? 2 * k + h : k;
+          for (u32 y = 0; y < 7; y++) w[y * 16384 + (kk / 16) * 2048 + m * 16 + kk % 16] = (uint8_t)(v >> (8 * y));
+        }
+      }
+    if (cudaMalloc(&dw, TCW_BYTES) != cudaSuccess ||
+        cudaMemcpy(dw, w.data(), TCW_BYTES, cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaFree(d);
+      cudaFree(dd);
+      if (dw) cudaFree(dw);
+      return nullptr;
+    }
+  }
   NttDev* T = new NttDev;
+  T->tcw = dw;
   T->fwd_d = dd;
   T->fwd_h = dd + n;
   T->inv_d = dd + 2 * n;

@@ -30,7 +30,11 @@ struct NttDev {
   const double* inv_d;
   const double* inv_h;
   double qd, q2d, qinv, ninv_d, ninv_h;
+  // The forward transform as a byte matrix for the tensor cores (n = 64 or
+  // 128, q < 2^50; ntt_tc.cu), else null.
+  const uint8_t* tcw;
 };
+constexpr size_t TCW_BYTES = 7 * 128 * 128;
 
 // Tables for (n, q) on the current device, built once and kept for the
 // process lifetime (thread-safe).  Returns nullptr when q has no 2n-th root.

@@ -56,16 +56,8 @@ __global__ void __launch_bounds__(ImgGeom<LOGN>::THREADS) ntt_img_kernel(ImgDigi
   // digit transform takes 16 source elements and both digits (d = 128: one
   // CTA, digit = local element & 1), or one digit per CTA
   constexpr u32 SEL = DIG ? 16 : EL;  // source elements per CTA
-  u64 blk = blockIdx.x;
-  u32 dig = 0;
-  if (DIG && JG == 1) {
-    dig = (u32)(blk & 1);
-    blk >>= 1;
-  }
-  const u64 per_row = R.width / SEL;
-  const u32 k = (u32)(blk / per_row);
-  const u64 e0 = (blk % per_row) * SEL;
-  const u64* src = R.src[k] + e0 * D;
+  if (R.gate && !*R.gate) return;
+  const u64 nblk = R.rows * (R.width / SEL) * (DIG && JG == 1 ? 2 : 1);
   u32 rlog = 0;
   u64 mask = 0, mag = 0;
   if (DIG) {
@@ -78,156 +70,169 @@ __global__ void __launch_bounds__(ImgGeom<LOGN>::THREADS) ntt_img_kernel(ImgDigi
       if (a.radix_out) *a.radix_out = 1ULL << rlog;
     }
   }
-  // output row of the (split) digit or source space for group jg
-  auto out_row = [&](u32 jg) -> u32 { return DIG ? 2 * k + (JG == 2 ? jg : dig) : k; };
-  const u32 out_rows = DIG ? 2 * R.rows : R.rows;
+  for (u64 b0 = blockIdx.x; b0 < nblk; b0 += gridDim.x) {
+    u64 blk = b0;
+    u32 dig = 0;
+    if (DIG && JG == 1) {
+      dig = (u32)(blk & 1);
+      blk >>= 1;
+    }
+    u32 k;
+    u64 e0;
+    img_item(R, im, SEL == 32 ? 5 : 4, (u32)blk, k, e0);
+    const u64* src = R.src[k] + e0 * D;
+    // output row of the (split) digit or source space for group jg
+    auto out_row = [&](u32 jg) -> u32 { return DIG ? 2 * k + (JG == 2 ? jg : dig) : k; };
+    const u32 out_rows = DIG ? 2 * R.rows : R.rows;
 
-  // ---- transform; the words end in the exchange tile ----
-  u64* words = (u64*)ni_smem;
-  if constexpr (LOGN == 6) {
-    double2* sm = (double2*)ni_smem;
-    const u32 el = tid >> 3, r = tid & 7;
-    const u32 sel = DIG ? el >> 1 : el, c = DIG ? el & 1 : 0;
-    double x0[8], x1[8];
+    // ---- transform; the words end in the exchange tile ----
+    u64* words = (u64*)ni_smem;
+    if constexpr (LOGN == 6) {
+      double2* sm = (double2*)ni_smem;
+      const u32 el = tid >> 3, r = tid & 7;
+      const u32 sel = DIG ? el >> 1 : el, c = DIG ? el & 1 : 0;
+      double x0[8], x1[8];
 #pragma unroll
-    for (u32 kk = 0; kk < 8; kk++) {
-      const u32 e = r + 8 * kk;
-      ulonglong2 v = __ldg((const ulonglong2*)(src + sel * D + 2 * e));
-      if (DIG) {
-        long long d0, d1;
-        v.x = img_digit(v.x, q, c * rlog, mask, d0);
-        v.y = img_digit(v.y, q, c * rlog, mask, d1);
-        if (a.coef)
-          *(int2*)(a.coef + ((u64)(2 * k + c) * R.width + e0 + sel) * D + 2 * e) = make_int2((int)d0, (int)d1);
-      } else if (R.mag_or) {
-        mag |= nr_mag(v.x, q) | nr_mag(v.y, q);
-      }
-      x0[kk] = fp_from_word(v.x);
-      x1[kk] = fp_from_word(v.y);
-    }
-    np6_forward(x0, x1, sm, el, r, true, T);
-    const double qd = T.qd, qinv = T.qinv;
-    u64 w0[8], w1[8];
-#pragma unroll
-    for (u32 kk = 0; kk < 8; kk++) {
-      w0[kk] = fp_to_word(x0[kk], qinv, qd);
-      w1[kk] = fp_to_word(x1[kk], qinv, qd);
-    }
-    if (R.slots) {
-      u64* d0 = R.slots + ((u64)out_row(c) * R.width + e0 + sel) * D + 8 * r;
-#pragma unroll
-      for (u32 h = 0; h < 2; h++) {
-        const u64* w = h ? w1 : w0;
-        st_v4_u64(d0 + h * N, w[0], w[1], w[2], w[3]);
-        st_v4_u64(d0 + h * N + 4, w[4], w[5], w[6], w[7]);
-      }
-    }
-    // a thread rewrites the exchange positions it read itself
-    ulonglong2* smw = (ulonglong2*)ni_smem;
-#pragma unroll
-    for (u32 kk = 0; kk < 8; kk++) smw[np6_pos(el, 8 * r + kk)] = make_ulonglong2(w0[kk], w1[kk]);
-  } else {
-    constexpr int PL = ph_count(LOGN) - 1;
-    double* sm = (double*)ni_smem;
-    u32 unit, tu;
-    nr_map<LOGN, true>(tid, unit, tu);
-    u64 w[16];
-    double x[16];
-    nr_load_global<LOGN, true, false>(w, src, unit, tu);
-#pragma unroll
-    for (u32 i = 0; i < 16; i++) {
-      if (DIG) {
-        long long d0;
-        w[i] = img_digit(w[i], q, dig * rlog, mask, d0);
-        if (a.coef) {
-          constexpr u32 K0 = 1u << ph_size(LOGN, 0);
-          const u32 e = nr_elem<LOGN, 0, false>(tu, i / K0, i % K0);
-          a.coef[((u64)(2 * k + dig) * R.width + e0 + (unit >> 1)) * D + 2 * e + (unit & 1)] = (int)d0;
+      for (u32 kk = 0; kk < 8; kk++) {
+        const u32 e = r + 8 * kk;
+        ulonglong2 v = __ldg((const ulonglong2*)(src + sel * D + 2 * e));
+        if (DIG) {
+          long long d0, d1;
+          v.x = img_digit(v.x, q, c * rlog, mask, d0);
+          v.y = img_digit(v.y, q, c * rlog, mask, d1);
+          if (a.coef)
+            *(int2*)(a.coef + ((u64)(2 * k + c) * R.width + e0 + sel) * D + 2 * e) = make_int2((int)d0, (int)d1);
+        } else if (R.mag_or) {
+          mag |= nr_mag(v.x, q) | nr_mag(v.y, q);
         }
-      } else if (R.mag_or) {
-        mag |= nr_mag(w[i], q);
+        x0[kk] = fp_from_word(v.x);
+        x1[kk] = fp_from_word(v.y);
       }
-      x[i] = fp_from_word(w[i]);
+      np6_forward(x0, x1, sm, el, r, true, T);
+      const double qd = T.qd, qinv = T.qinv;
+      u64 w0[8], w1[8];
+#pragma unroll
+      for (u32 kk = 0; kk < 8; kk++) {
+        w0[kk] = fp_to_word(x0[kk], qinv, qd);
+        w1[kk] = fp_to_word(x1[kk], qinv, qd);
+      }
+      if (R.slots) {
+        u64* d0 = R.slots + ((u64)out_row(c) * R.width + e0 + sel) * D + 8 * r;
+#pragma unroll
+        for (u32 h = 0; h < 2; h++) {
+          const u64* w = h ? w1 : w0;
+          st_v4_u64(d0 + h * N, w[0], w[1], w[2], w[3]);
+          st_v4_u64(d0 + h * N + 4, w[4], w[5], w[6], w[7]);
+        }
+      }
+      // a thread rewrites the exchange positions it read itself
+      ulonglong2* smw = (ulonglong2*)ni_smem;
+#pragma unroll
+      for (u32 kk = 0; kk < 8; kk++) smw[np6_pos(el, 8 * r + kk)] = make_ulonglong2(w0[kk], w1[kk]);
+    } else {
+      constexpr int PL = ph_count(LOGN) - 1;
+      double* sm = (double*)ni_smem;
+      u32 unit, tu;
+      nr_map<LOGN, true>(tid, unit, tu);
+      u64 w[16];
+      double x[16];
+      nr_load_global<LOGN, true, false>(w, src, unit, tu);
+#pragma unroll
+      for (u32 i = 0; i < 16; i++) {
+        if (DIG) {
+          long long d0;
+          w[i] = img_digit(w[i], q, dig * rlog, mask, d0);
+          if (a.coef) {
+            constexpr u32 K0 = 1u << ph_size(LOGN, 0);
+            const u32 e = nr_elem<LOGN, 0, false>(tu, i / K0, i % K0);
+            a.coef[((u64)(2 * k + dig) * R.width + e0 + (unit >> 1)) * D + 2 * e + (unit & 1)] = (int)d0;
+          }
+        } else if (R.mag_or) {
+          mag |= nr_mag(w[i], q);
+        }
+        x[i] = fp_from_word(w[i]);
+      }
+      nf_compute<LOGN, 0, false>(x, tu, T);
+      nr_store_smem<LOGN, 0, false>(x, sm, unit, tu);
+      __syncthreads();
+      nf_mid<LOGN, 1, PL, false>(x, sm, unit, tu, true, T);
+      nr_load_smem<LOGN, PL, false>(x, sm, unit, tu);
+      nf_compute<LOGN, PL, false>(x, tu, T);
+#pragma unroll
+      for (u32 i = 0; i < 16; i++) w[i] = fp_to_word(x[i], T.qinv, T.qd);
+      if (R.slots) {
+        constexpr u32 KL = 1u << ph_size(LOGN, PL);
+        u64* d0 = R.slots + ((u64)out_row(0) * R.width + e0) * D + (u64)unit * N;
+#pragma unroll
+        for (u32 i = 0; i < 16; i += 2)
+          *(ulonglong2*)(d0 + nr_elem<LOGN, PL, false>(tu, i / KL, i % KL)) = make_ulonglong2(w[i], w[i + 1]);
+      }
+      nr_store_smem<LOGN, PL, false>(w, words, unit, tu);
     }
-    nf_compute<LOGN, 0, false>(x, tu, T);
-    nr_store_smem<LOGN, 0, false>(x, sm, unit, tu);
     __syncthreads();
-    nf_mid<LOGN, 1, PL, false>(x, sm, unit, tu, true, T);
-    nr_load_smem<LOGN, PL, false>(x, sm, unit, tu);
-    nf_compute<LOGN, PL, false>(x, tu, T);
-#pragma unroll
-    for (u32 i = 0; i < 16; i++) w[i] = fp_to_word(x[i], T.qinv, T.qd);
-    if (R.slots) {
-      constexpr u32 KL = 1u << ph_size(LOGN, PL);
-      u64* d0 = R.slots + ((u64)out_row(0) * R.width + e0) * D + (u64)unit * N;
-#pragma unroll
-      for (u32 i = 0; i < 16; i += 2)
-        *(ulonglong2*)(d0 + nr_elem<LOGN, PL, false>(tu, i / KL, i % KL)) = make_ulonglong2(w[i], w[i + 1]);
-    }
-    nr_store_smem<LOGN, PL, false>(w, words, unit, tu);
-  }
-  __syncthreads();
 
-  // ---- byte rows of (slot s, half h, group jg) ----
-  constexpr u32 US = Geo::IU;
-  u32 s, h, jg;
-  if constexpr (LOGN == 6) {
-    h = tid & 1;
-    s = (tid >> 1) & (N - 1);
-    jg = tid >> 7;
-  } else {
-    s = tid & (N - 1);
-    h = tid >> LOGN;
-    jg = 0;
-  }
-  uint4 pl[7];
+    // ---- byte rows of (slot s, half h, group jg) ----
+    constexpr u32 US = Geo::IU;
+    u32 s, h, jg;
+    if constexpr (LOGN == 6) {
+      h = tid & 1;
+      s = (tid >> 1) & (N - 1);
+      jg = tid >> 7;
+    } else {
+      s = tid & (N - 1);
+      h = tid >> LOGN;
+      jg = 0;
+    }
+    uint4 pl[7];
 #pragma unroll
-  for (u32 q4 = 0; q4 < 4; q4++) {
-    u32 lo[4], hi[4], p[8];
+    for (u32 q4 = 0; q4 < 4; q4++) {
+      u32 lo[4], hi[4], p[8];
 #pragma unroll
-    for (u32 e = 0; e < 4; e++) {
-      const u32 t = 4 * q4 + e;
-      u64 w;
-      if constexpr (LOGN == 6) {
-        const u32 el = DIG ? 2 * t + jg : 16 * jg + t;
-        w = words[2 * np6_pos(el, s) + h];
-      } else {
-        w = words[npad((2 * t + h) * N + s)];
+      for (u32 e = 0; e < 4; e++) {
+        const u32 t = 4 * q4 + e;
+        u64 w;
+        if constexpr (LOGN == 6) {
+          const u32 el = DIG ? 2 * t + jg : 16 * jg + t;
+          w = words[2 * np6_pos(el, s) + h];
+        } else {
+          w = words[npad((2 * t + h) * N + s)];
+        }
+        lo[e] = (u32)w;
+        hi[e] = (u32)(w >> 32);
       }
-      lo[e] = (u32)w;
-      hi[e] = (u32)(w >> 32);
+      img_transpose4(lo[0], lo[1], lo[2], lo[3], p[0], p[1], p[2], p[3]);
+      img_transpose4(hi[0], hi[1], hi[2], hi[3], p[4], p[5], p[6], p[7]);
+#pragma unroll
+      for (u32 y = 0; y < 7; y++) {
+        if (q4 == 0) pl[y].x = p[y];
+        if (q4 == 1) pl[y].y = p[y];
+        if (q4 == 2) pl[y].z = p[y];
+        if (q4 == 3) pl[y].w = p[y];
+      }
     }
-    img_transpose4(lo[0], lo[1], lo[2], lo[3], p[0], p[1], p[2], p[3]);
-    img_transpose4(hi[0], hi[1], hi[2], hi[3], p[4], p[5], p[6], p[7]);
+    __syncthreads();
+    uint4* tile = (uint4*)ni_smem;
 #pragma unroll
-    for (u32 y = 0; y < 7; y++) {
-      if (q4 == 0) pl[y].x = p[y];
-      if (q4 == 1) pl[y].y = p[y];
-      if (q4 == 2) pl[y].z = p[y];
-      if (q4 == 3) pl[y].w = p[y];
+    for (u32 y = 0; y < 7; y++) tile[s * US + jg * 14 + h * 7 + y] = pl[y];
+    __syncthreads();
+    // image units of the JG groups: 14 units per (slot, group)
+    const u64 w2 = R.split ? R.width / 2 : R.width;
+    u64 base[JG];
+#pragma unroll
+    for (u32 g = 0; g < JG; g++) {
+      const u64 i = DIG ? e0 : e0 + 16 * g;
+      const u32 row = out_row(g);
+      const bool second = i >= w2;
+      base[g] = cki_unit(im, R.k0 + row + (second ? out_rows : 0), second ? i - w2 : i);
     }
-  }
-  __syncthreads();
-  uint4* tile = (uint4*)ni_smem;
-#pragma unroll
-  for (u32 y = 0; y < 7; y++) tile[s * US + jg * 14 + h * 7 + y] = pl[y];
-  __syncthreads();
-  // image units of the JG groups: 14 units per (slot, group)
-  const u64 w2 = R.split ? R.width / 2 : R.width;
-  u64 base[JG];
-#pragma unroll
-  for (u32 g = 0; g < JG; g++) {
-    const u64 i = DIG ? e0 : e0 + 16 * g;
-    const u32 row = out_row(g);
-    const bool second = i >= w2;
-    base[g] = cki_unit(im, R.k0 + row + (second ? out_rows : 0), second ? i - w2 : i);
-  }
-  uint4* out = (uint4*)im.p;
-  const u32 sstride = 4 * im.VP;
-  for (u32 u = tid; u < N * 14 * JG; u += Geo::THREADS) {
-    const u32 ss = u / (14 * JG), rem = u % (14 * JG);
-    const u32 g = JG == 2 && rem >= 14 ? 1 : 0;
-    out[(g ? base[JG - 1] : base[0]) + (u64)ss * sstride + (rem - 14 * g)] = tile[ss * US + rem];
+    uint4* out = (uint4*)im.p;
+    const u32 sstride = 4 * im.VP;
+    for (u32 u = tid; u < N * 14 * JG; u += Geo::THREADS) {
+      const u32 ss = u / (14 * JG), rem = u % (14 * JG);
+      const u32 g = JG == 2 && rem >= 14 ? 1 : 0;
+      out[(g ? base[JG - 1] : base[0]) + (u64)ss * sstride + (rem - 14 * g)] = tile[ss * US + rem];
+    }
+    __syncthreads();
   }
   if (!DIG && R.mag_or) {
 #pragma unroll
@@ -252,7 +257,9 @@ int img_go(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStream_t 
   const int tr = salsaa_trace_begin(DIG ? "ntt_digits_kernel" : "ntt_kernel", st,
                                     coeffs * (DIG ? 8 + 2 * (7 + 4 + (a.rows.slots ? 8 : 0))
                                                   : 15 + (a.rows.slots ? 8 : 0)));
-  kern<<<(unsigned)blocks, Geo::THREADS, Geo::SMEM, st>>>(a, im, T);
+  // gated: a grid that leaves quickly when the gate is closed
+  const u64 grid = a.rows.gate && blocks > 444 ? 444 : blocks;
+  kern<<<(unsigned)grid, Geo::THREADS, Geo::SMEM, st>>>(a, im, T);
   salsaa_trace_end(tr, st);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();

@@ -18,7 +18,7 @@ namespace salsaa {
 // layout (16-byte K slices of VP rows each), one bulk copy.
 struct CkImage {
   uint8_t* p;
-  u32 R, G, VP, n, btlog, nlc, nhg;
+  u32 R, G, VP, n, btlog, nlc, nhg, glog;  // glog: log2 G
   u64 width;
 };
 constexpr u32 CKI_CHUNK = 64;
@@ -35,11 +35,9 @@ bool cki_ok(u32 R, u64 width, u32 n, u32 ck_bt, u64 q);
 
 // 16-byte unit index of (image row k, element i, slot 0, byte row 0); i a multiple of 16.
 __device__ __forceinline__ u64 cki_unit(const CkImage& im, u32 k, u64 i) {
-  const u64 hi = i >> im.btlog;
-  const u32 lo = (u32)(i & ((1ull << im.btlog) - 1));
-  const u32 g = (u32)(hi & (im.G - 1));  // G is a power of two
-  const u64 hg = hi / im.G;
-  return (((hg * im.nlc + (lo >> 6)) * im.n) * 4 + ((lo >> 4) & 3)) * im.VP + (g * im.R + k) * 14;
+  const u32 hi = (u32)(i >> im.btlog), lo = (u32)i & ((1u << im.btlog) - 1);
+  const u32 g = hi & (im.G - 1), hg = hi >> im.glog;
+  return (u64)((hg * im.nlc + (lo >> 6)) * im.n * 4 + ((lo >> 4) & 3)) * im.VP + (g * im.R + k) * 14;
 }
 
 // Forward incomplete transform of coefficient-form rows (canonical words)
@@ -52,8 +50,22 @@ struct ImgRows {
   u64 width;
   u64* slots;        // slot-form words too (rows x width), or null
   u64* mag_or;       // OR of the centred magnitudes of the source, or null
+  const u32* gate;   // run only if *gate != 0 (the tensor-core transform gave up), or null
 };
 int ntt_img_launch(const ImgRows& a, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// Source row k and first element e0 of item `item` (2^sellog elements, at most
+// 64).  All rows of one tile (source rows, halves, stacked key blocks) come
+// from consecutive items, so the 224-byte runs that they write side by side
+// meet in L2.  32-bit arithmetic: a 64-bit division costs hundreds of clocks.
+__device__ __forceinline__ void img_item(const ImgRows& R, const CkImage& im, u32 sellog, u32 item, u32& k, u64& e0) {
+  const u32 slog = R.split ? 1 : 0, t = item / (R.rows << (slog + im.glog));
+  u32 f = item - t * (R.rows << (slog + im.glog));
+  const u32 f2 = f / R.rows, hs = f2 & slog, g = f2 >> slog;
+  k = f - f2 * R.rows;
+  const u32 pl = im.btlog - sellog, lg = t & ((1u << pl) - 1), hg = t >> pl;
+  e0 = (hs ? R.width / 2 : 0) + ((u64)((hg << im.glog) + g) << im.btlog) + ((u64)lg << sellog);
+}
 
 // The same for the two decomposition digits of each source row: digit c of
 // row r is row 2 r + c of the digit space (2 rows x width), whose halves
@@ -67,6 +79,28 @@ struct ImgDigits {
   int* coef;
 };
 int ntt_img_digits_launch(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// The same transforms on the tensor cores, for short values (ntt_tc.cu; d =
+// 128 or 256): source values of 8 bits (limbs = 1) or 16 (limbs = 2) or, with
+// bw_or, the two digits when they are at most 7 bits.  Values that do not fit
+// set *flag (zeroed by the caller; digits write it), and the image is then
+// incomplete: launch ntt_img_launch / ntt_img_digits_launch gated on it.
+// c8: the short values themselves (8 bits), same rows and order as the
+// source (digits: row 2 r + c), or null.
+struct TcArgs {
+  ImgRows rows;  // slots and mag_or are not used
+  u32* flag;
+  int8_t* c8;
+  const u64* bw_or;  // digits only
+  u64* rlog_out;
+  u64* radix_out;
+};
+bool ntt_tc_ok(const NttDev& T);
+int ntt_tc_launch(const TcArgs& a, int limbs, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// Transform of rows that are usually short: on the tensor cores when the
+// shapes allow, else (or, gated on *flag, when a value does not fit) FP64.
+int ntt_short_img_launch(const ImgRows& a, u32* flag, const CkImage& im, const NttDev& T, cudaStream_t st);
 
 // Key rows x image (q < 2^50): the sums of key row r and witness row k are
 // added to acc row r * R + k (slot form, zeroed by the caller).

@@ -1879,7 +1879,7 @@ extern "C" int salsaa_commit(salsaa_ctx* c, const uint64_t* d_w, uint64_t rows, 
     for (u32 k = 0; k < rows; k++) r.src[k] = d_w + (u64)k * width * d;
     r.rows = (u32)rows;
     r.width = width;
-    TRY(ntt_img_launch(r, im, *c->T, st));
+    TRY(ntt_short_img_launch(r, &ds->tc_flag, im, *c->T, st));
     a.img = &im;
   } else {
     TRY(ntt_launch(d_w, ws, rows * width, *c->T, true, false, st));

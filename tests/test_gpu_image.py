@@ -40,3 +40,30 @@ def test_commit_image(api, oracle, d, ms, width, wit_len, rows, top):
     ctx = api.Context(p, crs_seed=9)
     got = api.to_host(ctx.parallel_dot_series_matrix(api.to_dev(w)))
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("d,ms,width,rows,lo,hi,odd", [
+    (128, 12, 1 << 14, 1, -128, 128, None),   # every value that fits a byte
+    (128, 4, 64, 3, -128, 128, None),         # the fewest elements
+    (128, 4, 1 << 14, 2, -1, 2, 128),         # ternary but for one value past the byte, late in the rows
+    (128, 4, 1 << 14, 2, -1, 2, -129),
+    (256, 7, 1 << 13, 2, -128, 128, None),
+    (256, 3, 1 << 13, 1, -128, -127, None),   # all at the lower end: the largest sums
+    (256, 3, 1 << 13, 1, -1, 2, 128),
+    (128, 3, 1 << 13, 1, -128, -127, None),
+    (128, 3, 1 << 15, 4, -128, 128, None),    # tens of items per CTA: every ring of the pipeline wraps
+    (256, 3, 1 << 14, 4, -128, 128, None),
+])
+def test_commit_short_values(api, oracle, d, ms, width, rows, lo, hi, odd):
+    """Short witnesses go through the byte transform on the tensor cores; one
+    value outside [-128, 127] sends the whole witness to the FP64 transform."""
+    q = Q[d]
+    p = P.make_params(d, q, ms, max(width, 128), 1)
+    v = np.random.default_rng(width + rows).integers(lo, hi, size=(rows, width, d))
+    if odd is not None:
+        v[-1, -5, d - 3] = odd
+    w = np.where(v < 0, q + v, v).astype(np.uint64)
+    want = oracle.commit_ck(p, 2, w)
+    ctx = api.Context(p, crs_seed=2)
+    got = api.to_host(ctx.parallel_dot_series_matrix(api.to_dev(w)))
+    assert np.array_equal(got, want)
