@@ -1514,7 +1514,8 @@ __global__ void fold_pre_kernel(const u64* c, u32 rows, u32 n, ModQ M, const u64
 constexpr u32 FOLD_EL = 4;
 
 __global__ void __launch_bounds__(256) fold_fp_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M,
-                                                      const u64* __restrict__ pre, u64* out) {
+                                                      const u64* __restrict__ pre, u64* out, const u32* gate) {
+  if (gate && !*gate) return;
   const u32 n = 1u << logn, hn = n >> 1;
   const u64 groups = (width + FOLD_EL - 1) / FOLD_EL;
   const u64 tot = groups << (logn - 1);
@@ -1574,7 +1575,8 @@ __global__ void __launch_bounds__(256) fold_fp_kernel(RowSet w, u32 rows, u64 wi
 // per-row terms (each below 4q) are summed without reduction and reduced once.
 template <bool LAZY>
 __global__ void fold_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M, const u64* __restrict__ pre,
-                            u64* out) {
+                            u64* out, const u32* gate) {
+  if (gate && !*gate) return;
   const u32 n = 1u << logn;
   const u64 tot = width << logn, q = M.q, q2 = 2 * q;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
@@ -1617,7 +1619,8 @@ __global__ void fold_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M, con
 // rows and output).
 template <bool LAZY>
 __global__ void __launch_bounds__(256) fold_vec_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M,
-                                                       const u64* __restrict__ pre, u64* out) {
+                                                       const u64* __restrict__ pre, u64* out, const u32* gate) {
+  if (gate && !*gate) return;
   const u32 n = 1u << logn, hn = n >> 1;
   const u64 tot = width << (logn - 1), q = M.q, q2 = 2 * q;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
@@ -1676,7 +1679,7 @@ __global__ void __launch_bounds__(256) fold_vec_kernel(RowSet w, u32 rows, u64 w
 }
 
 int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ& M, const u64* c_slot, u64* pre,
-                u64* out_slot, cudaStream_t st) {
+                u64* out_slot, cudaStream_t st, const u32* gate) {
   if (rows == 0 || rows > MAX_WROWS) return salsaa_set_error(-2, "fold: bad row count");
   if (w_slot.narrow) return salsaa_set_error(-2, "fold: slot-form rows must be canonical words");
   const bool lazy = M.q < (1ULL << 57);
@@ -1688,19 +1691,20 @@ int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ&
   if (rc) return rc;
   if (fp) {
     fold_fp_kernel<<<grid_1d((width + FOLD_EL - 1) / FOLD_EL * T.n / 2, 256), 256, 0, st>>>(w_slot, rows, width,
-                                                                                            T.logn, M, pre, out_slot);
+                                                                                            T.logn, M, pre, out_slot,
+                                                                                            gate);
     return check_launch("fold");
   }
   if (vec) {
     const unsigned g = grid_1d(width * T.n / 2, 256);
-    if (lazy) fold_vec_kernel<true><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot);
-    else fold_vec_kernel<false><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot);
+    if (lazy) fold_vec_kernel<true><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
+    else fold_vec_kernel<false><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
     return check_launch("fold");
   }
   if (lazy)
-    fold_kernel<true><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot);
+    fold_kernel<true><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
   else
-    fold_kernel<false><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot);
+    fold_kernel<false><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
   return check_launch("fold");
 }
 

@@ -55,6 +55,9 @@ struct DevState {
   u64 bw_or[16];   // decomposition: OR of centred magnitudes, per decomposition index
   u64 rlog[16];    // decomposition: radix log2, per decomposition index
   u64 proj_flag;   // projection: set when a witness value does not fit int8
+  // per round: the witness rows (projected row) do not fit the byte-tile steps
+  // (zeroed with bw_or when a proof starts); the word steps run instead
+  u32 wide[16], wide_p[16];
   u32 tc_flag;     // tensor-core transform of a single call: set when a value does not fit int8
 };
 
@@ -174,9 +177,10 @@ int launch_project_umma(RowSet in, u32 rows, u64 nch, u32 d, u64 q, u32 cw, cons
                         cudaStream_t st);
 
 int launch_fold_challenge(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, cudaStream_t st);
-// pre: scratch of rows x n x 6 words (Shoup constants of the challenges)
+// pre: scratch of rows x n x 6 words (Shoup constants of the challenges); with
+// gate the products run only if *gate != 0
 int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ& M, const u64* c_slot, u64* pre,
-                u64* out_slot, cudaStream_t st);
+                u64* out_slot, cudaStream_t st, const u32* gate = nullptr);
 
 // <statement rows, witness rows> in slot form.  acc: (nck + nsc) x rows x d
 // scratch; out_slot: results in statement order given by `order`.

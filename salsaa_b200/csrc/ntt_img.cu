@@ -285,7 +285,56 @@ int img_launch(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStrea
   }
 }
 
+// Gated inverse incomplete transform (ntt_fp_kernel's, one 4096-coefficient
+// tile per step of a grid that leaves quickly when the gate is closed).
+template <int LOGN>
+__global__ void __launch_bounds__(256) ntt_inv_gated_kernel(const u64* in, u64* out, u64 units, NttDev T,
+                                                            const u32* gate, u64* mag_or) {
+  constexpr int PL = ph_count(LOGN) - 1;
+  constexpr u32 UPT = NR_TILE >> LOGN;
+  __shared__ double sm[NR_TILE + NR_TILE / 16];
+  if (!*gate) return;
+  u32 unit, tu;
+  nr_map<LOGN, true>(threadIdx.x, unit, tu);
+  u64 mag = 0;
+  for (u64 b = blockIdx.x; b * UPT < units; b += gridDim.x) {
+    const u64 ug = b * UPT + unit;
+    const bool active = ug < units;
+    double x[16];
+    if (active) {
+      nf_load_global<LOGN, true, true>(x, in, ug, tu, T.q, nullptr);
+      nf_compute<LOGN, 0, true>(x, tu, T);
+      nr_store_smem<LOGN, 0, true>(x, sm, unit, tu);
+    }
+    __syncthreads();
+    if (active) {
+      nr_load_smem<LOGN, PL, true>(x, sm, unit, tu);
+      nf_compute<LOGN, PL, true>(x, tu, T);
+      nf_store_global<LOGN, true, true>(x, out, ug, tu, T, mag_or ? &mag : nullptr);
+    }
+    __syncthreads();
+  }
+  if (mag_or) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mag |= __shfl_xor_sync(0xffffffffu, mag, o);
+    if ((threadIdx.x & 31) == 0 && mag) atomicOr((unsigned long long*)mag_or, (unsigned long long)mag);
+  }
+}
+
 }  // namespace
+
+int ntt_inv_gated_launch(const u64* in, u64* out, u64 count, const NttDev& T, const u32* gate, u64* mag_or,
+                         cudaStream_t st) {
+  if ((T.logn != 6 && T.logn != 7) || T.q >= NR_RELAX_Q || (uintptr_t)in % 16 || (uintptr_t)out % 16 || !gate)
+    return salsaa_set_error(-2, "ntt_inv_gated: shape or alignment not supported");
+  const u64 units = 2 * count, tiles = (units * T.n + NR_TILE - 1) / NR_TILE;
+  const unsigned grid = (unsigned)(tiles < 592 ? tiles : 592);
+  if (T.logn == 6) ntt_inv_gated_kernel<6><<<grid, 256, 0, st>>>(in, out, units, T, gate, mag_or);
+  else ntt_inv_gated_kernel<7><<<grid, 256, 0, st>>>(in, out, units, T, gate, mag_or);
+  salsaa_count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "ntt_inv_gated launch");
+}
 
 int ntt_img_launch(const ImgRows& a, const CkImage& im, const NttDev& T, cudaStream_t st) {
   ImgDigits d{};

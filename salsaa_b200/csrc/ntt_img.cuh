@@ -85,22 +85,37 @@ int ntt_img_digits_launch(const ImgDigits& a, const CkImage& im, const NttDev& T
 // bw_or, the two digits when they are at most 7 bits.  Values that do not fit
 // set *flag (zeroed by the caller; digits write it), and the image is then
 // incomplete: launch ntt_img_launch / ntt_img_digits_launch gated on it.
-// c8: the short values themselves (8 bits), same rows and order as the
-// source (digits: row 2 r + c), or null.
+// c8: the short values themselves as byte tiles (see below), rows as the
+// source's (digits: row 2 r + c; two limbs: rows 2 r and 2 r + 1, low and high
+// byte, both signed), or null.
 struct TcArgs {
-  ImgRows rows;  // slots and mag_or are not used
+  ImgRows rows;  // slots are not used
   u32* flag;
   int8_t* c8;
+  int* coef;         // the digits as centred int32 in source order, or null
   const u64* bw_or;  // digits only
   u64* rlog_out;
   u64* radix_out;
 };
+// Byte tiles of a row of width x d values: 64 elements each, 16-position
+// slices of 64 x 16 bytes,
+//   offset(i, p) = (i / 64) 64 d + (p / 16) 1024 + (i % 64) 16 + p % 16.
+// One tile is contiguous and an operand as it lies: K-major with elements as
+// rows and positions as K, or MN-major with positions as rows and elements as K.
+__host__ __device__ inline u64 c8_offset(u64 i, u32 p, u32 d) {
+  return (i >> 6) * 64 * d + (u64)(p >> 4) * 1024 + (i & 63) * 16 + (p & 15);
+}
 bool ntt_tc_ok(const NttDev& T);
 int ntt_tc_launch(const TcArgs& a, int limbs, const CkImage& im, const NttDev& T, cudaStream_t st);
 
 // Transform of rows that are usually short: on the tensor cores when the
 // shapes allow, else (or, gated on *flag, when a value does not fit) FP64.
 int ntt_short_img_launch(const ImgRows& a, u32* flag, const CkImage& im, const NttDev& T, cudaStream_t st);
+
+// Inverse incomplete transform of `count` elements (n = 64 or 128, q < 2^50),
+// run only if *gate != 0; mag_or as in ntt_launch.
+int ntt_inv_gated_launch(const u64* in, u64* out, u64 count, const NttDev& T, const u32* gate, u64* mag_or,
+                         cudaStream_t st);
 
 // Key rows x image (q < 2^50): the sums of key row r and witness row k are
 // added to acc row r * R + k (slot form, zeroed by the caller).

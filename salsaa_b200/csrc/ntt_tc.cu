@@ -155,8 +155,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
   using Geo = TcGeom<LOGN, MODE>;
   constexpr u32 N = Geo::N, D = Geo::D, SEL = Geo::SEL, SELLOG = Geo::SELLOG, SUB = Geo::SUB, WPT = Geo::WPT, JG = Geo::JG, US = Geo::IU;
   constexpr u32 EPI = MODE == TC_LIMBS ? 128 : 256;  // threads per unit
+  // a barrier pair per set of threads that shares units, so each set sees
+  // every phase of its own (a parity wait cannot skip one)
+  constexpr u32 NBAR = TC_EPI / EPI;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], acc_full[2], acc_empty[2], w_bar;
+  __shared__ uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], acc_full[NBAR], acc_empty[NBAR], w_bar;
   __shared__ uint64_t raw_full[TC_RAW], raw_empty[TC_RAW];
   __shared__ uint32_t tslot;
   const u32 tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
       umma::mbar_init(&full_bar[i], TC_CONV);
       umma::mbar_init(&empty_bar[i], 1);
     }
-    for (u32 i = 0; i < 2; i++) {
+    for (u32 i = 0; i < NBAR; i++) {
       umma::mbar_init(&acc_full[i], 1);
       umma::mbar_init(&acc_empty[i], EPI);
     }
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
   const u32 tmem = tslot;
 
   if (warp >= TC_EPI / 32 && warp < (TC_EPI + TC_CONV) / 32) {
-    u32 fit = 0, fith = 0;
+    u32 fit = 0, fith = 0, mag = 0;
     bool ok = true;
     u32 it = 0;
     u32 ri = 0;  // items so far: the parity of their source ring uses
@@ -292,7 +295,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
         } else {
           u32 x[4];
 #pragma unroll
-          for (u32 e = 0; e < 4; e++) x[e] = centred(v[e], fit, fith);
+          for (u32 e = 0; e < 4; e++) {
+            x[e] = centred(v[e], fit, fith);
+            if (MODE == TC_LIMBS) {
+              const int c = (int)(x[e] - BIAS);
+              mag |= (u32)(c < 0 ? -c : c);
+            }
+          }
           const u32 x01 = __byte_perm(x[0], x[1], 0x5140), x23 = __byte_perm(x[2], x[3], 0x5140);
           pk[i][0] = __byte_perm(x01, x23, 0x5410) ^ 0x80808080u;
           if (MODE == TC_LIMBS) pk[i][MODE == TC_BYTES ? 0 : 1] = __byte_perm(x01, x23, 0x7632) ^ 0x80808080u;
@@ -337,19 +346,40 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
       umma::fence_proxy_async();
 #pragma unroll
       for (u32 sub = 0; sub < SUB; sub++, it++) umma::mbar_arrive(&full_bar[it % TC_STAGES]);
-      // the short coefficients themselves, four bytes per lane (after the
-      // fence, which would wait for these stores)
+      // the short values themselves, four per lane (after the fence, which
+      // would wait for these stores)
       if (a.c8) {
 #pragma unroll
         for (u32 i = 0; i < WPT / 4; i++) {
           u32 el, p;
           quad(i, ct, el, p);
-          const u64 o = ((e0 + el) * D + p) / 4;
+          const u64 o = c8_offset(e0 + el, p, D);
 #pragma unroll
-          for (u32 c = 0; c < (MODE == TC_DIGITS ? 2u : 1u); c++)
-            ((u32*)a.c8)[(u64)(MODE == TC_DIGITS ? 2 * k + c : k) * (R.width * D / 4) + o] = pk[i][c];
+          for (u32 c = 0; c < (MODE == TC_BYTES ? 1u : 2u); c++)
+            *(u32*)(a.c8 + (u64)(MODE == TC_BYTES ? k : 2 * k + c) * R.width * D + o) = pk[i][c];
         }
       }
+      if (MODE == TC_DIGITS && a.coef) {
+#pragma unroll
+        for (u32 i = 0; i < WPT / 4; i++) {
+          u32 el, p;
+          quad(i, ct, el, p);
+#pragma unroll
+          for (u32 c = 0; c < 2; c++) {
+            const u32 x = pk[i][MODE == TC_BYTES ? 0 : c];
+            *(int4*)(a.coef + ((u64)(2 * k + c) * R.width + e0 + el) * D + p) =
+                make_int4((int)(int8_t)x, (int)(int8_t)(x >> 8), (int)(int8_t)(x >> 16), (int)(int8_t)(x >> 24));
+          }
+        }
+      }
+    }
+    if (MODE != TC_DIGITS && R.mag_or) {
+      // magnitudes of a thread whose values all fit (else the FP64 kernel
+      // collects them)
+      if (unfit(fit, fith)) mag = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mag |= __shfl_xor_sync(0xffffffffu, mag, o);
+      if (lane == 0 && mag) atomicOr((unsigned long long*)R.mag_or, (unsigned long long)mag);
     }
     if (MODE != TC_DIGITS && unfit(fit, fith)) *a.flag = 1;
   } else if (warp == (TC_EPI + TC_CONV) / 32 + 1) {
@@ -383,7 +413,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
 #pragma unroll
       for (u32 sub = 0; sub < SUB; sub++, it++) {
         const u32 nb = it & 1;
-        if (it >= 2 && !(ok = umma::mbar_wait(&acc_empty[nb], ((it >> 1) - 1) & 1, err, 23))) break;
+        // TMEM buffer nb was last used by unit it - 2
+        if (it >= 2 && !(ok = umma::mbar_wait(&acc_empty[(it - 2) % NBAR], ((it - 2) / NBAR) & 1, err, 23))) break;
         if (!(ok = umma::mbar_wait(&full_bar[st], par, err, 24))) break;
         umma::fence_after_sync();
         const uint64_t bd = bd0 + st * (TC_BTILE >> 4);
@@ -395,7 +426,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
               umma::mma_i8_u(tmem + nb * (7 * TC_COLS) + y * TC_COLS, ad0 + y * 1024 + ks * 256,
                              bd + ks * (2 * TC_SLICE >> 4), idesc, ks > 0 ? 1u : 0u);
           umma::commit(&empty_bar[st]);
-          umma::commit(&acc_full[nb]);
+          umma::commit(&acc_full[it % NBAR]);
         }
         __syncwarp();
         if (++st == TC_STAGES) {
@@ -405,7 +436,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
       }
     }
     // MMAs still in flight complete before TMEM is freed
-    for (u32 c = it >= 2 ? it - 2 : 0; c < it; c++) umma::mbar_wait(&acc_full[c & 1], (c >> 1) & 1, err, 25);
+    for (u32 c = it >= 2 ? it - 2 : 0; c < it; c++) umma::mbar_wait(&acc_full[c % NBAR], (c / NBAR) & 1, err, 25);
   } else {
     // group eg takes the units it = eg mod 2; TMEM lane m; ch: half of the
     // columns, or (two limbs) of the group's units
@@ -432,7 +463,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
         // all threads of the unit stop together, also when only some of them
         // gave up; the barrier also orders the copies out of this tile before
         // its new rows
-        ok = umma::mbar_wait(&acc_full[nb], (it >> 1) & 1, err, 26);
+        ok = umma::mbar_wait(&acc_full[it % NBAR], (it / NBAR) & 1, err, 26);
         if (!(ok = bar_tc_and<EPI>(ok, bar))) break;
         umma::fence_after_sync();
         const u32 tb = tmem + (((warp & 3) * 32) << 16) + nb * (7 * TC_COLS) + (MODE == TC_LIMBS ? 0 : ch * 16);
@@ -456,7 +487,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
           }
           if (q4 == 3) {
             umma::fence_before_sync();
-            umma::mbar_arrive(&acc_empty[nb]);
+            umma::mbar_arrive(&acc_empty[it % NBAR]);
           }
           u64 wv[4];
 #pragma unroll
@@ -554,7 +585,8 @@ int ntt_tc_launch(const TcArgs& a, int limbs, const CkImage& im, const NttDev& T
   const bool digits = a.bw_or != nullptr;
   const u64 w2 = R.split ? R.width / 2 : R.width;
   const u32 out_rows = (digits ? 2 : 1) * R.rows;
-  if (!ntt_tc_ok(T) || !a.flag || !im.p || im.n != T.n || im.width != w2 ||
+  // magnitudes are collected for two limbs only
+  if (!ntt_tc_ok(T) || !a.flag || (R.mag_or && (digits || limbs != 2)) || !im.p || im.n != T.n || im.width != w2 ||
       R.k0 + out_rows * (R.split ? 2 : 1) > im.R || R.rows == 0 || R.rows > MAX_WROWS || w2 < CKI_CHUNK ||
       (R.width & (R.width - 1)) || limbs < 1 || limbs > 2 || (digits && !a.rlog_out))
     return salsaa_set_error(-2, "ntt_tc: rows outside the image");

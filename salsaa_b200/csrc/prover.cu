@@ -17,6 +17,7 @@
 #include "host_math.h"
 #include "kernels.cuh"
 #include "ntt_img.cuh"
+#include "short_tc.cuh"
 
 using namespace salsaa;
 
@@ -172,7 +173,14 @@ struct Shapes {
   u32 nsc_total = 0;         // scalar rows pushed by the whole proof
   bool use_img = false;      // every key-row product of the proof goes through a byte image
   u64 max_img = 0;           // its largest image, bytes
+  bool use_short = false;    // short rows go through the tensor-core transforms and steps
 };
+
+// Words of a slot's byte-tile buffers: the witness rows, the projected row's
+// two limbs, the fold challenges' blocks.
+static u64 short_words(u64 d_rows_width, u64 fp_width, u64 d) {
+  return d_rows_width * d / 8 + 2 * fp_width * d / 8 + fold_tz_bytes(8, (u32)d) / 8;
+}
 
 static Shapes walk(const salsaa_params* p) {
   Shapes S;
@@ -289,6 +297,14 @@ static Shapes walk(const salsaa_params* p) {
   if (K > S.max_rows) S.max_rows = (u32)K;
   if (!p->folding) w += K * width * d;
   S.proof_words = w;
+  // The image and the byte tiles live in what the slot-form projected row and
+  // the sumcheck's former full-length buffers took; a set for which that is
+  // not enough (no rounds, one folded row) keeps the slot-form path, so no
+  // slot needs more memory than it did.
+  const u64 room = (S.max_fp_width + S.max_nc_rows_width * 7 / 8 + S.max_nc_rows_width / 2 - S.max_nc_rows_width / 128) * d;
+  S.use_short = S.use_img && (d == 128 || d == 256) && q > (1ULL << 49) && (u32)q >= (1u << 16) &&
+                S.max_img / 8 + short_words(S.max_d_rows_width, S.max_fp_width, d) <= room;
+  S.use_img = S.use_img && S.max_img / 8 <= room;
   if (!S.use_img) S.max_img = 0;
   S.ok = true;
   return S;
@@ -428,6 +444,9 @@ struct salsaa_prover {
   u64 *Dc = nullptr, *Ds = nullptr, *Fc = nullptr, *Fs = nullptr, *Pc = nullptr;
   u64* Ps = nullptr;       // slot form of the projected row; null with an image (only the key rows read it)
   uint8_t* img = nullptr;  // byte image of the key rows' witness (ntt_img.cuh), or null
+  int8_t* c8 = nullptr;    // the round's short witness rows as byte tiles, or null
+  int8_t* p8 = nullptr;    // the projected row's two byte limbs, likewise
+  int8_t* tz = nullptr;    // Toeplitz blocks of the fold challenges
   SumcheckBufs sc{};
   u64* row_base = nullptr;  // TENSOR row bases, nsc_total x d
   u64* row_cj = nullptr;    // PERIODIC row scalars, rounds x CK_BLOCK
@@ -486,6 +505,7 @@ extern "C" uint64_t salsaa_workspace_bytes(const salsaa_params* p) {
   words += 2 * S.max_d_rows_width * d;        // Dc, Ds
   words += (S.use_img ? 3 : 4) * S.max_fp_width * d;  // Fc, Fs, Pc, and Ps without an image
   words += S.max_img / 8;                     // byte image of the key rows' witness
+  if (S.use_short) words += short_words(S.max_d_rows_width, S.max_fp_width, d);  // byte tiles
   words += S.max_nc_rows_width * d / 8;       // sumcheck a
   words += S.max_nc_rows_width * d / 128;     // sumcheck b
   words += (u64)MAX_WROWS * 256 + 1;          // sumcheck Gram matrices
@@ -537,6 +557,9 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (rc = m.alloc(&pr->Fs, S.max_fp_width * d, "Fs")) || (rc = m.alloc(&pr->Pc, S.max_fp_width * d, "Pc")) ||
       (!S.use_img && (rc = m.alloc(&pr->Ps, S.max_fp_width * d, "Ps"))) ||
       (S.use_img && (rc = m.alloc(&pr->img, S.max_img, "key-row image"))) ||
+      (S.use_short && (rc = m.alloc(&pr->c8, S.max_d_rows_width * d, "byte tiles"))) ||
+      (S.use_short && (rc = m.alloc(&pr->p8, 2 * S.max_fp_width * d, "projected row's limbs"))) ||
+      (S.use_short && (rc = m.alloc(&pr->tz, fold_tz_bytes(8, (u32)d), "fold challenge blocks"))) ||
       (rc = m.alloc(&pr->sc.a, S.max_nc_rows_width * d / 8 + 1, "sumcheck a")) ||
       (rc = m.alloc(&pr->sc.b, S.max_nc_rows_width * d / 128 + 1, "sumcheck b")) ||
       (rc = m.alloc(&pr->sc.sums, 2ULL * 64 * MAX_WROWS * 3, "sumcheck sums")) ||
@@ -651,7 +674,14 @@ extern "C" int salsaa_prover_set_overlap(salsaa_prover* pr, int on) {
   return 0;
 }
 
-__global__ void set_seed_kernel(DevState* ds, u64 seed) { ds->seed = seed; }
+__global__ void set_seed_kernel(DevState* ds, u64 seed) {
+  const u32 t = threadIdx.x;
+  if (t == 0) ds->seed = seed;
+  if (t < 16) {
+    ds->bw_or[t] = 0;
+    ds->wide[t] = ds->wide_p[t] = 0;
+  }
+}
 
 // <statement rows [0, nck) ++ scalar rows [sc_first, sc_first + nsc), witness rows>
 // -> slot-form ring elements in pr->cout, row-major (statement, witness).
@@ -721,10 +751,26 @@ static RowSet rows_of_narrow(const u64* base, u32 rows, u64 width, u32 d) {
   return r;
 }
 
+// The K split (or unsplit) rows of the witness in pr->c8.
+static C8Rows c8_rows(const int8_t* c8, u32 K, u64 width, u32 d, bool split) {
+  C8Rows r{};
+  r.p = c8;
+  r.stride = (split ? 2 : 1) * width * d;
+  r.rows = K;
+  r.width = width;
+  for (u32 k = 0; k < K; k++) {
+    r.row[k] = split ? k % (K / 2) : k;
+    r.off[k] = split && k >= K / 2 ? width : 0;
+  }
+  return r;
+}
+
 // decomp_ell into two digits, as centred int32 coefficients (Dc), the image
-// rows and, with slots, slot-form words.
+// rows and, with slots, slot-form words.  With wide, digits of at most 7 bits
+// go through the tensor cores (and to pr->c8, without slot-form words); else
+// *wide is raised and the FP64 kernel does the round.
 static int decompose_image(salsaa_prover* pr, const RowSet& src, u32 rows, u64 width, u32 didx, bool split, u64* slots,
-                           u64* proof_radix, const CkImage& im) {
+                           u64* proof_radix, const CkImage& im, u32* wide) {
   ImgDigits a{};
   for (u32 k = 0; k < rows; k++) a.rows.src[k] = src.p[k];
   a.rows.rows = rows;
@@ -735,6 +781,19 @@ static int decompose_image(salsaa_prover* pr, const RowSet& src, u32 rows, u64 w
   a.rlog_out = &pr->ds->rlog[didx];
   a.radix_out = proof_radix;
   a.coef = (int*)pr->Dc;
+  if (wide) {
+    TcArgs t{};
+    t.rows = a.rows;
+    t.flag = wide;
+    t.c8 = pr->c8;
+    t.coef = a.coef;
+    t.bw_or = a.bw_or;
+    t.rlog_out = a.rlog_out;
+    t.radix_out = a.radix_out;
+    t.rows.slots = nullptr;
+    TRY(ntt_tc_launch(t, 1, im, *pr->ctx->T, pr->st));
+    a.rows.gate = wide;
+  }
   return ntt_img_digits_launch(a, im, *pr->ctx->T, pr->st);
 }
 
@@ -752,7 +811,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
   cudaError_t e = cudaMemcpyAsync(proof, pr->header_pinned, 8 * sizeof(u64), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: header");
   cur = 8;
-  set_seed_kernel<<<1, 1, 0, st>>>(pr->ds, seed);
+  set_seed_kernel<<<1, 32, 0, st>>>(pr->ds, seed);
   salsaa_count_launch();
   u32 K = (u32)P.init_wit_rep;
   u64 width = L;
@@ -784,10 +843,33 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     r.mag_or = mag;
     return ntt_img_launch(r, im, T, s);
   };
+  // Short rows (every witness of the relation) go through the tensor cores:
+  // image, byte tiles and fold.  A row that does not fit raises the round's
+  // flag, and the FP64 transforms and the slot-form fold, launched after them
+  // and gated on it, do the round.
+  const bool sh = c->S.use_short && ntt_tc_ok(T);
+  auto short_rows = [&](const RowSet& src, u32 rows, u64 w, u32 k0, bool split, int limbs, int8_t* c8, u32* flag,
+                        u64* slots, u64* mag, cudaStream_t s) {
+    TcArgs t{};
+    for (u32 k = 0; k < rows; k++) t.rows.src[k] = src.p[k];
+    t.rows.rows = rows;
+    t.rows.k0 = k0;
+    t.rows.split = split ? 1 : 0;
+    t.rows.width = w;
+    t.rows.mag_or = mag;
+    t.flag = flag;
+    t.c8 = c8;
+    TRY(ntt_tc_launch(t, limbs, im, T, s));
+    ImgRows g = t.rows;
+    g.gate = flag;
+    g.slots = slots;
+    return ntt_img_launch(g, im, T, s);
+  };
   if (imp) {
     const bool split = !P.folding && P.nof_rounds > 0;
     image(split ? 2 * K + 1 : K, split ? width / 2 : width);
-    TRY(image_rows(Wc, K, width, 0, split, pr->Ds, nullptr, st));
+    if (sh) TRY(short_rows(Wc, K, width, 0, split, 1, pr->c8, &pr->ds->wide[0], pr->Ds, nullptr, st));
+    else TRY(image_rows(Wc, K, width, 0, split, pr->Ds, nullptr, st));
   } else {
     TRY(ntt_launch(wbase, pr->Ds, (u64)K * width, T, true, false, st));
   }
@@ -811,7 +893,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       if (imp) {
         if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
         image(2 * parts * K + 1, width / 2);
-        TRY(decompose_image(pr, Wc, K, width, didx++, true, pr->Ds, proof + cur, im));
+        TRY(decompose_image(pr, Wc, K, width, didx++, true, pr->Ds, proof + cur, im, sh ? &pr->ds->wide[rd] : nullptr));
         narrow = true;
       } else {
         TRY(launch_decompose_ntt(Wc, K, width, d, q, parts, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
@@ -843,7 +925,8 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       Wc = rows_of(pr->Dc, K, width, d);
       if (imp) {
         image(2 * K + 1, width / 2);
-        TRY(image_rows(Wc, K, width, 0, true, pr->Ds, nullptr, st));
+        if (sh) TRY(short_rows(Wc, K, width, 0, true, 1, pr->c8, &pr->ds->wide[rd], pr->Ds, nullptr, st));
+        else TRY(image_rows(Wc, K, width, 0, true, pr->Ds, nullptr, st));
       }
       Ws = rows_of(pr->Ds, K, width, d);
     }
@@ -888,12 +971,13 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     if (next_decomp && didx < 16 && (imp || ntt_mag_ok(pr->Pc, pr->Ps, T, true)) &&
         ntt_mag_ok(pr->Fs, pr->Fc, T, true)) {
       mag = &pr->ds->bw_or[didx];
-      e = cudaMemsetAsync(mag, 0, sizeof(u64), ps);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: magnitude OR");
     }
     if (imp) {
       if (P.folding) image(1, width2);
-      TRY(image_rows(rows_of(pr->Pc, 1, width2, d), 1, width2, P.folding ? 0 : K2, false, nullptr, mag, ps));
+      const RowSet prow = rows_of(pr->Pc, 1, width2, d);
+      const u32 pk0 = P.folding ? 0 : K2;
+      if (sh) TRY(short_rows(prow, 1, width2, pk0, false, 2, nullptr, &pr->ds->wide_p[rd], nullptr, mag, ps));
+      else TRY(image_rows(prow, 1, width2, pk0, false, nullptr, mag, ps));
     } else {
       TRY(ntt_launch(pr->Pc, pr->Ps, width2, T, true, false, ps, mag));
     }
@@ -992,10 +1076,20 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     nsc += 1;  // witness_lhs joins the statement
     // fold (src/subroutines/fold.rs:22-27)
     TRY(mark(pr, PH_FOLD));
-    TRY(launch_fold_challenge(pr->ds, rd, K, d, q, pr->c_coef, st));
-    TRY(ntt_launch(pr->c_coef, pr->c_slot, K, T, true, false, st));
-    TRY(launch_fold(Ws, K, width, T, M, pr->c_slot, pr->fold_pre, pr->Fs, st));
-    TRY(ntt_launch(pr->Fs, pr->Fc, width, T, true, true, st, mag));
+    if (sh) {
+      u32* wide = &pr->ds->wide[rd];
+      const C8Rows w8 = c8_rows(pr->c8, K, width, d, !P.folding);
+      TRY(launch_fold_challenge_tz(pr->ds, rd, K, d, q, pr->c_coef, pr->tz, st));
+      TRY(launch_fold_tc(w8, d, q, pr->tz, pr->Fc, mag, wide, st));
+      TRY(ntt_launch(pr->c_coef, pr->c_slot, K, T, true, false, st));
+      TRY(launch_fold(Ws, K, width, T, M, pr->c_slot, pr->fold_pre, pr->Fs, st, wide));
+      TRY(ntt_inv_gated_launch(pr->Fs, pr->Fc, width, T, wide, mag, st));
+    } else {
+      TRY(launch_fold_challenge(pr->ds, rd, K, d, q, pr->c_coef, st));
+      TRY(ntt_launch(pr->c_coef, pr->c_slot, K, T, true, false, st));
+      TRY(launch_fold(Ws, K, width, T, M, pr->c_slot, pr->fold_pre, pr->Fs, st));
+      TRY(ntt_launch(pr->Fs, pr->Fc, width, T, true, true, st, mag));
+    }
     mag_ready = mag != nullptr;
     // send_cross_terms_before_join (src/subroutines/project.rs:229-245)
     RowSet Fr = rows_of(pr->Fs, 1, width, d), Frc = rows_of(pr->Fc, 1, width, d);
@@ -1023,7 +1117,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       if (imp) {
         if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
         image(2 * K, width);
-        TRY(decompose_image(pr, Wc, K, width, didx++, false, nullptr, proof + cur, im));
+        TRY(decompose_image(pr, Wc, K, width, didx++, false, nullptr, proof + cur, im, sh ? &pr->ds->wide[rd + 1] : nullptr));
         narrow = true;
       } else {
         TRY(launch_decompose_ntt(Wc, K, width, d, q, 2, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
@@ -1416,7 +1510,7 @@ static int verify_impl(salsaa_prover* pr, u64 seed, const u64* proof, int* verdi
   u64* dslot = pr->Ds;
   if ((e = cudaMemcpyAsync(dcoef, proof, words * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return salsaa_set_cuda_error(e, "verify: proof upload");
-  set_seed_kernel<<<1, 1, 0, st>>>(pr->ds, seed);  // the challenges drawn on the device
+  set_seed_kernel<<<1, 32, 0, st>>>(pr->ds, seed);  // the challenges drawn on the device
   salsaa_count_launch();
   std::vector<std::pair<u64, u64>> seg;
   proof_segments(P, seg);
@@ -1982,7 +2076,7 @@ extern "C" int salsaa_sumcheck(const uint64_t* d_w, uint64_t rows, uint64_t n, u
   t.want(&B.gram, rows * 256 + 1);
   t.want(&ds, 1);
   TRY(t.alloc());
-  set_seed_kernel<<<1, 1, 0, st>>>(ds, seed);
+  set_seed_kernel<<<1, 32, 0, st>>>(ds, seed);
   const u64 nr = ilog2u(n);
   RowSet w = rows_of(d_w, (u32)rows, n / d, (u32)d);
   return launch_sumcheck(w, (u32)rows, n, (u32)d, make_modq(q), ds, (u32)round, B, d_claims, d_polys,
@@ -2018,7 +2112,7 @@ extern "C" int salsaa_project(const uint64_t* d_w, uint64_t rows, uint64_t width
   t.want(&nm, 256 * cw / 32);
   t.want(&J, 256 * cw);
   TRY(t.alloc());
-  set_seed_kernel<<<1, 1, 0, st>>>(ds, seed);
+  set_seed_kernel<<<1, 32, 0, st>>>(ds, seed);
   TRY(launch_proj_tables(ds, (u32)round, (u32)cw, pm, nm, J, nullptr, q, st));
   RowSet w = rows_of(d_w, (u32)rows, width, (u32)d);
   return launch_project(w, (u32)rows, width, (u32)d, q, pm, nm, J, ds, d_out, st);

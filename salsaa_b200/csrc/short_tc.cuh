@@ -1,0 +1,31 @@
+// short_tc.cuh — prover steps over short witness rows (byte tiles, see
+// ntt_img.cuh) on the tensor cores.  Each takes a flag word: the rows were
+// short, and the step runs, only while it is zero.
+#pragma once
+#include "ntt_img.cuh"
+
+namespace salsaa {
+
+// Rows of byte tiles: row k at p + k stride (stride bytes a row), of which
+// elements off[k] .. off[k] + width - 1 are used (off a multiple of 64).
+struct C8Rows {
+  const int8_t* p;
+  u64 stride;
+  u32 row[MAX_WROWS];
+  u64 off[MAX_WROWS];
+  u32 rows;
+  u64 width;
+};
+
+// Fold challenges of (seed, round) as coefficients c (rows x d words) and as
+// the negacyclic Toeplitz blocks the fold multiplies by (fold_tz_bytes).
+inline u64 fold_tz_bytes(u32 rows, u32 d) { return (u64)rows * 32 * d; }
+int launch_fold_challenge_tz(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, int8_t* tz,
+                             cudaStream_t st);
+// out (width x d canonical words) = sum_k c_k w_k in R_q, coefficient form;
+// d = 128 or 256, at most 8 rows.  mag_or: OR of the outputs' centred magnitudes.
+bool fold_tc_ok(const C8Rows& w, u32 d);
+int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u64* mag_or, const u32* flag,
+                   cudaStream_t st);
+
+}  // namespace salsaa

@@ -67,3 +67,41 @@ def test_commit_short_values(api, oracle, d, ms, width, rows, lo, hi, odd):
     ctx = api.Context(p, crs_seed=2)
     got = api.to_host(ctx.parallel_dot_series_matrix(api.to_dev(w)))
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("d,folding,rounds,log_wit,bound", [
+    (128, False, 3, 14, 1),         # the relation's ternary witness
+    (128, False, 3, 14, 127),       # the largest that stays short in round 0; digits above 7 bits later
+    (128, False, 3, 14, 128),       # round 0 wide, later rounds on their own sizes
+    (128, False, 2, 13, 40000),     # every round wide, the projected row beyond two limbs
+    (128, True, 1, 12, 1),
+    (128, True, 1, 12, 127),
+    (128, True, 1, 12, 5000),
+    (256, False, 2, 13, 1),
+    (256, False, 2, 13, 200),
+    (256, True, 1, 11, 127),
+])
+def test_prove_short_and_wide(api, oracle, d, folding, rounds, log_wit, bound):
+    """A proof's rounds take the byte steps while the witness is short and the
+    word steps once it is not; the bytes are the oracle's either way."""
+    q = Q[d]
+    p = P.make_params(d, q, 3, 1 << log_wit, rounds, folding)
+    v = np.random.default_rng(bound + d).integers(-bound, bound + 1, size=(p.init_wit_rep, p.wit_len, d))
+    w = np.where(v < 0, q + v, v).astype(np.uint64)
+    rc, want, _ = oracle.prove(p, 5, 6, witness=w)
+    assert rc == 0
+    ctx = api.Context(p, crs_seed=5)
+    got = ctx.prove(6, witness=w)
+    assert np.array_equal(got, want)
+    pr = api.Prover(ctx)
+    pr.set_overlap()
+    pr.set_graph()
+    import torch
+    dw, out = api.to_dev(w), torch.zeros(ctx.proof_bytes, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        pr.enqueue(6, out, dw)
+        pr.sync()
+        assert np.array_equal(out.cpu().numpy(), want)
+    pr.close()
