@@ -701,9 +701,8 @@ int launch_project_umma(RowSet in, u32 rows, u64 nch, u32 d, u64 q, u32 cw, cons
 //   B (N = 128): coefficient positions, the centred witness split into three
 //     signed byte limbs (exact for |w| < 2^23), one MMA chain per limb,
 //   D_l[(r,x)][pos] = sum_i byte_x(s_lo(i)) limb_l(w(i, pos)),
-// and the row sum is sum_{x,l} 2^(8(x+l)) D_l mod q.  A CTA that meets a
-// larger value adds nothing and flags itself; sc_exact_kernel then redoes
-// exactly the flagged CTAs on CUDA cores.  The sums land in the coefficient-
+// and the row sum is sum_{x,l} 2^(8(x+l)) D_l mod q.  A work item that meets a
+// larger value is redone exactly on CUDA cores.  The sums land in the coefficient-
 // form accumulators that launch_commit moves to slot form.
 // ---------------------------------------------------------------------------
 constexpr u32 SU_POS = 128, SU_KS = 128, SU_LIMBS = 3;
@@ -716,8 +715,8 @@ __global__ void sc_img_kernel(const u64* s_lo, u32 Bw, ScRowList tl, uint8_t* im
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 b = (u32)(t % 16), row = (u32)((t / 16) % 128), sl = (u32)((t / 2048) % 8), cc = (u32)(t / 16384);
     uint8_t v = 0;
-    if (row < tl.n * 7) {
-      const u32 r = row / 7, x = row % 7;
+    if (row < tl.n * 8 && row % 8 < 7) {
+      const u32 r = row / 8, x = row % 8;
       v = (uint8_t)(s_lo[(u64)tl.idx[r] * Bw + cc * 128 + sl * 16 + b] >> (8 * x));
     }
     img[t] = v;
@@ -726,18 +725,15 @@ __global__ void sc_img_kernel(const u64* s_lo, u32 Bw, ScRowList tl, uint8_t* im
 
 __global__ void __launch_bounds__(512, 1)
     sc_umma_kernel(RowSet wc, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl,
-                   const uint8_t* __restrict__ img, const u64* s_hi, ModQ M, u64* acc, bool plain, u32* flags) {
+                   const uint8_t* __restrict__ img0, const u64* s_lo, const u64* s_hi, ModQ M, u64* acc, bool plain,
+                   ScGates gates) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[2], done_bar[2];
   __shared__ uint32_t tslot;
   const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // CTA: positions pb, element block hb (one s_hi factor), its part sub of split
-  const u32 pb = blockIdx.x, hb = blockIdx.y / split, sub = blockIdx.y % split, k = blockIdx.z;
+  if (gates.all_closed()) return;
   const u64 q = M.q, half_q = q >> 1;
-  const u32 nsteps = Bw / SU_KS / split, c0 = sub * nsteps;
-  const bool nar = (wc.narrow >> k) & 1;
-  const u64* src0 = row_advance(wc.p[k], nar, ((u64)hb * Bw + (u64)c0 * SU_KS) * d + (u64)pb * SU_POS);
-  img += (u64)c0 * SU_A;
+  const u32 nsteps = Bw / SU_KS / split;
   u32* err = &g_tc_error;
   if (tid == 0) {
     for (int b = 0; b < 2; b++) {
@@ -753,7 +749,20 @@ __global__ void __launch_bounds__(512, 1)
   const u32 tmem = tslot;
   // unsigned bytes (A) x signed bytes (B) -> s32, M = N = 128
   const u32 idesc = umma::idesc_u8(128, SU_POS) | (1u << 10);
-  bool bad = false, ok = true;
+  bool ok = true;
+  // work items: positions pb, element block hb (one s_hi factor), its part sub
+  // of split, witness row k; g0 counts the steps of earlier items
+  const u32 npb = d / SU_POS, items = npb * nhi * split * rows;
+  u32 g0 = 0;
+  for (u32 item = blockIdx.x; item < items; item += gridDim.x) {
+  const u32 pb = item % npb, hs = item / npb % (nhi * split), k = item / (npb * nhi * split);
+  const u32 hb = hs / split, sub = hs % split;
+  if (!gates.open(k)) continue;
+  const u32 c0 = sub * nsteps;
+  const bool nar = (wc.narrow >> k) & 1;
+  const u64* src0 = row_advance(wc.p[k], nar, ((u64)hb * Bw + (u64)c0 * SU_KS) * d + (u64)pb * SU_POS);
+  const uint8_t* img = img0 + (u64)c0 * SU_A;
+  bool bad = false;
   // task of this thread: 16 consecutive elements x 2 neighbouring positions,
   // one 16-byte load per element for word rows (two u64 values) and one
   // 8-byte load for narrow rows (two int32 values, kept in wv[e].x); one
@@ -774,9 +783,9 @@ __global__ void __launch_bounds__(512, 1)
   };
   load(0);
   for (u32 c = 0; c < nsteps; c++) {
-    const u32 st = c & 1;
+    const u32 g = g0 + c, st = g & 1;
     uint8_t* stage = smem + st * SU_STAGE;
-    if (c >= 2) ok &= umma::mbar_wait(&done_bar[st], ((c - 2) >> 1) & 1, err, 1);
+    if (g >= 2) ok &= umma::mbar_wait(&done_bar[st], ((g - 2) >> 1) & 1, err, 1);
     if (tid == 0) {
       umma::mbar_expect_tx(&full_bar[st], SU_A);
       umma::bulk_g2s(stage, img + (u64)c * SU_A, SU_A, &full_bar[st]);
@@ -821,7 +830,7 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     if (tid == 0) {
       umma::fence_after_sync();
-      ok &= umma::mbar_wait(&full_bar[st], (c >> 1) & 1, err, 2);
+      ok &= umma::mbar_wait(&full_bar[st], (g >> 1) & 1, err, 2);
 #pragma unroll
       for (u32 l = 0; l < SU_LIMBS; l++)
 #pragma unroll
@@ -834,17 +843,17 @@ __global__ void __launch_bounds__(512, 1)
       umma::commit(&done_bar[st]);
     }
   }
-  ok &= umma::mbar_wait(&done_bar[(nsteps - 1) & 1], ((nsteps - 1) >> 1) & 1, err, 3);
+  const u32 gl = g0 + nsteps - 1;
+  ok &= umma::mbar_wait(&done_bar[gl & 1], (gl >> 1) & 1, err, 3);
   ok = __syncthreads_and(ok);
   bad = __syncthreads_or(bad);
   umma::fence_after_sync();
-  const u32 cta = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if (bad && tid == 0) flags[cta] = 1;
+  g0 += nsteps;
   if (ok && !bad) {
     // per TMEM lane (row (r, x)), per position: sum_l 2^(8l) D_l, reduced, times 2^(8x)
     u64* Pm = (u64*)smem;  // 128 rows x 128 positions
     const u32 row = (warp & 3) * 32 + lane, quarter = warp >> 2;  // four groups of 32 positions
-    const u32 x = row % 7;
+    const u32 x = row % 8;  // column 7 of a row's eight is zero
     const u64 pw = ((u64)1 << (8 * x)) % q;
     const u64 cpos = ((((u64)1 << 62) / q) + 1) * q;
     for (u32 cb = quarter * 32; cb < quarter * 32 + 32; cb += 16) {
@@ -869,61 +878,60 @@ __global__ void __launch_bounds__(512, 1)
       const u32 r = t / SU_POS, pos = t % SU_POS;
       u64 v = 0;
 #pragma unroll
-      for (u32 x = 0; x < 7; x++) v = salsaa::add_mod(v, Pm[(u64)(r * 7 + x) * 128 + pos], q);
+      for (u32 x = 0; x < 7; x++) v = salsaa::add_mod(v, Pm[(u64)(r * 8 + x) * 128 + pos], q);
       const u32 j = tl.idx[r];
       v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
       atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
     }
   }
+  if (ok && bad) {  // exact CUDA-core sums of this item
+    for (u32 t = tid; t < tl.n * SU_POS; t += 512) {
+      const u32 r = t / SU_POS, pos = t % SU_POS, j = tl.idx[r];
+      u64 v = 0;
+      for (u32 i = 0; i < nsteps * SU_KS; i++)
+        v = salsaa::add_mod(v, mul_mod(M, s_lo[(u64)j * Bw + c0 * SU_KS + i], wres(src0, nar, (u64)i * d + pos, q)), q);
+      v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
+      atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
+    }
+  }
+  // the next item's copies and MMAs reuse the stages and TMEM read above
+  umma::fence_proxy_async();
   umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  if (!ok) break;
+  }
   __syncthreads();
   if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-// Exact CUDA-core sums for the CTAs sc_umma_kernel flagged (same grid).
-__global__ void sc_exact_kernel(RowSet wc, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl,
-                                const u64* s_lo, const u64* s_hi, ModQ M, u64* acc, bool plain, const u32* flags) {
-  const u32 cta = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if (!flags[cta]) return;
-  const u32 pb = blockIdx.x, hb = blockIdx.y / split, sub = blockIdx.y % split, k = blockIdx.z, pos = threadIdx.x;
-  const u32 i0 = sub * (Bw / split), i1 = i0 + Bw / split;
-  const bool nar = (wc.narrow >> k) & 1;
-  const u64* src = row_advance(wc.p[k], nar, ((u64)hb * Bw) * d + (u64)pb * SU_POS + pos);
-  for (u32 r = 0; r < tl.n; r++) {
-    const u32 j = tl.idx[r];
-    u64 v = 0;
-    for (u32 i = i0; i < i1; i++)
-      v = salsaa::add_mod(v, mul_mod(M, s_lo[(u64)j * Bw + i], wres(src, nar, (u64)i * d, M.q)), M.q);
-    v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
-    atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, M.q, plain);
-  }
-}
 
-int launch_sc_umma(const RowSet& wc, u32 rows, u64 width, u32 d, u32 Bw, u32 nhi, const ScRowList& tl,
-                   const u64* s_lo, const u64* s_hi, const ModQ& M, u64* acc, bool plain, uint8_t* img, u32* flags,
-                   u64 flag_cap, cudaStream_t st) {
-  // short witnesses: split each element block over several CTAs (linear sums)
-  // while the grid stays within one wave (one CTA per SM) and the flag scratch
-  const u64 base = (u64)(d / SU_POS) * nhi * rows;
-  u32 split = 1;
-  while (split * 2 <= Bw / SU_KS && base * split * 2 <= 148 && base * split * 2 <= flag_cap) split *= 2;
-  const u64 ctas = base * split;
-  if (ctas > flag_cap) return salsaa_set_error(-2, "sc_umma: flag scratch too small");
-  cudaError_t e = cudaMemsetAsync(flags, 0, ctas * sizeof(u32), st);
-  if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_umma flags");
-  u64 g = ((u64)Bw * 128 + 255) / 256;
+
+int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cudaStream_t st) {
+  const u64 g = ((u64)Bw * 128 + 255) / 256;
   sc_img_kernel<<<(unsigned)(g < 4096 ? g : 4096), 256, 0, st>>>(s_lo, Bw, tl, img);
   salsaa_count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_img launch");
+}
+
+int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_lo,
+                   const u64* s_hi, const ModQ& M, u64* acc, bool plain, const uint8_t* img, const ScGates& gates,
+                   cudaStream_t st) {
+  if (tl.n == 0 || tl.n > SC_UMMA_MAX_ROWS) return salsaa_set_error(-2, "sc_umma: too many rows in one pass");
+  // short witnesses: split each element block over several CTAs (linear sums)
+  // while the items stay within one wave (one CTA per SM)
+  const u64 base = (u64)(d / SU_POS) * nhi * rows;
+  u32 split = 1;
+  while (split * 2 <= Bw / SU_KS && base * split * 2 <= 148) split *= 2;
+  const u64 items = base * split;
   const size_t smem = 2 * (size_t)SU_STAGE;
-  e = cudaFuncSetAttribute(sc_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(sc_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_umma smem attribute");
-  dim3 grid(d / SU_POS, nhi * split, rows);
-  sc_umma_kernel<<<grid, 512, smem, st>>>(wc, rows, d, Bw, nhi, split, tl, img, s_hi, M, acc, plain, flags);
-  salsaa_count_launch();
-  sc_exact_kernel<<<grid, SU_POS, 0, st>>>(wc, rows, d, Bw, nhi, split, tl, s_lo, s_hi, M, acc, plain, flags);
+  sc_umma_kernel<<<(unsigned)(items < 148 ? items : 148), 512, smem, st>>>(wc, rows, d, Bw, nhi, split, tl, img, s_lo,
+                                                                           s_hi, M, acc, plain, gates);
   salsaa_count_launch();
   e = cudaGetLastError();
-  (void)width;
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_umma launch");
 }
 

@@ -11,6 +11,7 @@
 #include <vector>
 #include "kernels.cuh"
 #include "ntt_img.cuh"
+#include "short_tc.cuh"
 
 namespace salsaa {
 
@@ -1708,6 +1709,27 @@ int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ&
   return check_launch("fold");
 }
 
+__global__ void fold_slots_kernel(const u64* x, const u64* c, u32 K, u32 n, ModQ M, const u64* zeta, u64* out) {
+  const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  u64 ae = 0, ao = 0;
+#pragma unroll 4
+  for (u32 k = 0; k < K; k++) {
+    u64 e, o;
+    slot_mul(M, c[k * 2 * n + s], c[k * 2 * n + n + s], x[k * 2 * n + s], x[k * 2 * n + n + s], zeta[s], e, o);
+    ae = add_mod(ae, e, M.q);
+    ao = add_mod(ao, o, M.q);
+  }
+  out[s] = ae;
+  out[n + s] = ao;
+}
+
+int launch_fold_slots(const u64* x, const u64* c_slot, u32 K, const NttDev& T, const ModQ& M, u64* out,
+                      cudaStream_t st) {
+  fold_slots_kernel<<<(T.n + 63) / 64, 64, 0, st>>>(x, c_slot, K, T.n, M, T.zeta, out);
+  return check_launch("fold_slots");
+}
+
 // ---------------------------------------------------------------------------
 // Structured commitment <statement row, witness row> (parallel_dot_series_matrix,
 // src/arithmetic.rs:459-505), all rows in one pass over each witness chunk.
@@ -2385,29 +2407,30 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
       if (a.sc_types_host[j] == ROW_TENSOR) tl.idx[tl.n++] = (unsigned char)j;
       else ol.idx[ol.n++] = (unsigned char)j;
     }
-    // TENSOR rows: one tensor-core pass over the coefficient-form witness when
-    // the shapes fit, else CUDA cores.  Every scalar row weighs element i by
-    // s_hi[i / Bw] s_lo[i % Bw], so when that pass runs anyway the periodic /
-    // all-ones rows ride in it if they fit, and no column sums are needed.
-    const bool tc_ok = a.coef_sc && a.sc_img && a.sc_flags && M.q < (1ULL << 56) && d % 128 == 0 &&
-                       Bw % 128 == 0 && tl.n > 0 && tl.n <= SC_UMMA_MAX_ROWS && rowset_aligned(wsrc, a.rows, 16, 8);
+    // one tensor-core pass over the coefficient-form witness per 16 rows when
+    // the shapes fit (every scalar row weighs element i by s_hi[i / Bw]
+    // s_lo[i % Bw]), else CUDA cores, the periodic / all-ones rows over column
+    // sums; rows of byte tiles take the byte pass, the others this one
+    const bool tc_ok = a.coef_sc && a.sc_img && M.q < (1ULL << 56) && d % 128 == 0 && Bw % 128 == 0 &&
+                       rowset_aligned(wsrc, a.rows, 16, 8) && (tl.n > 0 || a.sc8);
     bool periodic_done = false;
     if (tc_ok) {
-      ScRowList gl = tl;
-      if (tl.n + ol.n <= SC_UMMA_MAX_ROWS) {
-        for (u32 i = 0; i < ol.n; i++) gl.idx[gl.n++] = ol.idx[i];
-        periodic_done = true;
-      }
-      rc = launch_sc_umma(wsrc, a.rows, a.width, d, Bw, nhi, gl, a.sc_lo, a.sc_hi, M, acc_sc, plain, a.sc_img,
-                          a.sc_flags, a.sc_flag_cap, ss);
-      if (rc) return rc;
-      if (!periodic_done && ol.n <= SC_UMMA_MAX_ROWS) {
-        // more rows than one pass holds: the periodic / all-ones rows in a second pass
-        rc = launch_sc_umma(wsrc, a.rows, a.width, d, Bw, nhi, ol, a.sc_lo, a.sc_hi, M, acc_sc, plain, a.sc_img,
-                            a.sc_flags, a.sc_flag_cap, ss);
+      for (u32 j0 = 0; j0 < a.nsc; j0 += SC_UMMA_MAX_ROWS) {
+        ScRowList gl{};
+        for (u32 j = j0; j < a.nsc && j < j0 + SC_UMMA_MAX_ROWS; j++) gl.idx[gl.n++] = (unsigned char)j;
+        rc = launch_sc_img(a.sc_lo, Bw, gl, a.sc_img, ss);
         if (rc) return rc;
-        periodic_done = true;
+        ScGates gates{};
+        gates.rows = a.rows;
+        if (a.sc8) {
+          for (u32 k = 0; k < a.rows; k++) gates.gate[k] = a.sc8->wide[k];
+          rc = launch_sc_tc(*a.sc8, a.rows, d, Bw, nhi, gl, a.sc_hi, M, acc_sc, a.sc_img, ss);
+          if (rc) return rc;
+        }
+        rc = launch_sc_umma(wsrc, a.rows, d, Bw, nhi, gl, a.sc_lo, a.sc_hi, M, acc_sc, plain, a.sc_img, gates, ss);
+        if (rc) return rc;
       }
+      periodic_done = true;
     } else {
       launch_sc_pass(a, wsrc, a.width, tl, true, d, Bw, nhi, (u32)CH, M, plain, acc_sc, ss);
       rc = check_launch("sc_commit (tensor rows)");

@@ -101,10 +101,23 @@ inline u64 ck_tk8_bytes(u32 nck, u32 n, u32 bt) { return (u64)bt * n * ck_tk8_nk
 int launch_ck_tk8(const u64* tlo, u32 nck, u32 n, u32 bt, bool packed, uint8_t* tk8, cudaStream_t st);
 // TENSOR rows on tcgen05 over the coefficient-form witness (see ck_umma.cu).
 constexpr u64 SC_IMG_BYTES = (u64)CK_BLOCK * 128;
-constexpr u32 SC_UMMA_MAX_ROWS = 18;
-int launch_sc_umma(const RowSet& wc, u32 rows, u64 width, u32 d, u32 Bw, u32 nhi, const ScRowList& tl,
-                   const u64* s_lo, const u64* s_hi, const ModQ& M, u64* acc, bool plain, uint8_t* img, u32* flags,
-                   u64 flag_cap, cudaStream_t st);
+constexpr u32 SC_UMMA_MAX_ROWS = 16;
+// Which witness rows a pass takes: row k runs if gate[k] is null or *gate[k] != 0.
+struct ScGates {
+  const u32* gate[MAX_WROWS];
+  u32 rows;
+  __device__ bool open(u32 k) const { return !gate[k] || *gate[k] != 0; }
+  __device__ bool all_closed() const {
+    for (u32 k = 0; k < rows; k++)
+      if (open(k)) return false;
+    return true;
+  }
+};
+// img: the byte image of the rows' scalars (launch_sc_img), 8 operand rows each.
+int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cudaStream_t st);
+int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_lo,
+                   const u64* s_hi, const ModQ& M, u64* acc, bool plain, const uint8_t* img, const ScGates& gates,
+                   cudaStream_t st);
 // First sumcheck pass (rounds 0..3 of both repetitions) on tcgen05 through the
 // Gram matrices of 16-element groups (see ck_umma.cu): launch_nc_gram writes
 // the folded vectors and the Gram matrices, or raises the flag word after them
@@ -182,6 +195,10 @@ int launch_fold_challenge(const DevState* ds, u32 round, u32 rows, u32 d, u64 q,
 int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ& M, const u64* c_slot, u64* pre,
                 u64* out_slot, cudaStream_t st, const u32* gate = nullptr);
 
+// out (one ring element, slot form) = sum_k c_slot[k] x[k] over K slot-form elements.
+int launch_fold_slots(const u64* x, const u64* c_slot, u32 K, const NttDev& T, const ModQ& M, u64* out,
+                      cudaStream_t st);
+
 // <statement rows, witness rows> in slot form.  acc: (nck + nsc) x rows x d
 // scratch; out_slot: results in statement order given by `order`.
 struct CkImage;
@@ -201,8 +218,7 @@ struct CommitArgs {
   const ScalarRowDesc* sc_desc_dev;  // nsc descriptors in device memory
   const int* sc_types_host;          // their types, on the host (required when nsc > 0)
   uint8_t* sc_img;   // scratch for the tcgen05 TENSOR-row pass (SC_IMG_BYTES), or null
-  u32* sc_flags;     // scratch: one word per CTA of that pass
-  u64 sc_flag_cap;   // words of sc_flags
+  const struct Sc8Rows* sc8;  // the rows wc as byte tiles where they are short (short_tc.cuh), or null
   cudaStream_t st2;  // optional: statement rows on this stream beside the key rows
   cudaEvent_t ev_fork, ev_join;
   const u64* const* sc_base_dev;     // nsc ring bases (slot form) or null (= 1)

@@ -454,8 +454,6 @@ struct salsaa_prover {
   int8_t* Jm = nullptr;  // projection challenge as int8, 256 x chunk width
   int8_t* Jc = nullptr;  // the same in the tcgen05 operand layout
   uint8_t* sc_img = nullptr;  // tcgen05 TENSOR-row pass: scalar byte image
-  u32* sc_flags = nullptr;    // and its per-CTA fallback flags
-  u64 sc_flag_words = 0;
   u64 *c_coef = nullptr, *c_slot = nullptr, *fold_pre = nullptr;
   ScalarRowDesc* sc_desc = nullptr;
   std::vector<int> sc_types;  // host copy of the scalar rows' types (launch tiling)
@@ -516,7 +514,7 @@ extern "C" uint64_t salsaa_workspace_bytes(const salsaa_params* p) {
   words += (u64)(S.max_rows + 1) * (L < CK_BLOCK ? L : CK_BLOCK) * d;
   words += 2 * 256ULL * CK_BLOCK / 8;          // projection J and its tensor-core image (bytes)
   words += (u64)MAX_WROWS * (d / 2) * 6;       // fold constants
-  words += SC_IMG_BYTES / 8 + (d / 128 + 1) * (L / CK_BLOCK + 1) * (S.max_rows + 2) / 2;  // scalar-row pass
+  words += SC_IMG_BYTES / 8;                   // scalar-row pass
   return words * 8 + (S.proof_words * 8);
 }
 
@@ -557,8 +555,7 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (rc = m.alloc(&pr->Fs, S.max_fp_width * d, "Fs")) || (rc = m.alloc(&pr->Pc, S.max_fp_width * d, "Pc")) ||
       (!S.use_img && (rc = m.alloc(&pr->Ps, S.max_fp_width * d, "Ps"))) ||
       (S.use_img && (rc = m.alloc(&pr->img, S.max_img, "key-row image"))) ||
-      (S.use_short && (rc = m.alloc(&pr->c8, S.max_d_rows_width * d, "byte tiles"))) ||
-      (S.use_short && (rc = m.alloc(&pr->p8, 2 * S.max_fp_width * d, "projected row's limbs"))) ||
+      (S.use_short && (rc = m.alloc(&pr->c8, (S.max_d_rows_width + 2 * S.max_fp_width) * d, "byte tiles"))) ||
       (S.use_short && (rc = m.alloc(&pr->tz, fold_tz_bytes(8, (u32)d), "fold challenge blocks"))) ||
       (rc = m.alloc(&pr->sc.a, S.max_nc_rows_width * d / 8 + 1, "sumcheck a")) ||
       (rc = m.alloc(&pr->sc.b, S.max_nc_rows_width * d / 128 + 1, "sumcheck b")) ||
@@ -572,8 +569,6 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (rc = m.alloc(&pr->Jm, 256ULL * CK_BLOCK, "projection J")) ||
       (rc = m.alloc(&pr->Jc, 256ULL * CK_BLOCK, "projection J (tensor-core layout)")) ||
       (rc = m.alloc(&pr->sc_img, SC_IMG_BYTES, "scalar-row byte image")) ||
-      (rc = m.alloc(&pr->sc_flags, pr->sc_flag_words = (u64)(d / 128 + 1) * (L / CK_BLOCK + 1) * (S.max_rows + 2),
-                    "scalar-row flags")) ||
       (rc = m.alloc(&pr->c_coef, (u64)MAX_WROWS * d, "fold c")) ||
       (rc = m.alloc(&pr->c_slot, (u64)MAX_WROWS * d, "fold c slot")) ||
       (rc = m.alloc(&pr->fold_pre, (u64)MAX_WROWS * (d / 2) * 6, "fold constants")) ||
@@ -586,6 +581,7 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (rc = m.alloc(&pr->cout, stmt * (MAX_WROWS + 1) * d, "commit out")) ||
       (rc = m.alloc(&pr->cout2, stmt * (MAX_WROWS + 1) * d, "commit out (coefficients)")))
     return fail(rc);
+  if (S.use_short) pr->p8 = pr->c8 + S.max_d_rows_width * d;
   // Scalar statement rows of the whole proof, in push order: per round
   // TENSOR(rep 0), TENSOR(rep 1), PERIODIC (witness_lhs), ONES (projected_lhs).
   std::vector<ScalarRowDesc> desc;
@@ -687,8 +683,9 @@ __global__ void set_seed_kernel(DevState* ds, u64 seed) {
 // -> slot-form ring elements in pr->cout, row-major (statement, witness).
 // wc: the same witness rows in coefficient form (scalar rows are summed there), or null.
 // img: their byte image for the key rows (ws is then not read), or null.
+// sc8: the rows as byte tiles for the scalar rows, or null.
 static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* wc, u32 rows, u64 width, u32 nck,
-                            u32 sc_first, u32 nsc, const CkImage* img = nullptr) {
+                            u32 sc_first, u32 nsc, const CkImage* img = nullptr, const Sc8Rows* sc8 = nullptr) {
   salsaa_ctx* c = pr->ctx;
   if ((u64)sc_first + nsc > c->S.nsc_total || nck > c->P.module_size)
     return salsaa_set_error(-9, "commit: statement row range outside the proof's rows");
@@ -717,11 +714,8 @@ static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* w
   a.tk8 = c->tk8;
   a.colsum = pr->colsum;
   a.colsum_rows = c->S.max_rows + 1;  // the merged split/projection pass has 2K + 1 rows
-  if ((u64)(c->d / 128) * (width / CK_BLOCK > 0 ? width / CK_BLOCK : 1) * rows <= pr->sc_flag_words) {
-    a.sc_img = pr->sc_img;
-    a.sc_flags = pr->sc_flags;
-    a.sc_flag_cap = pr->sc_flag_words;
-  }
+  a.sc_img = pr->sc_img;
+  a.sc8 = sc8;
   if (pr->overlap) {
     a.st2 = pr->st2;
     a.ev_fork = pr->ev_fork;
@@ -733,8 +727,9 @@ static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* w
 
 // Same, in coefficient form at proof_out.
 static int commit_rows(salsaa_prover* pr, const RowSet& ws, const RowSet* wc, u32 rows, u64 width, u32 nck,
-                       u32 sc_first, u32 nsc, u64* proof_out, const CkImage* img = nullptr) {
-  TRY(commit_rows_slot(pr, ws, wc, rows, width, nck, sc_first, nsc, img));
+                       u32 sc_first, u32 nsc, u64* proof_out, const CkImage* img = nullptr,
+                       const Sc8Rows* sc8 = nullptr) {
+  TRY(commit_rows_slot(pr, ws, wc, rows, width, nck, sc_first, nsc, img, sc8));
   return ntt_launch(pr->cout, proof_out, (u64)(nck + nsc) * rows, *pr->ctx->T, true, true, pr->st);
 }
 
@@ -761,6 +756,29 @@ static C8Rows c8_rows(const int8_t* c8, u32 K, u64 width, u32 d, bool split) {
   for (u32 k = 0; k < K; k++) {
     r.row[k] = split ? k % (K / 2) : k;
     r.off[k] = split && k >= K / 2 ? width : 0;
+  }
+  return r;
+}
+
+// The K rows of the witness (short while !*wide) and, with wide_p, the
+// projected row as witness row K (two limbs, short while !*wide_p).
+static Sc8Rows sc8_rows(const salsaa_prover* pr, u32 K, u64 width, u32 d, bool split, const u32* wide,
+                        const u32* wide_p) {
+  Sc8Rows r{};
+  r.w = c8_rows(pr->c8, K, width, d, split);
+  for (u32 k = 0; k < K; k++) {
+    r.dst[k] = k;
+    r.wide[k] = wide;
+  }
+  if (wide_p) {
+    for (u32 l = 0; l < 2; l++) {  // p8 lies behind c8
+      r.w.row[K + l] = 0;
+      r.w.off[K + l] = (u64)(pr->p8 - pr->c8) / d + l * width;
+      r.dst[K + l] = K;
+      r.shift[K + l] = 8 * l;
+    }
+    r.w.rows = K + 2;
+    r.wide[K] = wide_p;
   }
   return r;
 }
@@ -976,7 +994,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       if (P.folding) image(1, width2);
       const RowSet prow = rows_of(pr->Pc, 1, width2, d);
       const u32 pk0 = P.folding ? 0 : K2;
-      if (sh) TRY(short_rows(prow, 1, width2, pk0, false, 2, nullptr, &pr->ds->wide_p[rd], nullptr, mag, ps));
+      if (sh) TRY(short_rows(prow, 1, width2, pk0, false, 2, pr->p8, &pr->ds->wide_p[rd], nullptr, mag, ps));
       else TRY(image_rows(prow, 1, width2, pk0, false, nullptr, mag, ps));
     } else {
       TRY(ntt_launch(pr->Pc, pr->Ps, width2, T, true, false, ps, mag));
@@ -1021,7 +1039,8 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       RowSet both = Ws, bothc = Wc;
       both.p[K] = pr->Ps;
       bothc.p[K] = pr->Pc;
-      TRY(commit_rows_slot(pr, both, &bothc, K + 1, width, ms, 0, nsc + 2, imp));
+      const Sc8Rows sr = sc8_rows(pr, K, width, d, true, &pr->ds->wide[rd], &pr->ds->wide_p[rd]);
+      TRY(commit_rows_slot(pr, both, &bothc, K + 1, width, ms, 0, nsc + 2, imp, sh ? &sr : nullptr));
       TRY(ntt_launch(pr->cout, pr->cout2, (u64)(S + 2) * (K + 1), T, true, true, st));
       const size_t row_bytes = (size_t)(K + 1) * d * sizeof(u64);
       e = cudaMemcpy2DAsync(proof + cur, (size_t)K * d * sizeof(u64), pr->cout2, row_bytes,
@@ -1054,24 +1073,36 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
         pending = false;
       }
     } else {
-      TRY(commit_rows(pr, Pr, &Prc, 1, width, ms, 0, nsc, proof + cur, imp));
+      // the projected commitment; its two further rows, witness_lhs and
+      // projected_lhs, give the cross term l1 and projection_rhs
+      const Sc8Rows sr = sc8_rows(pr, 0, width, d, false, nullptr, &pr->ds->wide_p[rd]);
+      TRY(commit_rows_slot(pr, Pr, &Prc, 1, width, ms, 0, nsc + 2, imp, sh ? &sr : nullptr));
+      TRY(ntt_launch(pr->cout, pr->cout2, S + 2, T, true, true, st));
+      e = cudaMemcpyAsync(proof + cur, pr->cout2, (size_t)S * d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: projected commitment");
       cur += (u64)S * d;
     }
-    // batch_projections (src/subroutines/project.rs:131-203): witness_rhs, projection_rhs
-    const u64* l1_src = nullptr;  // <witness_lhs, projected> when the merged pass made it
+    // batch_projections (src/subroutines/project.rs:131-203): witness_rhs,
+    // projection_rhs; ones: projected_lhs x the witness rows, slot form (for l0)
+    const u64 *l1_src, *prhs_src, *ones;
     if (!P.folding) {
       const u64* wl = pr->cout2 + (u64)S * (K + 1) * d;  // witness_lhs x [split witness, P]
       const u64* pl = wl + (u64)(K + 1) * d;             // projected_lhs x [split witness, P]
       e = cudaMemcpyAsync(proof + cur, wl, (size_t)K * d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(proof + cur + (u64)K * d, pl + (u64)K * d, (size_t)d * sizeof(u64),
-                            cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: batch projections");
       l1_src = wl + (u64)K * d;
+      prhs_src = pl + (u64)K * d;
+      ones = pr->cout + (u64)(S + 1) * (K + 1) * d;
     } else {
-      TRY(commit_rows(pr, Ws, &Wc, K, width, 0, nsc, 1, proof + cur));
-      TRY(commit_rows(pr, Pr, &Prc, 1, width, 0, nsc + 1, 1, proof + cur + (u64)K * d));
+      l1_src = pr->cout2 + (u64)S * d;
+      prhs_src = l1_src + d;
+      const Sc8Rows sr = sc8_rows(pr, K, width, d, false, &pr->ds->wide[rd], nullptr);
+      TRY(commit_rows_slot(pr, Ws, &Wc, K, width, 0, nsc, 2, nullptr, sh ? &sr : nullptr));
+      TRY(ntt_launch(pr->cout, proof + cur, K, T, true, true, st));
+      ones = pr->cout + (u64)K * d;
     }
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(proof + cur + (u64)K * d, prhs_src, (size_t)d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: batch projections");
     cur += (u64)K * d + d;
     nsc += 1;  // witness_lhs joins the statement
     // fold (src/subroutines/fold.rs:22-27)
@@ -1091,16 +1122,13 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       TRY(ntt_launch(pr->Fs, pr->Fc, width, T, true, true, st, mag));
     }
     mag_ready = mag != nullptr;
-    // send_cross_terms_before_join (src/subroutines/project.rs:229-245)
-    RowSet Fr = rows_of(pr->Fs, 1, width, d), Frc = rows_of(pr->Fc, 1, width, d);
-    TRY(commit_rows(pr, Fr, &Frc, 1, width, 0, nsc, 1, proof + cur));  // l0 = <projected_lhs, folded>
+    // send_cross_terms_before_join (src/subroutines/project.rs:229-245): the
+    // fold is linear, so l0 = <projected_lhs, folded> = sum_k c_k <projected_lhs, w_k>
+    TRY(launch_fold_slots(ones, pr->c_slot, K, T, M, pr->acc, st));
+    TRY(ntt_launch(pr->acc, proof + cur, 1, T, true, true, st));
     cur += d;
-    if (l1_src) {  // l1 = <witness_lhs, projected>
-      e = cudaMemcpyAsync(proof + cur, l1_src, (size_t)d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: cross term");
-    } else {
-      TRY(commit_rows(pr, Pr, &Prc, 1, width, 0, nsc - 1, 1, proof + cur));
-    }
+    e = cudaMemcpyAsync(proof + cur, l1_src, (size_t)d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: cross term");
     cur += d;
     nsc += 1;  // projected_lhs joins the statement
     // join: witness = [folded, projected]
@@ -1128,7 +1156,8 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       K *= 2;
       Ws = rows_of(pr->Ds, K, width, d);
       const RowSet Dcr = narrow ? rows_of_narrow(pr->Dc, K, width, d) : rows_of(pr->Dc, K, width, d);
-      TRY(commit_rows(pr, Ws, &Dcr, K, width, ms, 0, nsc, proof + cur, imp));
+      const Sc8Rows sr = sc8_rows(pr, K, width, d, false, &pr->ds->wide[rd + 1], nullptr);
+      TRY(commit_rows(pr, Ws, &Dcr, K, width, ms, 0, nsc, proof + cur, imp, sh ? &sr : nullptr));
       cur += (u64)(ms + nsc) * K * d;
       break;
     }

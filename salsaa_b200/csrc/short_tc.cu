@@ -1,4 +1,4 @@
-// short_tc.cu — fold over short witness rows on the tensor cores.
+// short_tc.cu — fold and statement rows over short witness rows on the tensor cores.
 #include <cuda_runtime.h>
 
 #include "short_tc.cuh"
@@ -196,6 +196,169 @@ __global__ void fold_chal_tz_kernel(const DevState* ds, u32 round, u32 rows, u32
   tz[t] = (int8_t)v;
 }
 
+// ---------------------------------------------------------------------------
+// Statement rows (the scalar rows of parallel_dot_series_matrix,
+// src/arithmetic.rs:459-505) over byte rows.  Per (byte row, 128 positions,
+// element block of one s_hi factor or a part of it): D[position][8 j + x] =
+// sum_i w(i, position) byte_x(s_lo_j(i)), M = 128 positions (the byte tile
+// MN-major), N = 8 columns a row, K = elements; the row's sum is
+// s_hi sum_x 2^(8 x) D_x.  A CTA takes a run of items in element order and
+// keeps the residues in registers (lane = position, 8 rows a warp) until the
+// (byte row, positions) changes, then adds them to the accumulators.  Where
+// sc_umma_kernel turns every value into three byte limbs, here both operands
+// are bulk copies.  Bound by the copies' latency and L2 traffic: 16 KB per 64
+// elements with 16 rows.  Together with the products that the proof no longer
+// recomputes (<projected_lhs, folded> is a combination of <projected_lhs, w_k>):
+// 1222 -> 374 us of an 8-round proof over 2^19 elements, d = 128.
+// ---------------------------------------------------------------------------
+constexpr u32 ST_EPI = 256, ST_THREADS = ST_EPI + 64, ST_STAGES = 8;
+constexpr u32 ST_A = 64 * 128, ST_STAGE = ST_A + 64 * 128;
+
+__global__ void __launch_bounds__(ST_THREADS, 1)
+    sc_tc_kernel(Sc8Rows w, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl, const u64* s_hi, ModQ M,
+                 u64* acc, const uint8_t* __restrict__ img, u32* err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t full_bar[ST_STAGES], empty_bar[ST_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tslot;
+  const u32 tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const u32 npb = d / 128, per = nhi * split, items = w.w.rows * npb * per;
+  const u32 i0 = (u32)((u64)blockIdx.x * items / gridDim.x), i1 = (u32)((u64)(blockIdx.x + 1) * items / gridDim.x);
+  const u32 steps = Bw / 64 / split, np = (tl.n * 8 + 15) / 16 * 16;  // N, whole 16-column groups
+  auto open = [&](u32 item) { return *w.wide[w.dst[item / (npb * per)]] == 0; };
+  if (tid == 0) {
+    for (u32 i = 0; i < ST_STAGES; i++) {
+      umma::mbar_init(&full_bar[i], 1);
+      umma::mbar_init(&empty_bar[i], 1);
+    }
+    for (u32 i = 0; i < 2; i++) {
+      umma::mbar_init(&acc_full[i], 1);
+      umma::mbar_init(&acc_empty[i], ST_EPI);
+    }
+    umma::mbar_fence_init();
+  }
+  if (warp == 0) umma::tmem_alloc(&tslot, 256);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const u32 tmem = tslot;
+
+  if (warp == ST_EPI / 32) {
+    bool ok = true;
+    u32 it = 0, st = 0, par = 1;
+    for (u32 item = i0; ok && item < i1; item++) {
+      if (!open(item)) continue;
+      const u32 hs = item % per, rp = item / per, pb = rp % npb, r = rp / npb;
+      const u32 e0 = hs / split * Bw + hs % split * steps * 64, l0 = hs % split * steps * 64;
+      const int8_t* src = w.w.p + w.w.row[r] * w.w.stride + (w.w.off[r] + e0) * d + pb * ST_A;
+      for (u32 c = 0; c < steps; c++, it++) {
+        if (it >= ST_STAGES && !(ok = umma::mbar_wait(&empty_bar[st], par, err, 51))) break;
+        if (umma::elect_one()) {
+          uint8_t* stage = smem + st * ST_STAGE;
+          umma::mbar_expect_tx(&full_bar[st], ST_A + 4 * np * 16);
+          umma::bulk_g2s(stage, src + (u64)c * 64 * d, ST_A, &full_bar[st]);
+          const uint8_t* im = img + (u64)(l0 / 16 + 4 * c) * 2048;
+          for (u32 j = 0; j < 4; j++)
+            umma::bulk_g2s(stage + ST_A + j * 2048, im + j * 2048, np * 16, &full_bar[st]);
+        }
+        __syncwarp();
+        if (++st == ST_STAGES) {
+          st = 0;
+          par ^= 1;
+        }
+      }
+    }
+    for (u32 c = it >= ST_STAGES ? it - ST_STAGES : 0; c < it; c++)
+      umma::mbar_wait(&full_bar[c % ST_STAGES], (c / ST_STAGES) & 1, err, 52);
+  } else if (warp == ST_EPI / 32 + 1) {
+    // A: s8, MN-major (position slices 1024 apart, 8-element blocks 128);
+    // B: u8, K-major
+    const u32 idesc = (2u << 4) | (1u << 7) | (1u << 15) | ((np >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t ad0 = umma::desc_kmajor(umma::smem_u32(smem), 128, 1024);
+    const uint64_t bd0 = umma::desc_kmajor(umma::smem_u32(smem + ST_A), 2048, 128);
+    bool ok = true;
+    u32 it = 0, ui = 0, st = 0, par = 0;
+    for (u32 item = i0; ok && item < i1; item++) {
+      if (!open(item)) continue;
+      const u32 nb = ui & 1;
+      if (ui >= 2 && !(ok = umma::mbar_wait(&acc_empty[nb], ((ui >> 1) - 1) & 1, err, 53))) break;
+      umma::fence_after_sync();
+      for (u32 c = 0; c < steps; c++, it++) {
+        if (!(ok = umma::mbar_wait(&full_bar[st], par, err, 54))) break;
+        umma::fence_after_sync();
+        const uint64_t so = (uint64_t)st * (ST_STAGE >> 4);
+        if (umma::elect_one()) {
+#pragma unroll
+          for (u32 ks = 0; ks < 2; ks++)
+            umma::mma_i8_u(tmem + nb * 128, ad0 + so + ks * 32, bd0 + so + ks * 256, idesc, (c > 0 || ks > 0) ? 1u : 0u);
+          umma::commit(&empty_bar[st]);
+          if (c + 1 == steps) umma::commit(&acc_full[nb]);
+        }
+        __syncwarp();
+        if (++st == ST_STAGES) {
+          st = 0;
+          par ^= 1;
+        }
+      }
+      ui++;
+    }
+    for (u32 c = it >= ST_STAGES ? it - ST_STAGES : 0; c < it; c++)
+      umma::mbar_wait(&empty_bar[c % ST_STAGES], (c / ST_STAGES) & 1, err, 55);
+  } else {
+    const u32 m = (warp & 3) * 32 + lane, ch = warp >> 2;  // position; rows 8 ch .. + 7
+    const u64 q = M.q, p32 = ((u64)1 << 32) % q;
+    u64 sum[8];
+#pragma unroll
+    for (u32 j = 0; j < 8; j++) sum[j] = 0;
+    u32 ui = 0;
+    for (u32 item = i0; item < i1; item++) {
+      const u32 hs = item % per, rp = item / per;
+      if (open(item)) {
+        const u32 nb = ui & 1;
+        const bool ok = umma::mbar_wait(&acc_full[nb], (ui >> 1) & 1, err, 56);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        umma::fence_after_sync();
+        const u32 tb = tmem + (((warp & 3) * 32) << 16) + nb * 128 + ch * 64;
+        uint32_t v[4][16];
+#pragma unroll
+        for (u32 g = 0; g < 4; g++)
+          if (8 * ch + 2 * g < tl.n) umma::tmem_ld16(tb + g * 16, v[g]);
+        umma::tmem_wait_ld();
+        umma::fence_before_sync();
+        umma::mbar_arrive(&acc_empty[nb]);
+        ui++;
+#pragma unroll
+        for (u32 j = 0; j < 8; j++) {
+          if (8 * ch + j < tl.n) {
+            const uint32_t* D = &v[j / 2][8 * (j & 1)];
+            // |D_x| <= 2048 x 255 x 128 < 2^26
+            const long long lo = (long long)(int)D[0] + ((long long)(int)D[1] << 8) + ((long long)(int)D[2] << 16) +
+                                 ((long long)(int)D[3] << 24);
+            const long long hi = (long long)(int)D[4] + ((long long)(int)D[5] << 8) + ((long long)(int)D[6] << 16);
+            // |hi| < 2^43 < q; |lo| < 2^51 <= 16 q
+            u64 x = mul_mod(M, hi < 0 ? (u64)(hi + (long long)q) : (u64)hi, p32);
+            x = reduce64(M, x + (u64)(lo + (long long)(16 * q)));
+            x = mul_mod(M, x, __ldg(s_hi + (u64)tl.idx[8 * ch + j] * nhi + hs / split));
+            sum[j] = add_mod(sum[j], x, q);
+          }
+        }
+      }
+      if (item + 1 == i1 || rp != (item + 1) / per) {  // the run of this byte row and these positions ends
+        const u32 pb = rp % npb, r = rp / npb, k = w.dst[r];
+        const u64 sc = ((u64)1 << w.shift[r]) % q;
+#pragma unroll
+        for (u32 j = 0; j < 8; j++) {
+          if (8 * ch + j < tl.n && sum[j])
+            atomic_add_mod(acc + ((u64)tl.idx[8 * ch + j] * rows + k) * d + pb * 128 + m, mul_mod(M, sum[j], sc), q, true);
+          sum[j] = 0;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  umma::fence_after_sync();
+  if (warp == 0) umma::tmem_dealloc(tmem, 256);
+}
+
 }  // namespace
 
 int launch_fold_challenge_tz(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, int8_t* tz,
@@ -225,6 +388,28 @@ int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u6
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_tc launch");
+}
+
+int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_hi,
+                 const ModQ& M, u64* acc, const uint8_t* img, cudaStream_t st) {
+  // q above 2^47 for the bounds, below 2^50 so that plain adds of at most one
+  // residue per CTA and byte row cannot overflow
+  if ((d != 128 && d != 256) || Bw % 64 || tl.n == 0 || tl.n > SC_UMMA_MAX_ROWS || M.q >= (1ULL << 50) ||
+      M.q < (1ULL << 47) || w.w.rows == 0 || w.w.rows > (u32)MAX_WROWS || (u64)Bw * nhi > w.w.width)
+    return salsaa_set_error(-2, "sc_tc: rows outside the byte-tile path");
+  // few items: split each element block over several CTAs
+  const u64 base = (u64)w.w.rows * (d / 128) * nhi;
+  u32 split = 1;
+  while (split * 4 <= Bw / 64 && base * split < 148) split *= 2;
+  const u64 items = base * split;
+  const size_t smem = (size_t)ST_STAGES * ST_STAGE;
+  cudaError_t e = cudaFuncSetAttribute(sc_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tc smem attribute");
+  sc_tc_kernel<<<(unsigned)(items < 148 ? items : 148), ST_THREADS, smem, st>>>(w, rows, d, Bw, nhi, split, tl, s_hi, M,
+                                                                                acc, img, tc_error_word());
+  salsaa_count_launch();
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_tc launch");
 }
 
 }  // namespace salsaa

@@ -28,4 +28,15 @@ bool fold_tc_ok(const C8Rows& w, u32 d);
 int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u64* mag_or, const u32* flag,
                    cudaStream_t st);
 
+// Statement rows of launch_commit (kernels.cuh) over byte rows: byte row r
+// adds 2^shift[r] times its sums to witness row dst[r], unless *wide[dst[r]]
+// is nonzero (then launch_sc_umma takes that row).
+struct Sc8Rows {
+  C8Rows w;
+  u32 dst[MAX_WROWS], shift[MAX_WROWS];
+  const u32* wide[MAX_WROWS];  // per witness row
+};
+int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_hi,
+                 const ModQ& M, u64* acc, const uint8_t* img, cudaStream_t st);
+
 }  // namespace salsaa

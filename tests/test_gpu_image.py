@@ -73,6 +73,7 @@ def test_commit_short_values(api, oracle, d, ms, width, rows, lo, hi, odd):
     (128, False, 3, 14, 1),         # the relation's ternary witness
     (128, False, 3, 14, 127),       # the largest that stays short in round 0; digits above 7 bits later
     (128, False, 3, 14, 128),       # round 0 wide, later rounds on their own sizes
+    (128, False, 5, 16, 1),         # more statement rows than one tensor-core pass holds
     (128, False, 2, 13, 40000),     # every round wide, the projected row beyond two limbs
     (128, True, 1, 12, 1),
     (128, True, 1, 12, 127),
