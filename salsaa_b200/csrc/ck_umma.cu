@@ -528,8 +528,8 @@ int launch_ck_umma(const CommitArgs& a, u32 n, u32 Bw, u32 G, const ModQ& M, con
 // Projection on tcgen05 (project, src/subroutines/project.rs:50-103): per
 // chunk of cw witness elements, out[256 x d] = J (256 x cw, entries -1/0/1) x
 // W (cw x d, centre-lifted, int8).  CTA = (chunk, block of 128 coefficient
-// positions); per 128-element step thread 0 bulk-copies both 128-row halves
-// of J from their canonical image (Jc, see launch_proj_tables) and issues
+// positions); per 64-element step thread 0 bulk-copies the 256 rows of
+// J from their canonical image (Jc, see launch_proj_tables) and issues
 // 2 x 4 MMAs (kind::i8, signed x signed, M = 128 J rows, N = 128 positions,
 // K = 32) into two TMEM accumulators; the threads convert the witness step to
 // int8 in the canonical layout.  A value outside [-128, 127] sets the flag and
@@ -538,17 +538,17 @@ int launch_ck_umma(const CommitArgs& a, u32 n, u32 Bw, u32 G, const ModQ& M, con
 // step c run.
 // ---------------------------------------------------------------------------
 constexpr u32 PU_POS = 128, PU_KS = 64;
-constexpr u32 PU_IMG = 2 * 128 * 128;  // Jc: both J halves of one 128-element chunk (32 KiB)
 constexpr u32 PU_A = 2 * 128 * PU_KS;  // both J halves of one step (16 KiB)
 constexpr u32 PU_B = PU_POS * PU_KS;   // witness int8 tile (8 KiB)
 constexpr u32 PU_STAGE = PU_A + PU_B;
 
 __global__ void __launch_bounds__(256, 2)
     project_umma_kernel(RowSet in, u32 d, u64 q, u32 cw, u64 nch, const int8_t* __restrict__ Jc,
-                        u64* __restrict__ out, u64* flag) {
+                        u64* __restrict__ out, u64* flag, const u32* gate) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[2], done_bar[2];
   __shared__ uint32_t tslot;
+  if (gate && *(volatile const u32*)gate == 0) return;  // the byte rows were projected
   const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const u32 nblk = blockIdx.x;
   const u64 idx = blockIdx.y;
@@ -598,11 +598,9 @@ __global__ void __launch_bounds__(256, 2)
     const u32 st = c & 1;
     uint8_t* stage = smem + st * PU_STAGE;
     if (c >= 2) ok &= umma::mbar_wait(&done_bar[st], ((c - 2) >> 1) & 1, err, 1);
-    if (tid == 0) {  // K slices of this step from the chunk's image, one copy per J half
+    if (tid == 0) {  // K slices of this step from the image
       umma::mbar_expect_tx(&full_bar[st], PU_A);
-      const int8_t* img = Jc + (u64)(c / 2) * PU_IMG + (c % 2) * (PU_A / 2);
-      umma::bulk_g2s(stage, img, PU_A / 2, &full_bar[st]);
-      umma::bulk_g2s(stage + PU_A / 2, img + PU_IMG / 2, PU_A / 2, &full_bar[st]);
+      umma::bulk_g2s(stage, Jc + (u64)c * PU_A, PU_A, &full_bar[st]);
     }
     // witness step: 128 positions x 64 elements as int8, (k / 16, pos, k % 16):
     // the 16 bytes of one position are one 16-byte store
@@ -647,7 +645,7 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (u32 ks = 0; ks < PU_KS / 32; ks++) {
           const uint64_t ad =
-              umma::desc_kmajor(umma::smem_u32(stage + h * (PU_A / 2) + ks * 2 * 128 * 16), 128 * 16, 128);
+              umma::desc_kmajor(umma::smem_u32(stage + h * 128 * 16 + ks * 2 * 256 * 16), 256 * 16, 128);
           const uint64_t bd = umma::desc_kmajor(umma::smem_u32(B + ks * 2 * PU_POS * 16), PU_POS * 16, 128);
           umma::mma_i8(tmem + h * 128, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
         }
@@ -680,12 +678,12 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 int launch_project_umma(RowSet in, u32 rows, u64 nch, u32 d, u64 q, u32 cw, const int8_t* Jc, u64* out, u64* flag,
-                        cudaStream_t st) {
+                        const u32* gate, cudaStream_t st) {
   const size_t smem = 2 * (size_t)PU_STAGE;
   cudaError_t e = cudaFuncSetAttribute(project_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project_umma smem attribute");
   dim3 g(d / PU_POS, (unsigned)(rows * nch));
-  project_umma_kernel<<<g, 256, smem, st>>>(in, d, q, cw, nch, Jc, out, flag);
+  project_umma_kernel<<<g, 256, smem, st>>>(in, d, q, cw, nch, Jc, out, flag, gate);
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "project_umma launch");

@@ -1209,30 +1209,27 @@ int launch_decompose_ntt(RowSet in, u32 rows, u64 width, u32 d, u64 q, u32 parts
 // ---------------------------------------------------------------------------
 constexpr u32 PROJ_H = 256;
 
+// One thread per row and 16 elements, rows fastest: a warp's Jc stores are one run.
 __global__ void proj_tables_kernel(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32* neg_mask,
                                    int8_t* J, int8_t* Jc) {
-  const u32 words = cw / 32;
-  u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (u64)PROJ_H * words) return;
-  const u32 k = (u32)(t / words), w = (u32)(t % words);
+  const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= PROJ_H * (cw / 16)) return;
+  const u32 k = t % PROJ_H, sl = t / PROJ_H;
   const u64 key = prf_key(ds->seed, domain_id(DOM_PROJ, round, 0));
-  u32 pm = 0, nm = 0;
-  for (u32 b = 0; b < 32; b++) {
-    const u64 r = prf_at(key, (u64)k * cw + w * 32 + b);
+  u32 pm = 0, nm = 0, v[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (u32 b = 0; b < 16; b++) {
+    const u64 r = prf_at(key, (u64)k * cw + sl * 16 + b);
     const u32 iz = r & 1, sg = (r >> 1) & 1;
-    if (!iz) {
-      if (sg) pm |= 1u << b;
-      else nm |= 1u << b;
-    }
-    const int8_t v = iz ? 0 : (sg ? 1 : -1);
-    if (J) J[(u64)k * cw + w * 32 + b] = v;
-    if (Jc) {  // (chunk, half, 16-byte slice, row in half, byte)
-      const u32 l = w * 32 + b, cc = l / 128, sl = (l % 128) / 16, h = k / 128, r = k % 128;
-      Jc[((((u64)cc * 2 + h) * 8 + sl) * 128 + r) * 16 + (l % 16)] = v;
-    }
+    pm |= (u32)(!iz && sg) << b;
+    nm |= (u32)(!iz && !sg) << b;
+    v[b / 4] |= (iz ? 0u : (sg ? 1u : 0xffu)) << (8 * (b % 4));
   }
-  pos_mask[t] = pm;
-  neg_mask[t] = nm;
+  ((uint16_t*)pos_mask)[(u64)k * (cw / 16) + sl] = (uint16_t)pm;
+  ((uint16_t*)neg_mask)[(u64)k * (cw / 16) + sl] = (uint16_t)nm;
+  const uint4 v4 = make_uint4(v[0], v[1], v[2], v[3]);
+  if (J) *(uint4*)(J + (u64)k * cw + sl * 16) = v4;
+  if (Jc) *(uint4*)(Jc + ((u64)sl * PROJ_H + k) * 16) = v4;
 }
 
 // cj[l] = sum_k J[k][l]: one CTA per 32 columns (one mask word), 32 x 32
@@ -1259,8 +1256,8 @@ int launch_proj_tables(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32
                        u64 q, cudaStream_t st, int8_t* Jc) {
   if (cw % 32) return salsaa_set_error(-2, "project: chunk width must be a multiple of 32");
   if (Jc && cw % 128) Jc = nullptr;
-  u64 tot = (u64)PROJ_H * (cw / 32);
-  proj_tables_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(ds, round, cw, pos_mask, neg_mask, J, Jc);
+  u64 tot = (u64)PROJ_H * (cw / 16);
+  proj_tables_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(ds, round, cw, pos_mask, neg_mask, J, Jc);
   int rc = check_launch("proj_tables");
   if (rc) return rc;
   if (cj) {
@@ -1270,53 +1267,55 @@ int launch_proj_tables(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32
   return rc;
 }
 
-// One CTA per (chunk, tile of KT outputs); one thread per coefficient.
+// Work item: (chunk, tile of KT outputs); one thread per coefficient.
 // With q < 2^52 the +-1 sums (cw terms of value < q, negatives as q - w) fit
 // in 64 bits and are reduced once.
 template <int KT, bool LAZY>
-__global__ void project_kernel(RowSet in, u64 width, u32 d, u64 q, u32 cw, u64 nch, const u32* pos_mask,
+__global__ void project_kernel(RowSet in, u32 rows, u32 d, u64 q, u32 cw, u64 nch, const u32* pos_mask,
                                const u32* neg_mask, u64* out, const u64* gate) {
   extern __shared__ u32 msk[];  // KT x words (pos), then KT x words (neg)
   if (gate && *(volatile const u64*)gate == 0) return;  // the tensor-core pass was exact
-  const u32 words = cw / 32;
-  const u64 idx = blockIdx.x;
-  const u32 i = (u32)(idx / nch);
-  const u64 j = idx % nch;
-  const u32 k0 = blockIdx.y * KT;
-  for (u32 t = threadIdx.x; t < KT * words; t += blockDim.x) {
-    const u32 kk = t / words, w = t % words;
-    msk[t] = pos_mask[(u64)(k0 + kk) * words + w];
-    msk[KT * words + t] = neg_mask[(u64)(k0 + kk) * words + w];
-  }
-  __syncthreads();
-  const u32 pos = threadIdx.x;
-  if (pos >= d) return;
-  const bool nar = (in.narrow >> i) & 1;
-  const u64* chunk = row_advance(in.p[i], nar, (j * cw) * d);
-  u64 acc[KT];
-#pragma unroll
-  for (int kk = 0; kk < KT; kk++) acc[kk] = 0;
-  for (u32 w = 0; w < words; w++) {
-    u32 pm[KT], nm[KT];
-#pragma unroll
-    for (int kk = 0; kk < KT; kk++) {
-      pm[kk] = msk[kk * words + w];
-      nm[kk] = msk[KT * words + kk * words + w];
+  const u32 words = cw / 32, items = (u32)(rows * nch) * (PROJ_H / KT);
+  for (u32 item = blockIdx.x; item < items; item += gridDim.x) {
+    const u64 idx = item / (PROJ_H / KT);
+    const u32 i = (u32)(idx / nch);
+    const u64 j = idx % nch;
+    const u32 k0 = item % (PROJ_H / KT) * KT;
+    __syncthreads();
+    for (u32 t = threadIdx.x; t < KT * words; t += blockDim.x) {
+      const u32 kk = t / words, w = t % words;
+      msk[t] = pos_mask[(u64)(k0 + kk) * words + w];
+      msk[KT * words + t] = neg_mask[(u64)(k0 + kk) * words + w];
     }
-    for (u32 b = 0; b < 32; b++) {
-      const u64 x = wres(chunk, nar, (u64)(w * 32 + b) * d + pos, q);
-      const u64 nx = x ? q - x : 0;
+    __syncthreads();
+    const u32 pos = threadIdx.x;
+    const bool nar = (in.narrow >> i) & 1;
+    const u64* chunk = row_advance(in.p[i], nar, (j * cw) * d);
+    u64 acc[KT];
+#pragma unroll
+    for (int kk = 0; kk < KT; kk++) acc[kk] = 0;
+    for (u32 w = 0; w < words; w++) {
+      u32 pm[KT], nm[KT];
 #pragma unroll
       for (int kk = 0; kk < KT; kk++) {
-        u64 v = ((pm[kk] >> b) & 1) ? x : 0;
-        v = ((nm[kk] >> b) & 1) ? nx : v;
-        if (LAZY) acc[kk] += v;
-        else acc[kk] = add_mod(acc[kk], v, q);
+        pm[kk] = msk[kk * words + w];
+        nm[kk] = msk[KT * words + kk * words + w];
+      }
+      for (u32 b = 0; b < 32; b++) {
+        const u64 x = wres(chunk, nar, (u64)(w * 32 + b) * d + pos, q);
+        const u64 nx = x ? q - x : 0;
+#pragma unroll
+        for (int kk = 0; kk < KT; kk++) {
+          u64 v = ((pm[kk] >> b) & 1) ? x : 0;
+          v = ((nm[kk] >> b) & 1) ? nx : v;
+          if (LAZY) acc[kk] += v;
+          else acc[kk] = add_mod(acc[kk], v, q);
+        }
       }
     }
-  }
 #pragma unroll
-  for (int kk = 0; kk < KT; kk++) out[((idx * PROJ_H) + k0 + kk) * d + pos] = LAZY ? acc[kk] % q : acc[kk];
+    for (int kk = 0; kk < KT; kk++) out[((idx * PROJ_H) + k0 + kk) * d + pos] = LAZY ? acc[kk] % q : acc[kk];
+  }
 }
 
 // Tensor-core projection: per chunk, OUT (256 x d) = J (256 x cw) * W (cw x d)
@@ -1425,7 +1424,8 @@ __global__ void __launch_bounds__(256, 2) project_mma_kernel(RowSet in, u32 d, u
 }
 
 int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_mask, const u32* neg_mask,
-                   const int8_t* J, DevState* ds, u64* out, cudaStream_t st, const int8_t* Jc) {
+                   const int8_t* J, DevState* ds, u64* out, cudaStream_t st, const int8_t* Jc, const C8Rows* w8,
+                   const u32* wide) {
   const u32 cw = rows * PROJ_H;
   if (rows == 0 || rows > MAX_WROWS || cw > width || width % cw)
     return salsaa_set_error(-3, "project: chunk width exceeds witness width");
@@ -1436,7 +1436,11 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
   if (Jc && ds && d % 128 == 0 && cw % 128 == 0 && rowset_aligned(in, rows, 16, 8)) {
     cudaError_t e = cudaMemsetAsync(&ds->proj_flag, 0, sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project memset");
-    int rc = launch_project_umma(in, rows, nch, d, q, cw, Jc, out, &ds->proj_flag, st);
+    // short rows as byte tiles; then the words, only while they are wide
+    const bool tc = w8 && wide && project_tc_ok(*w8, d, cw);
+    int rc = tc ? launch_project_tc(*w8, d, q, cw, Jc, out, wide, st) : 0;
+    if (rc) return rc;
+    rc = launch_project_umma(in, rows, nch, d, q, cw, Jc, out, &ds->proj_flag, tc ? wide : nullptr, st);
     if (rc) return rc;
     gate = &ds->proj_flag;
   } else if (J && ds && d % PJ_BN == 0 && cw % PJ_KS == 0) {
@@ -1449,11 +1453,13 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
     gate = &ds->proj_flag;
   }
   constexpr int KT = 16;
-  dim3 g((unsigned)(rows * nch), PROJ_H / KT);
+  const u64 items = rows * nch * (PROJ_H / KT);
+  // behind a gate that is nearly always closed: few blocks to start and end
+  const unsigned g = (unsigned)(gate && items > 148 * 8 ? 148 * 8 : items);
   const size_t smem = 2ULL * KT * (cw / 32) * sizeof(u32);
   const bool lazy = q < (1ULL << 52) && cw <= 4096;
-  if (lazy) project_kernel<KT, true><<<g, d, smem, st>>>(in, width, d, q, cw, nch, pos_mask, neg_mask, out, gate);
-  else project_kernel<KT, false><<<g, d, smem, st>>>(in, width, d, q, cw, nch, pos_mask, neg_mask, out, gate);
+  if (lazy) project_kernel<KT, true><<<g, d, smem, st>>>(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
+  else project_kernel<KT, false><<<g, d, smem, st>>>(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
   return check_launch("project");
 }
 

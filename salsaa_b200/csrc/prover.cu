@@ -978,7 +978,9 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       const u32 cw = K2 * 256;
       u64* cj = pr->row_cj + (u64)rd * CK_BLOCK;
       TRY(launch_proj_tables(pr->ds, rd, cw, pr->pmask, pr->nmask, pr->Jm, cj, q, ps, pr->Jc));
-      TRY(launch_project(Wc2, K2, width2, d, q, pr->pmask, pr->nmask, pr->Jm, pr->ds, pr->Pc, ps, pr->Jc));
+      const C8Rows w8 = c8_rows(pr->c8, K2, width2, d, !P.folding);
+      TRY(launch_project(Wc2, K2, width2, d, q, pr->pmask, pr->nmask, pr->Jm, pr->ds, pr->Pc, ps, pr->Jc,
+                         sh ? &w8 : nullptr, &pr->ds->wide[rd]));
     }
     // the joined witness [folded, projected] is decomposed next: the two
     // transforms that read P and write the folded row collect the OR of its

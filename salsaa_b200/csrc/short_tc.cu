@@ -1,4 +1,4 @@
-// short_tc.cu — fold and statement rows over short witness rows on the tensor cores.
+// short_tc.cu — fold, projection and statement rows over short witness rows on the tensor cores.
 #include <cuda_runtime.h>
 
 #include "short_tc.cuh"
@@ -359,6 +359,138 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
+// ---------------------------------------------------------------------------
+// Projection (project, src/subroutines/project.rs:50-103) over byte rows: per
+// (chunk of cw elements, 128 positions) D[position][J row] = sum_l w(l,
+// position) J[row][l], M = 128 positions (the byte tile MN-major), N = 256 J
+// rows (their image K-major) or a part of them, K = elements, one item per
+// unit of a persistent grid, two accumulators.  A lane holds one position, so
+// each column is stored as whole sectors.  Bound by the words it writes (8
+// bytes for 256 / rows input bytes) and, with long chunks, by its copies from
+// L2: 24 KB per 64 elements.  Where project_umma_kernel converts the witness
+// words itself, here both operands are bulk copies: 789 -> 203 us of an
+// 8-round proof over 2^19 elements, d = 128.
+// ---------------------------------------------------------------------------
+constexpr u32 PT_EPI = 256, PT_THREADS = PT_EPI + 64, PT_STAGES = 8, PT_ROWS = 256;
+constexpr u32 PT_A = 64 * 128, PT_STAGE = PT_A + 64 * PT_ROWS;
+
+__global__ void __launch_bounds__(PT_THREADS, 1)
+    project_tc_kernel(C8Rows w, u32 d, u64 q, u32 cw, u32 nch, u32 nsplit, const int8_t* __restrict__ Jc,
+                      u64* __restrict__ out, const u32* wide, u32* err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t full_bar[PT_STAGES], empty_bar[PT_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tslot;
+  if (*(volatile const u32*)wide) return;
+  const u32 tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const u32 npb = d / 128, items = w.rows * nch * npb * nsplit, nr = PT_ROWS / nsplit, steps = cw / 64;
+  if (tid == 0) {
+    for (u32 i = 0; i < PT_STAGES; i++) {
+      umma::mbar_init(&full_bar[i], 1);
+      umma::mbar_init(&empty_bar[i], 1);
+    }
+    for (u32 i = 0; i < 2; i++) {
+      umma::mbar_init(&acc_full[i], 1);
+      umma::mbar_init(&acc_empty[i], PT_EPI);
+    }
+    umma::mbar_fence_init();
+  }
+  if (warp == 0) umma::tmem_alloc(&tslot, 512);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const u32 tmem = tslot;
+
+  if (warp == PT_EPI / 32) {
+    bool ok = true;
+    u32 it = 0, st = 0, par = 1;
+    for (u32 item = blockIdx.x; ok && item < items; item += gridDim.x) {
+      const u32 ns = item % nsplit, pb = item / nsplit % npb, idx = item / (nsplit * npb), r = idx / nch, j = idx % nch;
+      const int8_t* src = w.p + w.row[r] * w.stride + (w.off[r] + (u64)j * cw) * d + pb * PT_A;
+      for (u32 c = 0; c < steps; c++, it++) {
+        if (it >= PT_STAGES && !(ok = umma::mbar_wait(&empty_bar[st], par, err, 61))) break;
+        if (umma::elect_one()) {
+          uint8_t* stage = smem + st * PT_STAGE;
+          umma::mbar_expect_tx(&full_bar[st], PT_A + 64 * nr);
+          umma::bulk_g2s(stage, src + (u64)c * 64 * d, PT_A, &full_bar[st]);
+          const int8_t* im = Jc + (u64)c * 64 * PT_ROWS + ns * nr * 16;
+          if (nsplit == 1) umma::bulk_g2s(stage + PT_A, im, 64 * PT_ROWS, &full_bar[st]);
+          else
+            for (u32 x = 0; x < 4; x++)
+              umma::bulk_g2s(stage + PT_A + x * nr * 16, im + x * PT_ROWS * 16, nr * 16, &full_bar[st]);
+        }
+        __syncwarp();
+        if (++st == PT_STAGES) {
+          st = 0;
+          par ^= 1;
+        }
+      }
+    }
+    for (u32 c = it >= PT_STAGES ? it - PT_STAGES : 0; c < it; c++)
+      umma::mbar_wait(&full_bar[c % PT_STAGES], (c / PT_STAGES) & 1, err, 62);
+  } else if (warp == PT_EPI / 32 + 1) {
+    // A: s8, MN-major (position slices 1024 apart, 8-element blocks 128); B: s8, K-major
+    const u32 idesc = (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((nr >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t ad0 = umma::desc_kmajor(umma::smem_u32(smem), 128, 1024);
+    const uint64_t bd0 = umma::desc_kmajor(umma::smem_u32(smem + PT_A), nr * 16, 128);
+    bool ok = true;
+    u32 it = 0, ui = 0, st = 0, par = 0;
+    for (u32 item = blockIdx.x; ok && item < items; item += gridDim.x, ui++) {
+      const u32 nb = ui & 1;
+      if (ui >= 2 && !(ok = umma::mbar_wait(&acc_empty[nb], ((ui >> 1) - 1) & 1, err, 63))) break;
+      umma::fence_after_sync();
+      for (u32 c = 0; c < steps; c++, it++) {
+        if (!(ok = umma::mbar_wait(&full_bar[st], par, err, 64))) break;
+        umma::fence_after_sync();
+        const uint64_t so = (uint64_t)st * (PT_STAGE >> 4);
+        if (umma::elect_one()) {
+#pragma unroll
+          for (u32 ks = 0; ks < 2; ks++)
+            umma::mma_i8_u(tmem + nb * 256, ad0 + so + ks * 32, bd0 + so + ks * 2 * nr, idesc,
+                           (c > 0 || ks > 0) ? 1u : 0u);
+          umma::commit(&empty_bar[st]);
+          if (c + 1 == steps) umma::commit(&acc_full[nb]);
+        }
+        __syncwarp();
+        if (++st == PT_STAGES) {
+          st = 0;
+          par ^= 1;
+        }
+      }
+    }
+    for (u32 c = it >= PT_STAGES ? it - PT_STAGES : 0; c < it; c++)
+      umma::mbar_wait(&empty_bar[c % PT_STAGES], (c / PT_STAGES) & 1, err, 65);
+  } else {
+    const u32 m = (warp & 3) * 32 + lane, cols = nr / 2, c0 = (warp >> 2) * cols;
+    u32 ui = 0;
+    for (u32 item = blockIdx.x; item < items; item += gridDim.x, ui++) {
+      const u32 ns = item % nsplit, pb = item / nsplit % npb, idx = item / (nsplit * npb), nb = ui & 1;
+      const bool ok = umma::mbar_wait(&acc_full[nb], (ui >> 1) & 1, err, 66);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      umma::fence_after_sync();
+      const u32 tb = tmem + (((warp & 3) * 32) << 16) + nb * 256 + c0;
+      u64* dst = out + ((u64)idx * PT_ROWS + ns * nr + c0) * d + pb * 128 + m;
+      for (u32 g = 0; g < cols; g += 32) {
+        uint32_t v[2][16];
+        umma::tmem_ld16(tb + g, v[0]);
+        umma::tmem_ld16(tb + g + 16, v[1]);
+        umma::tmem_wait_ld();
+        if (g + 32 == cols) {
+          umma::fence_before_sync();
+          umma::mbar_arrive(&acc_empty[nb]);
+        }
+#pragma unroll
+        for (u32 e = 0; e < 32; e++) {
+          const int x = (int)v[e / 16][e % 16];
+          dst[(u64)(g + e) * d] = x >= 0 ? (u64)x : q - (u64)(-(long long)x);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  umma::fence_after_sync();
+  if (warp == 0) umma::tmem_dealloc(tmem, 512);
+}
+
 }  // namespace
 
 int launch_fold_challenge_tz(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, int8_t* tz,
@@ -388,6 +520,30 @@ int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u6
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_tc launch");
+}
+
+bool project_tc_ok(const C8Rows& w, u32 d, u32 cw) {
+  // 2^31 bounds the sums: cw x 128
+  return d % 128 == 0 && d <= 1024 && cw >= 64 && cw % 64 == 0 && cw <= (1u << 23) && w.rows > 0 &&
+         w.rows <= (u32)MAX_WROWS && w.width >= cw && w.width % cw == 0 && w.width / cw * w.rows <= 65535;
+}
+
+int launch_project_tc(const C8Rows& w, u32 d, u64 q, u32 cw, const int8_t* Jc, u64* out, const u32* wide,
+                      cudaStream_t st) {
+  if (!project_tc_ok(w, d, cw)) return salsaa_set_error(-2, "project_tc: rows outside the byte-tile path");
+  const u32 nch = (u32)(w.width / cw), base = w.rows * nch * (d / 128);
+  // few chunks: part of the J rows per CTA
+  u32 nsplit = 1;
+  while (nsplit < 4 && base * nsplit * 2 <= 148) nsplit *= 2;
+  const u32 items = base * nsplit;
+  const size_t smem = (size_t)PT_STAGES * PT_STAGE;
+  cudaError_t e = cudaFuncSetAttribute(project_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project_tc smem attribute");
+  project_tc_kernel<<<items < 148 ? items : 148, PT_THREADS, smem, st>>>(w, d, q, cw, nch, nsplit, Jc, out, wide,
+                                                                         tc_error_word());
+  salsaa_count_launch();
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "project_tc launch");
 }
 
 int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_hi,

@@ -28,6 +28,12 @@ bool fold_tc_ok(const C8Rows& w, u32 d);
 int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u64* mag_or, const u32* flag,
                    cudaStream_t st);
 
+// Projection of launch_project (kernels.cuh): rows w.rows, chunks of cw
+// elements, out word rows [(row, chunk)][256][d]; runs only while *wide == 0.
+bool project_tc_ok(const C8Rows& w, u32 d, u32 cw);
+int launch_project_tc(const C8Rows& w, u32 d, u64 q, u32 cw, const int8_t* Jc, u64* out, const u32* wide,
+                      cudaStream_t st);
+
 // Statement rows of launch_commit (kernels.cuh) over byte rows: byte row r
 // adds 2^shift[r] times its sums to witness row dst[r], unless *wide[dst[r]]
 // is nonzero (then launch_sc_umma takes that row).
