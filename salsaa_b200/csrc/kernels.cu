@@ -11,6 +11,7 @@
 #include <vector>
 #include "kernels.cuh"
 #include "ntt_img.cuh"
+#include "gram.cuh"
 #include "short_tc.cuh"
 
 namespace salsaa {
@@ -212,6 +213,7 @@ constexpr u32 SC_TAIL = 16384;   // vectors this short finish in one CTA (batche
 // vector is captured at length d by the tail); the tail then finishes in one
 // CTA per (repetition, row).
 constexpr u32 SC_TAIL_ONE = 2048;
+constexpr u32 SC_MAX_NR = 64;    // rounds of a vector
 
 // Lazy sums: with q < 2^50 each product is < 2^100 and a thread's sum of
 // far fewer than 2^27 products fits in 128 bits.
@@ -335,10 +337,9 @@ __device__ __forceinline__ void group_rounds(const ModQ& M, u64 (&x)[1 << T], co
 template <bool LAZY>
 __global__ void __launch_bounds__(256, 2) sc_first_kernel(RowSet w, u32 rows, u64 nlen, ModQ M, const DevState* ds,
                                                           u32 round, u64* out, u64 sout, u64* sums, u32 nr,
-                                                          bool plain, const u32* only_if) {
+                                                          bool plain) {
   constexpr u32 T = SC_T, G = 1u << T;
   __shared__ Sum128 red[SC_T * 3 * 32];
-  if (only_if && *only_if == 0) return;  // the tensor-core pass covered this launch
   const u32 k = blockIdx.y, rep = blockIdx.x & 1, bx = blockIdx.x >> 1, nbx = gridDim.x >> 1;
   const u64* x = w.p[k];
   const bool nar = (w.narrow >> k) & 1;
@@ -415,13 +416,18 @@ __global__ void __launch_bounds__(256) sc_round_kernel(const u64* in, u64 sin, u
 // T rounds of the tail on the vector v (length cur, shared memory): groups of
 // 2^T values v[g + m ng] per thread, sums of all T rounds in one block
 // reduction, folded values back to v[g] (only thread g touches v[g]).
-template <bool LAZY, u32 T>
-__device__ __forceinline__ void tail_step(u64* v, u64 cur, const ModQ& M, const DevState* ds, u32 round, u32 rep,
-                                          u32 j, u64* sums, u32 nr, u32 rows, u32 k, Sum128* red, u64* sch) {
+// ch: the challenges from this step's first round on, their Shoup companions
+// SC_MAX_NR behind; sums(t): where the three sums of its round t go.
+template <bool LAZY, u32 T, typename Sums>
+__device__ __forceinline__ void tail_step(u64* v, u64 cur, const ModQ& M, const u64* ch, Sums sums, Sum128* red) {
   constexpr u32 G = 1u << T;
-  const u64 q = M.q, ng = cur >> T;
+  const u64 ng = cur >> T;
   u64 c[T], cp[T];
-  shared_challenges<T>(sch, [&](u32 t) { return nc_challenge(ds, round, rep, j + t, q); }, q, c, cp);
+#pragma unroll
+  for (u32 t = 0; t < T; t++) {
+    c[t] = ch[t];
+    cp[t] = ch[SC_MAX_NR + t];
+  }
   ScAcc<LAZY> acc[T][3];
 #pragma unroll
   for (u32 t = 0; t < T; t++)
@@ -440,21 +446,92 @@ __device__ __forceinline__ void tail_step(u64* v, u64 cur, const ModQ& M, const 
 #pragma unroll
     for (u32 a = 0; a < 3; a++) flat[t * 3 + a] = acc[t][a];
   const u64 r = block_totals<LAZY, T * 3>(M, flat, red);  // its barriers also publish v
-  if (threadIdx.x < T * 3) sums[((rep * (u64)nr + j + threadIdx.x / 3) * rows + k) * 3 + threadIdx.x % 3] = r;
+  if (threadIdx.x < T * 3) sums(threadIdx.x / 3)[threadIdx.x % 3] = r;
 }
+template <bool LAZY, typename Sums>
+__device__ __forceinline__ void tail_steps(u32 T, u64* v, u64 cur, const ModQ& M, const u64* ch, Sums sums,
+                                           Sum128* red) {
+  switch (T) {
+    case 4: tail_step<LAZY, 4>(v, cur, M, ch, sums, red); break;
+    case 3: tail_step<LAZY, 3>(v, cur, M, ch, sums, red); break;
+    case 2: tail_step<LAZY, 2>(v, cur, M, ch, sums, red); break;
+    default: tail_step<LAZY, 1>(v, cur, M, ch, sums, red); break;
+  }
+}
+// A tail's challenges, all rounds at once: the companions are 128-bit divisions.
+template <typename Chal>
+__device__ __forceinline__ void tail_challenges(u64* ch, u32 nr, Chal chal, u64 q) {
+  for (u32 t = threadIdx.x; t < nr; t += blockDim.x) {
+    const u64 v = chal(t);
+    ch[t] = v;
+    ch[SC_MAX_NR + t] = (u64)((((unsigned __int128)v) << 64) / q);
+  }
+  __syncthreads();
+}
+// Round polynomial (and with claim the claim) from a round's raw sums.
+__device__ __forceinline__ void sc_poly(const u64* s, u64 q, u64* o, u64* claim) {
+  const u64 s00 = s[0] % q, s01 = s[1] % q, s11 = s[2] % q;
+  o[0] = s00;
+  o[1] = sub_mod(s01, s00, q);
+  o[2] = add_mod(sub_mod(sub_mod(s11, s01, q), s01, q), s00, q);
+  if (claim) *claim = add_mod(s00, s11, q);  // round 0: sum of squares
+}
+
+// Sums of a tensor-core pass's four rounds from its Gram matrix C (gram.cuh):
+// round t's sums are traces of its values' Gram matrix, which folds on both
+// sides with the round's challenge.  Every thread of a block of at least 256.
+template <typename Sums>
+__device__ __forceinline__ void gram_sums(const u64* gram, const ModQ& M, const u64* ch, Sums sums, u64* C) {
+  const u64 q = M.q;
+  const u32 tid = threadIdx.x;
+  __syncthreads();  // C may still be read by an earlier use
+  if (tid < 256) C[tid] = reduce64(M, gram[tid]);
+  __syncthreads();
+#pragma unroll
+  for (u32 t = 0; t < SC_T; t++) {
+    const u32 h = 8u >> t;
+    const u64 c = ch[t], cp = ch[SC_MAX_NR + t];
+    if (tid < 3) {
+      const u32 r0 = tid == 2 ? h : 0, c0 = tid == 0 ? 0 : h;
+      u64 s = 0;
+#pragma unroll
+      for (u32 j = 0; j < h; j++) s = add_mod(s, C[(r0 + j) * 16 + c0 + j], q);
+      sums(t)[tid] = s;
+    }
+    const u32 i = tid / h, j = tid % h;
+    u64 v = 0;
+    if (tid < h * h)
+      v = fold1(fold1(C[i * 16 + j], C[i * 16 + j + h], c, cp, q),
+                fold1(C[(i + h) * 16 + j], C[(i + h) * 16 + j + h], c, cp, q), c, cp, q);
+    __syncthreads();
+    if (tid < h * h) C[i * 16 + j] = v;
+    __syncthreads();
+  }
+}
+// Tensor-core passes of launch_sumcheck: first round, Gram matrices (one a row
+// for both repetitions when shared, else one a (rep, row)).
+struct GramList {
+  const u64* c[SC_GRAM_PASSES];
+  u32 j[SC_GRAM_PASSES], shared[SC_GRAM_PASSES];
+  u32 n;
+};
 
 template <bool LAZY>
 __global__ void __launch_bounds__(512) sc_tail_kernel(const u64* in, u64 sin, RowSet w0, u64 L, u32 rows, ModQ M,
                                                        const DevState* ds, u32 round, u32 j0, u64* sums, u32 nr,
-                                                       u32 d, u64* cap) {
+                                                       u32 d, u64* cap, GramList gl, u64* claims, u64* polys0,
+                                                       u64* polys1) {
   extern __shared__ u64 v[];
   __shared__ Sum128 red[SC_T * 3 * 32];
-  __shared__ u64 sch[2 * SC_T];
+  __shared__ u64 ch[2 * SC_MAX_NR], C[256];
   const u32 pair = blockIdx.x, rep = pair / rows, k = pair % rows;
   const u64* x = (j0 == 0) ? w0.p[k] : in + (u64)pair * sin;
   const bool nar = j0 == 0 && ((w0.narrow >> k) & 1);
   for (u32 i = threadIdx.x; i < L; i += blockDim.x) v[i] = wres(x, nar, i, M.q);
-  __syncthreads();
+  tail_challenges(ch, nr, [&](u32 t) { return nc_challenge(ds, round, rep, t, M.q); }, M.q);
+  for (u32 p = 0; p < gl.n; p++)
+    gram_sums(gl.c[p] + (u64)(gl.shared[p] ? k : pair) * 256, M, ch + gl.j[p],
+              [&](u32 t) { return sums + ((rep * (u64)nr + gl.j[p] + t) * rows + k) * 3; }, C);
   u64 cur = L;
   u32 j = j0;
   while (cur > 1) {
@@ -469,15 +546,16 @@ __global__ void __launch_bounds__(512) sc_tail_kernel(const u64* in, u64 sin, Ro
       T = td < T ? td : T;
     }
     T = T < SC_T ? T : SC_T;
-    switch (T) {
-      case 4: tail_step<LAZY, 4>(v, cur, M, ds, round, rep, j, sums, nr, rows, k, red, sch); break;
-      case 3: tail_step<LAZY, 3>(v, cur, M, ds, round, rep, j, sums, nr, rows, k, red, sch); break;
-      case 2: tail_step<LAZY, 2>(v, cur, M, ds, round, rep, j, sums, nr, rows, k, red, sch); break;
-      default: tail_step<LAZY, 1>(v, cur, M, ds, round, rep, j, sums, nr, rows, k, red, sch); break;
-    }
+    tail_steps<LAZY>(T, v, cur, M, ch + j, [&](u32 t) { return sums + ((rep * (u64)nr + j + t) * rows + k) * 3; },
+                     red);
     cur >>= T;
     j += T;
   }
+  // every round of this (rep, row) is summed: its claims and polynomials
+  __syncthreads();
+  for (u32 t = threadIdx.x; t < nr; t += blockDim.x)
+    sc_poly(sums + ((rep * (u64)nr + t) * rows + k) * 3, M.q, (rep ? polys1 : polys0) + ((u64)t * rows + k) * 3,
+            rep == 0 && t == 0 ? claims + k : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -489,16 +567,6 @@ __global__ void __launch_bounds__(512) sc_tail_kernel(const u64* in, u64 sin, Ro
 // memory), four rounds per pass; a final launch finishes every instance in
 // shared memory (one CTA each).
 // ---------------------------------------------------------------------------
-struct SbInst {
-  const u64* in;
-  u64* out;
-  u64 L;     // current length
-  u64 tile0; // first tile of this instance in the level's tile space
-  u32 j;     // index of the next round
-  u32 id;    // instance index: its challenge stream and its rows of sums
-};
-constexpr u32 SB_MAX_INST = 64, SB_GPT = 4, SB_TILE_GROUPS = 256 * SB_GPT;
-
 __device__ __forceinline__ u64 sb_challenge(u64 seed, u32 round, u32 inst, u64 j, u64 q) {
   return uni_mod(prf_at(prf_key(seed, domain_id(DOM_NC, round, inst)), j), q);
 }
@@ -549,62 +617,38 @@ __global__ void __launch_bounds__(256, 2) sb_pass_kernel(const SbInst* inst, u32
   }
 }
 
+// gram: per level (four rounds) SB_MAX_INST Gram matrices, for the levels that
+// the instance took on the tensor cores; or null.
 template <bool LAZY>
 __global__ void __launch_bounds__(1024) sb_tail_kernel(const SbInst* inst, ModQ M, u64 seed, u32 round, u64* sums,
-                                                       u32 nrmax) {
+                                                       u32 nrmax, const u64* gram, const u64* offs, u64* claims,
+                                                       u64* polys) {
   extern __shared__ u64 v[];
-  __shared__ Sum128 red[3 * 32];
-  __shared__ u64 sch[2];
+  __shared__ Sum128 red[SC_T * 3 * 32];
+  __shared__ u64 ch[2 * SC_MAX_NR], C[256];
   const u32 i = blockIdx.x;
   const SbInst I = inst[i];
   const u64 q = M.q;
   for (u64 e = threadIdx.x; e < I.L; e += blockDim.x) v[e] = I.in[e];
-  __syncthreads();
+  const u32 nr = I.j + 63u - (u32)__clzll((long long)I.L);
+  tail_challenges(ch, nr, [&](u32 t) { return sb_challenge(seed, round, i, t, q); }, q);
+  if (gram)
+    for (u32 j = 0; j < I.j; j += SC_T)
+      gram_sums(gram + ((u64)(j / SC_T) * SB_MAX_INST + i) * 256, M, ch + j,
+                [&](u32 t) { return sums + ((u64)i * nrmax + j + t) * 3; }, C);
   u64 cur = I.L;
   u32 j = I.j;
   while (cur > 1) {
-    const u64 h = cur / 2;
-    ScAcc<LAZY> a0, a1, a2;
-    a0.zero();
-    a1.zero();
-    a2.zero();
-    for (u64 e = threadIdx.x; e < h; e += blockDim.x) {
-      const u64 p0 = v[e], p1 = v[e + h];
-      a0.mac(M, p0, p0);
-      a1.mac(M, p0, p1);
-      a2.mac(M, p1, p1);
-    }
-    ScAcc<LAZY> tri[3] = {a0, a1, a2};
-    const u64 r = block_totals<LAZY, 3>(M, tri, red);
-    if (threadIdx.x < 3) sums[((u64)i * nrmax + j) * 3 + threadIdx.x] = r;
-    if (threadIdx.x == 0) {
-      const u64 cv = sb_challenge(seed, round, i, j, q);
-      sch[0] = cv;
-      sch[1] = shoup_dev(cv, q);
-    }
-    __syncthreads();
-    const u64 c = sch[0], cp = sch[1];
-    for (u64 e = threadIdx.x; e < h; e += blockDim.x) v[e] = fold1(v[e], v[e + h], c, cp, q);
-    __syncthreads();
-    cur = h;
-    j++;
+    u32 T = 63u - (u32)__clzll((long long)cur);
+    T = T < SC_T ? T : SC_T;
+    tail_steps<LAZY>(T, v, cur, M, ch + j, [&](u32 t) { return sums + ((u64)i * nrmax + j + t) * 3; }, red);
+    cur >>= T;
+    j += T;
   }
-}
-
-// polys: instance i's nr_i x 3 block starts at offs[i] * 3
-__global__ void sb_finalize_kernel(const u64* sums, const u32* nrs, const u64* offs, u32 ninst, u32 nrmax, u64 q,
-                                   u64* claims, u64* polys) {
-  const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (u64)ninst * nrmax) return;
-  const u32 i = (u32)(t / nrmax), j = (u32)(t % nrmax);
-  if (j >= nrs[i]) return;
-  const u64* s = sums + t * 3;
-  const u64 s00 = s[0] % q, s01 = s[1] % q, s11 = s[2] % q;
-  u64* o = polys + (offs[i] + j) * 3;
-  o[0] = s00;
-  o[1] = sub_mod(s01, s00, q);
-  o[2] = add_mod(sub_mod(sub_mod(s11, s01, q), s01, q), s00, q);
-  if (j == 0) claims[i] = add_mod(s00, s11, q);
+  __syncthreads();
+  // instance i's polynomials start at offs[i] * 3
+  for (u32 t = threadIdx.x; t < nr; t += blockDim.x)
+    sc_poly(sums + ((u64)i * nrmax + t) * 3, q, polys + (offs[i] + t) * 3, t == 0 ? claims + i : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -815,9 +859,20 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   } guard{nullptr, st};
   // one allocation: sums | descriptors | nrs | offs | the two areas
   auto up = [](u64 b) { return (b + 255) / 256 * 256; };
-  const u64 sum_b = up((u64)count * nrmax * 3 * 8), desc_b = up(desc_bytes), nr_b = up(count * 4), off_b = up(count * 8);
+  // levels on the tensor cores where the modulus allows (their vectors, longer
+  // than SC_TAIL, are whole tiles); their Gram matrices lie behind the sums
+  const bool tc = gram_words_ok(2 * SC_TAIL, M.q);
+  u64 glev = 0;
+  if (tc)
+    for (u32 i = 0; i < count; i++) {
+      u64 n = 0;
+      for (u64 L = lens[i]; L > SC_TAIL; L /= 16) n++;
+      glev = n > glev ? n : glev;
+    }
+  const u64 gram_b = up(glev * SB_MAX_INST * 256 * 8);
+  const u64 sum_b = up((u64)count * nrmax * 3 * 8) + gram_b, desc_b = up(desc_bytes), off_b = up(count * 8);
   {
-    cudaError_t ea = salsaa_scratch_alloc(&guard.p, sum_b + desc_b + nr_b + off_b + up(tot_a * 8) + tot_b * 8 + 256, st);
+    cudaError_t ea = salsaa_scratch_alloc(&guard.p, sum_b + desc_b + off_b + up(tot_a * 8) + tot_b * 8 + 256, st);
     if (ea != cudaSuccess) {
       guard.p = nullptr;
       return salsaa_set_cuda_error(ea, "sumcheck_batch: workspace");
@@ -826,11 +881,11 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   char* base = (char*)guard.p;
   u64* sums = (u64*)base;
   SbInst* ddesc = (SbInst*)(base + sum_b);
-  u32* dnrs = (u32*)(base + sum_b + desc_b);
-  u64* doffs = (u64*)(base + sum_b + desc_b + nr_b);
-  u64* bufa = (u64*)(base + sum_b + desc_b + nr_b + off_b);
+  u64* doffs = (u64*)(base + sum_b + desc_b);
+  u64* bufa = (u64*)(base + sum_b + desc_b + off_b);
   u64* bufb = (u64*)((char*)bufa + up(tot_a * 8));
-  cudaError_t e = cudaMemsetAsync(sums, 0, (u64)count * nrmax * 3 * 8, st);
+  u64* gram = (u64*)(base + sum_b - gram_b);
+  cudaError_t e = cudaMemsetAsync(sums, 0, sum_b, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: memset");
   // host plan: per level, the instances still longer than SC_TAIL, then the tail
   std::vector<SbInst> plan((maxlev + 1) * SB_MAX_INST);
@@ -885,12 +940,17 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     tail_max = cur_L[i] > tail_max ? cur_L[i] : tail_max;
   }
   e = cudaMemcpyAsync(ddesc, plan.data(), desc_bytes, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dnrs, nrs.data(), count * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(doffs, offs.data(), count * 8, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: plan");
   // (from pageable memory the copies are staged before cudaMemcpyAsync returns)
   for (u32 lev = 0; lev < nlev; lev++) {
     const u64 grid = lev_tiles[lev] < 296 ? lev_tiles[lev] : 296;
+    if (tc) {
+      if ((rc = launch_gram_batch(ddesc + lev * SB_MAX_INST, lev_n[lev], lev_tiles[lev], M, seed, round,
+                                  gram + (u64)lev * SB_MAX_INST * 256, st)))
+        return rc;
+      continue;
+    }
     if (lazy)
       sb_pass_kernel<true><<<(unsigned)grid, 256, 0, st>>>(ddesc + lev * SB_MAX_INST, lev_n[lev], lev_tiles[lev],
                                                             M, seed, round, sums, nrmax, plain);
@@ -905,35 +965,17 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     e = cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: tail smem");
   }
-  tail<<<count, 1024, smem, st>>>(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax);
-  if ((rc = check_launch("sb_tail"))) return rc;
-  const u64 tot = (u64)count * nrmax;
-  sb_finalize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(sums, dnrs, doffs, count, nrmax, M.q, claims,
-                                                                   polys);
-  return check_launch("sb_finalize");
+  tail<<<count, 1024, smem, st>>>(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
+                                   claims, polys);
+  return check_launch("sb_tail");
 }
 
-// Round polynomials and claims from the raw sums, canonical mod q.// Round polynomials and claims from the raw sums, canonical mod q.
-__global__ void sc_finalize_kernel(const u64* sums, u32 rows, u32 nr, u64 q, u64* claims, u64* polys0,
-                                   u64* polys1) {
-  u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2ULL * nr * rows) return;
-  const u32 rep = (u32)(t / ((u64)nr * rows));
-  const u64 jk = t % ((u64)nr * rows);
-  const u64* s = sums + t * 3;
-  const u64 s00 = s[0] % q, s01 = s[1] % q, s11 = s[2] % q;
-  const u64 f0 = s00, f1 = sub_mod(s01, s00, q);
-  const u64 f2 = add_mod(sub_mod(sub_mod(s11, s01, q), s01, q), s00, q);
-  u64* o = (rep ? polys1 : polys0) + jk * 3;
-  o[0] = f0;
-  o[1] = f1;
-  o[2] = f2;
-  if (rep == 0 && jk < rows) claims[jk] = add_mod(s00, s11, q);  // round 0: sum of squares
-}
+constexpr u64 SC_GRAM_TILES = 296;
 
 template <bool LAZY>
 static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
-                           SumcheckBufs B, u32 nr, bool plain, cudaStream_t st) {
+                           SumcheckBufs B, u32 nr, bool plain, cudaStream_t st, const C8Rows* w8, const u32* wide,
+                           u64* claims, u64* polys0, u64* polys1) {
   const u64 sa = nlen >> SC_T, sb = nlen >> (2 * SC_T);  // strides: a pass divides the length by 16
   u64 L = nlen;
   u32 j = 0;
@@ -948,18 +990,31 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     return (unsigned)(g < want ? (g ? g : 1) : want);
   };
   auto pass_ok = [d](u64 len) { return len > SC_TAIL_ONE && (len >> SC_T) >= d; };
+  GramList gl{};
+  u64 go = 2ULL * nr * rows * 3;  // words used behind the sums
+  auto gram_room = [&](u32 n) { return gl.n < SC_GRAM_PASSES && go + (u64)n * 256 <= B.sums_words; };
+  auto gram_take = [&](u32 n, u32 shared) {
+    u64* g = B.sums + go;
+    gl.c[gl.n] = g;
+    gl.j[gl.n] = j;
+    gl.shared[gl.n++] = shared;
+    go += (u64)n * 256;
+    return g;
+  };
   if (pass_ok(L)) {
-    // rounds 0..3 on the tensor cores when the shapes allow; the CUDA-core
-    // pass then runs only if a witness value did not fit the byte limbs
-    const bool tc = B.gram && nc_gram_ok(w, rows, L, M.q);
-    const u32* flag = tc ? (const u32*)(B.gram + (u64)rows * 256) : nullptr;
+    // on the tensor cores where modulus and length allow: the byte rows, or
+    // (gated on their flag) the words
     int rc = 0;
-    if (tc && (rc = launch_nc_gram(w, rows, L, M, ds, round, B.a, sa, B.gram, plain, st))) return rc;
-    dim3 g(2 * grid_for(L / (1u << SC_T), 2 * rows), rows);
-    sc_first_kernel<LAZY><<<g, 256, 0, st>>>(w, rows, L, M, ds, round, B.a, sa, B.sums, nr, plain, flag);
-    rc = check_launch("sc_first");
-    if (rc) return rc;
-    if (tc && (rc = launch_nc_gram_sums(B.gram, rows, M, ds, round, B.sums, nr, plain, st))) return rc;
+    if (gram_room(rows) && gram_words_ok(L, M.q)) {
+      u64* g = gram_take(rows, 1);
+      const bool c8 = w8 && wide && gram_c8_ok(*w8, d, M.q);
+      if (c8 && (rc = launch_gram_c8(*w8, d, M, ds, round, B.a, sa, g, wide, st))) return rc;
+      if ((rc = launch_gram_first(w, rows, L, M, ds, round, B.a, sa, g, c8 ? wide : nullptr, st))) return rc;
+    } else {
+      dim3 g(2 * grid_for(L / (1u << SC_T), 2 * rows), rows);
+      sc_first_kernel<LAZY><<<g, 256, 0, st>>>(w, rows, L, M, ds, round, B.a, sa, B.sums, nr, plain);
+      if ((rc = check_launch("sc_first"))) return rc;
+    }
     in = B.a;
     sin = sa;
     to_a = false;
@@ -968,10 +1023,15 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     while (pass_ok(L)) {
       u64* out = to_a ? B.a : B.b;
       const u64 so = to_a ? sa : sb;
-      dim3 gr(grid_for(L / (1u << SC_T), 2 * rows), 2 * rows);
-      sc_round_kernel<LAZY><<<gr, 256, 0, st>>>(in, sin, out, so, L, rows, M, ds, round, j, B.sums, nr, plain);
-      rc = check_launch("sc_round");
-      if (rc) return rc;
+      // a tile per CTA at least (16 us against 20 for 512 tiles); with fewer the
+      // CUDA cores' 8 us are what a tensor-core pass and its sums take to start
+      if (gl.n && gram_room(2 * rows) && gram_words_ok(L, M.q) && L / 16 / GRAM_TILE * 2 * rows >= SC_GRAM_TILES) {
+        if ((rc = launch_gram_round(in, sin, out, so, L, rows, M, ds, round, j, gram_take(2 * rows, 0), st))) return rc;
+      } else {
+        dim3 gr(grid_for(L / (1u << SC_T), 2 * rows), 2 * rows);
+        sc_round_kernel<LAZY><<<gr, 256, 0, st>>>(in, sin, out, so, L, rows, M, ds, round, j, B.sums, nr, plain);
+        if ((rc = check_launch("sc_round"))) return rc;
+      }
       in = out;
       sin = so;
       to_a = !to_a;
@@ -985,12 +1045,14 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tail smem attribute");
   }
-  kern<<<2 * rows, 512, smem, st>>>(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap);
+  kern<<<2 * rows, 512, smem, st>>>(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
+                                        claims, polys0, polys1);
   return check_launch("sc_tail");
 }
 
 int launch_sumcheck(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
-                    SumcheckBufs B, u64* proof_claims, u64* proof_rep0, u64* proof_rep1, cudaStream_t st) {
+                    SumcheckBufs B, u64* proof_claims, u64* proof_rep0, u64* proof_rep1, cudaStream_t st,
+                    const C8Rows* w8, const u32* wide) {
   if (nlen < 4 || (nlen & (nlen - 1)) || rows == 0 || rows > MAX_WROWS || nlen < d)
     return salsaa_set_error(-2, "sumcheck: bad shape");
   const u32 nr = 63u - (u32)__builtin_clzll(nlen);
@@ -998,15 +1060,16 @@ int launch_sumcheck(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const De
   // the lazy per-thread / per-block sums stay far below 2^128; with fewer than
   // 2^13 contributions per address the plain 64-bit atomics cannot overflow
   const bool plain = lazy;
-  cudaError_t e = cudaMemsetAsync(B.sums, 0, 2ULL * nr * rows * 3 * sizeof(u64), st);
+  // the Gram matrices lie behind the sums
+  const u64 used = 2ULL * nr * rows * 3, full = used + gram_words(rows);
+  cudaError_t e = cudaMemsetAsync(B.sums, 0, (full < B.sums_words ? full : B.sums_words) * sizeof(u64), st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck memset");
-  int rc = lazy ? sumcheck_passes<true>(w, rows, nlen, d, M, ds, round, B, nr, plain, st)
-                : sumcheck_passes<false>(w, rows, nlen, d, M, ds, round, B, nr, plain, st);
+  int rc = lazy ? sumcheck_passes<true>(w, rows, nlen, d, M, ds, round, B, nr, plain, st, w8, wide, proof_claims, proof_rep0,
+                                      proof_rep1)
+                : sumcheck_passes<false>(w, rows, nlen, d, M, ds, round, B, nr, plain, st, w8, wide, proof_claims, proof_rep0,
+                                      proof_rep1);
   if (rc) return rc;
-  u64 tot = 2ULL * nr * rows;
-  sc_finalize_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(B.sums, rows, nr, M.q, proof_claims,
-                                                                    proof_rep0, proof_rep1);
-  return check_launch("sc_finalize");
+  return 0;
 }
 
 // ---------------------------------------------------------------------------

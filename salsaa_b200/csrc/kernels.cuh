@@ -118,16 +118,6 @@ int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cu
 int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_lo,
                    const u64* s_hi, const ModQ& M, u64* acc, bool plain, const uint8_t* img, const ScGates& gates,
                    cudaStream_t st);
-// First sumcheck pass (rounds 0..3 of both repetitions) on tcgen05 through the
-// Gram matrices of 16-element groups (see ck_umma.cu): launch_nc_gram writes
-// the folded vectors and the Gram matrices, or raises the flag word after them
-// when a value does not fit four signed byte limbs; launch_nc_gram_sums adds
-// the round sums unless the flag is raised.
-bool nc_gram_ok(const RowSet& w, u32 rows, u64 nlen, u64 q);
-int launch_nc_gram(const RowSet& w, u32 rows, u64 nlen, const ModQ& M, const DevState* ds, u32 round, u64* out,
-                   u64 sout, u64* gram, bool plain, cudaStream_t st);
-int launch_nc_gram_sums(const u64* gram, u32 rows, const ModQ& M, const DevState* ds, u32 round, u64* sums, u32 nr,
-                        bool plain, cudaStream_t st);
 // Nonzero (and the last error set) when a tensor-core kernel's bounded wait gave up.
 int tc_error_check();
 // The current device's error word of the tensor-core kernels (null if unavailable).
@@ -143,12 +133,17 @@ int launch_pointwise_mul(u64* r, const u64* b, u64 n, u64 q, cudaStream_t st);
 struct SumcheckBufs {
   u64* a;     // 2 * rows * nlen/16
   u64* b;     // 2 * rows * nlen/256
-  u64* sums;  // 2 * nr * rows * 3 (zeroed by the launcher)
+  u64* sums;  // 2 * nr * rows * 3 words and, for tensor-core passes, Gram matrices
+              // behind them (gram_words(rows) for all); zeroed by the launcher
+  u64 sums_words;
   u64* cap;   // 2 * rows * d: vector after log2(width) rounds
-  u64* gram;  // rows * 256 + 1 (Gram matrices and a flag word) or null: first pass on tcgen05
 };
+constexpr u32 SC_GRAM_PASSES = 3;  // the first pass and up to two long later ones
+inline u64 gram_words(u64 rows) { return rows * 256 * (1 + 2 * (SC_GRAM_PASSES - 1)); }
+// w8 and wide (optional): the rows as byte tiles, valid while *wide is zero.
 int launch_sumcheck(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
-                    SumcheckBufs B, u64* proof_claims, u64* proof_rep0, u64* proof_rep1, cudaStream_t st);
+                    SumcheckBufs B, u64* proof_claims, u64* proof_rep0, u64* proof_rep1, cudaStream_t st,
+                    const struct C8Rows* w8 = nullptr, const u32* wide = nullptr);
 // Independent sumchecks of `count` <= 64 vectors of power-of-two lengths (one
 // repetition each; instance i uses the norm-check challenges of (round, i)):
 // claims[i] and the round polynomials of instance i at polys + 3 * sum_{i'<i} log2 len.

@@ -559,9 +559,9 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (S.use_short && (rc = m.alloc(&pr->tz, fold_tz_bytes(8, (u32)d), "fold challenge blocks"))) ||
       (rc = m.alloc(&pr->sc.a, S.max_nc_rows_width * d / 8 + 1, "sumcheck a")) ||
       (rc = m.alloc(&pr->sc.b, S.max_nc_rows_width * d / 128 + 1, "sumcheck b")) ||
-      (rc = m.alloc(&pr->sc.sums, 2ULL * 64 * MAX_WROWS * 3, "sumcheck sums")) ||
+      (rc = m.alloc(&pr->sc.sums, pr->sc.sums_words = 2ULL * 64 * MAX_WROWS * 3 + MAX_WROWS * 256 + 1,
+                    "sumcheck sums and Gram matrices")) ||
       (rc = m.alloc(&pr->sc.cap, 2ULL * MAX_WROWS * d, "sumcheck cap")) ||
-      (rc = m.alloc(&pr->sc.gram, (u64)MAX_WROWS * 256 + 1, "sumcheck gram")) ||
       (rc = m.alloc(&pr->row_base, (u64)S.nsc_total * d + 1, "row bases")) ||
       (rc = m.alloc(&pr->row_cj, (c->P.nof_rounds + 1) * (u64)CK_BLOCK, "row cj")) ||
       (rc = m.alloc(&pr->pmask, 256ULL * CK_BLOCK / 32, "pos mask")) ||
@@ -1014,7 +1014,9 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     u64* polys1 = rhs0 + (u64)K * d;
     u64* rhs1 = polys1 + nr * K * 3;
     cur = (u64)(rhs1 + (u64)K * d - proof);
-    TRY(launch_sumcheck(Wc, K, width * d, d, M, pr->ds, rd, pr->sc, claims, polys0, polys1, st));
+    const C8Rows n8 = c8_rows(pr->c8, K, width, d, false);
+    TRY(launch_sumcheck(Wc, K, width * d, d, M, pr->ds, rd, pr->sc, claims, polys0, polys1, st, sh ? &n8 : nullptr,
+                        &pr->ds->wide[rd]));
     TRY(mark(pr, PH_NORM3));
     TRY(launch_norm3(pr->sc.cap, K, (u32)nr, T, M, pr->ds, rd, rhs0, rhs1, pr->row_base + (u64)nsc * d,
                      pr->row_base + (u64)(nsc + 1) * d, st));
@@ -2102,9 +2104,8 @@ extern "C" int salsaa_sumcheck(const uint64_t* d_w, uint64_t rows, uint64_t n, u
   DevState* ds;
   t.want(&B.a, rows * n / 8);
   t.want(&B.b, rows * n / 128);
-  t.want(&B.sums, 2ULL * 64 * rows * 3);
+  t.want(&B.sums, B.sums_words = 2ULL * 64 * rows * 3 + gram_words(rows));
   t.want(&B.cap, 2ULL * rows * d);
-  t.want(&B.gram, rows * 256 + 1);
   t.want(&ds, 1);
   TRY(t.alloc());
   set_seed_kernel<<<1, 32, 0, st>>>(ds, seed);
