@@ -136,6 +136,7 @@ template <u32 E, u32 PAIRS>
 __global__ void __launch_bounds__(CKI_THREADS, 1)
     ck_img_kernel(const uint8_t* __restrict__ tk8, CkImage im, CkImgTiles t, u32 nck, u32 nkp, u32 nkc,
                   const u64* thi, u32 nhi_t, ModQ M, const u64* zeta, u64* acc, bool plain, u32* err) {
+  pdl_wait();
   // finishing tasks per thread: 4 lanes per (virtual row, key row)
   constexpr u32 NIT = (CKI_MAX_V * 4 * PAIRS * 4 + CKI_EPI - 1) / CKI_EPI;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -398,7 +399,7 @@ int launch_ck_img(const CkImgArgs& a, const CkImage& im, const ModQ& M, const u6
   salsaa_trace_alias(tr, "ck_umma_kernel:int8", 2.0 * 196.0 * a.nck * im.R * (double)im.width * im.n);
   salsaa_trace_alias(tr, "ck_umma_kernel:mac", (double)a.nck * im.R * (double)im.width * 2 * im.n);
   const u32 grid = t.ntiles < 148 ? t.ntiles : 148;
-  kern<<<grid, CKI_THREADS, smem, st>>>(a.tk8, im, t, a.nck, nkp, nkc, a.thi, a.ck_nhi, M, zeta, a.acc,
+  pdl(kern, grid, CKI_THREADS, smem, st)(a.tk8, im, t, a.nck, nkp, nkc, a.thi, a.ck_nhi, M, zeta, a.acc,
                                                  plain, tc_error_word());
   salsaa_trace_end(tr, st);
   salsaa_count_launch();

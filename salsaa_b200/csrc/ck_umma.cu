@@ -18,6 +18,7 @@ namespace {
 // MMAs are issued by one thread, and the accumulator is read back from TMEM.
 __global__ void __launch_bounds__(128) umma_selftest_kernel(const uint8_t* A, const uint8_t* B, u32 N, u32 K,
                                                             int32_t* out, u32* err) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
@@ -107,6 +108,7 @@ constexpr u32 CKU_CONV = 448;  // witness-converting threads (warps 0..13); warp
 constexpr u32 CKU_ATILE = 128 * CKU_CHUNK;  // witness byte tile of one slot
 
 __global__ void ck_tk8_kernel(const u64* tlo, u32 nck, u32 n, u32 bt, u32 nkp, bool packed, uint8_t* tk8) {
+  pdl_wait();
   const u64 tot = (u64)bt * n * nkp;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 b = (u32)(t % 16);
@@ -370,6 +372,7 @@ __device__ __forceinline__ void ck_umma_body(const uint8_t* __restrict__ tk8, co
 __global__ void __launch_bounds__(CKU_THREADS, 1)
     ck_umma_kernel(const uint8_t* __restrict__ tk8, RowSet w, u32 rows, u32 G, u32 nck, u32 nkp, u32 n, u32 bt,
                    u32 Bw, const u64* thi, u32 nhi_t, ModQ M, const u64* zeta, u64* acc, bool plain) {
+  pdl_wait();
   ck_umma_body(tk8, w, rows, G, nck, nkp, n, bt, Bw, thi, nhi_t, M, zeta, acc, rows, 0, plain, blockIdx.y);
 }
 
@@ -388,6 +391,7 @@ struct CkMulti {
 __global__ void __launch_bounds__(CKU_THREADS, 1)
     ck_umma_multi_kernel(const uint8_t* __restrict__ tk8, CkMulti m, u32 nck, u32 nkp, u32 n, u32 bt,
                          const u64* thi, u32 nhi_t, ModQ M, const u64* zeta) {
+  pdl_wait();
   u32 i = 0;
   while (i + 1 < m.count && m.ystart[i + 1] <= blockIdx.y) i++;
   ck_umma_body(tk8, m.w[i], m.rows[i], m.G[i], nck, nkp, n, bt, m.Bw[i], thi, nhi_t, M, zeta, m.acc[i], m.rows[i],
@@ -403,7 +407,7 @@ int launch_ck_tk8(const u64* tlo, u32 nck, u32 n, u32 bt, bool packed, uint8_t* 
   const u64 tot = (u64)bt * n * nkp;
   u64 g = (tot + 255) / 256;
   if (g > 65535 * 16) g = 65535 * 16;
-  ck_tk8_kernel<<<(unsigned)g, 256, 0, st>>>(tlo, nck, n, bt, nkp, packed, tk8);
+  pdl(ck_tk8_kernel, (unsigned)g, 256, 0, st)(tlo, nck, n, bt, nkp, packed, tk8);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "ck_tk8");
@@ -484,7 +488,7 @@ int launch_ck_umma_multi(const CommitArgs* a, u32 ninst, u32 n, const ModQ& M, c
   const int tr = salsaa_trace_begin("ck_umma_kernel", st, wit_bytes + out_bytes);
   salsaa_trace_alias(tr, "ck_umma_kernel:int8", ops);
   salsaa_trace_alias(tr, "ck_umma_kernel:mac", macs);
-  ck_umma_multi_kernel<<<dim3(n / 2, y), CKU_THREADS, smem, st>>>(a[0].tk8, m, nck, nkp, n, a[0].ck_bt, a[0].thi,
+  pdl(ck_umma_multi_kernel, dim3(n / 2, y), CKU_THREADS, smem, st)(a[0].tk8, m, nck, nkp, n, a[0].ck_bt, a[0].thi,
                                                                    a[0].ck_nhi, M, zeta);
   salsaa_trace_end(tr, st);
   salsaa_count_launch();
@@ -516,7 +520,7 @@ int launch_ck_umma(const CommitArgs& a, u32 n, u32 Bw, u32 G, const ModQ& M, con
   const int tr = salsaa_trace_begin("ck_umma_kernel", st, wit_bytes + out_bytes);
   salsaa_trace_alias(tr, "ck_umma_kernel:int8", 2.0 * 196.0 * a.nck * a.rows * (double)a.width * n);
   salsaa_trace_alias(tr, "ck_umma_kernel:mac", (double)a.nck * a.rows * (double)a.width * 2 * n);
-  ck_umma_kernel<<<g, CKU_THREADS, smem, st>>>(a.tk8, a.w, a.rows, G, a.nck, nkp, n, a.ck_bt, Bw, a.thi, a.ck_nhi,
+  pdl(ck_umma_kernel, g, CKU_THREADS, smem, st)(a.tk8, a.w, a.rows, G, a.nck, nkp, n, a.ck_bt, Bw, a.thi, a.ck_nhi,
                                                M, zeta, a.acc, plain);
   salsaa_trace_end(tr, st);
   salsaa_count_launch();
@@ -545,6 +549,7 @@ constexpr u32 PU_STAGE = PU_A + PU_B;
 __global__ void __launch_bounds__(256, 2)
     project_umma_kernel(RowSet in, u32 d, u64 q, u32 cw, u64 nch, const int8_t* __restrict__ Jc,
                         u64* __restrict__ out, u64* flag, const u32* gate) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[2], done_bar[2];
   __shared__ uint32_t tslot;
@@ -683,7 +688,7 @@ int launch_project_umma(RowSet in, u32 rows, u64 nch, u32 d, u64 q, u32 cw, cons
   cudaError_t e = cudaFuncSetAttribute(project_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project_umma smem attribute");
   dim3 g(d / PU_POS, (unsigned)(rows * nch));
-  project_umma_kernel<<<g, 256, smem, st>>>(in, d, q, cw, nch, Jc, out, flag, gate);
+  pdl(project_umma_kernel, g, 256, smem, st)(in, d, q, cw, nch, Jc, out, flag, gate);
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "project_umma launch");
@@ -709,6 +714,7 @@ constexpr u32 SU_B = SU_POS * SU_KS;                // one limb tile (16 KiB)
 constexpr u32 SU_STAGE = SU_A + SU_LIMBS * SU_B;    // 64 KiB
 
 __global__ void sc_img_kernel(const u64* s_lo, u32 Bw, ScRowList tl, uint8_t* img) {
+  pdl_wait();
   const u64 tot = (u64)Bw * 128;  // (chunk, slice, row, byte) = Bw / 128 x 8 x 128 x 16
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 b = (u32)(t % 16), row = (u32)((t / 16) % 128), sl = (u32)((t / 2048) % 8), cc = (u32)(t / 16384);
@@ -725,6 +731,7 @@ __global__ void __launch_bounds__(512, 1)
     sc_umma_kernel(RowSet wc, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl,
                    const uint8_t* __restrict__ img0, const u64* s_lo, const u64* s_hi, ModQ M, u64* acc, bool plain,
                    ScGates gates) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[2], done_bar[2];
   __shared__ uint32_t tslot;
@@ -907,7 +914,7 @@ __global__ void __launch_bounds__(512, 1)
 
 int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cudaStream_t st) {
   const u64 g = ((u64)Bw * 128 + 255) / 256;
-  sc_img_kernel<<<(unsigned)(g < 4096 ? g : 4096), 256, 0, st>>>(s_lo, Bw, tl, img);
+  pdl(sc_img_kernel, (unsigned)(g < 4096 ? g : 4096), 256, 0, st)(s_lo, Bw, tl, img);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_img launch");
@@ -926,7 +933,7 @@ int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScR
   const size_t smem = 2 * (size_t)SU_STAGE;
   cudaError_t e = cudaFuncSetAttribute(sc_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_umma smem attribute");
-  sc_umma_kernel<<<(unsigned)(items < 148 ? items : 148), 512, smem, st>>>(wc, rows, d, Bw, nhi, split, tl, img, s_lo,
+  pdl(sc_umma_kernel, (unsigned)(items < 148 ? items : 148), 512, smem, st)(wc, rows, d, Bw, nhi, split, tl, img, s_lo,
                                                                            s_hi, M, acc, plain, gates);
   salsaa_count_launch();
   e = cudaGetLastError();
@@ -968,7 +975,7 @@ extern "C" int salsaa_selftest_umma_i8(const uint8_t* d_a, const uint8_t* d_b, u
   const size_t smem = (size_t)(128 + n) * k;
   e = cudaFuncSetAttribute(umma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) {
-    umma_selftest_kernel<<<1, 128, smem, st>>>(d_a, d_b, n, k, d_out, err);
+    pdl(umma_selftest_kernel, 1, 128, smem, st)(d_a, d_b, n, k, d_out, err);
     salsaa_count_launch();
     e = cudaGetLastError();
   }

@@ -35,6 +35,7 @@ constexpr u32 DENSE_GROUP = CKU_MAX_WROWS;
 
 __global__ void dense_tables_kernel(const u64* a_slot, u32 nrows, u64 m, u32 n, ModQ M, const u64* zeta,
                                     bool packed, u64* tlo, u64* thi) {
+  pdl_wait();
   const u64 tot = (u64)nrows * m * n;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 s = (u32)(t % n);
@@ -101,7 +102,7 @@ extern "C" int salsaa_dense_key_create(const uint64_t* d_a, uint64_t nrows, uint
   const bool packed = q < (1ULL << 50);
   u64 tot = nrows * m * (d / 2), g = (tot + 255) / 256;
   if (g > 65535ull * 16) g = 65535ull * 16;
-  dense_tables_kernel<<<(unsigned)g, 256, 0, st>>>(a_slot, (u32)nrows, m, (u32)(d / 2), k->M, T->zeta, packed,
+  pdl(dense_tables_kernel, (unsigned)g, 256, 0, st)(a_slot, (u32)nrows, m, (u32)(d / 2), k->M, T->zeta, packed,
                                                     k->tlo, k->thi);
   salsaa_count_launch();
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "dense_key_create: tables");

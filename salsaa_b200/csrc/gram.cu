@@ -65,6 +65,7 @@ enum GwMode { GW_FIRST, GW_ROUND, GW_BATCH };
 
 template <int MODE>
 __global__ void __launch_bounds__(GR_THREADS, 2) gram_words_kernel(const __grid_constant__ GwArgs a, ModQ M, u32* err) {
+  pdl_wait();
   constexpr u32 REPS = MODE == GW_FIRST ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t full_bar, done_bar;
@@ -287,7 +288,7 @@ int gw_launch(GwArgs& a, const ModQ& M, cudaStream_t st) {
   a.plain = M.q < (1ULL << 50) && a.ntiles / GW_SEG + grid + SB_MAX_INST < (1u << 13);
   cudaError_t e = cudaFuncSetAttribute(gram_words_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GW_SMEM);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "gram_words smem attribute");
-  gram_words_kernel<MODE><<<grid, GR_THREADS, GW_SMEM, st>>>(a, M, tc_error_word());
+  pdl(gram_words_kernel<MODE>, grid, GR_THREADS, GW_SMEM, st)(a, M, tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "gram_words launch");
@@ -314,6 +315,7 @@ constexpr u32 GC_MAX = 1000;  // steps a CTA: 128^2 x 128 x 1000 < 2^31
 __global__ void __launch_bounds__(GR_THREADS, 2)
     gram_c8_kernel(C8Rows w, u32 d, ModQ M, const DevState* ds, u32 round, u64* out, u64 sout, u64* gram,
                    const u32* wide, u64 w32p, bool plain, u32* err) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar, done_bar;
   __shared__ uint32_t tslot;
@@ -516,7 +518,7 @@ int launch_gram_c8(const C8Rows& w, u32 d, const ModQ& M, const DevState* ds, u3
   if (nb > steps) nb = steps;
   const u64 w32p = (u64)(((unsigned __int128)(((u64)1 << 32) % M.q) << 64) / M.q);
   const bool plain = M.q < (1ULL << 50) && nb < (1u << 13);
-  gram_c8_kernel<<<dim3(nb, w.rows), GR_THREADS, GC_SMEM, st>>>(w, d, M, ds, round, out, sout, gram, wide, w32p, plain,
+  pdl(gram_c8_kernel, dim3(nb, w.rows), GR_THREADS, GC_SMEM, st)(w, d, M, ds, round, out, sout, gram, wide, w32p, plain,
                                                                 tc_error_word());
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();

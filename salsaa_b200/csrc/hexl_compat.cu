@@ -97,6 +97,7 @@ enum EwOp { EW_MUL, EW_ADD, EW_SUB, EW_FMA, EW_RED };
 
 __global__ void eltwise_kernel(int op, uint64_t* r, const uint64_t* a, const uint64_t* b, uint64_t s, uint64_t n,
                                ModQ M) {
+  pdl_wait();
   const uint64_t q = M.q;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t x = a[i] % q;
@@ -113,11 +114,13 @@ __global__ void eltwise_kernel(int op, uint64_t* r, const uint64_t* a, const uin
 }
 
 __global__ void pointwise_mul_kernel(uint64_t* a, const uint64_t* b, uint64_t n, ModQ M) {
+  pdl_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     a[i] = mul_mod(M, a[i], b[i]);
 }
 
 __global__ void sum_kernel(const uint64_t* a, uint64_t n, ModQ M, int square, uint64_t* out) {
+  pdl_wait();
   __shared__ uint64_t sm[32];
   const uint64_t q = M.q;
   uint64_t acc = 0;
@@ -160,7 +163,7 @@ void run_eltwise(int op, uint64_t* r, const uint64_t* a, const uint64_t* b, uint
   if (b) cudaMemcpyAsync(db, b, n * 8, cudaMemcpyHostToDevice, st);
   unsigned g = (unsigned)((n + 255) / 256);
   if (g > 4096) g = 4096;
-  eltwise_kernel<<<g, 256, 0, st>>>(op, dr, da, b ? db : da, s, n, make_modq(q));
+  pdl(eltwise_kernel, g, 256, 0, st)(op, dr, da, b ? db : da, s, n, make_modq(q));
   cudaMemcpyAsync(r, dr, n * 8, cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) salsaa_set_cuda_error(e, "eltwise");
@@ -179,7 +182,7 @@ uint64_t run_sum(const uint64_t* a, uint64_t n, uint64_t q, int square) {
   cudaMemsetAsync(d + n, 0, 8, st);
   unsigned g = (unsigned)((n + 255) / 256);
   if (g > 1024) g = 1024;
-  sum_kernel<<<g, 256, 0, st>>>(d, n, make_modq(q), square, d + n);
+  pdl(sum_kernel, g, 256, 0, st)(d, n, make_modq(q), square, d + n);
   uint64_t out = 0;
   cudaMemcpyAsync(&out, d + n, 8, cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);
@@ -222,10 +225,10 @@ void run_poly_mul(uint64_t* r, const uint64_t* a, const uint64_t* b, uint64_t n,
   uint64_t *da = d, *db = d + n;
   cudaMemcpyAsync(da, a, n * 8, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(db, b, n * 8, cudaMemcpyHostToDevice, st);
-  eltwise_kernel<<<1, 256, 0, st>>>(EW_RED, da, da, da, 0, n, M);
-  eltwise_kernel<<<1, 256, 0, st>>>(EW_RED, db, db, db, 0, n, M);
+  pdl(eltwise_kernel, 1, 256, 0, st)(EW_RED, da, da, da, 0, n, M);
+  pdl(eltwise_kernel, 1, 256, 0, st)(EW_RED, db, db, db, 0, n, M);
   if (ntt_launch(da, da, 1, *T, false, false, st) || ntt_launch(db, db, 1, *T, false, false, st)) return;
-  pointwise_mul_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(da, db, n, M);
+  pdl(pointwise_mul_kernel, (unsigned)((n + 255) / 256), 256, 0, st)(da, db, n, M);
   if (ntt_launch(da, da, 1, *T, false, true, st)) return;
   cudaMemcpyAsync(r, da, n * 8, cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);

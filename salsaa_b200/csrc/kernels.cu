@@ -46,6 +46,7 @@ __device__ __forceinline__ u64 nc_challenge(const DevState* ds, u32 round, u32 r
 // so that m^(i+1) = thi[i / B] * tlo[i % B].
 // ---------------------------------------------------------------------------
 __global__ void gen_crs_kernel(u64* m, u32 rows, u32 d, u64 q, u64 crs_seed) {
+  pdl_wait();
   u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (u64)rows * d) return;
   u32 r = (u32)(t / d), i = (u32)(t % d);
@@ -54,7 +55,7 @@ __global__ void gen_crs_kernel(u64* m, u32 rows, u32 d, u64 q, u64 crs_seed) {
 
 int launch_gen_crs(u64* m_coef, u32 rows, u32 d, u64 q, u64 crs_seed, cudaStream_t st) {
   u64 tot = (u64)rows * d;
-  gen_crs_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(m_coef, rows, d, q, crs_seed);
+  pdl(gen_crs_kernel, (unsigned)((tot + 255) / 256), 256, 0, st)(m_coef, rows, d, q, crs_seed);
   return check_launch("gen_crs");
 }
 
@@ -73,6 +74,7 @@ __device__ void slot_pow(const ModQ& M, u64 z, u64 be, u64 bo, u64 e, u64& re, u
 __device__ __forceinline__ u64 pack25(u64 v) { return ((v >> 25) << 32) | (v & 0x1FFFFFFull); }
 
 __global__ void ck_tlo_kernel(const u64* ms, u32 rows, u32 n, u32 B, ModQ M, const u64* zeta, u64* tlo) {
+  pdl_wait();
   u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (u64)rows * B * n) return;
   u32 s = (u32)(t % n);
@@ -96,6 +98,7 @@ __global__ void ck_tlo_kernel(const u64* ms, u32 rows, u32 n, u32 B, ModQ M, con
 
 __global__ void ck_thi_kernel(const u64* ms, u32 rows, u32 n, u32 B, u32 nhi, ModQ M, const u64* zeta,
                               u64* thi) {
+  pdl_wait();
   u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (u64)rows * nhi * n) return;
   u32 s = (u32)(t % n);
@@ -115,11 +118,11 @@ int launch_ck_tables(const u64* m_slot, u32 rows, const NttDev& T, const ModQ& M
   const u32 B = (u32)(L < CK_KEY_BLOCK ? L : CK_KEY_BLOCK);
   const u32 nhi = (u32)(L / B);
   u64 tot = (u64)rows * B * n;
-  ck_tlo_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(m_slot, rows, n, B, M, T.zeta, tlo);
+  pdl(ck_tlo_kernel, (unsigned)((tot + 255) / 256), 256, 0, st)(m_slot, rows, n, B, M, T.zeta, tlo);
   int rc = check_launch("ck_tlo");
   if (rc) return rc;
   tot = (u64)rows * nhi * n;
-  ck_thi_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(m_slot, rows, n, B, nhi, M, T.zeta, thi);
+  pdl(ck_thi_kernel, (unsigned)((tot + 255) / 256), 256, 0, st)(m_slot, rows, n, B, nhi, M, T.zeta, thi);
   return check_launch("ck_thi");
 }
 
@@ -127,6 +130,7 @@ int launch_ck_tables(const u64* m_slot, u32 rows, const NttDev& T, const ModQ& M
 // Witness: random_bounded(2) coefficients (0 w.p. 1/2, +-1 w.p. 1/4 each).
 // ---------------------------------------------------------------------------
 __global__ void gen_witness_kernel(u64* w, u32 rows, u64 per_row, u64 q, const DevState* ds) {
+  pdl_wait();
   const u64 seed = ds->seed;
   for (u32 k = 0; k < rows; k++) {
     const u64 key = prf_key(seed, domain_id(DOM_WIT, 0, k));
@@ -140,13 +144,14 @@ __global__ void gen_witness_kernel(u64* w, u32 rows, u64 per_row, u64 q, const D
 
 int launch_gen_witness(u64* w, u32 rows, u64 width, u32 d, u64 q, const DevState* ds, cudaStream_t st) {
   const u64 per_row = width * d;
-  gen_witness_kernel<<<grid_1d(per_row, 256), 256, 0, st>>>(w, rows, per_row, q, ds);
+  pdl(gen_witness_kernel, grid_1d(per_row, 256), 256, 0, st)(w, rows, per_row, q, ds);
   return check_launch("gen_witness");
 }
 
 // Short witness sent as centred int8 coefficients: out[i] = in[i] mod q.
 // Four coefficients per thread step (one 4-byte load, two 16-byte stores).
 __global__ void expand_i8_kernel(const int8_t* __restrict__ in, u64 n, u64 q, u64* __restrict__ out) {
+  pdl_wait();
   const u64 stride = (u64)gridDim.x * blockDim.x, n4 = n / 4;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < n4; t += stride) {
     const u32 w = __ldg((const u32*)in + t);
@@ -168,27 +173,29 @@ __global__ void expand_i8_kernel(const int8_t* __restrict__ in, u64 n, u64 q, u6
 int launch_expand_i8(const int8_t* in, u64 n, u64 q, u64* out, cudaStream_t st) {
   if (!n) return 0;
   if ((uintptr_t)in % 4 || (uintptr_t)out % 16) return salsaa_set_error(-2, "expand_i8: misaligned buffers");
-  expand_i8_kernel<<<grid_1d((n + 3) / 4, 256), 256, 0, st>>>(in, n, q, out);
+  pdl(expand_i8_kernel, grid_1d((n + 3) / 4, 256), 256, 0, st)(in, n, q, out);
   return check_launch("expand_i8");
 }
 
 __global__ void fill_kernel(u64* p, u64 n, u64 v) {
+  pdl_wait();
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (u64)gridDim.x * blockDim.x) p[t] = v;
 }
 int launch_fill(u64* p, u64 n, u64 v, cudaStream_t st) {
   if (!n) return 0;
-  fill_kernel<<<grid_1d(n, 256), 256, 0, st>>>(p, n, v);
+  pdl(fill_kernel, grid_1d(n, 256), 256, 0, st)(p, n, v);
   return check_launch("fill");
 }
 
 __global__ void pointwise_mul_kernel(u64* r, const u64* b, u64 n, ModQ M) {
+  pdl_wait();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
     r[i] = mul_mod(M, r[i], b[i]);
 }
 
 int launch_pointwise_mul(u64* r, const u64* b, u64 n, u64 q, cudaStream_t st) {
   if (!n) return 0;
-  pointwise_mul_kernel<<<grid_1d(n, 256), 256, 0, st>>>(r, b, n, make_modq(q));
+  pdl(pointwise_mul_kernel, grid_1d(n, 256), 256, 0, st)(r, b, n, make_modq(q));
   return check_launch("pointwise_mul");
 }
 
@@ -338,6 +345,7 @@ template <bool LAZY>
 __global__ void __launch_bounds__(256, 2) sc_first_kernel(RowSet w, u32 rows, u64 nlen, ModQ M, const DevState* ds,
                                                           u32 round, u64* out, u64 sout, u64* sums, u32 nr,
                                                           bool plain) {
+  pdl_wait();
   constexpr u32 T = SC_T, G = 1u << T;
   __shared__ Sum128 red[SC_T * 3 * 32];
   const u32 k = blockIdx.y, rep = blockIdx.x & 1, bx = blockIdx.x >> 1, nbx = gridDim.x >> 1;
@@ -377,6 +385,7 @@ template <bool LAZY>
 __global__ void __launch_bounds__(256) sc_round_kernel(const u64* in, u64 sin, u64* out, u64 sout, u64 L, u32 rows,
                                                        ModQ M, const DevState* ds, u32 round, u32 j, u64* sums,
                                                        u32 nr, bool plain) {
+  pdl_wait();
   constexpr u32 T = SC_T, G = 1u << T;
   __shared__ Sum128 red[SC_T * 3 * 32];
   const u32 pair = blockIdx.y, rep = pair / rows, k = pair % rows;
@@ -521,6 +530,7 @@ __global__ void __launch_bounds__(512) sc_tail_kernel(const u64* in, u64 sin, Ro
                                                        const DevState* ds, u32 round, u32 j0, u64* sums, u32 nr,
                                                        u32 d, u64* cap, GramList gl, u64* claims, u64* polys0,
                                                        u64* polys1) {
+  pdl_wait();
   extern __shared__ u64 v[];
   __shared__ Sum128 red[SC_T * 3 * 32];
   __shared__ u64 ch[2 * SC_MAX_NR], C[256];
@@ -574,6 +584,7 @@ __device__ __forceinline__ u64 sb_challenge(u64 seed, u32 round, u32 inst, u64 j
 template <bool LAZY>
 __global__ void __launch_bounds__(256, 2) sb_pass_kernel(const SbInst* inst, u32 ninst, u64 ntiles, ModQ M,
                                                          u64 seed, u32 round, u64* sums, u32 nrmax, bool plain) {
+  pdl_wait();
   constexpr u32 T = SC_T, G = 1u << T;
   __shared__ Sum128 red[SC_T * 3 * 32];
   __shared__ u64 t0s[SB_MAX_INST + 1];
@@ -623,6 +634,7 @@ template <bool LAZY>
 __global__ void __launch_bounds__(1024) sb_tail_kernel(const SbInst* inst, ModQ M, u64 seed, u32 round, u64* sums,
                                                        u32 nrmax, const u64* gram, const u64* offs, u64* claims,
                                                        u64* polys) {
+  pdl_wait();
   extern __shared__ u64 v[];
   __shared__ Sum128 red[SC_T * 3 * 32];
   __shared__ u64 ch[2 * SC_MAX_NR], C[256];
@@ -685,6 +697,7 @@ __device__ __forceinline__ void qe_mul_dev(const ModQ& M, u64 s, u64 a0, u64 a1,
 
 __global__ void __launch_bounds__(256) fq2_level_kernel(Fq2Level L, ModQ M, u64 shift, u64 seed, u32 round,
                                                         u64* sums, u32 nrmax) {
+  pdl_wait();
   __shared__ u64 red[6][8];
   const u64 q = M.q;
   const u64 total = L.start[L.count];
@@ -744,6 +757,7 @@ __global__ void __launch_bounds__(256) fq2_level_kernel(Fq2Level L, ModQ M, u64 
 }
 
 __global__ void fq2_claims_kernel(const u64* sums, u32 count, u32 nrmax, u64 q, u64* claims) {
+  pdl_wait();
   const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const u64* f = sums + (u64)i * nrmax * 6;  // round 0: real parts f0, f1, f2 at 0, 2, 4
@@ -804,7 +818,7 @@ int launch_sumcheck_fq2_batch(const u64* const* vecs, const u64* lens, u32 count
     L.count = k;
     u64 blocks = start / BS;
     if (blocks > 148ULL * 16) blocks = 148ULL * 16;
-    fq2_level_kernel<<<(unsigned)blocks, BS, 0, st>>>(L, M, shift, seed, round, sums, nrmax);
+    pdl(fq2_level_kernel, (unsigned)blocks, BS, 0, st)(L, M, shift, seed, round, sums, nrmax);
     int rc = check_launch("sumcheck_fq2 level");
     if (rc) return rc;
   }
@@ -817,7 +831,7 @@ int launch_sumcheck_fq2_batch(const u64* const* vecs, const u64* lens, u32 count
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_fq2: polys");
     po += (u64)nr * 6;
   }
-  fq2_claims_kernel<<<(count + 63) / 64, 64, 0, st>>>(sums, count, nrmax, M.q, claims);
+  pdl(fq2_claims_kernel, (count + 63) / 64, 64, 0, st)(sums, count, nrmax, M.q, claims);
   return check_launch("sumcheck_fq2 claims");
 }
 
@@ -952,10 +966,10 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       continue;
     }
     if (lazy)
-      sb_pass_kernel<true><<<(unsigned)grid, 256, 0, st>>>(ddesc + lev * SB_MAX_INST, lev_n[lev], lev_tiles[lev],
+      pdl(sb_pass_kernel<true>, (unsigned)grid, 256, 0, st)(ddesc + lev * SB_MAX_INST, lev_n[lev], lev_tiles[lev],
                                                             M, seed, round, sums, nrmax, plain);
     else
-      sb_pass_kernel<false><<<(unsigned)grid, 256, 0, st>>>(ddesc + lev * SB_MAX_INST, lev_n[lev],
+      pdl(sb_pass_kernel<false>, (unsigned)grid, 256, 0, st)(ddesc + lev * SB_MAX_INST, lev_n[lev],
                                                              lev_tiles[lev], M, seed, round, sums, nrmax, plain);
     if ((rc = check_launch("sb_pass"))) return rc;
   }
@@ -965,7 +979,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     e = cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: tail smem");
   }
-  tail<<<count, 1024, smem, st>>>(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
+  pdl(tail, count, 1024, smem, st)(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
                                    claims, polys);
   return check_launch("sb_tail");
 }
@@ -1012,7 +1026,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
       if ((rc = launch_gram_first(w, rows, L, M, ds, round, B.a, sa, g, c8 ? wide : nullptr, st))) return rc;
     } else {
       dim3 g(2 * grid_for(L / (1u << SC_T), 2 * rows), rows);
-      sc_first_kernel<LAZY><<<g, 256, 0, st>>>(w, rows, L, M, ds, round, B.a, sa, B.sums, nr, plain);
+      pdl(sc_first_kernel<LAZY>, g, 256, 0, st)(w, rows, L, M, ds, round, B.a, sa, B.sums, nr, plain);
       if ((rc = check_launch("sc_first"))) return rc;
     }
     in = B.a;
@@ -1029,7 +1043,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
         if ((rc = launch_gram_round(in, sin, out, so, L, rows, M, ds, round, j, gram_take(2 * rows, 0), st))) return rc;
       } else {
         dim3 gr(grid_for(L / (1u << SC_T), 2 * rows), 2 * rows);
-        sc_round_kernel<LAZY><<<gr, 256, 0, st>>>(in, sin, out, so, L, rows, M, ds, round, j, B.sums, nr, plain);
+        pdl(sc_round_kernel<LAZY>, gr, 256, 0, st)(in, sin, out, so, L, rows, M, ds, round, j, B.sums, nr, plain);
         if ((rc = check_launch("sc_round"))) return rc;
       }
       in = out;
@@ -1045,7 +1059,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tail smem attribute");
   }
-  kern<<<2 * rows, 512, smem, st>>>(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
+  pdl(kern, 2 * rows, 512, smem, st)(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
                                         claims, polys0, polys1);
   return check_launch("sc_tail");
 }
@@ -1118,6 +1132,7 @@ __device__ void blk_ntt(u64* a, u32 units, const NttDev& T, bool inverse) {
 
 __global__ void norm3_kernel(const u64* cap, u32 rows, u32 nr, NttDev T, ModQ M, const DevState* ds, u32 round,
                              u64* rhs0, u64* rhs1, u64* base0, u64* base1) {
+  pdl_wait();
   extern __shared__ u64 sm[];
   const u32 n = T.n, d = 2 * n, logd = T.logn + 1;
   const u32 pair = blockIdx.x, rep = pair / rows, k = pair % rows;
@@ -1165,7 +1180,7 @@ int launch_norm3(const u64* cap, u32 rows, u32 nr, const NttDev& T, const ModQ& 
                  u32 round, u64* proof_rep0, u64* proof_rep1, u64* base0, u64* base1, cudaStream_t st) {
   const u32 d = 2 * T.n;
   const size_t smem = 3ULL * d * sizeof(u64);
-  norm3_kernel<<<2 * rows, d < 256 ? d : 256, smem, st>>>(cap, rows, nr, T, M, ds, round, proof_rep0, proof_rep1,
+  pdl(norm3_kernel, 2 * rows, d < 256 ? d : 256, smem, st)(cap, rows, nr, T, M, ds, round, proof_rep0, proof_rep1,
                                                           base0, base1);
   return check_launch("norm3");
 }
@@ -1177,6 +1192,7 @@ int launch_norm3(const u64* cap, u32 rows, u32 nr, const NttDev& T, const ModQ& 
 // output row index = row*parts + c.  The OR and the radix stay on the device.
 // ---------------------------------------------------------------------------
 __global__ void decomp_or_kernel(RowSet in, u32 rows, u64 per_row, u64 q, u64* bw_or) {
+  pdl_wait();
   u64 acc = 0;
   for (u32 k = 0; k < rows; k++) {
     const u64* x = in.p[k];
@@ -1196,6 +1212,7 @@ __device__ __forceinline__ u32 radix_log_of(u64 orv, u32 parts) {
 
 __global__ void decomp_digits_kernel(RowSet in, u32 rows, u64 per_row, u64 q, u32 parts, DevState* ds, u32 didx,
                                      u64* out, u64* proof_radix) {
+  pdl_wait();
   const u32 rlog = radix_log_of(ds->bw_or[didx], parts);
   const u64 mask = (rlog >= 64) ? ~0ULL : ((1ULL << rlog) - 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1228,11 +1245,11 @@ int launch_decompose(RowSet in, u32 rows, u64 width, u32 d, u64 q, u32 parts, u3
   if (!mag_ready) {
     cudaError_t e = cudaMemsetAsync(&ds->bw_or[didx], 0, sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "decompose memset");
-    decomp_or_kernel<<<grid_1d(per_row, 256), 256, 0, st>>>(in, rows, per_row, q, &ds->bw_or[didx]);
+    pdl(decomp_or_kernel, grid_1d(per_row, 256), 256, 0, st)(in, rows, per_row, q, &ds->bw_or[didx]);
     rc = check_launch("decomp_or");
     if (rc) return rc;
   }
-  decomp_digits_kernel<<<grid_1d(per_row, 256), 256, 0, st>>>(in, rows, per_row, q, parts, ds, didx, out,
+  pdl(decomp_digits_kernel, grid_1d(per_row, 256), 256, 0, st)(in, rows, per_row, q, parts, ds, didx, out,
                                                                 proof_radix);
   return check_launch("decomp_digits");
 }
@@ -1251,7 +1268,7 @@ int launch_decompose_ntt(RowSet in, u32 rows, u64 width, u32 d, u64 q, u32 parts
   if (!mag_ready) {
     cudaError_t e = cudaMemsetAsync(&ds->bw_or[didx], 0, sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "decompose memset");
-    decomp_or_kernel<<<grid_1d(width * d, 256), 256, 0, st>>>(in, rows, width * d, q, &ds->bw_or[didx]);
+    pdl(decomp_or_kernel, grid_1d(width * d, 256), 256, 0, st)(in, rows, width * d, q, &ds->bw_or[didx]);
     int rc = check_launch("decomp_or");
     if (rc) return rc;
   }
@@ -1275,6 +1292,7 @@ constexpr u32 PROJ_H = 256;
 // One thread per row and 16 elements, rows fastest: a warp's Jc stores are one run.
 __global__ void proj_tables_kernel(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32* neg_mask,
                                    int8_t* J, int8_t* Jc) {
+  pdl_wait();
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= PROJ_H * (cw / 16)) return;
   const u32 k = t % PROJ_H, sl = t / PROJ_H;
@@ -1299,6 +1317,7 @@ __global__ void proj_tables_kernel(const DevState* ds, u32 round, u32 cw, u32* p
 // threads, thread (x, y) summing rows y, y + 32, ... of column x.
 __global__ void __launch_bounds__(1024) proj_cj_kernel(u32 cw, const u32* pos_mask, const u32* neg_mask, u64* cj,
                                                        u64 q) {
+  pdl_wait();
   __shared__ int part[32][33];
   const u32 x = threadIdx.x & 31, y = threadIdx.x >> 5, wd = blockIdx.x, words = cw / 32;
   int v = 0;
@@ -1320,11 +1339,11 @@ int launch_proj_tables(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32
   if (cw % 32) return salsaa_set_error(-2, "project: chunk width must be a multiple of 32");
   if (Jc && cw % 128) Jc = nullptr;
   u64 tot = (u64)PROJ_H * (cw / 16);
-  proj_tables_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(ds, round, cw, pos_mask, neg_mask, J, Jc);
+  pdl(proj_tables_kernel, (unsigned)((tot + 127) / 128), 128, 0, st)(ds, round, cw, pos_mask, neg_mask, J, Jc);
   int rc = check_launch("proj_tables");
   if (rc) return rc;
   if (cj) {
-    proj_cj_kernel<<<cw / 32, 1024, 0, st>>>(cw, pos_mask, neg_mask, cj, q);
+    pdl(proj_cj_kernel, cw / 32, 1024, 0, st)(cw, pos_mask, neg_mask, cj, q);
     rc = check_launch("proj_cj");
   }
   return rc;
@@ -1336,6 +1355,7 @@ int launch_proj_tables(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32
 template <int KT, bool LAZY>
 __global__ void project_kernel(RowSet in, u32 rows, u32 d, u64 q, u32 cw, u64 nch, const u32* pos_mask,
                                const u32* neg_mask, u64* out, const u64* gate) {
+  pdl_wait();
   extern __shared__ u32 msk[];  // KT x words (pos), then KT x words (neg)
   if (gate && *(volatile const u64*)gate == 0) return;  // the tensor-core pass was exact
   const u32 words = cw / 32, items = (u32)(rows * nch) * (PROJ_H / KT);
@@ -1401,6 +1421,7 @@ __device__ __forceinline__ void mma_s8_16832(int (&c)[4], u32 a0, u32 a1, u32 a2
 __global__ void __launch_bounds__(256, 2) project_mma_kernel(RowSet in, u32 d, u64 q, u32 cw, u64 nch,
                                                              const int8_t* __restrict__ J, u64* __restrict__ out,
                                                              u64* flag) {
+  pdl_wait();
   __shared__ __align__(16) int8_t As[PJ_BM * PJ_LD];
   __shared__ __align__(16) int8_t Bs[PJ_BN * PJ_LD];
   const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1510,7 +1531,7 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
     cudaError_t e = cudaMemsetAsync(&ds->proj_flag, 0, sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project memset");
     dim3 gm(2 * (d / PJ_BN), (unsigned)(rows * nch));
-    project_mma_kernel<<<gm, 256, 0, st>>>(in, d, q, cw, nch, J, out, &ds->proj_flag);
+    pdl(project_mma_kernel, gm, 256, 0, st)(in, d, q, cw, nch, J, out, &ds->proj_flag);
     int rc = check_launch("project_mma");
     if (rc) return rc;
     gate = &ds->proj_flag;
@@ -1521,8 +1542,8 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
   const unsigned g = (unsigned)(gate && items > 148 * 8 ? 148 * 8 : items);
   const size_t smem = 2ULL * KT * (cw / 32) * sizeof(u32);
   const bool lazy = q < (1ULL << 52) && cw <= 4096;
-  if (lazy) project_kernel<KT, true><<<g, d, smem, st>>>(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
-  else project_kernel<KT, false><<<g, d, smem, st>>>(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
+  if (lazy) pdl(project_kernel<KT, true>, g, d, smem, st)(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
+  else pdl(project_kernel<KT, false>, g, d, smem, st)(in, rows, d, q, cw, nch, pos_mask, neg_mask, out, gate);
   return check_launch("project");
 }
 
@@ -1531,6 +1552,7 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
 // (random_biased: q-1, 0, 1 uniformly) and new_w[i] = sum_k w_k[i] * c_k.
 // ---------------------------------------------------------------------------
 __global__ void fold_chal_kernel(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c) {
+  pdl_wait();
   u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (u64)rows * d) return;
   const u64 r = prf_at(prf_key(ds->seed, domain_id(DOM_FOLD, round, 0)), t);
@@ -1540,7 +1562,7 @@ __global__ void fold_chal_kernel(const DevState* ds, u32 round, u32 rows, u32 d,
 
 int launch_fold_challenge(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, cudaStream_t st) {
   u64 tot = (u64)rows * d;
-  fold_chal_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(ds, round, rows, d, q, c_coef);
+  pdl(fold_chal_kernel, (unsigned)((tot + 255) / 256), 256, 0, st)(ds, round, rows, d, q, c_coef);
   return check_launch("fold_challenge");
 }
 
@@ -1552,6 +1574,7 @@ int launch_fold_challenge(const DevState* ds, u32 round, u32 rows, u32 d, u64 q,
 // FP: the same six planes for the FP64 products (q < 2^50): each constant as
 // a double and its quotient fl(c / 2q), stored as the doubles' bits.
 __global__ void fold_pre_kernel(const u64* c, u32 rows, u32 n, ModQ M, const u64* zeta, u64* pre, bool fp) {
+  pdl_wait();
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= rows * n) return;
   const u32 k = t / n, s = t % n;
@@ -1585,6 +1608,7 @@ constexpr u32 FOLD_EL = 4;
 
 __global__ void __launch_bounds__(256) fold_fp_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M,
                                                       const u64* __restrict__ pre, u64* out, const u32* gate) {
+  pdl_wait();
   if (gate && !*gate) return;
   const u32 n = 1u << logn, hn = n >> 1;
   const u64 groups = (width + FOLD_EL - 1) / FOLD_EL;
@@ -1646,6 +1670,7 @@ __global__ void __launch_bounds__(256) fold_fp_kernel(RowSet w, u32 rows, u64 wi
 template <bool LAZY>
 __global__ void fold_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M, const u64* __restrict__ pre,
                             u64* out, const u32* gate) {
+  pdl_wait();
   if (gate && !*gate) return;
   const u32 n = 1u << logn;
   const u64 tot = width << logn, q = M.q, q2 = 2 * q;
@@ -1690,6 +1715,7 @@ __global__ void fold_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M, con
 template <bool LAZY>
 __global__ void __launch_bounds__(256) fold_vec_kernel(RowSet w, u32 rows, u64 width, u32 logn, ModQ M,
                                                        const u64* __restrict__ pre, u64* out, const u32* gate) {
+  pdl_wait();
   if (gate && !*gate) return;
   const u32 n = 1u << logn, hn = n >> 1;
   const u64 tot = width << (logn - 1), q = M.q, q2 = 2 * q;
@@ -1756,29 +1782,30 @@ int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ&
   bool vec = T.n >= 2 && (uintptr_t)out_slot % 16 == 0 && (uintptr_t)pre % 16 == 0 && ((u64)rows * T.n) % 2 == 0;
   for (u32 k = 0; k < rows; k++) vec = vec && (uintptr_t)w_slot.p[k] % 16 == 0;
   const bool fp = vec && M.q < (1ULL << 50) && fold_choice() == 1;
-  fold_pre_kernel<<<(rows * T.n + 127) / 128, 128, 0, st>>>(c_slot, rows, T.n, M, T.zeta, pre, fp);
+  pdl(fold_pre_kernel, (rows * T.n + 127) / 128, 128, 0, st)(c_slot, rows, T.n, M, T.zeta, pre, fp);
   int rc = check_launch("fold_pre");
   if (rc) return rc;
   if (fp) {
-    fold_fp_kernel<<<grid_1d((width + FOLD_EL - 1) / FOLD_EL * T.n / 2, 256), 256, 0, st>>>(w_slot, rows, width,
+    pdl(fold_fp_kernel, grid_1d((width + FOLD_EL - 1) / FOLD_EL * T.n / 2, 256), 256, 0, st)(w_slot, rows, width,
                                                                                             T.logn, M, pre, out_slot,
                                                                                             gate);
     return check_launch("fold");
   }
   if (vec) {
     const unsigned g = grid_1d(width * T.n / 2, 256);
-    if (lazy) fold_vec_kernel<true><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
-    else fold_vec_kernel<false><<<g, 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
+    if (lazy) pdl(fold_vec_kernel<true>, g, 256, 0, st)(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
+    else pdl(fold_vec_kernel<false>, g, 256, 0, st)(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
     return check_launch("fold");
   }
   if (lazy)
-    fold_kernel<true><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
+    pdl(fold_kernel<true>, grid_1d(width * T.n, 256), 256, 0, st)(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
   else
-    fold_kernel<false><<<grid_1d(width * T.n, 256), 256, 0, st>>>(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
+    pdl(fold_kernel<false>, grid_1d(width * T.n, 256), 256, 0, st)(w_slot, rows, width, T.logn, M, pre, out_slot, gate);
   return check_launch("fold");
 }
 
 __global__ void fold_slots_kernel(const u64* x, const u64* c, u32 K, u32 n, ModQ M, const u64* zeta, u64* out) {
+  pdl_wait();
   const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   u64 ae = 0, ao = 0;
@@ -1795,7 +1822,7 @@ __global__ void fold_slots_kernel(const u64* x, const u64* c, u32 K, u32 n, ModQ
 
 int launch_fold_slots(const u64* x, const u64* c_slot, u32 K, const NttDev& T, const ModQ& M, u64* out,
                       cudaStream_t st) {
-  fold_slots_kernel<<<(T.n + 63) / 64, 64, 0, st>>>(x, c_slot, K, T.n, M, T.zeta, out);
+  pdl(fold_slots_kernel, (T.n + 63) / 64, 64, 0, st)(x, c_slot, K, T.n, M, T.zeta, out);
   return check_launch("fold_slots");
 }
 
@@ -1812,6 +1839,7 @@ template <int RT, int KT, bool LIMB>
 __global__ void __launch_bounds__(256) ck_commit_kernel(RowSet w, u32 rows, u32 nck, const u64* tlo,
                                                         const u64* thi, u32 Bt, u32 nhi_t, u32 CH, ModQ M,
                                                         const u64* zeta, u64* acc, bool plain) {
+  pdl_wait();
   // grid: x = row tile (fastest, so co-scheduled CTAs share the witness chunk in L2),
   //       y = element chunk, z = witness-row tile
   const u32 n = blockDim.x, s = threadIdx.x, d = 2 * n;
@@ -1932,6 +1960,7 @@ template <int RT, int KT, bool LIMB>
 __global__ void __launch_bounds__(512) sc_commit_kernel(RowSet w, u32 rows, ScRowList list, const u64* s_lo,
                                                         const u64* s_hi, u32 Bw, u32 nhi, u32 CH, ModQ M, u64* acc,
                                                         bool plain) {
+  pdl_wait();
   const u32 d = blockDim.x, p = threadIdx.x;
   const u32 t0 = blockIdx.x * RT, k0 = blockIdx.z * KT;
   u32 row[RT];  // statement rows of this tile (the last one repeated past the list's end)
@@ -2055,6 +2084,7 @@ __global__ void __launch_bounds__(512) sc_commit_kernel(RowSet w, u32 rows, ScRo
 // Column sums U_k[lo] = sum_h W_k[h*Bw + lo] (mod q) for the rows whose
 // weights repeat with a period dividing Bw (witness_lhs and projected_lhs).
 __global__ void colsum_kernel(RowSet w, u32 rows, u64 width, u32 Bw, u32 d, ModQ M, u64* out) {
+  pdl_wait();
   const u64 per = (u64)Bw * d, tot = rows * per, nhi = width / Bw;
   const bool lazy = M.q < (1ULL << 50) && nhi <= 4096;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
@@ -2077,6 +2107,7 @@ __global__ void colsum_kernel(RowSet w, u32 rows, u64 width, u32 Bw, u32 d, ModQ
 // s(i) = prod_t (bit ? c : 1 - c); split at Bw into s_hi (high bits), s_lo.
 __global__ void sc_tables_kernel(const ScalarRowDesc* desc, u32 nsc, u64 width, u32 Bw, u32 nhi, ModQ M,
                                  const DevState* ds, u64* s_lo, u64* s_hi) {
+  pdl_wait();
   const u32 r = blockIdx.y;
   const ScalarRowDesc D = desc[r];
   const u64 q = M.q;
@@ -2105,6 +2136,7 @@ __global__ void sc_tables_kernel(const ScalarRowDesc* desc, u32 nsc, u64 width, 
 
 __global__ void commit_finalize_kernel(const u64* acc, u32 nck, u32 nsc, u32 rows, u32 n, ModQ M,
                                        const u64* zeta, const u64* const* bases, u64* out) {
+  pdl_wait();
   const u64 tot = (u64)(nck + nsc) * rows * n;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 s = (u32)(t % n);
@@ -2135,6 +2167,7 @@ __global__ void commit_finalize_kernel(const u64* acc, u32 nck, u32 nsc, u32 row
 constexpr u32 CKM_KS = 128, CKM_LD = 144;
 
 __global__ void ck_tl8_kernel(const u64* tlo, u32 nck, u32 n, u32 bt, u32 nmt, bool packed, uint8_t* tl8) {
+  pdl_wait();
   const u64 tot = (u64)n * nmt * CKM_BM * bt;
   for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
     const u32 lo = (u32)(t % bt);
@@ -2157,7 +2190,7 @@ __global__ void ck_tl8_kernel(const u64* tlo, u32 nck, u32 n, u32 bt, u32 nmt, b
 
 int launch_ck_tl8(const u64* tlo, u32 nck, u32 n, u32 bt, bool packed, uint8_t* tl8, cudaStream_t st) {
   const u32 nmt = (nck + CKM_ROWS - 1) / CKM_ROWS;
-  ck_tl8_kernel<<<grid_1d((u64)n * nmt * CKM_BM * bt, 256), 256, 0, st>>>(tlo, nck, n, bt, nmt, packed, tl8);
+  pdl(ck_tl8_kernel, grid_1d((u64)n * nmt * CKM_BM * bt, 256), 256, 0, st)(tlo, nck, n, bt, nmt, packed, tl8);
   return check_launch("ck_tl8");
 }
 
@@ -2189,6 +2222,7 @@ template <int NTW>
 __global__ void __launch_bounds__(256) ck_mma_kernel(const uint8_t* __restrict__ tl8, RowSet w, u32 rows, u64 width,
                                                      u32 nck, u32 nmt, u32 n, u32 bt, u32 Bw, const u64* thi,
                                                      u32 nhi_t, ModQ M, const u64* zeta, u64* acc, bool plain) {
+  pdl_wait();
   constexpr u32 NP = 2 * NTW * 8;
   constexpr u32 TPT = 3;  // witness staging tasks per thread (rows <= 12)
   extern __shared__ __align__(16) uint8_t smem[];
@@ -2353,7 +2387,7 @@ static int launch_ck_mma_t(const CommitArgs& a, u32 n, u32 Bw, const ModQ& M, co
   // algorithmic work: the exact byte-limb products, 3 key components x 7 bytes
   // against 2 witness parts x 7 bytes per (key row, witness row, element, slot)
   const int tr = salsaa_trace_begin("ck_mma_kernel", st, 2.0 * 294.0 * a.nck * a.rows * (double)a.width * n);
-  kern<<<g, 256, smem, st>>>(a.tl8, a.w, a.rows, a.width, a.nck, nmt, n, a.ck_bt, Bw, a.thi, a.ck_nhi, M, zeta,
+  pdl(kern, g, 256, smem, st)(a.tl8, a.w, a.rows, a.width, a.nck, nmt, n, a.ck_bt, Bw, a.thi, a.ck_nhi, M, zeta,
                              a.acc, plain);
   salsaa_trace_end(tr, st);
   return check_launch("ck_mma");
@@ -2379,10 +2413,10 @@ static void launch_ck_variant(const CommitArgs& a, u32 n, u32 Bt, u32 nhi_t, u32
                               const u64* zeta, bool plain, cudaStream_t st) {
   dim3 g((a.nck + RT - 1) / RT, (unsigned)(a.width / CH), (a.rows + KT - 1) / KT);
   if (M.q < (1ULL << 50))
-    ck_commit_kernel<RT, KT, true><<<g, n, 0, st>>>(a.w, a.rows, a.nck, a.tlo, a.thi, Bt, nhi_t, CH, M, zeta, a.acc,
+    pdl(ck_commit_kernel<RT, KT, true>, g, n, 0, st)(a.w, a.rows, a.nck, a.tlo, a.thi, Bt, nhi_t, CH, M, zeta, a.acc,
                                                    plain);
   else
-    ck_commit_kernel<RT, KT, false><<<g, n, 0, st>>>(a.w, a.rows, a.nck, a.tlo, a.thi, Bt, nhi_t, CH, M, zeta,
+    pdl(ck_commit_kernel<RT, KT, false>, g, n, 0, st)(a.w, a.rows, a.nck, a.tlo, a.thi, Bt, nhi_t, CH, M, zeta,
                                                     a.acc, plain);
 }
 
@@ -2391,9 +2425,9 @@ static void launch_sc_variant(const CommitArgs& a, const RowSet& w, u64 width, c
                               u32 nhi, u32 CH, const ModQ& M, bool plain, u64* acc_sc, cudaStream_t st) {
   dim3 g((list.n + RT - 1) / RT, (unsigned)(width / CH), (a.rows + KT - 1) / KT);
   if (M.q < (1ULL << 50))
-    sc_commit_kernel<RT, KT, true><<<g, d, 0, st>>>(w, a.rows, list, a.sc_lo, a.sc_hi, Bw, nhi, CH, M, acc_sc, plain);
+    pdl(sc_commit_kernel<RT, KT, true>, g, d, 0, st)(w, a.rows, list, a.sc_lo, a.sc_hi, Bw, nhi, CH, M, acc_sc, plain);
   else
-    sc_commit_kernel<RT, KT, false><<<g, d, 0, st>>>(w, a.rows, list, a.sc_lo, a.sc_hi, Bw, nhi, CH, M, acc_sc,
+    pdl(sc_commit_kernel<RT, KT, false>, g, d, 0, st)(w, a.rows, list, a.sc_lo, a.sc_hi, Bw, nhi, CH, M, acc_sc,
                                                     plain);
 }
 
@@ -2409,6 +2443,7 @@ static void launch_sc_pass(const CommitArgs& a, const RowSet& w, u64 width, cons
 }
 
 __global__ void reduce_inplace_kernel(u64* x, u64 n, ModQ M) {
+  pdl_wait();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
     x[i] = reduce64(M, x[i]);
 }
@@ -2463,7 +2498,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
   }
   if (a.nsc) {
     dim3 gt((Bw + nhi + 255) / 256, a.nsc);
-    sc_tables_kernel<<<gt, 256, 0, ss>>>(a.sc_desc_dev, a.nsc, a.width, Bw, nhi, M, ds, a.sc_lo, a.sc_hi);
+    pdl(sc_tables_kernel, gt, 256, 0, ss)(a.sc_desc_dev, a.nsc, a.width, Bw, nhi, M, ds, a.sc_lo, a.sc_hi);
     int rc = check_launch("sc_tables");
     if (rc) return rc;
     u64* acc_sc = a.acc + (u64)a.nck * a.rows * d;
@@ -2510,7 +2545,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
       RowSet u = wsrc;
       if (nhi > 1) {
         if (!a.colsum || a.rows > a.colsum_rows) return salsaa_set_error(-2, "commit: column-sum scratch too small");
-        colsum_kernel<<<grid_1d((u64)a.rows * Bw * d, 256), 256, 0, ss>>>(wsrc, a.rows, a.width, Bw, d, M,
+        pdl(colsum_kernel, grid_1d((u64)a.rows * Bw * d, 256), 256, 0, ss)(wsrc, a.rows, a.width, Bw, d, M,
                                                                          a.colsum);
         rc = check_launch("colsum");
         if (rc) return rc;
@@ -2526,7 +2561,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
     }
     if (a.coef_sc) {
       const u64 cnt = (u64)a.nsc * a.rows;
-      reduce_inplace_kernel<<<grid_1d(cnt * d, 256), 256, 0, ss>>>(acc_sc, cnt * d, M);
+      pdl(reduce_inplace_kernel, grid_1d(cnt * d, 256), 256, 0, ss)(acc_sc, cnt * d, M);
       rc = check_launch("reduce");
       if (rc) return rc;
       rc = ntt_launch(acc_sc, acc_sc, cnt, T, true, false, ss);
@@ -2539,7 +2574,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "commit: join");
   }
   const u64 tot = (u64)(a.nck + a.nsc) * a.rows * n;
-  commit_finalize_kernel<<<grid_1d(tot, 256), 256, 0, st>>>(a.acc, a.nck, a.nsc, a.rows, n, M, T.zeta,
+  pdl(commit_finalize_kernel, grid_1d(tot, 256), 256, 0, st)(a.acc, a.nck, a.nsc, a.rows, n, M, T.zeta,
                                                           a.sc_base_dev, a.out_slot);
   return check_launch("commit_finalize");
 }
@@ -2547,7 +2582,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
 int launch_commit_finalize(const u64* acc, u32 nck, u32 rows, const NttDev& T, const ModQ& M, u64* out,
                            cudaStream_t st) {
   const u64 tot = (u64)nck * rows * T.n;
-  commit_finalize_kernel<<<grid_1d(tot, 256), 256, 0, st>>>(acc, nck, 0, rows, T.n, M, T.zeta, nullptr, out);
+  pdl(commit_finalize_kernel, grid_1d(tot, 256), 256, 0, st)(acc, nck, 0, rows, T.n, M, T.zeta, nullptr, out);
   return check_launch("commit_finalize");
 }
 
@@ -2555,6 +2590,7 @@ int launch_commit_finalize(const u64* acc, u32 nck, u32 rows, const NttDev& T, c
 // Derived commitments (see launch_derive in kernels.cuh).
 // ---------------------------------------------------------------------------
 __global__ void derive_kernel(DeriveArgs a, u32 n, ModQ M, const u64* zeta, const DevState* ds) {
+  pdl_wait();
   const u64 tot = (u64)(a.nck + a.nsc) * a.K * n;
   const u32 d = 2 * n;
   const u32 logw = 63u - (u32)__clzll((long long)a.w);
@@ -2604,7 +2640,7 @@ __global__ void derive_kernel(DeriveArgs a, u32 n, ModQ M, const u64* zeta, cons
 int launch_derive(const DeriveArgs& a, const NttDev& T, const ModQ& M, const DevState* ds, cudaStream_t st) {
   if (a.w < 2 || (a.w & (a.w - 1)) || a.ncols < 2 * a.K) return salsaa_set_error(-2, "derive: bad shape");
   const u64 tot = (u64)(a.nck + a.nsc) * a.K * T.n;
-  derive_kernel<<<grid_1d(tot, 256), 256, 0, st>>>(a, T.n, M, T.zeta, ds);
+  pdl(derive_kernel, grid_1d(tot, 256), 256, 0, st)(a, T.n, M, T.zeta, ds);
   return check_launch("derive");
 }
 

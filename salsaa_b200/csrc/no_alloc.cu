@@ -45,7 +45,8 @@ unsigned char* g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
 typedef int (*CtxGetCurrentFn)(void**);
 CtxGetCurrentFn g_ctx_get_current = nullptr;
 
-__global__ void noalloc_seed_kernel(DevState* ds, u64 seed) { ds->seed = seed; }
+__global__ void noalloc_seed_kernel(DevState* ds, u64 seed) {
+  pdl_wait(); ds->seed = seed; }
 
 // The current driver context, through the runtime's driver entry-point lookup
 // (no link-time dependency on the driver library).
@@ -110,7 +111,7 @@ extern "C" int salsaa_project_noalloc(const uint64_t* d_w, uint64_t rows, uint64
   // The array keeps the previous call's contents: the seed is written here
   // and the projection clears its overflow flag itself before use; the masks
   // and J are fully rewritten for this call's chunk width.
-  noalloc_seed_kernel<<<1, 1, 0, st>>>(ds, seed);
+  pdl(noalloc_seed_kernel, 1, 1, 0, st)(ds, seed);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project_noalloc: seed");
   rc = launch_proj_tables(ds, (u32)round, (u32)cw, pm, nm, J, nullptr, q, st);

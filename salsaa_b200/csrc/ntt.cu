@@ -159,6 +159,7 @@ const NttDev* ntt_tables(u32 n, u64 q) {
 template <bool INCOMPLETE, bool INVERSE>
 __global__ void __launch_bounds__(256) ntt_kernel(const u64* in, u64* out, u64 count,
                                                   NttDev T, u32 epb) {
+  pdl_wait();
   extern __shared__ u64 sm[];
   const u32 n = T.n, logn = T.logn;
   const u32 logd = INCOMPLETE ? logn + 1 : logn;
@@ -401,6 +402,7 @@ __device__ __forceinline__ void nr_tile(const u64* in, u64* out, u64 units, u64 
 
 template <int LOGN, bool INC, bool INV, bool RELAX>
 __global__ void __launch_bounds__(256) ntt_reg_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or) {
+  pdl_wait();
   __shared__ u64 sm[NR_TILE + NR_TILE / 16];
   nr_tile<LOGN, INC, INV, RELAX>(in, out, units, blockIdx.x, T, mag_or, sm);
 }
@@ -478,6 +480,7 @@ __device__ __forceinline__ void nf_tile(const u64* in, u64* out, u64 units, u64 
 
 template <int LOGN, bool INC, bool INV>
 __global__ void __launch_bounds__(256) ntt_fp_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or) {
+  pdl_wait();
   __shared__ double sm[NR_TILE + NR_TILE / 16];
   nf_tile<LOGN, INC, INV>(in, out, units, blockIdx.x, T, mag_or, sm);
 }
@@ -486,6 +489,7 @@ __global__ void __launch_bounds__(256) ntt_fp_kernel(const u64* in, u64* out, u6
 
 template <bool INV>
 __global__ void __launch_bounds__(256) ntt_fp6_kernel(const u64* in, u64* out, u64 count, NttDev T, u64* mag_or) {
+  pdl_wait();
   __shared__ double2 sm[NP6_EL * NP6_ROW];
   const u32 el = threadIdx.x >> 3, r = threadIdx.x & 7;
   const u64 eg = (u64)blockIdx.x * NP6_EL + el;
@@ -562,6 +566,7 @@ __global__ void __launch_bounds__(256) ntt_fp6_kernel(const u64* in, u64* out, u
 // ntt_reg_kernel<6, false, INV, RELAX>.
 template <bool INV, bool RELAX>
 __global__ void __launch_bounds__(256) ntt_int6_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or) {
+  pdl_wait();
   __shared__ ulonglong2 sm[NP6_EL * NP6_ROW];
   const u32 el = threadIdx.x >> 3, r = threadIdx.x & 7;
   const u64 u0 = 2 * ((u64)blockIdx.x * NP6_EL + el);
@@ -661,6 +666,7 @@ bool np6_aligned(const u64* in, const u64* out, bool inverse) {
 // FP: FP64 butterflies (q < 2^50, the nf_* code), else the integer ones.
 template <int LOGN, bool INC, bool INV, bool RELAX, int STAGES, bool FP>
 __global__ void __launch_bounds__(256) ntt_pipe_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or) {
+  pdl_wait();
   using Wd = typename std::conditional<FP, double, u64>::type;
   constexpr u32 N = 1u << LOGN, UPT = NR_TILE / N;
   constexpr int NPH = ph_count(LOGN);
@@ -786,6 +792,7 @@ struct NttMulti {
 
 template <int LOGN, bool INC, bool INV, bool RELAX, bool FP>
 __global__ void __launch_bounds__(256) ntt_multi_kernel(NttMulti m, NttDev T) {
+  pdl_wait();
   __shared__ u64 sm[NR_TILE + NR_TILE / 16];
   const u64 b = blockIdx.x;
   u32 lo = 0, hi = m.count;  // invariant: bstart[lo] <= b < bstart[hi]
@@ -811,6 +818,7 @@ template <int LOGN, bool RELAX, bool FP>
 __global__ void __launch_bounds__(256)
     ntt_digits_kernel(NttSrcRows src, u64 width, u32 parts, const u64* bw_or, u64* rlog_out, u64* radix_out, u64* dc,
                       u64* ds, u64 units, NttDev T, bool narrow) {
+  pdl_wait();
   // FP: the FP64 butterflies (q < 2^50), else the integer ones.  narrow: the
   // coefficient-form digits go to dc as centred int32 values (parts >= 2, so
   // |digit| < radix <= 2^25), else as canonical words.
@@ -899,6 +907,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     ntt_digits6_kernel(NttSrcRows src, u64 width, u32 parts, const u64* bw_or, u64* rlog_out, u64* radix_out,
                        u64* dc, u64* ds, u64 count, NttDev T, bool narrow) {
+  pdl_wait();
   __shared__ double2 sm[NP6_EL * NP6_ROW];
   const u32 el = threadIdx.x >> 3, r = threadIdx.x & 7;
   const u64 re = (u64)blockIdx.x * NP6_EL + el;  // ring element of the digit space
@@ -955,6 +964,7 @@ __global__ void __launch_bounds__(256)
 template <int LOGN, bool RELAX>
 __global__ void __launch_bounds__(256) ntt_mul_kernel(const u64* a, const u64* b, u64* r, u64 units, NttDev T,
                                                       ModQ M) {
+  pdl_wait();
   constexpr u32 N = 1u << LOGN, UPT = NR_TILE / N;
   constexpr int NPH = ph_count(LOGN), PL = NPH - 1, SL = ph_size(LOGN, PL);
   constexpr u32 MBL = 16 >> SL, KL = 1u << SL;
@@ -1037,7 +1047,7 @@ int nm_launch(const u64* a, const u64* b, u64* r, u64 count, const NttDev& T, cu
   auto go = [&](auto kern) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ntt_mul smem attribute");
-    kern<<<(unsigned)blocks, 256, smem, st>>>(a, b, r, count, T, make_modq(T.q));
+    pdl(kern, (unsigned)blocks, 256, smem, st)(a, b, r, count, T, make_modq(T.q));
     return 0;
   };
   return T.q < NR_RELAX_Q ? go(ntt_mul_kernel<LOGN, true>) : go(ntt_mul_kernel<LOGN, false>);
@@ -1073,7 +1083,7 @@ int np_go(const u64* in, u64* out, u64 units, const NttDev& T, cudaStream_t st, 
   const u64 tiles = (units + UPT - 1) / UPT;
   const u64 cap = (u64)nsm * (u64)per_sm;
   const u64 blocks = tiles < cap ? tiles : cap;
-  kern<<<(unsigned)blocks, 256, smem, st>>>(in, out, units, T, mag_or);
+  pdl(kern, (unsigned)blocks, 256, smem, st)(in, out, units, T, mag_or);
   return 0;
 }
 
@@ -1107,13 +1117,13 @@ int nr_launch(const u64* in, u64* out, u64 units, const NttDev& T, bool incomple
   const NttChoice ch = ntt_choice(LOGN, incomplete, inverse, !relax, units * (1ULL << LOGN) >= NTT_LARGE_COEFFS);
   if (ch.variant == 1 && relax) {  // FP64 butterflies
     auto gof = [&](auto kern) -> int {
-      kern<<<(unsigned)blocks, 256, 0, st>>>(in, out, units, T, mag_or);
+      pdl(kern, (unsigned)blocks, 256, 0, st)(in, out, units, T, mag_or);
       return 0;
     };
     if (LOGN == 6 && incomplete && np6_aligned(in, out, inverse)) {
       const u64 count = units / 2, g6 = (count + NP6_EL - 1) / NP6_EL;
-      if (inverse) ntt_fp6_kernel<true><<<(unsigned)g6, 256, 0, st>>>(in, out, count, T, mag_or);
-      else ntt_fp6_kernel<false><<<(unsigned)g6, 256, 0, st>>>(in, out, count, T, mag_or);
+      if (inverse) pdl(ntt_fp6_kernel<true>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or);
+      else pdl(ntt_fp6_kernel<false>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or);
       return 0;
     }
     if (incomplete) {
@@ -1141,18 +1151,18 @@ int nr_launch(const u64* in, u64* out, u64 units, const NttDev& T, bool incomple
     }
   }
   auto go = [&](auto kern) -> int {
-    kern<<<(unsigned)blocks, 256, 0, st>>>(in, out, units, T, mag_or);
+    pdl(kern, (unsigned)blocks, 256, 0, st)(in, out, units, T, mag_or);
     return 0;
   };
   // full 64-point transforms: the paired layout when the contiguous side is 32-byte aligned
   if (LOGN == 6 && !incomplete && (uintptr_t)(inverse ? in : out) % 32 == 0) {
     const unsigned g6 = (unsigned)((units + 2 * NP6_EL - 1) / (2 * NP6_EL));
     if (inverse) {
-      if (relax) ntt_int6_kernel<true, true><<<g6, 256, 0, st>>>(in, out, units, T, mag_or);
-      else ntt_int6_kernel<true, false><<<g6, 256, 0, st>>>(in, out, units, T, mag_or);
+      if (relax) pdl(ntt_int6_kernel<true, true>, g6, 256, 0, st)(in, out, units, T, mag_or);
+      else pdl(ntt_int6_kernel<true, false>, g6, 256, 0, st)(in, out, units, T, mag_or);
     } else {
-      if (relax) ntt_int6_kernel<false, true><<<g6, 256, 0, st>>>(in, out, units, T, mag_or);
-      else ntt_int6_kernel<false, false><<<g6, 256, 0, st>>>(in, out, units, T, mag_or);
+      if (relax) pdl(ntt_int6_kernel<false, true>, g6, 256, 0, st)(in, out, units, T, mag_or);
+      else pdl(ntt_int6_kernel<false, false>, g6, 256, 0, st)(in, out, units, T, mag_or);
     }
     return 0;
   }
@@ -1178,7 +1188,7 @@ int nm_multi_go(const NttMulti& m, u64 blocks, const NttDev& T, bool incomplete,
   const bool relax = T.q < NR_RELAX_Q;
   const bool fp = relax && ntt_choice(LOGN, incomplete, inverse, false, large).fp64();
   auto go = [&](auto kern) -> int {
-    kern<<<(unsigned)blocks, 256, 0, st>>>(m, T);
+    pdl(kern, (unsigned)blocks, 256, 0, st)(m, T);
     return 0;
   };
   if (incomplete) {
@@ -1246,7 +1256,7 @@ int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incompl
     }
     // algorithmic bytes: every coefficient read once and written once
     const int tr = salsaa_trace_begin("ntt_kernel", st, 16.0 * (double)count * d);
-    kern<<<(unsigned)blocks, 256, smem, st>>>(in, out, count, T, epb);
+    pdl(kern, (unsigned)blocks, 256, smem, st)(in, out, count, T, epb);
     salsaa_trace_end(tr, st);
     salsaa_count_launch();
     cudaError_t e = cudaGetLastError();
@@ -1317,16 +1327,16 @@ int nd_launch(const NttSrcRows& src, u32 rows, u64 width, u32 parts, const u64* 
   for (u32 k = 0; k < rows && k < 16; k++) src16 = src16 && (uintptr_t)src.p[k] % 16 == 0;
   if (fp && LOGN == 6 && (uintptr_t)ds % 32 == 0 && src16) {
     const u64 count = units / 2;
-    ntt_digits6_kernel<<<(unsigned)((count + NP6_EL - 1) / NP6_EL), 256, 0, st>>>(src, width, parts, bw_or, rlog_out,
+    pdl(ntt_digits6_kernel, (unsigned)((count + NP6_EL - 1) / NP6_EL), 256, 0, st)(src, width, parts, bw_or, rlog_out,
                                                                                    radix_out, dc, ds, count, T, narrow);
   } else if (fp)
-    ntt_digits_kernel<LOGN, true, true><<<(unsigned)blocks, 256, 0, st>>>(src, width, parts, bw_or, rlog_out,
+    pdl(ntt_digits_kernel<LOGN, true, true>, (unsigned)blocks, 256, 0, st)(src, width, parts, bw_or, rlog_out,
                                                                            radix_out, dc, ds, units, T, narrow);
   else if (relax)
-    ntt_digits_kernel<LOGN, true, false><<<(unsigned)blocks, 256, 0, st>>>(src, width, parts, bw_or, rlog_out,
+    pdl(ntt_digits_kernel<LOGN, true, false>, (unsigned)blocks, 256, 0, st)(src, width, parts, bw_or, rlog_out,
                                                                             radix_out, dc, ds, units, T, narrow);
   else
-    ntt_digits_kernel<LOGN, false, false><<<(unsigned)blocks, 256, 0, st>>>(src, width, parts, bw_or, rlog_out,
+    pdl(ntt_digits_kernel<LOGN, false, false>, (unsigned)blocks, 256, 0, st)(src, width, parts, bw_or, rlog_out,
                                                                              radix_out, dc, ds, units, T, narrow);
   return 0;
 }

@@ -46,6 +46,7 @@ __device__ __forceinline__ u64 img_digit(u64 v, u64 q, u32 sh, u64 mask, long lo
 
 template <int LOGN, bool DIG>
 __global__ void __launch_bounds__(ImgGeom<LOGN>::THREADS) ntt_img_kernel(ImgDigits a, CkImage im, NttDev T) {
+  pdl_wait();
   using Geo = ImgGeom<LOGN>;
   constexpr u32 N = Geo::N, D = Geo::D, JG = Geo::JG, EL = Geo::EL;
   extern __shared__ __align__(16) unsigned char ni_smem[];
@@ -259,7 +260,7 @@ int img_go(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStream_t 
                                                   : 15 + (a.rows.slots ? 8 : 0)));
   // gated: a grid that leaves quickly when the gate is closed
   const u64 grid = a.rows.gate && blocks > 444 ? 444 : blocks;
-  kern<<<(unsigned)grid, Geo::THREADS, Geo::SMEM, st>>>(a, im, T);
+  pdl(kern, (unsigned)grid, Geo::THREADS, Geo::SMEM, st)(a, im, T);
   salsaa_trace_end(tr, st);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
@@ -290,6 +291,7 @@ int img_launch(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStrea
 template <int LOGN>
 __global__ void __launch_bounds__(256) ntt_inv_gated_kernel(const u64* in, u64* out, u64 units, NttDev T,
                                                             const u32* gate, u64* mag_or) {
+  pdl_wait();
   constexpr int PL = ph_count(LOGN) - 1;
   constexpr u32 UPT = NR_TILE >> LOGN;
   __shared__ double sm[NR_TILE + NR_TILE / 16];
@@ -329,8 +331,8 @@ int ntt_inv_gated_launch(const u64* in, u64* out, u64 count, const NttDev& T, co
     return salsaa_set_error(-2, "ntt_inv_gated: shape or alignment not supported");
   const u64 units = 2 * count, tiles = (units * T.n + NR_TILE - 1) / NR_TILE;
   const unsigned grid = (unsigned)(tiles < 592 ? tiles : 592);
-  if (T.logn == 6) ntt_inv_gated_kernel<6><<<grid, 256, 0, st>>>(in, out, units, T, gate, mag_or);
-  else ntt_inv_gated_kernel<7><<<grid, 256, 0, st>>>(in, out, units, T, gate, mag_or);
+  if (T.logn == 6) pdl(ntt_inv_gated_kernel<6>, grid, 256, 0, st)(in, out, units, T, gate, mag_or);
+  else pdl(ntt_inv_gated_kernel<7>, grid, 256, 0, st)(in, out, units, T, gate, mag_or);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "ntt_inv_gated launch");

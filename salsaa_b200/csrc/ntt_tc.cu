@@ -152,6 +152,7 @@ __device__ __forceinline__ bool bar_tc_and(bool p, u32 bar) {
 template <int LOGN, int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage im, const uint8_t* __restrict__ tcw,
                                                                u64 q, TcRed red, u32* err) {
+  pdl_wait();
   using Geo = TcGeom<LOGN, MODE>;
   constexpr u32 N = Geo::N, D = Geo::D, SEL = Geo::SEL, SELLOG = Geo::SELLOG, SUB = Geo::SUB, WPT = Geo::WPT, JG = Geo::JG, US = Geo::IU;
   constexpr u32 EPI = MODE == TC_LIMBS ? 128 : 256;  // threads per unit
@@ -566,7 +567,7 @@ int tc_go(const TcArgs& a, const CkImage& im, const NttDev& T, cudaStream_t st) 
   const double coeffs = (double)a.rows.rows * a.rows.width * Geo::D;
   const int tr = salsaa_trace_begin(MODE == TC_DIGITS ? "ntt_digits_kernel" : "ntt_kernel", st,
                                     coeffs * (8 + (MODE == TC_DIGITS ? 2 : 1) * (a.c8 ? 8 : 7)));
-  kern<<<(unsigned)(items < 148 ? items : 148), TC_THREADS, Geo::SMEM, st>>>(a, im, T.tcw, T.q,
+  pdl(kern, (unsigned)(items < 148 ? items : 148), TC_THREADS, Geo::SMEM, st)(a, im, T.tcw, T.q,
                                                                              tc_red(T.q, LOGN == 6 && MODE != TC_LIMBS),
                                                                              tc_error_word());
   salsaa_trace_end(tr, st);

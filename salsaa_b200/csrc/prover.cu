@@ -671,6 +671,7 @@ extern "C" int salsaa_prover_set_overlap(salsaa_prover* pr, int on) {
 }
 
 __global__ void set_seed_kernel(DevState* ds, u64 seed) {
+  pdl_wait();
   const u32 t = threadIdx.x;
   if (t == 0) ds->seed = seed;
   if (t < 16) {
@@ -829,7 +830,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
   cudaError_t e = cudaMemcpyAsync(proof, pr->header_pinned, 8 * sizeof(u64), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: header");
   cur = 8;
-  set_seed_kernel<<<1, 32, 0, st>>>(pr->ds, seed);
+  pdl(set_seed_kernel, 1, 32, 0, st)(pr->ds, seed);
   salsaa_count_launch();
   u32 K = (u32)P.init_wit_rep;
   u64 width = L;
@@ -1543,7 +1544,7 @@ static int verify_impl(salsaa_prover* pr, u64 seed, const u64* proof, int* verdi
   u64* dslot = pr->Ds;
   if ((e = cudaMemcpyAsync(dcoef, proof, words * 8, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return salsaa_set_cuda_error(e, "verify: proof upload");
-  set_seed_kernel<<<1, 32, 0, st>>>(pr->ds, seed);  // the challenges drawn on the device
+  pdl(set_seed_kernel, 1, 32, 0, st)(pr->ds, seed);  // the challenges drawn on the device
   salsaa_count_launch();
   std::vector<std::pair<u64, u64>> seg;
   proof_segments(P, seg);
@@ -2108,7 +2109,7 @@ extern "C" int salsaa_sumcheck(const uint64_t* d_w, uint64_t rows, uint64_t n, u
   t.want(&B.cap, 2ULL * rows * d);
   t.want(&ds, 1);
   TRY(t.alloc());
-  set_seed_kernel<<<1, 32, 0, st>>>(ds, seed);
+  pdl(set_seed_kernel, 1, 32, 0, st)(ds, seed);
   const u64 nr = ilog2u(n);
   RowSet w = rows_of(d_w, (u32)rows, n / d, (u32)d);
   return launch_sumcheck(w, (u32)rows, n, (u32)d, make_modq(q), ds, (u32)round, B, d_claims, d_polys,
@@ -2144,7 +2145,7 @@ extern "C" int salsaa_project(const uint64_t* d_w, uint64_t rows, uint64_t width
   t.want(&nm, 256 * cw / 32);
   t.want(&J, 256 * cw);
   TRY(t.alloc());
-  set_seed_kernel<<<1, 32, 0, st>>>(ds, seed);
+  pdl(set_seed_kernel, 1, 32, 0, st)(ds, seed);
   TRY(launch_proj_tables(ds, (u32)round, (u32)cw, pm, nm, J, nullptr, q, st));
   RowSet w = rows_of(d_w, (u32)rows, width, (u32)d);
   return launch_project(w, (u32)rows, width, (u32)d, q, pm, nm, J, ds, d_out, st);

@@ -45,6 +45,7 @@ template <u32 D>
 __global__ void __launch_bounds__(FT_THREADS, 1)
     fold_tc_kernel(C8Rows w, const int8_t* __restrict__ tz, u64 q, u64* __restrict__ out, u64* mag_or,
                    const u32* flag, u32* err) {
+  pdl_wait();
   using Geo = FtGeom<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[Geo::STAGES], empty_bar[Geo::STAGES], acc_full[2], acc_empty[2], tz_bar;
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
 // Byte (r8, kk) of block b of row k: coefficient delta = d - 8 - 8 b + r8 - kk
 // of the challenge, negated and moved by d when delta < 0.
 __global__ void fold_chal_tz_kernel(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c, int8_t* tz) {
+  pdl_wait();
   const u64 key = prf_key(ds->seed, domain_id(DOM_FOLD, round, 0));
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < rows * d) {
@@ -217,6 +219,7 @@ constexpr u32 ST_A = 64 * 128, ST_STAGE = ST_A + 64 * 128;
 __global__ void __launch_bounds__(ST_THREADS, 1)
     sc_tc_kernel(Sc8Rows w, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl, const u64* s_hi, ModQ M,
                  u64* acc, const uint8_t* __restrict__ img, u32* err) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[ST_STAGES], empty_bar[ST_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tslot;
@@ -377,6 +380,7 @@ constexpr u32 PT_A = 64 * 128, PT_STAGE = PT_A + 64 * PT_ROWS;
 __global__ void __launch_bounds__(PT_THREADS, 1)
     project_tc_kernel(C8Rows w, u32 d, u64 q, u32 cw, u32 nch, u32 nsplit, const int8_t* __restrict__ Jc,
                       u64* __restrict__ out, const u32* wide, u32* err) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[PT_STAGES], empty_bar[PT_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tslot;
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1)
 int launch_fold_challenge_tz(const DevState* ds, u32 round, u32 rows, u32 d, u64 q, u64* c_coef, int8_t* tz,
                              cudaStream_t st) {
   const u32 tot = rows * 32 * d;
-  fold_chal_tz_kernel<<<(tot + 255) / 256, 256, 0, st>>>(ds, round, rows, d, q, c_coef, tz);
+  pdl(fold_chal_tz_kernel, (tot + 255) / 256, 256, 0, st)(ds, round, rows, d, q, c_coef, tz);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_challenge_tz");
@@ -516,7 +520,7 @@ int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u6
   auto kern = d == 128 ? fold_tc_kernel<128> : fold_tc_kernel<256>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "fold_tc smem attribute");
-  kern<<<grid, FT_THREADS, smem, st>>>(w, tz, q, out, mag_or, flag, tc_error_word());
+  pdl(kern, grid, FT_THREADS, smem, st)(w, tz, q, out, mag_or, flag, tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_tc launch");
@@ -539,7 +543,7 @@ int launch_project_tc(const C8Rows& w, u32 d, u64 q, u32 cw, const int8_t* Jc, u
   const size_t smem = (size_t)PT_STAGES * PT_STAGE;
   cudaError_t e = cudaFuncSetAttribute(project_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project_tc smem attribute");
-  project_tc_kernel<<<items < 148 ? items : 148, PT_THREADS, smem, st>>>(w, d, q, cw, nch, nsplit, Jc, out, wide,
+  pdl(project_tc_kernel, items < 148 ? items : 148, PT_THREADS, smem, st)(w, d, q, cw, nch, nsplit, Jc, out, wide,
                                                                          tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();
@@ -561,7 +565,7 @@ int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRow
   const size_t smem = (size_t)ST_STAGES * ST_STAGE;
   cudaError_t e = cudaFuncSetAttribute(sc_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tc smem attribute");
-  sc_tc_kernel<<<(unsigned)(items < 148 ? items : 148), ST_THREADS, smem, st>>>(w, rows, d, Bw, nhi, split, tl, s_hi, M,
+  pdl(sc_tc_kernel, (unsigned)(items < 148 ? items : 148), ST_THREADS, smem, st)(w, rows, d, Bw, nhi, split, tl, s_hi, M,
                                                                                 acc, img, tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();
