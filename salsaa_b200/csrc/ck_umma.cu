@@ -713,22 +713,22 @@ constexpr u32 SU_A = 128 * SU_KS;                   // scalar byte tile (16 KiB)
 constexpr u32 SU_B = SU_POS * SU_KS;                // one limb tile (16 KiB)
 constexpr u32 SU_STAGE = SU_A + SU_LIMBS * SU_B;    // 64 KiB
 
-__global__ void sc_img_kernel(const u64* s_lo, u32 Bw, ScRowList tl, uint8_t* img) {
+__global__ void sc_img_kernel(const u64* s_lo, u32 Bw, ScRange rg, uint8_t* img) {
   pdl_wait();
-  const u64 tot = (u64)Bw * 128;  // (chunk, slice, row, byte) = Bw / 128 x 8 x 128 x 16
-  for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (u64)gridDim.x * blockDim.x) {
-    const u32 b = (u32)(t % 16), row = (u32)((t / 16) % 128), sl = (u32)((t / 2048) % 8), cc = (u32)(t / 16384);
+  const u32 tot = Bw * 128 * rg.groups();  // (group, chunk, slice, row, byte) = groups x Bw / 128 x 8 x 128 x 16
+  for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += gridDim.x * blockDim.x) {
+    const u32 b = t % 16, row = t / 16 % 128, sl = t / 2048 % 8, cc = t / 16384 % (Bw / 128), g = t / (Bw * 128);
     uint8_t v = 0;
-    if (row < tl.n * 8 && row % 8 < 7) {
+    if (row < rg.rows(g) * 8 && row % 8 < 7) {
       const u32 r = row / 8, x = row % 8;
-      v = (uint8_t)(s_lo[(u64)tl.idx[r] * Bw + cc * 128 + sl * 16 + b] >> (8 * x));
+      v = (uint8_t)(s_lo[(u64)(rg.first(g) + r) * Bw + cc * 128 + sl * 16 + b] >> (8 * x));
     }
     img[t] = v;
   }
 }
 
 __global__ void __launch_bounds__(512, 1)
-    sc_umma_kernel(RowSet wc, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl,
+    sc_umma_kernel(RowSet wc, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRange rg,
                    const uint8_t* __restrict__ img0, const u64* s_lo, const u64* s_hi, ModQ M, u64* acc, bool plain,
                    ScGates gates) {
   pdl_wait();
@@ -757,16 +757,18 @@ __global__ void __launch_bounds__(512, 1)
   bool ok = true;
   // work items: positions pb, element block hb (one s_hi factor), its part sub
   // of split, witness row k; g0 counts the steps of earlier items
-  const u32 npb = d / SU_POS, items = npb * nhi * split * rows;
+  // and group of scalar rows
+  const u32 npb = d / SU_POS, per = npb * nhi * split * rows, items = per * rg.groups();
   u32 g0 = 0;
   for (u32 item = blockIdx.x; item < items; item += gridDim.x) {
-  const u32 pb = item % npb, hs = item / npb % (nhi * split), k = item / (npb * nhi * split);
+  const u32 pb = item % npb, hs = item / npb % (nhi * split), k = item / (npb * nhi * split) % rows;
+  const u32 grp = item / per, nrow = rg.rows(grp), j0 = rg.first(grp);
   const u32 hb = hs / split, sub = hs % split;
   if (!gates.open(k)) continue;
   const u32 c0 = sub * nsteps;
   const bool nar = (wc.narrow >> k) & 1;
   const u64* src0 = row_advance(wc.p[k], nar, ((u64)hb * Bw + (u64)c0 * SU_KS) * d + (u64)pb * SU_POS);
-  const uint8_t* img = img0 + (u64)c0 * SU_A;
+  const uint8_t* img = img0 + (u64)grp * Bw * 128 + (u64)c0 * SU_A;
   bool bad = false;
   // task of this thread: 16 consecutive elements x 2 neighbouring positions,
   // one 16-byte load per element for word rows (two u64 values) and one
@@ -879,19 +881,19 @@ __global__ void __launch_bounds__(512, 1)
   __syncthreads();
   if (ok && !bad) {
     const u64* Pm = (const u64*)smem;
-    for (u32 t = tid; t < tl.n * SU_POS; t += 512) {
+    for (u32 t = tid; t < nrow * SU_POS; t += 512) {
       const u32 r = t / SU_POS, pos = t % SU_POS;
       u64 v = 0;
 #pragma unroll
       for (u32 x = 0; x < 7; x++) v = salsaa::add_mod(v, Pm[(u64)(r * 8 + x) * 128 + pos], q);
-      const u32 j = tl.idx[r];
+      const u32 j = j0 + r;
       v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
       atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
     }
   }
   if (ok && bad) {  // exact CUDA-core sums of this item
-    for (u32 t = tid; t < tl.n * SU_POS; t += 512) {
-      const u32 r = t / SU_POS, pos = t % SU_POS, j = tl.idx[r];
+    for (u32 t = tid; t < nrow * SU_POS; t += 512) {
+      const u32 r = t / SU_POS, pos = t % SU_POS, j = j0 + r;
       u64 v = 0;
       for (u32 i = 0; i < nsteps * SU_KS; i++)
         v = salsaa::add_mod(v, mul_mod(M, s_lo[(u64)j * Bw + c0 * SU_KS + i], wres(src0, nar, (u64)i * d + pos, q)), q);
@@ -912,28 +914,27 @@ __global__ void __launch_bounds__(512, 1)
 
 
 
-int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cudaStream_t st) {
-  const u64 g = ((u64)Bw * 128 + 255) / 256;
-  pdl(sc_img_kernel, (unsigned)(g < 4096 ? g : 4096), 256, 0, st)(s_lo, Bw, tl, img);
+int launch_sc_img(const u64* s_lo, u32 Bw, const ScRange& rg, uint8_t* img, cudaStream_t st) {
+  const u64 g = ((u64)Bw * 128 * rg.groups() + 255) / 256;
+  pdl(sc_img_kernel, (unsigned)(g < 4096 ? g : 4096), 256, 0, st)(s_lo, Bw, rg, img);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_img launch");
 }
 
-int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_lo,
+int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRange& rg, const u64* s_lo,
                    const u64* s_hi, const ModQ& M, u64* acc, bool plain, const uint8_t* img, const ScGates& gates,
                    cudaStream_t st) {
-  if (tl.n == 0 || tl.n > SC_UMMA_MAX_ROWS) return salsaa_set_error(-2, "sc_umma: too many rows in one pass");
   // short witnesses: split each element block over several CTAs (linear sums)
   // while the items stay within one wave (one CTA per SM)
   const u64 base = (u64)(d / SU_POS) * nhi * rows;
   u32 split = 1;
   while (split * 2 <= Bw / SU_KS && base * split * 2 <= 148) split *= 2;
-  const u64 items = base * split;
+  const u64 items = base * split * rg.groups();
   const size_t smem = 2 * (size_t)SU_STAGE;
   cudaError_t e = cudaFuncSetAttribute(sc_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_umma smem attribute");
-  pdl(sc_umma_kernel, (unsigned)(items < 148 ? items : 148), 512, smem, st)(wc, rows, d, Bw, nhi, split, tl, img, s_lo,
+  pdl(sc_umma_kernel, (unsigned)(items < 148 ? items : 148), 512, smem, st)(wc, rows, d, Bw, nhi, split, rg, img, s_lo,
                                                                            s_hi, M, acc, plain, gates);
   salsaa_count_launch();
   e = cudaGetLastError();

@@ -986,6 +986,12 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
 
 constexpr u64 SC_GRAM_TILES = 296;
 
+static bool sc_pass_ok(u64 len, u32 d) { return len > SC_TAIL_ONE && (len >> SC_T) >= d; }
+
+bool sumcheck_reads_bytes(const C8Rows& w8, u64 nlen, u32 d, u64 q) {
+  return sc_pass_ok(nlen, d) && gram_words_ok(nlen, q) && gram_c8_ok(w8, d, q);
+}
+
 template <bool LAZY>
 static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
                            SumcheckBufs B, u32 nr, bool plain, cudaStream_t st, const C8Rows* w8, const u32* wide,
@@ -1003,7 +1009,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     u64 g = (groups + 255) / 256;
     return (unsigned)(g < want ? (g ? g : 1) : want);
   };
-  auto pass_ok = [d](u64 len) { return len > SC_TAIL_ONE && (len >> SC_T) >= d; };
+  auto pass_ok = [d](u64 len) { return sc_pass_ok(len, d); };
   GramList gl{};
   u64 go = 2ULL * nr * rows * 3;  // words used behind the sums
   auto gram_room = [&](u32 n) { return gl.n < SC_GRAM_PASSES && go + (u64)n * 256 <= B.sums_words; };
@@ -1021,7 +1027,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     int rc = 0;
     if (gram_room(rows) && gram_words_ok(L, M.q)) {
       u64* g = gram_take(rows, 1);
-      const bool c8 = w8 && wide && gram_c8_ok(*w8, d, M.q);
+      const bool c8 = w8 && wide && sumcheck_reads_bytes(*w8, L, d, M.q);
       if (c8 && (rc = launch_gram_c8(*w8, d, M, ds, round, B.a, sa, g, wide, st))) return rc;
       if ((rc = launch_gram_first(w, rows, L, M, ds, round, B.a, sa, g, c8 ? wide : nullptr, st))) return rc;
     } else {
@@ -2511,7 +2517,7 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
       if (a.sc_types_host[j] == ROW_TENSOR) tl.idx[tl.n++] = (unsigned char)j;
       else ol.idx[ol.n++] = (unsigned char)j;
     }
-    // one tensor-core pass over the coefficient-form witness per 16 rows when
+    // one tensor-core pass over the coefficient-form witness per 16 or 32 rows when
     // the shapes fit (every scalar row weighs element i by s_hi[i / Bw]
     // s_lo[i % Bw]), else CUDA cores, the periodic / all-ones rows over column
     // sums; rows of byte tiles take the byte pass, the others this one
@@ -2519,19 +2525,19 @@ int launch_commit(const CommitArgs& a, const NttDev& T, const ModQ& M, const Dev
                        rowset_aligned(wsrc, a.rows, 16, 8) && (tl.n > 0 || a.sc8);
     bool periodic_done = false;
     if (tc_ok) {
-      for (u32 j0 = 0; j0 < a.nsc; j0 += SC_UMMA_MAX_ROWS) {
-        ScRowList gl{};
-        for (u32 j = j0; j < a.nsc && j < j0 + SC_UMMA_MAX_ROWS; j++) gl.idx[gl.n++] = (unsigned char)j;
-        rc = launch_sc_img(a.sc_lo, Bw, gl, a.sc_img, ss);
+      const u32 pass = SC_UMMA_MAX_ROWS * (a.sc_img_groups > 1 ? 2 : 1);
+      for (u32 j0 = 0; j0 < a.nsc; j0 += pass) {
+        const ScRange rg{j0, a.nsc - j0 < pass ? a.nsc - j0 : pass};
+        rc = launch_sc_img(a.sc_lo, Bw, rg, a.sc_img, ss);
         if (rc) return rc;
         ScGates gates{};
         gates.rows = a.rows;
         if (a.sc8) {
           for (u32 k = 0; k < a.rows; k++) gates.gate[k] = a.sc8->wide[k];
-          rc = launch_sc_tc(*a.sc8, a.rows, d, Bw, nhi, gl, a.sc_hi, M, acc_sc, a.sc_img, ss);
+          rc = launch_sc_tc(*a.sc8, a.rows, d, Bw, nhi, rg, a.sc_hi, M, acc_sc, a.sc_img, ss);
           if (rc) return rc;
         }
-        rc = launch_sc_umma(wsrc, a.rows, d, Bw, nhi, gl, a.sc_lo, a.sc_hi, M, acc_sc, plain, a.sc_img, gates, ss);
+        rc = launch_sc_umma(wsrc, a.rows, d, Bw, nhi, rg, a.sc_lo, a.sc_hi, M, acc_sc, plain, a.sc_img, gates, ss);
         if (rc) return rc;
       }
       periodic_done = true;

@@ -102,6 +102,17 @@ int launch_ck_tk8(const u64* tlo, u32 nck, u32 n, u32 bt, bool packed, uint8_t* 
 // TENSOR rows on tcgen05 over the coefficient-form witness (see ck_umma.cu).
 constexpr u64 SC_IMG_BYTES = (u64)CK_BLOCK * 128;
 constexpr u32 SC_UMMA_MAX_ROWS = 16;
+// The n <= 32 statement rows from j0 on, in groups of SC_UMMA_MAX_ROWS (one
+// image of Bw x 128 bytes and one accumulator each) of one launch.
+struct ScRange {
+  u32 j0, n;
+  __host__ __device__ u32 groups() const { return (n + SC_UMMA_MAX_ROWS - 1) / SC_UMMA_MAX_ROWS; }
+  __host__ __device__ u32 first(u32 g) const { return j0 + g * SC_UMMA_MAX_ROWS; }
+  __host__ __device__ u32 rows(u32 g) const {
+    const u32 r = n - g * SC_UMMA_MAX_ROWS;
+    return r < SC_UMMA_MAX_ROWS ? r : SC_UMMA_MAX_ROWS;
+  }
+};
 // Which witness rows a pass takes: row k runs if gate[k] is null or *gate[k] != 0.
 struct ScGates {
   const u32* gate[MAX_WROWS];
@@ -114,8 +125,8 @@ struct ScGates {
   }
 };
 // img: the byte image of the rows' scalars (launch_sc_img), 8 operand rows each.
-int launch_sc_img(const u64* s_lo, u32 Bw, const ScRowList& tl, uint8_t* img, cudaStream_t st);
-int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_lo,
+int launch_sc_img(const u64* s_lo, u32 Bw, const ScRange& rg, uint8_t* img, cudaStream_t st);
+int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRange& rg, const u64* s_lo,
                    const u64* s_hi, const ModQ& M, u64* acc, bool plain, const uint8_t* img, const ScGates& gates,
                    cudaStream_t st);
 // Nonzero (and the last error set) when a tensor-core kernel's bounded wait gave up.
@@ -144,6 +155,8 @@ inline u64 gram_words(u64 rows) { return rows * 256 * (1 + 2 * (SC_GRAM_PASSES -
 int launch_sumcheck(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const DevState* ds, u32 round,
                     SumcheckBufs B, u64* proof_claims, u64* proof_rep0, u64* proof_rep1, cudaStream_t st,
                     const struct C8Rows* w8 = nullptr, const u32* wide = nullptr);
+// Whether launch_sumcheck reads the byte tiles only while they are valid.
+bool sumcheck_reads_bytes(const struct C8Rows& w8, u64 nlen, u32 d, u64 q);
 // Independent sumchecks of `count` <= 64 vectors of power-of-two lengths (one
 // repetition each; instance i uses the norm-check challenges of (round, i)):
 // claims[i] and the round polynomials of instance i at polys + 3 * sum_{i'<i} log2 len.
@@ -215,7 +228,8 @@ struct CommitArgs {
   u32 nsc;           // scalar rows
   const ScalarRowDesc* sc_desc_dev;  // nsc descriptors in device memory
   const int* sc_types_host;          // their types, on the host (required when nsc > 0)
-  uint8_t* sc_img;   // scratch for the tcgen05 TENSOR-row pass (SC_IMG_BYTES), or null
+  uint8_t* sc_img;   // scratch of the tensor-core passes over statement rows, or null
+  u32 sc_img_groups; // groups of rows it holds (SC_IMG_BYTES each): those of one pass
   const struct Sc8Rows* sc8;  // the rows wc as byte tiles where they are short (short_tc.cuh), or null
   cudaStream_t st2;  // optional: statement rows on this stream beside the key rows
   cudaEvent_t ev_fork, ev_join;

@@ -177,9 +177,9 @@ struct Shapes {
 };
 
 // Words of a slot's byte-tile buffers: the witness rows, the projected row's
-// two limbs, the fold challenges' blocks.
+// two limbs, the fold challenges' blocks, a second group of statement rows.
 static u64 short_words(u64 d_rows_width, u64 fp_width, u64 d) {
-  return d_rows_width * d / 8 + 2 * fp_width * d / 8 + fold_tz_bytes(8, (u32)d) / 8;
+  return d_rows_width * d / 8 + 2 * fp_width * d / 8 + fold_tz_bytes(8, (u32)d) / 8 + SC_IMG_BYTES / 8;
 }
 
 static Shapes walk(const salsaa_params* p) {
@@ -568,7 +568,7 @@ extern "C" int salsaa_prover_create(salsaa_ctx* c, salsaa_prover** out) {
       (rc = m.alloc(&pr->nmask, 256ULL * CK_BLOCK / 32, "neg mask")) ||
       (rc = m.alloc(&pr->Jm, 256ULL * CK_BLOCK, "projection J")) ||
       (rc = m.alloc(&pr->Jc, 256ULL * CK_BLOCK, "projection J (tensor-core layout)")) ||
-      (rc = m.alloc(&pr->sc_img, SC_IMG_BYTES, "scalar-row byte image")) ||
+      (rc = m.alloc(&pr->sc_img, SC_IMG_BYTES * (S.use_short ? 2 : 1), "scalar-row byte images")) ||
       (rc = m.alloc(&pr->c_coef, (u64)MAX_WROWS * d, "fold c")) ||
       (rc = m.alloc(&pr->c_slot, (u64)MAX_WROWS * d, "fold c slot")) ||
       (rc = m.alloc(&pr->fold_pre, (u64)MAX_WROWS * (d / 2) * 6, "fold constants")) ||
@@ -716,6 +716,7 @@ static int commit_rows_slot(salsaa_prover* pr, const RowSet& ws, const RowSet* w
   a.colsum = pr->colsum;
   a.colsum_rows = c->S.max_rows + 1;  // the merged split/projection pass has 2K + 1 rows
   a.sc_img = pr->sc_img;
+  a.sc_img_groups = c->S.use_short ? 2 : 1;
   a.sc8 = sc8;
   if (pr->overlap) {
     a.st2 = pr->st2;
@@ -787,9 +788,10 @@ static Sc8Rows sc8_rows(const salsaa_prover* pr, u32 K, u64 width, u32 d, bool s
 // decomp_ell into two digits, as centred int32 coefficients (Dc), the image
 // rows and, with slots, slot-form words.  With wide, digits of at most 7 bits
 // go through the tensor cores (and to pr->c8, without slot-form words); else
-// *wide is raised and the FP64 kernel does the round.
+// *wide is raised and the FP64 kernel does the round.  words: something reads
+// Dc also while the digits are short.
 static int decompose_image(salsaa_prover* pr, const RowSet& src, u32 rows, u64 width, u32 didx, bool split, u64* slots,
-                           u64* proof_radix, const CkImage& im, u32* wide) {
+                           u64* proof_radix, const CkImage& im, u32* wide, bool words) {
   ImgDigits a{};
   for (u32 k = 0; k < rows; k++) a.rows.src[k] = src.p[k];
   a.rows.rows = rows;
@@ -805,7 +807,7 @@ static int decompose_image(salsaa_prover* pr, const RowSet& src, u32 rows, u64 w
     t.rows = a.rows;
     t.flag = wide;
     t.c8 = pr->c8;
-    t.coef = a.coef;
+    t.coef = words ? a.coef : nullptr;
     t.bw_or = a.bw_or;
     t.rlog_out = a.rlog_out;
     t.radix_out = a.radix_out;
@@ -912,7 +914,12 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       if (imp) {
         if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
         image(2 * parts * K + 1, width / 2);
-        TRY(decompose_image(pr, Wc, K, width, didx++, true, pr->Ds, proof + cur, im, sh ? &pr->ds->wide[rd] : nullptr));
+        // every step of a round over byte tiles leaves Dc alone, but for the
+        // norm check and the statement rows of the narrowest witnesses
+        const bool words = !sh || !sumcheck_reads_bytes(c8_rows(pr->c8, parts * K, width, d, false), width * d, d, q) ||
+                           width % 256;
+        TRY(decompose_image(pr, Wc, K, width, didx++, true, pr->Ds, proof + cur, im, sh ? &pr->ds->wide[rd] : nullptr,
+                            words));
         narrow = true;
       } else {
         TRY(launch_decompose_ntt(Wc, K, width, d, q, parts, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,
@@ -1150,7 +1157,8 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       if (imp) {
         if (!mag_ready) return salsaa_set_error(-9, "enqueue: digits before their magnitudes");
         image(2 * K, width);
-        TRY(decompose_image(pr, Wc, K, width, didx++, false, nullptr, proof + cur, im, sh ? &pr->ds->wide[rd + 1] : nullptr));
+        TRY(decompose_image(pr, Wc, K, width, didx++, false, nullptr, proof + cur, im,
+                            sh ? &pr->ds->wide[rd + 1] : nullptr, !sh || width % 128));
         narrow = true;
       } else {
         TRY(launch_decompose_ntt(Wc, K, width, d, q, 2, didx++, pr->ds, pr->Dc, pr->Ds, proof + cur, T, st,

@@ -209,7 +209,7 @@ __global__ void fold_chal_tz_kernel(const DevState* ds, u32 round, u32 rows, u32
 // (byte row, positions) changes, then adds them to the accumulators.  Where
 // sc_umma_kernel turns every value into three byte limbs, here both operands
 // are bulk copies.  Bound by the copies' latency and L2 traffic: 16 KB per 64
-// elements with 16 rows.  Together with the products that the proof no longer
+// elements with 16 rows; a launch takes two groups of 16 rows.  Together with the products that the proof no longer
 // recomputes (<projected_lhs, folded> is a combination of <projected_lhs, w_k>):
 // 1222 -> 374 us of an 8-round proof over 2^19 elements, d = 128.
 // ---------------------------------------------------------------------------
@@ -217,17 +217,21 @@ constexpr u32 ST_EPI = 256, ST_THREADS = ST_EPI + 64, ST_STAGES = 8;
 constexpr u32 ST_A = 64 * 128, ST_STAGE = ST_A + 64 * 128;
 
 __global__ void __launch_bounds__(ST_THREADS, 1)
-    sc_tc_kernel(Sc8Rows w, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRowList tl, const u64* s_hi, ModQ M,
+    sc_tc_kernel(Sc8Rows w, u32 rows, u32 d, u32 Bw, u32 nhi, u32 split, ScRange rg, const u64* s_hi, ModQ M,
                  u64* acc, const uint8_t* __restrict__ img, u32* err) {
   pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[ST_STAGES], empty_bar[ST_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tslot;
   const u32 tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const u32 npb = d / 128, per = nhi * split, items = w.w.rows * npb * per;
+  const u32 npb = d / 128, per = nhi * split, items = w.w.rows * npb * per * rg.groups();
   const u32 i0 = (u32)((u64)blockIdx.x * items / gridDim.x), i1 = (u32)((u64)(blockIdx.x + 1) * items / gridDim.x);
-  const u32 steps = Bw / 64 / split, np = (tl.n * 8 + 15) / 16 * 16;  // N, whole 16-column groups
-  auto open = [&](u32 item) { return *w.wide[w.dst[item / (npb * per)]] == 0; };
+  const u32 steps = Bw / 64 / split;
+  // item: (group of scalar rows, byte row, positions, elements)
+  auto brow = [&](u32 rp) { return rp / npb % w.w.rows; };
+  auto group = [&](u32 rp) { return rp / npb / w.w.rows; };
+  auto open = [&](u32 item) { return *w.wide[w.dst[brow(item / per)]] == 0; };
+  auto ncol = [&](u32 g) { return (rg.rows(g) * 8 + 15) / 16 * 16; };  // N, whole 16-column groups
   if (tid == 0) {
     for (u32 i = 0; i < ST_STAGES; i++) {
       umma::mbar_init(&full_bar[i], 1);
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
     u32 it = 0, st = 0, par = 1;
     for (u32 item = i0; ok && item < i1; item++) {
       if (!open(item)) continue;
-      const u32 hs = item % per, rp = item / per, pb = rp % npb, r = rp / npb;
+      const u32 hs = item % per, rp = item / per, pb = rp % npb, r = brow(rp), g = group(rp), np = ncol(g);
       const u32 e0 = hs / split * Bw + hs % split * steps * 64, l0 = hs % split * steps * 64;
       const int8_t* src = w.w.p + w.w.row[r] * w.w.stride + (w.w.off[r] + e0) * d + pb * ST_A;
       for (u32 c = 0; c < steps; c++, it++) {
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
           uint8_t* stage = smem + st * ST_STAGE;
           umma::mbar_expect_tx(&full_bar[st], ST_A + 4 * np * 16);
           umma::bulk_g2s(stage, src + (u64)c * 64 * d, ST_A, &full_bar[st]);
-          const uint8_t* im = img + (u64)(l0 / 16 + 4 * c) * 2048;
+          const uint8_t* im = img + (u64)g * Bw * 128 + (u64)(l0 / 16 + 4 * c) * 2048;
           for (u32 j = 0; j < 4; j++)
             umma::bulk_g2s(stage + ST_A + j * 2048, im + j * 2048, np * 16, &full_bar[st]);
         }
@@ -275,7 +279,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
   } else if (warp == ST_EPI / 32 + 1) {
     // A: s8, MN-major (position slices 1024 apart, 8-element blocks 128);
     // B: u8, K-major
-    const u32 idesc = (2u << 4) | (1u << 7) | (1u << 15) | ((np >> 3) << 17) | ((128u >> 4) << 24);
     const uint64_t ad0 = umma::desc_kmajor(umma::smem_u32(smem), 128, 1024);
     const uint64_t bd0 = umma::desc_kmajor(umma::smem_u32(smem + ST_A), 2048, 128);
     bool ok = true;
@@ -283,6 +286,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
     for (u32 item = i0; ok && item < i1; item++) {
       if (!open(item)) continue;
       const u32 nb = ui & 1;
+      const u32 idesc = (2u << 4) | (1u << 7) | (1u << 15) | ((ncol(group(item / per)) >> 3) << 17) | ((128u >> 4) << 24);
       if (ui >= 2 && !(ok = umma::mbar_wait(&acc_empty[nb], ((ui >> 1) - 1) & 1, err, 53))) break;
       umma::fence_after_sync();
       for (u32 c = 0; c < steps; c++, it++) {
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
     for (u32 j = 0; j < 8; j++) sum[j] = 0;
     u32 ui = 0;
     for (u32 item = i0; item < i1; item++) {
-      const u32 hs = item % per, rp = item / per;
+      const u32 hs = item % per, rp = item / per, grp = group(rp), nrow = rg.rows(grp), j0 = rg.first(grp) + 8 * ch;
       if (open(item)) {
         const u32 nb = ui & 1;
         const bool ok = umma::mbar_wait(&acc_full[nb], (ui >> 1) & 1, err, 56);
@@ -324,14 +328,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
         uint32_t v[4][16];
 #pragma unroll
         for (u32 g = 0; g < 4; g++)
-          if (8 * ch + 2 * g < tl.n) umma::tmem_ld16(tb + g * 16, v[g]);
+          if (8 * ch + 2 * g < nrow) umma::tmem_ld16(tb + g * 16, v[g]);
         umma::tmem_wait_ld();
         umma::fence_before_sync();
         umma::mbar_arrive(&acc_empty[nb]);
         ui++;
 #pragma unroll
         for (u32 j = 0; j < 8; j++) {
-          if (8 * ch + j < tl.n) {
+          if (8 * ch + j < nrow) {
             const uint32_t* D = &v[j / 2][8 * (j & 1)];
             // |D_x| <= 2048 x 255 x 128 < 2^26
             const long long lo = (long long)(int)D[0] + ((long long)(int)D[1] << 8) + ((long long)(int)D[2] << 16) +
@@ -340,18 +344,18 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
             // |hi| < 2^43 < q; |lo| < 2^51 <= 16 q
             u64 x = mul_mod(M, hi < 0 ? (u64)(hi + (long long)q) : (u64)hi, p32);
             x = reduce64(M, x + (u64)(lo + (long long)(16 * q)));
-            x = mul_mod(M, x, __ldg(s_hi + (u64)tl.idx[8 * ch + j] * nhi + hs / split));
+            x = mul_mod(M, x, __ldg(s_hi + (u64)(j0 + j) * nhi + hs / split));
             sum[j] = add_mod(sum[j], x, q);
           }
         }
       }
       if (item + 1 == i1 || rp != (item + 1) / per) {  // the run of this byte row and these positions ends
-        const u32 pb = rp % npb, r = rp / npb, k = w.dst[r];
+        const u32 pb = rp % npb, r = brow(rp), k = w.dst[r];
         const u64 sc = ((u64)1 << w.shift[r]) % q;
 #pragma unroll
         for (u32 j = 0; j < 8; j++) {
-          if (8 * ch + j < tl.n && sum[j])
-            atomic_add_mod(acc + ((u64)tl.idx[8 * ch + j] * rows + k) * d + pb * 128 + m, mul_mod(M, sum[j], sc), q, true);
+          if (8 * ch + j < nrow && sum[j])
+            atomic_add_mod(acc + ((u64)(j0 + j) * rows + k) * d + pb * 128 + m, mul_mod(M, sum[j], sc), q, true);
           sum[j] = 0;
         }
       }
@@ -550,22 +554,22 @@ int launch_project_tc(const C8Rows& w, u32 d, u64 q, u32 cw, const int8_t* Jc, u
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "project_tc launch");
 }
 
-int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_hi,
+int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRange& rg, const u64* s_hi,
                  const ModQ& M, u64* acc, const uint8_t* img, cudaStream_t st) {
   // q above 2^47 for the bounds, below 2^50 so that plain adds of at most one
   // residue per CTA and byte row cannot overflow
-  if ((d != 128 && d != 256) || Bw % 64 || tl.n == 0 || tl.n > SC_UMMA_MAX_ROWS || M.q >= (1ULL << 50) ||
+  if ((d != 128 && d != 256) || Bw % 64 || rg.n == 0 || rg.groups() > 2 || M.q >= (1ULL << 50) ||
       M.q < (1ULL << 47) || w.w.rows == 0 || w.w.rows > (u32)MAX_WROWS || (u64)Bw * nhi > w.w.width)
     return salsaa_set_error(-2, "sc_tc: rows outside the byte-tile path");
   // few items: split each element block over several CTAs
   const u64 base = (u64)w.w.rows * (d / 128) * nhi;
   u32 split = 1;
   while (split * 4 <= Bw / 64 && base * split < 148) split *= 2;
-  const u64 items = base * split;
+  const u64 items = base * split * rg.groups();
   const size_t smem = (size_t)ST_STAGES * ST_STAGE;
   cudaError_t e = cudaFuncSetAttribute(sc_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tc smem attribute");
-  pdl(sc_tc_kernel, (unsigned)(items < 148 ? items : 148), ST_THREADS, smem, st)(w, rows, d, Bw, nhi, split, tl, s_hi, M,
+  pdl(sc_tc_kernel, (unsigned)(items < 148 ? items : 148), ST_THREADS, smem, st)(w, rows, d, Bw, nhi, split, rg, s_hi, M,
                                                                                 acc, img, tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();

@@ -42,7 +42,7 @@ struct Sc8Rows {
   u32 dst[MAX_WROWS], shift[MAX_WROWS];
   const u32* wide[MAX_WROWS];  // per witness row
 };
-int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRowList& tl, const u64* s_hi,
+int launch_sc_tc(const Sc8Rows& w, u32 rows, u32 d, u32 Bw, u32 nhi, const ScRange& rg, const u64* s_hi,
                  const ModQ& M, u64* acc, const uint8_t* img, cudaStream_t st);
 
 }  // namespace salsaa
