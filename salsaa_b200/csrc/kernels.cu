@@ -1523,7 +1523,13 @@ int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_
   const u64 nch = width / cw;
   if ((u64)rows * nch > 65535) return salsaa_set_error(-2, "project: too many chunks");
   const u64* gate = nullptr;
-  if (Jc && ds && d % 128 == 0 && cw % 128 == 0 && rowset_aligned(in, rows, 16, 8)) {
+  if (Jc && w8 && wide && !ds) {
+    // byte tiles made for this call: the exact kernel takes rows that do not fit
+    if (!project_tc_ok(*w8, d, cw)) return salsaa_set_error(-2, "project: byte tiles outside the tensor-core path");
+    int rc = launch_project_tc(*w8, d, q, cw, Jc, out, wide, st);
+    if (rc) return rc;
+    gate = (const u64*)wide;
+  } else if (Jc && ds && d % 128 == 0 && cw % 128 == 0 && rowset_aligned(in, rows, 16, 8)) {
     cudaError_t e = cudaMemsetAsync(&ds->proj_flag, 0, sizeof(u64), st);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "project memset");
     // short rows as byte tiles; then the words, only while they are wide

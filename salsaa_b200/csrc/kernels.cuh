@@ -191,7 +191,8 @@ int launch_proj_tables(const DevState* ds, u32 round, u32 cw, u32* pos_mask, u32
                        u64 q, cudaStream_t st, int8_t* Jc = nullptr);
 // Tensor-core path when d is a multiple of 128 and J is given; exact CUDA-core
 // recomputation (chosen on the device) whenever a value does not fit int8.
-// w8 and wide: the rows as byte tiles, valid while *wide is zero.
+// w8 and wide: the rows as byte tiles, valid while *wide is zero; without ds
+// the words are only read by the exact kernel, behind *wide (then 64 bits).
 int launch_project(RowSet in, u32 rows, u64 width, u32 d, u64 q, const u32* pos_mask, const u32* neg_mask,
                    const int8_t* J, DevState* ds, u64* out, cudaStream_t st, const int8_t* Jc = nullptr,
                    const struct C8Rows* w8 = nullptr, const u32* wide = nullptr);

@@ -367,6 +367,46 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
+// Words to byte tiles.  A warp takes 16 elements x 16 positions: eight lanes
+// read the 128 bytes of an element's 16 words, and after each lane has put
+// its bytes together (two a word pair, then eight lanes' by shuffles) every
+// 16-byte unit is one store and the warp's 256 bytes are one run.  Bound by
+// HBM: nine bytes a value.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u32 d, u64 q, int8_t* c8, u32* wide) {
+  pdl_wait();
+  const u32 lane = threadIdx.x & 31, k = blockIdx.y, npg = d / 16;
+  const u64 tasks = width / 16 * npg, half_q = q >> 1;
+  const u64* x = src.p[k];
+  int8_t* out = c8 + (u64)k * width * d;
+  bool bad = false;
+  for (u64 t = (u64)blockIdx.x * 8 + (threadIdx.x >> 5); t < tasks; t += (u64)gridDim.x * 8) {
+    const u64 eg = t / npg;
+    const u32 pg = (u32)(t % npg);
+    ulonglong2 v[4];
+#pragma unroll
+    for (u32 i = 0; i < 4; i++)
+      v[i] = __ldg((const ulonglong2*)(x + (eg * 16 + 4 * i + (lane >> 3)) * d + pg * 16 + 2 * (lane & 7)));
+#pragma unroll
+    for (u32 i = 0; i < 4; i++) {
+      const u64 a = v[i].x + 128 - (v[i].x > half_q ? q : 0), b = v[i].y + 128 - (v[i].y > half_q ? q : 0);
+      bad |= (a | b) > 255;
+      u32 p = ((u32)a & 255) | ((u32)b & 255) << 8;  // two bytes, then four, eight, sixteen
+      p ^= 0x8080u;
+      p |= __shfl_down_sync(0xffffffffu, p, 1) << 16;
+      const u32 p1 = __shfl_down_sync(0xffffffffu, p, 2);
+      const u32 p2 = __shfl_down_sync(0xffffffffu, p, 4);
+      const u32 p3 = __shfl_down_sync(0xffffffffu, p, 6);
+      if ((lane & 7) == 0) {
+        const u64 e = eg * 16 + 4 * i + (lane >> 3);
+        *(uint4*)(out + c8_offset(e, pg * 16, d)) = make_uint4(p, p1, p2, p3);
+      }
+    }
+  }
+  if (bad) *wide = 1;
+}
+
+// ---------------------------------------------------------------------------
 // Projection (project, src/subroutines/project.rs:50-103) over byte rows: per
 // (chunk of cw elements, 128 positions) D[position][J row] = sum_l w(l,
 // position) J[row][l], M = 128 positions (the byte tile MN-major), N = 256 J
@@ -528,6 +568,17 @@ int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u6
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_tc launch");
+}
+
+int launch_words_to_c8(const RowSet& src, u32 rows, u64 width, u32 d, u64 q, int8_t* c8, u32* wide, cudaStream_t st) {
+  if (src.narrow || rows == 0 || rows > (u32)MAX_WROWS || width % 64 || d % 16 || !rowset_aligned(src, rows, 16, 16))
+    return salsaa_set_error(-2, "words_to_c8: bad rows");
+  const u64 tasks = width / 16 * (d / 16);
+  const u64 want = (tasks + 7) / 8, most = 148 * 8;
+  pdl(words_to_c8_kernel, dim3((unsigned)(want < most ? want : most), rows), 256, 0, st)(src, width, d, q, c8, wide);
+  salsaa_count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "words_to_c8 launch");
 }
 
 bool project_tc_ok(const C8Rows& w, u32 d, u32 cw) {

@@ -34,6 +34,10 @@ bool project_tc_ok(const C8Rows& w, u32 d, u32 cw);
 int launch_project_tc(const C8Rows& w, u32 d, u64 q, u32 cw, const int8_t* Jc, u64* out, const u32* wide,
                       cudaStream_t st);
 
+// Byte tiles (rows one after the other) of the word rows src; raises *wide
+// when a value does not fit a byte.  width a multiple of 64, d of 16.
+int launch_words_to_c8(const RowSet& src, u32 rows, u64 width, u32 d, u64 q, int8_t* c8, u32* wide, cudaStream_t st);
+
 // Statement rows of launch_commit (kernels.cuh) over byte rows: byte row r
 // adds 2^shift[r] times its sums to witness row dst[r], unless *wide[dst[r]]
 // is nonzero (then launch_sc_umma takes that row).

@@ -106,3 +106,23 @@ def test_prove_short_and_wide(api, oracle, d, folding, rounds, log_wit, bound):
         pr.sync()
         assert np.array_equal(out.cpu().numpy(), want)
     pr.close()
+
+
+@pytest.mark.parametrize("d,rows,width,lo,hi,odd", [
+    (128, 1, 1 << 16, -128, 128, None),   # more chunks than CTAs: both accumulators and every ring wrap
+    (128, 8, 1 << 13, -128, -127, None),  # long chunks, a part of the output rows per CTA, the largest sums
+    (256, 3, 768 * 5, -128, 128, None),
+    (512, 2, 512, -1, 2, 128),            # one value past the byte
+    (128, 4, 4096, -1, 2, -129),
+])
+def test_project_tiles(api, oracle, d, rows, width, lo, hi, odd):
+    """Projection of word rows through byte tiles, or exactly when a value does not fit."""
+    from helpers import proj_challenge
+    q = Q[d]
+    v = np.random.default_rng(width + d).integers(lo, hi, size=(rows, width, d))
+    if odd is not None:
+        v[-1, -3, d - 5] = odd
+    w = np.where(v < 0, q + v, v).astype(np.uint64)
+    iz, sg = proj_challenge(5, 2, rows * 256)
+    want = oracle.project(w, q, iz, sg)
+    assert np.array_equal(api.to_host(api.project(api.to_dev(w), q, 5, 2)), want)
