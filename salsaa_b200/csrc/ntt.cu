@@ -479,8 +479,10 @@ __device__ __forceinline__ void nf_tile(const u64* in, u64* out, u64 units, u64 
 }
 
 template <int LOGN, bool INC, bool INV>
-__global__ void __launch_bounds__(256) ntt_fp_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or) {
+__global__ void __launch_bounds__(256) ntt_fp_kernel(const u64* in, u64* out, u64 units, NttDev T, u64* mag_or,
+                                                     const u32* gate) {
   pdl_wait();
+  if (gate && !*gate) return;
   __shared__ double sm[NR_TILE + NR_TILE / 16];
   nf_tile<LOGN, INC, INV>(in, out, units, blockIdx.x, T, mag_or, sm);
 }
@@ -488,8 +490,10 @@ __global__ void __launch_bounds__(256) ntt_fp_kernel(const u64* in, u64* out, u6
 // ---------------------------------------------------------------------------
 
 template <bool INV>
-__global__ void __launch_bounds__(256) ntt_fp6_kernel(const u64* in, u64* out, u64 count, NttDev T, u64* mag_or) {
+__global__ void __launch_bounds__(256) ntt_fp6_kernel(const u64* in, u64* out, u64 count, NttDev T, u64* mag_or,
+                                                      const u32* gate) {
   pdl_wait();
+  if (gate && !*gate) return;
   __shared__ double2 sm[NP6_EL * NP6_ROW];
   const u32 el = threadIdx.x >> 3, r = threadIdx.x & 7;
   const u64 eg = (u64)blockIdx.x * NP6_EL + el;
@@ -1109,21 +1113,22 @@ int np_launch(const u64* in, u64* out, u64 units, const NttDev& T, cudaStream_t 
 
 template <int LOGN>
 int nr_launch(const u64* in, u64* out, u64 units, const NttDev& T, bool incomplete, bool inverse, cudaStream_t st,
-              u64* mag_or) {
+              u64* mag_or, const u32* gate) {
   constexpr u32 UPT = NR_TILE >> LOGN;
   const u64 blocks = (units + UPT - 1) / UPT;
   if (blocks > 0x7fffffffULL) return salsaa_set_error(-2, "ntt: batch too large");
   const bool relax = T.q < NR_RELAX_Q;
   const NttChoice ch = ntt_choice(LOGN, incomplete, inverse, !relax, units * (1ULL << LOGN) >= NTT_LARGE_COEFFS);
-  if (ch.variant == 1 && relax) {  // FP64 butterflies
+  if (gate && (!relax || LOGN < 6 || LOGN > 7)) return salsaa_set_error(-2, "ntt: no gated transform of this shape");
+  if ((ch.variant == 1 || gate) && relax) {  // FP64 butterflies
     auto gof = [&](auto kern) -> int {
-      pdl(kern, (unsigned)blocks, 256, 0, st)(in, out, units, T, mag_or);
+      pdl(kern, (unsigned)blocks, 256, 0, st)(in, out, units, T, mag_or, gate);
       return 0;
     };
     if (LOGN == 6 && incomplete && np6_aligned(in, out, inverse)) {
       const u64 count = units / 2, g6 = (count + NP6_EL - 1) / NP6_EL;
-      if (inverse) pdl(ntt_fp6_kernel<true>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or);
-      else pdl(ntt_fp6_kernel<false>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or);
+      if (inverse) pdl(ntt_fp6_kernel<true>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or, gate);
+      else pdl(ntt_fp6_kernel<false>, (unsigned)g6, 256, 0, st)(in, out, count, T, mag_or, gate);
       return 0;
     }
     if (incomplete) {
@@ -1217,8 +1222,16 @@ bool ntt_mag_ok(const u64* in, const u64* out, const NttDev& T, bool incomplete)
   return aligned && T.n >= 16 && T.n <= (incomplete ? 2048u : 4096u);
 }
 
+bool ntt_gate_ok(const NttDev& T) {
+  if ((T.logn != 6 && T.logn != 7) || T.q >= NR_RELAX_Q) return false;
+  for (int large = 0; large < 2; large++)
+    for (int inv = 0; inv < 2; inv++)
+      if (ntt_choice(T.logn, true, inv != 0, false, large != 0).variant != 1) return false;
+  return true;
+}
+
 int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incomplete, bool inverse,
-               cudaStream_t st, u64* mag_or) {
+               cudaStream_t st, u64* mag_or, const u32* gate) {
   if (count == 0) return 0;
   const u32 d = incomplete ? 2 * T.n : T.n;
   if (ntt_mag_ok(in, out, T, incomplete)) {
@@ -1226,15 +1239,15 @@ int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incompl
     const int tr = salsaa_trace_begin("ntt_kernel", st, 16.0 * (double)count * d);
     int rc = 0;
     switch (T.logn) {
-      case 4: rc = nr_launch<4>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 5: rc = nr_launch<5>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 6: rc = nr_launch<6>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 7: rc = nr_launch<7>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 8: rc = nr_launch<8>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 9: rc = nr_launch<9>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 10: rc = nr_launch<10>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      case 11: rc = nr_launch<11>(in, out, units, T, incomplete, inverse, st, mag_or); break;
-      default: rc = nr_launch<12>(in, out, units, T, incomplete, inverse, st, mag_or); break;
+      case 4: rc = nr_launch<4>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 5: rc = nr_launch<5>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 6: rc = nr_launch<6>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 7: rc = nr_launch<7>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 8: rc = nr_launch<8>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 9: rc = nr_launch<9>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 10: rc = nr_launch<10>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      case 11: rc = nr_launch<11>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
+      default: rc = nr_launch<12>(in, out, units, T, incomplete, inverse, st, mag_or, gate); break;
     }
     salsaa_trace_end(tr, st);
     if (rc) return rc;
@@ -1242,7 +1255,7 @@ int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incompl
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "ntt launch");
   }
-  if (mag_or) return salsaa_set_error(-2, "ntt: magnitude OR needs the register path");
+  if (mag_or || gate) return salsaa_set_error(-2, "ntt: magnitude OR and gate need the register path");
   // 32 KiB of elements per CTA (at least one element).
   u32 epb = 4096 / d;
   if (epb == 0) epb = 1;

@@ -65,7 +65,10 @@ int ntt_error_check();  // a bounded wait of the pipelined transform gave up
 // magnitudes min(v, q - v) of the coefficient-form side (the input of a
 // forward, the output of an inverse transform) is OR-ed into *mag_or.
 int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incomplete, bool inverse,
-               cudaStream_t st, u64* mag_or = nullptr);
+               cudaStream_t st, u64* mag_or = nullptr, const u32* gate = nullptr);
+// Whether incomplete transforms of T take a gate: they then run only while
+// *gate is nonzero (16-byte aligned pointers).
+bool ntt_gate_ok(const NttDev& T);
 bool ntt_mag_ok(const u64* in, const u64* out, const NttDev& T, bool incomplete);
 
 // Up to NTT_MULTI_MAX batches (count[i] units of n, or ring elements of 2n in

@@ -1123,7 +1123,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       u32* wide = &pr->ds->wide[rd];
       const C8Rows w8 = c8_rows(pr->c8, K, width, d, !P.folding);
       TRY(launch_fold_challenge_tz(pr->ds, rd, K, d, q, pr->c_coef, pr->tz, st));
-      TRY(launch_fold_tc(w8, d, q, pr->tz, pr->Fc, mag, wide, st));
+      TRY(launch_fold_tc(w8, d, q, pr->tz, width, pr->Fc, mag, wide, st));
       TRY(ntt_launch(pr->c_coef, pr->c_slot, K, T, true, false, st));
       TRY(launch_fold(Ws, K, width, T, M, pr->c_slot, pr->fold_pre, pr->Fs, st, wide));
       TRY(ntt_inv_gated_launch(pr->Fs, pr->Fc, width, T, wide, mag, st));
@@ -2191,8 +2191,42 @@ extern "C" int salsaa_fold(const uint64_t* d_w, uint64_t rows, uint64_t width, u
   const NttDev* T = ntt_tables((u32)(d / 2), q);
   if (!T) return salsaa_set_error(-1, "fold: no NTT for (d, q)");
   cudaStream_t st = (cudaStream_t)stream;
-  Tmp t(st);
   u64 *ws, *cs, *fs, *pre;
+  // Long folds on the tensor cores in coefficient form, through byte tiles of
+  // the rows (an eighth of them more memory); rows or challenges that do not
+  // fit raise the flag and the transforms run, else they leave at once.  Those
+  // launches cost some 15 us, what the tensor cores win at 2^22 coefficients;
+  // 8 rows of 20001 x 128: 139 -> 64 us.
+  const RowSet w = rows_of(d_w, (u32)rows, width, (u32)d);
+  C8Rows b = c8_rows(nullptr, (u32)rows, c8_width(width), (u32)d, false);
+  if (rows * width * d >= (1ULL << 23) && rows <= 8 && (d == 128 || d == 256) && fold_tc_ok(b, (u32)d) &&
+      ntt_gate_ok(*T) && q > (1ULL << 32) && rowset_aligned(w, (u32)rows, 16, 16) &&
+      ((uintptr_t)d_c | (uintptr_t)d_out) % 16 == 0) {
+    Tmp t(st);
+    int8_t *c8, *tz;
+    u32* wide;
+    t.want(&ws, rows * width * d);
+    t.want(&cs, rows * d);
+    t.want(&fs, width * d);
+    t.want(&pre, rows * (d / 2) * 6);
+    t.want(&c8, rows * b.width * d);
+    t.want(&tz, fold_tz_bytes((u32)rows, (u32)d));
+    t.want(&wide, 2);
+    if (t.alloc() == 0) {
+      b.p = c8;
+      cudaError_t e = cudaMemsetAsync(wide, 0, sizeof(u32), st);
+      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "fold memset");
+      TRY(launch_fold_words_tz(d_c, (u32)rows, (u32)d, q, tz, wide, st));
+      TRY(launch_words_to_c8(w, (u32)rows, width, (u32)d, q, c8, wide, st));
+      TRY(launch_fold_tc(b, (u32)d, q, tz, width, d_out, nullptr, wide, st));
+      TRY(ntt_launch(d_w, ws, rows * width, *T, true, false, st, nullptr, wide));
+      TRY(ntt_launch(d_c, cs, rows, *T, true, false, st, nullptr, wide));
+      TRY(launch_fold(rows_of(ws, (u32)rows, width, (u32)d), (u32)rows, width, *T, make_modq(q), cs, pre, fs, st, wide));
+      return ntt_launch(fs, d_out, width, *T, true, true, st, nullptr, wide);
+    }
+    cudaGetLastError();  // no room for the tiles
+  }
+  Tmp t(st);
   t.want(&ws, rows * width * d);
   t.want(&cs, rows * d);
   t.want(&fs, width * d);

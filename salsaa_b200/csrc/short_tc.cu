@@ -43,7 +43,7 @@ struct FtGeom {
 
 template <u32 D>
 __global__ void __launch_bounds__(FT_THREADS, 1)
-    fold_tc_kernel(C8Rows w, const int8_t* __restrict__ tz, u64 q, u64* __restrict__ out, u64* mag_or,
+    fold_tc_kernel(C8Rows w, const int8_t* __restrict__ tz, u64 q, u64 nout, u64* __restrict__ out, u64* mag_or,
                    const u32* flag, u32* err) {
   pdl_wait();
   using Geo = FtGeom<D>;
@@ -155,12 +155,14 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
           umma::fence_before_sync();
           umma::mbar_arrive(&acc_empty[nb]);
         }
-        u64* dst = out + ((u64)unit * FT_EL + half * 32) * D + mt * 128 + p0;
+        const u64 e0 = (u64)unit * FT_EL + half * 32;
+        const u32 left = e0 + 32 <= nout ? 32 : (e0 < nout ? (u32)(nout - e0) : 0);
+        u64* dst = out + e0 * D + mt * 128 + p0;
 #pragma unroll
         for (u32 i = 0; i < 32; i++) {
           const int c = (int)v[i];
           mag |= (u32)(c < 0 ? -c : c);
-          dst[(u64)i * D] = (u64)(long long)c + (c < 0 ? q : 0);
+          if (i < left) dst[(u64)i * D] = (u64)(long long)c + (c < 0 ? q : 0);
         }
       }
     }
@@ -366,6 +368,23 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
+// The same blocks from words.
+__global__ void fold_words_tz_kernel(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* wide) {
+  pdl_wait();
+  const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= rows * 32 * d) return;
+  const u32 k = t / (32 * d), b = t / 128 % (d / 4), r8 = t / 16 % 8, kk = t % 16;
+  const int delta = (int)(d - 8 - 8 * b + r8) - (int)kk;
+  long long v = 0;
+  if (delta > -(int)d && delta < (int)d) {
+    const u64 x = c[(u64)k * d + (u32)(delta < 0 ? delta + (int)d : delta)];
+    v = (long long)(x - (x > (q >> 1) ? q : 0));
+    if (v > 127 || v < -127) *wide = 1;
+    if (delta < 0) v = -v;
+  }
+  tz[t] = (int8_t)v;
+}
+
 // ---------------------------------------------------------------------------
 // Words to byte tiles.  A warp takes 16 elements x 16 positions: eight lanes
 // read the 128 bytes of an element's 16 words, and after each lane has put
@@ -373,20 +392,24 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
 // 16-byte unit is one store and the warp's 256 bytes are one run.  Bound by
 // HBM: nine bytes a value.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u32 d, u64 q, int8_t* c8, u32* wide) {
+__global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u64 wpad, u32 d, u64 q, int8_t* c8, u32* wide) {
   pdl_wait();
   const u32 lane = threadIdx.x & 31, k = blockIdx.y, npg = d / 16;
-  const u64 tasks = width / 16 * npg, half_q = q >> 1;
+  const u64 tasks = wpad / 16 * npg, half_q = q >> 1;
   const u64* x = src.p[k];
-  int8_t* out = c8 + (u64)k * width * d;
-  bool bad = false;
+  int8_t* out = c8 + (u64)k * wpad * d;
   for (u64 t = (u64)blockIdx.x * 8 + (threadIdx.x >> 5); t < tasks; t += (u64)gridDim.x * 8) {
+    // a warp that meets a wide value stops, and so do those that see the flag
+    if (__any_sync(0xffffffffu, *(volatile u32*)wide != 0)) break;
+    bool bad = false;
     const u64 eg = t / npg;
     const u32 pg = (u32)(t % npg);
     ulonglong2 v[4];
 #pragma unroll
-    for (u32 i = 0; i < 4; i++)
-      v[i] = __ldg((const ulonglong2*)(x + (eg * 16 + 4 * i + (lane >> 3)) * d + pg * 16 + 2 * (lane & 7)));
+    for (u32 i = 0; i < 4; i++) {
+      const u64 e = eg * 16 + 4 * i + (lane >> 3);
+      v[i] = e < width ? __ldg((const ulonglong2*)(x + e * d + pg * 16 + 2 * (lane & 7))) : make_ulonglong2(0, 0);
+    }
 #pragma unroll
     for (u32 i = 0; i < 4; i++) {
       const u64 a = v[i].x + 128 - (v[i].x > half_q ? q : 0), b = v[i].y + 128 - (v[i].y > half_q ? q : 0);
@@ -402,8 +425,9 @@ __global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width,
         *(uint4*)(out + c8_offset(e, pg * 16, d)) = make_uint4(p, p1, p2, p3);
       }
     }
+    if (bad) *(volatile u32*)wide = 1;
+    if (__any_sync(0xffffffffu, bad)) break;
   }
-  if (bad) *wide = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -554,9 +578,16 @@ bool fold_tc_ok(const C8Rows& w, u32 d) {
   return (d == 128 || d == 256) && w.rows >= 1 && w.rows <= 8 && w.width >= FT_EL && w.width % FT_EL == 0;
 }
 
-int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u64* mag_or, const u32* flag,
+int launch_fold_words_tz(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* wide, cudaStream_t st) {
+  pdl(fold_words_tz_kernel, (rows * 32 * d + 255) / 256, 256, 0, st)(c, rows, d, q, tz, wide);
+  salsaa_count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_words_tz launch");
+}
+
+int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64 nout, u64* out, u64* mag_or, const u32* flag,
                    cudaStream_t st) {
-  if (!fold_tc_ok(w, d) || !flag) return salsaa_set_error(-2, "fold_tc: rows outside the byte-tile path");
+  if (!fold_tc_ok(w, d) || !flag || nout > w.width) return salsaa_set_error(-2, "fold_tc: rows outside the byte-tile path");
   const size_t smem = (size_t)w.rows * 32 * d + (d == 128 ? (size_t)FtGeom<128>::STAGES * FtGeom<128>::TILE
                                                           : (size_t)FtGeom<256>::STAGES * FtGeom<256>::TILE);
   const u64 units = w.width / FT_EL;
@@ -564,18 +595,19 @@ int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64* out, u6
   auto kern = d == 128 ? fold_tc_kernel<128> : fold_tc_kernel<256>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "fold_tc smem attribute");
-  pdl(kern, grid, FT_THREADS, smem, st)(w, tz, q, out, mag_or, flag, tc_error_word());
+  pdl(kern, grid, FT_THREADS, smem, st)(w, tz, q, nout, out, mag_or, flag, tc_error_word());
   salsaa_count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "fold_tc launch");
 }
 
 int launch_words_to_c8(const RowSet& src, u32 rows, u64 width, u32 d, u64 q, int8_t* c8, u32* wide, cudaStream_t st) {
-  if (src.narrow || rows == 0 || rows > (u32)MAX_WROWS || width % 64 || d % 16 || !rowset_aligned(src, rows, 16, 16))
+  if (src.narrow || rows == 0 || rows > (u32)MAX_WROWS || width == 0 || d % 16 || !rowset_aligned(src, rows, 16, 16))
     return salsaa_set_error(-2, "words_to_c8: bad rows");
-  const u64 tasks = width / 16 * (d / 16);
+  const u64 wpad = c8_width(width), tasks = wpad / 16 * (d / 16);
   const u64 want = (tasks + 7) / 8, most = 148 * 8;
-  pdl(words_to_c8_kernel, dim3((unsigned)(want < most ? want : most), rows), 256, 0, st)(src, width, d, q, c8, wide);
+  pdl(words_to_c8_kernel, dim3((unsigned)(want < most ? want : most), rows), 256, 0, st)(src, width, wpad, d, q, c8,
+                                                                                         wide);
   salsaa_count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "words_to_c8 launch");

@@ -126,3 +126,26 @@ def test_project_tiles(api, oracle, d, rows, width, lo, hi, odd):
     iz, sg = proj_challenge(5, 2, rows * 256)
     want = oracle.project(w, q, iz, sg)
     assert np.array_equal(api.to_host(api.project(api.to_dev(w), q, 5, 2)), want)
+
+
+@pytest.mark.parametrize("d,rows,width,lo,hi,c_hi,odd", [
+    (128, 8, 8193, -31, 32, 1, None),      # ternary challenges, one element past a tile
+    (128, 8, 8255, -128, -127, 127, None),  # the largest sums, one element short of a tile
+    (128, 4, 16385, -128, 128, 127, 128),  # a row value past the byte: the transforms
+    (128, 4, 16400, -1, 2, 128, None),     # a challenge past it
+    (128, 1, 1 << 16, -128, 128, 1, None),
+    (256, 8, 4097, -128, 128, 1, None),
+    (256, 8, 4100, -1, 2, 1, -129),
+])
+def test_fold_tiles(api, oracle, d, rows, width, lo, hi, c_hi, odd):
+    """Long folds of word rows through byte tiles, or the transforms when a value does not fit."""
+    q = Q[d]
+    rng = np.random.default_rng(width + d)
+    v = rng.integers(lo, hi, size=(rows, width, d))
+    if odd is not None:
+        v[-1, -1, d - 5] = odd
+    cv = rng.integers(-c_hi, c_hi + 1, size=(rows, d)) if c_hi != 127 else np.full((rows, d), 127)
+    cv[0, 1] = c_hi
+    w, c = (np.where(x < 0, q + x, x).astype(np.uint64) for x in (v, cv))
+    got = api.to_host(api.fold(api.to_dev(w), q, api.to_dev(c)))
+    assert np.array_equal(got, oracle.fold(w, q, c))
