@@ -419,52 +419,73 @@ __global__ void __launch_bounds__(256) sc_round_kernel(const u64* in, u64 sin, u
   }
 }
 
-// One CTA per (rep,row) finishes rounds j0.. from v_{j0} (length L: at most
-// SC_TAIL_ONE, or 16 d when norm_check_3's vector is longer),
-// reading either a per-pair buffer or (j0 = 0) the witness row itself.
-// T rounds of the tail on the vector v (length cur, shared memory): groups of
-// 2^T values v[g + m ng] per thread, sums of all T rounds in one block
-// reduction, folded values back to v[g] (only thread g touches v[g]).
-// ch: the challenges from this step's first round on, their Shoup companions
-// SC_MAX_NR behind; sums(t): where the three sums of its round t go.
-template <bool LAZY, u32 T, typename Sums>
-__device__ __forceinline__ void tail_step(u64* v, u64 cur, const ModQ& M, const u64* ch, Sums sums, Sum128* red) {
-  constexpr u32 G = 1u << T;
-  const u64 ng = cur >> T;
-  u64 c[T], cp[T];
+// Tails: a block finishes the rounds of one vector v of `cur` values in shared
+// memory, one round per step of a loop.  The code of a tail runs once per
+// launch, so its size counts: with four rounds unrolled per step the block
+// spent most of 30 us fetching instructions, the loop takes 17 (256
+// values left, one Gram matrix, d = 128).  Thread e alone reads and writes
+// v[e], and the partial sums alternate between two buffers, so a round has
+// one barrier.
+// ch: challenges from the next round on, their Shoup companions SC_MAX_NR
+// behind; sums(t): where the three sums of round t go; at(cur): called before
+// each round, v complete.
+constexpr u32 TAIL_THREADS = 512;
+template <bool LAZY, typename Sums, typename At>
+__device__ __forceinline__ void tail_rounds(u64* v, u64 cur, const ModQ& M, const u64* ch, Sums sums, At at,
+                                            Sum128 (*red)[3 * TAIL_THREADS / 32]) {
+  const u32 tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const u64 q = M.q;
+#pragma unroll 1
+  for (u32 t = 0; cur > 1; t++, cur >>= 1) {
+    at(cur);
+    const u64 h = cur >> 1, c = ch[t], cp = ch[SC_MAX_NR + t];
+    const u32 nw = (u32)((h < TAIL_THREADS ? h : TAIL_THREADS) + 31) >> 5;
+    Sum128* const part = red[t & 1];
+    if (wid < nw) {
+      ScAcc<LAZY> acc[3];
 #pragma unroll
-  for (u32 t = 0; t < T; t++) {
-    c[t] = ch[t];
-    cp[t] = ch[SC_MAX_NR + t];
-  }
-  ScAcc<LAZY> acc[T][3];
+      for (u32 a = 0; a < 3; a++) acc[a].zero();
+#pragma unroll 1
+      for (u64 e = tid; e < h; e += TAIL_THREADS) {
+        const u64 x = v[e], y = v[e + h];
+        acc[0].mac(M, x, x);
+        acc[1].mac(M, x, y);
+        acc[2].mac(M, y, y);
+        v[e] = fold1(x, y, c, cp, q);
+      }
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-  for (u32 t = 0; t < T; t++)
+        for (u32 a = 0; a < 3; a++) {
+          if (LAZY) {
+            Sum128 u;
+            u.lo = __shfl_xor_sync(0xffffffffu, acc[a].s.lo, o);
+            u.hi = __shfl_xor_sync(0xffffffffu, acc[a].s.hi, o);
+            s128_add(acc[a].s, u);
+          } else {
+            acc[a].g = add_mod(acc[a].g, __shfl_xor_sync(0xffffffffu, acc[a].g, o), q);
+          }
+        }
+      }
+      if (lane == 0) {
 #pragma unroll
-    for (u32 a = 0; a < 3; a++) acc[t][a].zero();
-  for (u64 g = threadIdx.x; g < ng; g += blockDim.x) {
-    u64 x[G];
-#pragma unroll
-    for (u32 m = 0; m < G; m++) x[m] = v[g + m * ng];
-    group_rounds<LAZY, T>(M, x, c, cp, acc, 0);
-    v[g] = x[0];
-  }
-  ScAcc<LAZY> flat[T * 3];
-#pragma unroll
-  for (u32 t = 0; t < T; t++)
-#pragma unroll
-    for (u32 a = 0; a < 3; a++) flat[t * 3 + a] = acc[t][a];
-  const u64 r = block_totals<LAZY, T * 3>(M, flat, red);  // its barriers also publish v
-  if (threadIdx.x < T * 3) sums(threadIdx.x / 3)[threadIdx.x % 3] = r;
-}
-template <bool LAZY, typename Sums>
-__device__ __forceinline__ void tail_steps(u32 T, u64* v, u64 cur, const ModQ& M, const u64* ch, Sums sums,
-                                           Sum128* red) {
-  switch (T) {
-    case 4: tail_step<LAZY, 4>(v, cur, M, ch, sums, red); break;
-    case 3: tail_step<LAZY, 3>(v, cur, M, ch, sums, red); break;
-    case 2: tail_step<LAZY, 2>(v, cur, M, ch, sums, red); break;
-    default: tail_step<LAZY, 1>(v, cur, M, ch, sums, red); break;
+        for (u32 a = 0; a < 3; a++) {
+          if (LAZY) part[3 * wid + a] = acc[a].s;
+          else part[3 * wid + a].lo = acc[a].g;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < 3) {
+      Sum128 s = part[tid];
+      u64 g = s.lo;
+#pragma unroll 1
+      for (u32 w = 1; w < nw; w++) {
+        if (LAZY) s128_add(s, part[3 * w + tid]);
+        else g = add_mod(g, part[3 * w + tid].lo, q);
+      }
+      sums(t)[tid] = LAZY ? reduce128_any(M, s.hi, s.lo) : g;
+    }
   }
 }
 // A tail's challenges, all rounds at once: the companions are 128-bit divisions.
@@ -478,8 +499,8 @@ __device__ __forceinline__ void tail_challenges(u64* ch, u32 nr, Chal chal, u64 
   __syncthreads();
 }
 // Round polynomial (and with claim the claim) from a round's raw sums.
-__device__ __forceinline__ void sc_poly(const u64* s, u64 q, u64* o, u64* claim) {
-  const u64 s00 = s[0] % q, s01 = s[1] % q, s11 = s[2] % q;
+__device__ __forceinline__ void sc_poly(const u64* s, const ModQ& M, u64* o, u64* claim) {
+  const u64 q = M.q, s00 = reduce64(M, s[0]), s01 = reduce64(M, s[1]), s11 = reduce64(M, s[2]);
   o[0] = s00;
   o[1] = sub_mod(s01, s00, q);
   o[2] = add_mod(sub_mod(sub_mod(s11, s01, q), s01, q), s00, q);
@@ -496,16 +517,15 @@ __device__ __forceinline__ void gram_sums(const u64* gram, const ModQ& M, const 
   __syncthreads();  // C may still be read by an earlier use
   if (tid < 256) C[tid] = reduce64(M, gram[tid]);
   __syncthreads();
-#pragma unroll
+#pragma unroll 1
   for (u32 t = 0; t < SC_T; t++) {
     const u32 h = 8u >> t;
     const u64 c = ch[t], cp = ch[SC_MAX_NR + t];
-    if (tid < 3) {
-      const u32 r0 = tid == 2 ? h : 0, c0 = tid == 0 ? 0 : h;
-      u64 s = 0;
-#pragma unroll
-      for (u32 j = 0; j < h; j++) s = add_mod(s, C[(r0 + j) * 16 + c0 + j], q);
-      sums(t)[tid] = s;
+    if (tid < 32) {  // lane (sum a, diagonal entry e)
+      const u32 a = tid >> 3, e = tid & 7;
+      u64 x = a < 3 && e < h ? C[(e + (a == 2 ? h : 0)) * 16 + e + (a == 0 ? 0 : h)] : 0;
+      for (int o = 4; o > 0; o >>= 1) x = add_mod(x, __shfl_xor_sync(0xffffffffu, x, o), q);
+      if (a < 3 && e == 0) sums(t)[a] = x;
     }
     const u32 i = tid / h, j = tid % h;
     u64 v = 0;
@@ -525,47 +545,41 @@ struct GramList {
   u32 n;
 };
 
+// One CTA per (rep,row) finishes rounds j0.. from v_{j0} (length L: at most
+// SC_TAIL_ONE, or 16 d when norm_check_3's vector is longer), reading either a
+// per-pair buffer or (j0 = 0) the witness row itself.  cap: the vector when it
+// is d long (norm_check_3).
 template <bool LAZY>
-__global__ void __launch_bounds__(512) sc_tail_kernel(const u64* in, u64 sin, RowSet w0, u64 L, u32 rows, ModQ M,
-                                                       const DevState* ds, u32 round, u32 j0, u64* sums, u32 nr,
-                                                       u32 d, u64* cap, GramList gl, u64* claims, u64* polys0,
-                                                       u64* polys1) {
+__global__ void __launch_bounds__(TAIL_THREADS) sc_tail_kernel(const u64* in, u64 sin, RowSet w0, u64 L, u32 rows,
+                                                               ModQ M, const DevState* ds, u32 round, u32 j0,
+                                                               u64* sums, u32 nr, u32 d, u64* cap, GramList gl,
+                                                               u64* claims, u64* polys0, u64* polys1) {
   pdl_wait();
   extern __shared__ u64 v[];
-  __shared__ Sum128 red[SC_T * 3 * 32];
+  __shared__ Sum128 red[2][3 * TAIL_THREADS / 32];
   __shared__ u64 ch[2 * SC_MAX_NR], C[256];
   const u32 pair = blockIdx.x, rep = pair / rows, k = pair % rows;
   const u64* x = (j0 == 0) ? w0.p[k] : in + (u64)pair * sin;
   const bool nar = j0 == 0 && ((w0.narrow >> k) & 1);
-  for (u32 i = threadIdx.x; i < L; i += blockDim.x) v[i] = wres(x, nar, i, M.q);
+#pragma unroll 1
+  for (u32 i = threadIdx.x; i < L; i += TAIL_THREADS) v[i] = wres(x, nar, i, M.q);
   tail_challenges(ch, nr, [&](u32 t) { return nc_challenge(ds, round, rep, t, M.q); }, M.q);
-  for (u32 p = 0; p < gl.n; p++)
-    gram_sums(gl.c[p] + (u64)(gl.shared[p] ? k : pair) * 256, M, ch + gl.j[p],
-              [&](u32 t) { return sums + ((rep * (u64)nr + gl.j[p] + t) * rows + k) * 3; }, C);
-  u64 cur = L;
-  u32 j = j0;
-  while (cur > 1) {
-    if (cur == d) {
-      for (u32 i = threadIdx.x; i < d; i += blockDim.x) cap[(u64)pair * d + i] = v[i];
-      __syncthreads();
-    }
-    // up to four rounds per step, stopping at length d (norm_check_3's vector)
-    u32 T = 63u - (u32)__clzll((long long)cur);
-    if (cur > d) {
-      const u32 td = 63u - (u32)__clzll((long long)(cur / d));
-      T = td < T ? td : T;
-    }
-    T = T < SC_T ? T : SC_T;
-    tail_steps<LAZY>(T, v, cur, M, ch + j, [&](u32 t) { return sums + ((rep * (u64)nr + j + t) * rows + k) * 3; },
-                     red);
-    cur >>= T;
-    j += T;
+  auto sums_of = [&](u32 t) { return sums + ((rep * (u64)nr + t) * rows + k) * 3; };
+#pragma unroll 1
+  for (u32 p = 0; p < gl.n; p++) {
+    const u32 jp = gl.j[p];
+    gram_sums(gl.c[p] + (u64)(gl.shared[p] ? k : pair) * 256, M, ch + jp, [&](u32 t) { return sums_of(jp + t); }, C);
   }
+  tail_rounds<LAZY>(v, L, M, ch + j0, [&](u32 t) { return sums_of(j0 + t); },
+                    [&](u64 cur) {
+                      if (cur == d)
+                        for (u32 i = threadIdx.x; i < d; i += TAIL_THREADS) cap[(u64)pair * d + i] = v[i];
+                    },
+                    red);
   // every round of this (rep, row) is summed: its claims and polynomials
   __syncthreads();
-  for (u32 t = threadIdx.x; t < nr; t += blockDim.x)
-    sc_poly(sums + ((rep * (u64)nr + t) * rows + k) * 3, M.q, (rep ? polys1 : polys0) + ((u64)t * rows + k) * 3,
-            rep == 0 && t == 0 ? claims + k : nullptr);
+  for (u32 t = threadIdx.x; t < nr; t += TAIL_THREADS)
+    sc_poly(sums_of(t), M, (rep ? polys1 : polys0) + ((u64)t * rows + k) * 3, rep == 0 && t == 0 ? claims + k : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -631,36 +645,29 @@ __global__ void __launch_bounds__(256, 2) sb_pass_kernel(const SbInst* inst, u32
 // gram: per level (four rounds) SB_MAX_INST Gram matrices, for the levels that
 // the instance took on the tensor cores; or null.
 template <bool LAZY>
-__global__ void __launch_bounds__(1024) sb_tail_kernel(const SbInst* inst, ModQ M, u64 seed, u32 round, u64* sums,
-                                                       u32 nrmax, const u64* gram, const u64* offs, u64* claims,
-                                                       u64* polys) {
+__global__ void __launch_bounds__(TAIL_THREADS) sb_tail_kernel(const SbInst* inst, ModQ M, u64 seed, u32 round,
+                                                               u64* sums, u32 nrmax, const u64* gram, const u64* offs,
+                                                               u64* claims, u64* polys) {
   pdl_wait();
   extern __shared__ u64 v[];
-  __shared__ Sum128 red[SC_T * 3 * 32];
+  __shared__ Sum128 red[2][3 * TAIL_THREADS / 32];
   __shared__ u64 ch[2 * SC_MAX_NR], C[256];
   const u32 i = blockIdx.x;
   const SbInst I = inst[i];
-  const u64 q = M.q;
-  for (u64 e = threadIdx.x; e < I.L; e += blockDim.x) v[e] = I.in[e];
+#pragma unroll 4
+  for (u64 e = threadIdx.x; e < I.L; e += TAIL_THREADS) v[e] = __ldg(I.in + e);
   const u32 nr = I.j + 63u - (u32)__clzll((long long)I.L);
-  tail_challenges(ch, nr, [&](u32 t) { return sb_challenge(seed, round, i, t, q); }, q);
+  tail_challenges(ch, nr, [&](u32 t) { return sb_challenge(seed, round, i, t, M.q); }, M.q);
+  auto sums_of = [&](u32 t) { return sums + ((u64)i * nrmax + t) * 3; };
   if (gram)
+#pragma unroll 1
     for (u32 j = 0; j < I.j; j += SC_T)
-      gram_sums(gram + ((u64)(j / SC_T) * SB_MAX_INST + i) * 256, M, ch + j,
-                [&](u32 t) { return sums + ((u64)i * nrmax + j + t) * 3; }, C);
-  u64 cur = I.L;
-  u32 j = I.j;
-  while (cur > 1) {
-    u32 T = 63u - (u32)__clzll((long long)cur);
-    T = T < SC_T ? T : SC_T;
-    tail_steps<LAZY>(T, v, cur, M, ch + j, [&](u32 t) { return sums + ((u64)i * nrmax + j + t) * 3; }, red);
-    cur >>= T;
-    j += T;
-  }
+      gram_sums(gram + ((u64)(j / SC_T) * SB_MAX_INST + i) * 256, M, ch + j, [&](u32 t) { return sums_of(j + t); }, C);
+  tail_rounds<LAZY>(v, I.L, M, ch + I.j, [&](u32 t) { return sums_of(I.j + t); }, [](u64) {}, red);
   __syncthreads();
   // instance i's polynomials start at offs[i] * 3
-  for (u32 t = threadIdx.x; t < nr; t += blockDim.x)
-    sc_poly(sums + ((u64)i * nrmax + t) * 3, q, polys + (offs[i] + t) * 3, t == 0 ? claims + i : nullptr);
+  for (u32 t = threadIdx.x; t < nr; t += TAIL_THREADS)
+    sc_poly(sums_of(t), M, polys + (offs[i] + t) * 3, t == 0 ? claims + i : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -979,7 +986,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     e = cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: tail smem");
   }
-  pdl(tail, count, 1024, smem, st)(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
+  pdl(tail, count, TAIL_THREADS, smem, st)(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
                                    claims, polys);
   return check_launch("sb_tail");
 }
@@ -1065,7 +1072,7 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tail smem attribute");
   }
-  pdl(kern, 2 * rows, 512, smem, st)(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
+  pdl(kern, 2 * rows, TAIL_THREADS, smem, st)(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
                                         claims, polys0, polys1);
   return check_launch("sc_tail");
 }
@@ -1147,10 +1154,13 @@ __global__ void norm3_kernel(const u64* cap, u32 rows, u32 nr, NttDev T, ModQ M,
   u64* ext = sm;          // d
   u64* bs = sm + d;       // d: base, slot layout after NTT
   u64* vs = sm + 2 * d;   // d: vector, slot layout after NTT
+  __shared__ u64 ch[16];
+  if (threadIdx.x < logd) ch[threadIdx.x] = nc_challenge(ds, round, rep, K + threadIdx.x, q);
+  __syncthreads();
   for (u32 i = threadIdx.x; i < d; i += blockDim.x) {
     u64 v = 1 % q;
     for (u32 b = 0; b < logd; b++) {
-      const u64 c = nc_challenge(ds, round, rep, K + b, q);
+      const u64 c = ch[b];
       const u32 bit = (i >> (logd - 1 - b)) & 1;
       v = mul_mod(M, v, bit ? c : sub_mod(1 % q, c, q));
     }
