@@ -1836,6 +1836,26 @@ int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ&
   return check_launch("fold");
 }
 
+__global__ void __launch_bounds__(256) copies_kernel(CopyList l) {
+  pdl_wait();
+  const auto& c = l.c[blockIdx.y];
+  for (u32 t = blockIdx.x * 256 + threadIdx.x; t < c.rows * c.cols; t += gridDim.x * 256) {
+    const u32 r = t / c.cols, x = t % c.cols;
+    c.dst[(u64)r * c.dst_stride + x] = c.src[(u64)r * c.src_stride + x];
+  }
+}
+
+int launch_copies(const CopyList& l, cudaStream_t st) {
+  u32 most = 1;
+  for (u32 i = 0; i < l.n; i++) {
+    const u32 b = (l.c[i].rows * l.c[i].cols + 255) / 256;
+    most = b > most ? b : most;
+  }
+  if (l.n == 0 || l.n > CopyList::MAX) return salsaa_set_error(-2, "copies: 1..6 of them");
+  pdl(copies_kernel, dim3(most < 148 ? most : 148, l.n), 256, 0, st)(l);
+  return check_launch("copies");
+}
+
 __global__ void fold_slots_kernel(const u64* x, const u64* c, u32 K, u32 n, ModQ M, const u64* zeta, u64* out) {
   pdl_wait();
   const u32 s = blockIdx.x * blockDim.x + threadIdx.x;

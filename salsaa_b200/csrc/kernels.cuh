@@ -207,6 +207,27 @@ int launch_fold_challenge(const DevState* ds, u32 round, u32 rows, u32 d, u64 q,
 int launch_fold(RowSet w_slot, u32 rows, u64 width, const NttDev& T, const ModQ& M, const u64* c_slot, u64* pre,
                 u64* out_slot, cudaStream_t st, const u32* gate = nullptr);
 
+// Up to CopyList::MAX strided copies of words in one launch (a round's results
+// to their places in the proof: one launch of 3 us for five copies of 2).
+struct CopyList {
+  static constexpr u32 MAX = 6;
+  struct {
+    const u64* src;
+    u64* dst;
+    u32 rows, cols, src_stride, dst_stride;
+  } c[MAX];
+  u32 n;
+  void add(const u64* src, u32 src_stride, u64* dst, u32 dst_stride, u32 rows, u32 cols) {
+    c[n].src = src;
+    c[n].dst = dst;
+    c[n].rows = rows;
+    c[n].cols = cols;
+    c[n].src_stride = src_stride;
+    c[n++].dst_stride = dst_stride;
+  }
+};
+int launch_copies(const CopyList& l, cudaStream_t st);
+
 // out (one ring element, slot form) = sum_k c_slot[k] x[k] over K slot-form elements.
 int launch_fold_slots(const u64* x, const u64* c_slot, u32 K, const NttDev& T, const ModQ& M, u64* out,
                       cudaStream_t st);

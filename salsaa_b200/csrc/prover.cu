@@ -1039,6 +1039,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     RowSet Pr = rows_of(pr->Ps, 1, width, d);
     RowSet Prc = rows_of(pr->Pc, 1, width, d);
     const u32 S = ms + nsc;
+    CopyList copies{};  // out of pr->cout2
     if (!P.folding) {
       // split rhs and projected commitment in one pass over the statement
       // rows: witness columns L_0..L_{K/2-1}, R_0..R_{K/2-1}, P.  The
@@ -1054,14 +1055,9 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       const Sc8Rows sr = sc8_rows(pr, K, width, d, true, &pr->ds->wide[rd], &pr->ds->wide_p[rd]);
       TRY(commit_rows_slot(pr, both, &bothc, K + 1, width, ms, 0, nsc + 2, imp, sh ? &sr : nullptr));
       TRY(ntt_launch(pr->cout, pr->cout2, (u64)(S + 2) * (K + 1), T, true, true, st));
-      const size_t row_bytes = (size_t)(K + 1) * d * sizeof(u64);
-      e = cudaMemcpy2DAsync(proof + cur, (size_t)K * d * sizeof(u64), pr->cout2, row_bytes,
-                            (size_t)K * d * sizeof(u64), S, cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: split rhs");
+      copies.add(pr->cout2, (K + 1) * d, proof + cur, K * d, S, K * d);  // split rhs
       cur += (u64)S * K * d;
-      e = cudaMemcpy2DAsync(proof + cur, (size_t)d * sizeof(u64), pr->cout2 + (u64)K * d, row_bytes,
-                            (size_t)d * sizeof(u64), S, cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: projected commitment");
+      copies.add(pr->cout2 + (u64)K * d, (K + 1) * d, proof + cur, d, S, d);  // projected commitment
       cur += (u64)S * d;
       if (pending) {
         // commitment of the unsplit witness (initial commitment or decomp rhs)
@@ -1090,8 +1086,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       const Sc8Rows sr = sc8_rows(pr, 0, width, d, false, nullptr, &pr->ds->wide_p[rd]);
       TRY(commit_rows_slot(pr, Pr, &Prc, 1, width, ms, 0, nsc + 2, imp, sh ? &sr : nullptr));
       TRY(ntt_launch(pr->cout, pr->cout2, S + 2, T, true, true, st));
-      e = cudaMemcpyAsync(proof + cur, pr->cout2, (size_t)S * d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: projected commitment");
+      copies.add(pr->cout2, d, proof + cur, d, S, d);
       cur += (u64)S * d;
     }
     // batch_projections (src/subroutines/project.rs:131-203): witness_rhs,
@@ -1100,7 +1095,7 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     if (!P.folding) {
       const u64* wl = pr->cout2 + (u64)S * (K + 1) * d;  // witness_lhs x [split witness, P]
       const u64* pl = wl + (u64)(K + 1) * d;             // projected_lhs x [split witness, P]
-      e = cudaMemcpyAsync(proof + cur, wl, (size_t)K * d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
+      copies.add(wl, 0, proof + cur, 0, 1, K * d);
       l1_src = wl + (u64)K * d;
       prhs_src = pl + (u64)K * d;
       ones = pr->cout + (u64)(S + 1) * (K + 1) * d;
@@ -1112,9 +1107,9 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
       TRY(ntt_launch(pr->cout, proof + cur, K, T, true, true, st));
       ones = pr->cout + (u64)K * d;
     }
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(proof + cur + (u64)K * d, prhs_src, (size_t)d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: batch projections");
+    copies.add(prhs_src, 0, proof + cur + (u64)K * d, 0, 1, d);
+    copies.add(l1_src, 0, proof + cur + (u64)(K + 2) * d, 0, 1, d);  // the cross term behind l0
+    TRY(launch_copies(copies, st));
     cur += (u64)K * d + d;
     nsc += 1;  // witness_lhs joins the statement
     // fold (src/subroutines/fold.rs:22-27)
@@ -1139,8 +1134,6 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
     TRY(launch_fold_slots(ones, pr->c_slot, K, T, M, pr->acc, st));
     TRY(ntt_launch(pr->acc, proof + cur, 1, T, true, true, st));
     cur += d;
-    e = cudaMemcpyAsync(proof + cur, l1_src, (size_t)d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: cross term");
     cur += d;
     nsc += 1;  // projected_lhs joins the statement
     // join: witness = [folded, projected]
