@@ -732,7 +732,15 @@ static int commit_rows(salsaa_prover* pr, const RowSet& ws, const RowSet* wc, u3
                        u32 sc_first, u32 nsc, u64* proof_out, const CkImage* img = nullptr,
                        const Sc8Rows* sc8 = nullptr) {
   TRY(commit_rows_slot(pr, ws, wc, rows, width, nck, sc_first, nsc, img, sc8));
-  return ntt_launch(pr->cout, proof_out, (u64)(nck + nsc) * rows, *pr->ctx->T, true, true, pr->st);
+  const NttDev& T = *pr->ctx->T;
+  const u64 count = (u64)(nck + nsc) * rows;
+  if (ntt_mag_ok(pr->cout, proof_out, T, true) || !ntt_mag_ok(pr->cout, pr->cout2, T, true))
+    return ntt_launch(pr->cout, proof_out, count, T, true, true, pr->st);
+  // off the fast transforms' alignment: beside, then moved
+  TRY(ntt_launch(pr->cout, pr->cout2, count, T, true, true, pr->st));
+  CopyList l{};
+  l.add(pr->cout2, 0, proof_out, 0, 1, (u32)count * pr->ctx->d);
+  return launch_copies(l, pr->st);
 }
 
 static RowSet rows_of(const u64* base, u32 rows, u64 width, u32 d) {
@@ -1077,7 +1085,14 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
         da.out = pr->acc;
         if (da.K != pend_K) return salsaa_set_error(-9, "enqueue: derived commitment shape mismatch");
         TRY(launch_derive(da, T, M, pr->ds, st));
-        TRY(ntt_launch(pr->acc, proof + pend_off, (u64)pend_rows * pend_K, T, true, true, st));
+        // every other section of a proof lies 8 bytes off the transform's
+        // alignment, where only the generic kernel writes (20 us against 6)
+        if (ntt_mag_ok(pr->acc, proof + pend_off, T, true) || !ntt_mag_ok(pr->acc, pr->acc, T, true)) {
+          TRY(ntt_launch(pr->acc, proof + pend_off, (u64)pend_rows * pend_K, T, true, true, st));
+        } else {
+          TRY(ntt_launch(pr->acc, pr->acc, (u64)pend_rows * pend_K, T, true, true, st));
+          copies.add(pr->acc, 0, proof + pend_off, 0, 1, pend_rows * pend_K * d);
+        }
         pending = false;
       }
     } else {
