@@ -1035,8 +1035,10 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     if (gram_room(rows) && gram_words_ok(L, M.q)) {
       u64* g = gram_take(rows, 1);
       const bool c8 = w8 && wide && sumcheck_reads_bytes(*w8, L, d, M.q);
+      const int tr = salsaa_trace_begin("nc_gram_kernel", st, (double)rows * L * 8.0 * (1.0 + 2.0 / 16.0));
       if (c8 && (rc = launch_gram_c8(*w8, d, M, ds, round, B.a, sa, g, wide, st))) return rc;
       if ((rc = launch_gram_first(w, rows, L, M, ds, round, B.a, sa, g, c8 ? wide : nullptr, st))) return rc;
+      salsaa_trace_end(tr, st);
     } else {
       dim3 g(2 * grid_for(L / (1u << SC_T), 2 * rows), rows);
       pdl(sc_first_kernel<LAZY>, g, 256, 0, st)(w, rows, L, M, ds, round, B.a, sa, B.sums, nr, plain);
