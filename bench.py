@@ -902,13 +902,13 @@ def roofline_ntt(ntt, peak, kind):
             "algorithmic_bytes_per_launch": 16 * 128 * f["elements"], "frac_per_size": per}
 
 
-# DRAM bytes (read + write) of ck_umma_kernel per launch, mean over the eight
+# DRAM bytes (read + write) of ck_img_kernel per launch, mean over the eight
 # launches of one A0 proof (dram__bytes_read.sum + dram__bytes_write.sum), from
 # one ncu capture made by CK_TRAFFIC_CMD; ncu cannot run inside this process,
 # so the figure is carried with the command that measured it.
-CK_TRAFFIC_A0 = 653.8e6
+CK_TRAFFIC_A0 = 440.7e6
 CK_TRAFFIC_CMD = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum "
-                  "--clock-control none -k regex:ck_umma -c 8 --csv python bench.py --steps 1 --warmup 1 "
+                  "--clock-control none -k regex:ck_img -c 8 --csv python bench.py --steps 1 --warmup 1 "
                   "--slots 1 --plain-proofs 1 --no-e2e --no-ntt --no-serve --no-cpu-baseline --no-dense")
 
 
@@ -934,7 +934,7 @@ def roofline_ck(traced, elapsed_ms, a0):
     ops = t8["work"] / t8["launches"]
     tops = ops / (per_ms * 1e-3) / 1e12
     macs = tm["work"] / tm["launches"]
-    return {"kernel": "ck_umma_kernel (exact int8 limb-split commitment, tcgen05.mma kind::i8, TMEM)",
+    return {"kernel": "ck_img_kernel (exact int8 limb-split commitment, tcgen05.mma kind::i8, TMEM; traced as ck_umma_kernel)",
             "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "peak_kind": hbm_kind + " copy bandwidth",
             "traffic": CK_TRAFFIC_A0 if a0 else None,
