@@ -200,18 +200,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
     img_item(R, im, SELLOG, item, k, e0);
     return R.src[k] + e0 * D;
   };
-  // Centred value + 128 (one limb) or + 2^15 + 2^7 (two: its bytes are the
-  // signed limbs + 128).  A short residue has a zero high word or, as q minus
-  // at most 2^16 <= q mod 2^32, that of q: fit collects what contradicts.
-  constexpr u32 BIAS = MODE == TC_LIMBS ? 0x8080u : 0x80u;
+  // Centred value, plus 2^15 + 2^7 with two limbs (its bytes are then the signed
+  // limbs + 128).  A short residue has a zero high word or, as q minus at most
+  // 2^16 <= q mod 2^32, that of q, and the difference of the low words to 0 or
+  // q is negative in the second case only: a low word near 2^32 above a zero
+  // high word, or a small one above q's, is a value far from zero.  fit and
+  // fith collect what contradicts.
+  constexpr u32 BIAS = MODE == TC_LIMBS ? 0x8080u : 0u;
   auto centred = [&](u64 v, u32& fit, u32& fith) -> u32 {
     const u32 hi = (u32)(v >> 32);
-    const u32 t = (u32)v - (hi ? qlo : 0u) + BIAS;
-    fit |= t;
     if (hi) fith |= hi ^ qhi;
-    return t;
+    if (MODE == TC_LIMBS) {
+      const u32 s = (u32)v - (hi ? qlo : 0u);
+      fit |= s + BIAS;
+      fith |= (hi ? ~s : s) & 0x80000000u;
+      return s + BIAS;
+    }
+    const u32 w = (u32)v - (hi ? qlo - 128u : 0u);  // 0 .. 127 from 0 or from -128
+    fit |= w;
+    return hi ? w ^ 128u : w;  // its low byte
   };
-  auto unfit = [&](u32 fit, u32 fith) { return (fit >> (MODE == TC_LIMBS ? 16 : 8)) != 0 || fith != 0; };
+  auto unfit = [&](u32 fit, u32 fith) { return (fit >> (MODE == TC_LIMBS ? 16 : 7)) != 0 || fith != 0; };
 
   // a CTA whose first item does not fit leaves before it starts
   if (MODE != TC_DIGITS) {
@@ -304,7 +313,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
             }
           }
           const u32 x01 = __byte_perm(x[0], x[1], 0x5140), x23 = __byte_perm(x[2], x[3], 0x5140);
-          pk[i][0] = __byte_perm(x01, x23, 0x5410) ^ 0x80808080u;
+          pk[i][0] = __byte_perm(x01, x23, 0x5410) ^ (MODE == TC_LIMBS ? 0x80808080u : 0u);
           if (MODE == TC_LIMBS) pk[i][MODE == TC_BYTES ? 0 : 1] = __byte_perm(x01, x23, 0x7632) ^ 0x80808080u;
         }
 #pragma unroll

@@ -149,3 +149,36 @@ def test_fold_tiles(api, oracle, d, rows, width, lo, hi, c_hi, odd):
     w, c = (np.where(x < 0, q + x, x).astype(np.uint64) for x in (v, cv))
     got = api.to_host(api.fold(api.to_dev(w), q, api.to_dev(c)))
     assert np.array_equal(got, oracle.fold(w, q, c))
+
+
+def near_short(q):
+    """Residues far from zero whose low 32 bits look like a short value's."""
+    hi = (q >> 32) << 32
+    return [(1 << 32) - 32896, (1 << 32) - 129, (1 << 32) - 128, (1 << 32) - 1, 1 << 32, (1 << 32) + 1, hi, hi + 0x7880,
+            q - (1 << 32), q - (1 << 32) + 1, q >> 1, (q >> 1) + 1]
+
+
+@pytest.mark.parametrize("d", [128, 256])
+def test_values_near_short(api, oracle, d):
+    """One such residue among ternary values, and (proofs) alone, so that the
+    projected row holds it and its negative: everything is the oracle's."""
+    q = Q[d]
+    p = P.make_params(d, q, 3, 1 << 13, 2)
+    ctx, pc = api.Context(p, crs_seed=5), P.make_params(d, q, 3, 128, 1)
+    rng = np.random.default_rng(d)
+    A = rand_mod(rng, (3, 128, d), q)
+    key, small = api.DenseKey(api.to_dev(A), q), api.Context(pc, crs_seed=5)
+    tern = rng.integers(-1, 2, size=(1, 1 << 13, d))
+    tern = np.where(tern < 0, q + tern, tern).astype(np.uint64)
+    for v in near_short(q):
+        w = tern[:, :128].copy()
+        w[0, 77, 9] = v
+        assert np.array_equal(api.to_host(small.parallel_dot_series_matrix(api.to_dev(w))), oracle.commit_ck(pc, 5, w)), v
+        assert np.array_equal(api.to_host(key.commit(api.to_dev(w))), oracle.dense_commit(A, w, q)), v
+        for base in (tern, np.zeros_like(tern)):
+            w = base.copy()
+            w[0, 4321, 3] = v
+            rc, want, _ = oracle.prove(p, 5, 6, witness=w)
+            assert rc == 0
+            assert np.array_equal(ctx.prove(6, witness=w), want), (v, int(base.any()))
+    key.close()
