@@ -849,6 +849,12 @@ static int enqueue_impl(salsaa_prover* pr, u64 seed, const u64* d_witness, u64* 
   if (!wbase) {
     TRY(launch_gen_witness(pr->Dc, K, width, d, q, pr->ds, st));
     wbase = pr->Dc;
+  } else if (c->S.use_img && (uintptr_t)wbase % 16) {
+    // the transforms to the image read 16 bytes at a time; the digit buffer
+    // holds the initial witness and is free until the first digits
+    e = cudaMemcpyAsync(pr->Dc, wbase, K * width * d * sizeof(u64), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return salsaa_set_cuda_error(e, "enqueue: witness");
+    wbase = pr->Dc;
   }
   Wc = rows_of(wbase, K, width, d);
   // With use_img the key rows read the witness as a byte image, written by the

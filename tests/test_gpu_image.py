@@ -182,3 +182,31 @@ def test_values_near_short(api, oracle, d):
             assert rc == 0
             assert np.array_equal(ctx.prove(6, witness=w), want), (v, int(base.any()))
     key.close()
+
+
+@pytest.mark.parametrize("d,folding,log_wit,rounds", [(128, False, 13, 2), (128, True, 12, 1), (256, False, 13, 2),
+                                                      (512, False, 13, 2)])
+def test_prove_word_aligned_witness(api, oracle, cuda, d, folding, log_wit, rounds):
+    """A device witness on any word boundary gives the oracle's proof, by
+    direct launches and by graph replay, and stays as it was."""
+    q = Q[d]
+    p = P.make_params(d, q, 3, 1 << log_wit, rounds, folding)
+    v = np.random.default_rng(d).integers(-1, 2, size=(p.init_wit_rep, p.wit_len, d))
+    w = np.where(v < 0, q + v, v).astype(np.uint64)
+    rc, want, _ = oracle.prove(p, 5, 6, witness=w)
+    assert rc == 0
+    ctx = api.Context(p, crs_seed=5)
+    dw = api.to_dev(np.concatenate([[0], w.reshape(-1)]))[1:]
+    assert dw.data_ptr() % 16 == 8
+    out = cuda.zeros(ctx.proof_bytes, dtype=cuda.uint8, device="cuda")
+    for graph in (False, True):
+        pr = api.Prover(ctx)
+        pr.set_graph(graph)
+        for _ in range(2):
+            out.zero_()
+            cuda.cuda.synchronize()
+            pr.enqueue(6, out, dw)
+            pr.sync()
+            assert np.array_equal(out.cpu().numpy(), want)
+        pr.close()
+    assert np.array_equal(api.to_host(dw), w.reshape(-1))
