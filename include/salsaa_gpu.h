@@ -331,7 +331,8 @@ int salsaa_dense_key_create(const uint64_t* d_a, uint64_t n, uint64_t m, uint64_
 void salsaa_dense_key_destroy(salsaa_dense_key* key);
 /* d_w: r columns of m ring elements each (r x m x d, coefficient form);
  * d_c: n x r ring elements (coefficient form, row j = key row j).  d_w_slot is
- * an optional r x m x d workspace for W's NTT (NULL: allocated on the stream).
+ * an optional r x m x d workspace for W's NTT (NULL: allocated on the stream;
+ * d_w itself: W is overwritten); what it holds after the call is not specified.
  * Calls sharing one key must not overlap on the GPU (the key holds the
  * accumulators). */
 int salsaa_dense_commit(salsaa_dense_key* key, const uint64_t* d_w, uint64_t r, uint64_t* d_c, uint64_t* d_w_slot,

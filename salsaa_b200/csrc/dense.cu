@@ -155,8 +155,11 @@ extern "C" int salsaa_dense_commit(salsaa_dense_key* k, const uint64_t* d_w, uin
     }
   } free_tmp{tmp, st};
   // columns as a byte image (never larger than their words) when the shapes
-  // allow, else in slot form
-  const bool img = k->tk8 && (uintptr_t)d_w % 16 == 0 && (uintptr_t)d_w_slot % 16 == 0 &&
+  // allow, else in slot form; the image lies in another order than the words,
+  // so a workspace that overlaps them (W transformed in place) takes slot form
+  const u64 words = r * m * d;
+  const bool apart = d_w_slot + words <= d_w || d_w + words <= d_w_slot;
+  const bool img = apart && k->tk8 && (uintptr_t)d_w % 16 == 0 && (uintptr_t)d_w_slot % 16 == 0 &&
                    cki_ok(1, m, k->n, (u32)m, k->q);
   int rc = 0;
   if (!img && (rc = ntt_launch(d_w, d_w_slot, r * m, *k->T, true, false, st))) return rc;

@@ -68,3 +68,16 @@ def test_dense_commit_rejects_bad_shapes(api):
     from salsaa_b200.api import SalsaaError
     with pytest.raises(SalsaaError):
         api.DenseKey(api.to_dev(np.zeros((2, 100, 16), dtype=np.uint64)), P.Q0)
+
+
+@pytest.mark.parametrize("d,q,digits", [(128, P.Q0, 16), (128, P.Q0, 0), (256, P.Q1, 16), (512, P.Q2, 16)])
+def test_dense_commit_in_place(api, oracle, d, q, digits):
+    """The columns' own buffer as the workspace."""
+    n, m, r = 2, 2048, 3
+    rng = np.random.default_rng(d)
+    A = rand_mod(rng, (n, m, d), q)
+    W = small_signed(rng, (r, m, d), digits // 2, q) if digits else rand_mod(rng, (r, m, d), q)
+    key = api.DenseKey(api.to_dev(A), q)
+    w = api.to_dev(W)
+    assert np.array_equal(api.to_host(key.commit(w, w_slot=w)), oracle.dense_commit(A, W, q))
+    key.close()
