@@ -1412,15 +1412,23 @@ __global__ void project_kernel(RowSet in, u32 rows, u32 d, u64 q, u32 cw, u64 nc
         pm[kk] = msk[kk * words + w];
         nm[kk] = msk[KT * words + kk * words + w];
       }
-      for (u32 b = 0; b < 32; b++) {
-        const u64 x = wres(chunk, nar, (u64)(w * 32 + b) * d + pos, q);
-        const u64 nx = x ? q - x : 0;
+      // four loads ahead of their sums: one at a time, the item loop had cost
+      // 2 rows x 8192 x 512 1340 -> 1447 us; 1122 this way
+#pragma unroll 1
+      for (u32 b0 = 0; b0 < 32; b0 += 4) {
+        u64 xs[4];
 #pragma unroll
-        for (int kk = 0; kk < KT; kk++) {
-          u64 v = ((pm[kk] >> b) & 1) ? x : 0;
-          v = ((nm[kk] >> b) & 1) ? nx : v;
-          if (LAZY) acc[kk] += v;
-          else acc[kk] = add_mod(acc[kk], v, q);
+        for (u32 e = 0; e < 4; e++) xs[e] = wres(chunk, nar, (u64)(w * 32 + b0 + e) * d + pos, q);
+#pragma unroll
+        for (u32 e = 0; e < 4; e++) {
+          const u64 x = xs[e], nx = x ? q - x : 0;
+#pragma unroll
+          for (int kk = 0; kk < KT; kk++) {
+            u64 v = ((pm[kk] >> (b0 + e)) & 1) ? x : 0;
+            v = ((nm[kk] >> (b0 + e)) & 1) ? nx : v;
+            if (LAZY) acc[kk] += v;
+            else acc[kk] = add_mod(acc[kk], v, q);
+          }
         }
       }
     }
