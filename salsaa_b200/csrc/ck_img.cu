@@ -384,13 +384,14 @@ int launch_ck_img(const CkImgArgs& a, const CkImage& im, const ModQ& M, const u6
   const size_t epi = (size_t)V * 14 * (2 * a.nck + 1) * 16;
   // the MMA reads 128 rows of the last 16-byte slice: up to 2 KiB past the
   // stage's own bytes, inside the next stage or the partial sums
-  const size_t room = 225 * 1024 - (epi > 2048 ? epi : 2048);
+  constexpr size_t most = 225 * 1024;
+  const size_t room = most - (epi > 2048 ? epi : 2048);
   t.nst = (u32)(room / t.stage_bytes);
   if (t.nst > CKI_MAX_STAGES) t.nst = CKI_MAX_STAGES;
   if (t.nst < 2) return salsaa_set_error(-2, "ck_img: stages do not fit shared memory");
   const size_t smem = (size_t)t.nst * t.stage_bytes + (epi > 2048 ? epi : 2048);
   auto kern = t.E == 2 ? ck_img_kernel<2, 3> : a.nck <= 12 ? ck_img_kernel<1, 3> : ck_img_kernel<1, 5>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = smem_limit(kern, most);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ck_img smem attribute");
   const bool plain = M.q < (1ULL << 50) && im.width / t.Bw < (1ULL << 13);
   const double wit_bytes = 8.0 * im.R * (double)im.width * 2 * im.n;

@@ -422,6 +422,14 @@ static int ck_carveout(size_t smem) {
   return pct > 100 ? 100 : (int)pct;
 }
 
+// Dynamic shared memory for nck key rows: two stages, or the epilogue's sums over them.
+static size_t cku_smem(u32 nck) {
+  const size_t stage = 2 * (size_t)CKU_ATILE + 2 * (size_t)ck_tk8_nkp(nck) * CKU_CHUNK;
+  const size_t epi = 2 * 128 * (size_t)(2 * nck) * sizeof(u64);
+  return 2 * stage > epi ? 2 * stage : epi;
+}
+static const size_t CKU_MAX_SMEM = cku_smem(CKU_MAX_KEYS);
+
 bool ck_umma_ok(const CommitArgs& a, u32 n) {
   if (!a.tk8 || a.rows == 0 || a.rows > CKU_MAX_WROWS || a.nck == 0 || a.nck > CKU_MAX_KEYS || (n & 1)) return false;
   if (a.width < CKU_CHUNK || a.ck_bt < CKU_CHUNK) return false;
@@ -477,11 +485,8 @@ int launch_ck_umma_multi(const CommitArgs* a, u32 ninst, u32 n, const ModQ& M, c
   m.ystart[ninst] = y;
   m.count = ninst;
   const u32 nck = a[0].nck, nkp = ck_tk8_nkp(nck);
-  const size_t stage = 2 * (size_t)CKU_ATILE + 2 * (size_t)nkp * CKU_CHUNK;
-  const size_t epi = 2 * 128 * (size_t)(2 * nck) * sizeof(u64);
-  const size_t smem = 2 * stage > epi ? 2 * stage : epi;
-  cudaError_t e =
-      cudaFuncSetAttribute(ck_umma_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = cku_smem(nck);
+  cudaError_t e = smem_limit(ck_umma_multi_kernel, CKU_MAX_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ck_umma_multi_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, ck_carveout(smem));
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ck_umma_multi smem attribute");
@@ -502,10 +507,8 @@ int launch_ck_umma(const CommitArgs& a, u32 n, u32 Bw, u32 G, const ModQ& M, con
       a.ck_bt % Bw || a.width % ((u64)Bw * G))
     return salsaa_set_error(-2, "ck_umma: bad block grouping");
   const u32 nkp = ck_tk8_nkp(a.nck);
-  const size_t stage = 2 * (size_t)CKU_ATILE + 2 * (size_t)nkp * CKU_CHUNK;
-  const size_t epi = 2 * 128 * (size_t)(2 * a.nck) * sizeof(u64);
-  const size_t smem = 2 * stage > epi ? 2 * stage : epi;
-  cudaError_t e = cudaFuncSetAttribute(ck_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = cku_smem(a.nck);
+  cudaError_t e = smem_limit(ck_umma_kernel, CKU_MAX_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ck_umma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, ck_carveout(smem));
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ck_umma smem attribute");

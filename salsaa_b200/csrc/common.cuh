@@ -75,6 +75,15 @@ __host__ inline PdlLaunch<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block,
   return l;
 }
 
+// The most dynamic shared memory that `kernel` is ever launched with.  A
+// constant of the kernel and never the size of one call: the limit belongs to
+// the function, so a smaller one set by another host thread between this call
+// and its launch would fail the launch.
+template <typename... P>
+__host__ inline cudaError_t smem_limit(void (*kernel)(P...), size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 __host__ inline u64 shoup_pre(u64 w, u64 q) { return (u64)((((unsigned __int128)w) << 64) / q); }
 
 __device__ __forceinline__ u64 add_mod(u64 a, u64 b, u64 q) {

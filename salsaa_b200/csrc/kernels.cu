@@ -983,7 +983,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   const size_t smem = tail_max * sizeof(u64);
   auto tail = lazy ? sb_tail_kernel<true> : sb_tail_kernel<false>;
   if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = smem_limit(tail, SC_TAIL * sizeof(u64));
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: tail smem");
   }
   pdl(tail, count, TAIL_THREADS, smem, st)(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
@@ -1071,7 +1071,8 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
   const size_t smem = L * sizeof(u64);
   auto kern = sc_tail_kernel<LAZY>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t most = 128 * 1024;  // the next power of two is out of reach
+    cudaError_t e = smem_limit(kern, smem > most ? smem : most);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sc_tail smem attribute");
   }
   pdl(kern, 2 * rows, TAIL_THREADS, smem, st)(in, sin, w, L, rows, M, ds, round, j, B.sums, nr, d, B.cap, gl,
@@ -2437,12 +2438,15 @@ static int launch_ck_mma_t(const CommitArgs& a, u32 n, u32 Bw, const ModQ& M, co
                            cudaStream_t st) {
   constexpr u32 NP = 2 * NTW * 8;
   const u32 nmt = (a.nck + CKM_ROWS - 1) / CKM_ROWS;
-  const size_t stage = (size_t)(CKM_BM + NP) * CKM_LD;
-  const size_t epi = (size_t)CKM_BM * NP * sizeof(int) + (size_t)CKM_ROWS * a.rows * 28 * sizeof(u64);
-  const size_t smem = stage > epi ? stage : epi;
+  auto bytes = [](u32 rows) {
+    const size_t stage = (size_t)(CKM_BM + NP) * CKM_LD;
+    const size_t epi = (size_t)CKM_BM * NP * sizeof(int) + (size_t)CKM_ROWS * rows * 28 * sizeof(u64);
+    return stage > epi ? stage : epi;
+  };
+  const size_t smem = bytes(a.rows);
   auto kern = ck_mma_kernel<NTW>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = smem_limit(kern, bytes(MAX_WROWS));
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ck_mma smem attribute");
   }
   dim3 g(n, nmt, (unsigned)(a.width / Bw));

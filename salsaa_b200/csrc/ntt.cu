@@ -1264,7 +1264,8 @@ int ntt_launch(const u64* in, u64* out, u64 count, const NttDev& T, bool incompl
   if (blocks > 0x7fffffffULL) return salsaa_set_error(-2, "ntt: batch too large");
   auto launch = [&](auto kern) -> int {
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      constexpr size_t most = 128 * 1024;  // the next power of two is out of reach
+      cudaError_t e = smem_limit(kern, smem > most ? smem : most);
       if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ntt smem attribute");
     }
     // algorithmic bytes: every coefficient read once and written once

@@ -30,7 +30,7 @@ __host__ __device__ constexpr u32 idesc_s8(u32 M, u32 N) { return IDESC_S8 | ((N
 // Bound by HBM: 8 bytes out and one per row in a coefficient, against 16 per
 // row and 32 more for the slot-form fold and its inverse transform.
 // ---------------------------------------------------------------------------
-constexpr u32 FT_EPI = 256, FT_THREADS = FT_EPI + 64, FT_EL = 64;
+constexpr u32 FT_EPI = 256, FT_THREADS = FT_EPI + 64, FT_EL = 64, FT_MAX_ROWS = 8;
 
 template <u32 D>
 struct FtGeom {
@@ -579,7 +579,7 @@ int launch_fold_challenge_tz(const DevState* ds, u32 round, u32 rows, u32 d, u64
 }
 
 bool fold_tc_ok(const C8Rows& w, u32 d) {
-  return (d == 128 || d == 256) && w.rows >= 1 && w.rows <= 8 && w.width >= FT_EL && w.width % FT_EL == 0;
+  return (d == 128 || d == 256) && w.rows >= 1 && w.rows <= FT_MAX_ROWS && w.width >= FT_EL && w.width % FT_EL == 0;
 }
 
 int launch_fold_words_tz(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* wide, cudaStream_t st) {
@@ -592,12 +592,13 @@ int launch_fold_words_tz(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* 
 int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64 nout, u64* out, u64* mag_or, const u32* flag,
                    cudaStream_t st) {
   if (!fold_tc_ok(w, d) || !flag || nout > w.width) return salsaa_set_error(-2, "fold_tc: rows outside the byte-tile path");
-  const size_t smem = (size_t)w.rows * 32 * d + (d == 128 ? (size_t)FtGeom<128>::STAGES * FtGeom<128>::TILE
-                                                          : (size_t)FtGeom<256>::STAGES * FtGeom<256>::TILE);
+  const size_t ring = d == 128 ? (size_t)FtGeom<128>::STAGES * FtGeom<128>::TILE
+                               : (size_t)FtGeom<256>::STAGES * FtGeom<256>::TILE;
+  const size_t smem = (size_t)w.rows * 32 * d + ring;
   const u64 units = w.width / FT_EL;
   const unsigned grid = (unsigned)(units < 148 ? units : 148);
   auto kern = d == 128 ? fold_tc_kernel<128> : fold_tc_kernel<256>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = smem_limit(kern, (size_t)FT_MAX_ROWS * 32 * d + ring);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "fold_tc smem attribute");
   pdl(kern, grid, FT_THREADS, smem, st)(w, tz, q, nout, out, mag_or, flag, tc_error_word());
   salsaa_count_launch();

@@ -210,3 +210,37 @@ def test_prove_word_aligned_witness(api, oracle, cuda, d, folding, log_wit, roun
             assert np.array_equal(out.cpu().numpy(), want)
         pr.close()
     assert np.array_equal(api.to_host(dw), w.reshape(-1))
+
+
+def test_commits_of_many_threads(api, oracle):
+    """Host threads whose launches need different amounts of shared memory."""
+    import ctypes
+    import threading
+    import torch
+    from salsaa_b200 import lib
+    q, p = P.Q0, P.make_params(128, P.Q0, 12, 1 << 9, 1)
+    ctx = api.Context(p, crs_seed=5)
+    wants, errors = {}, []
+    for rows in (1, 9):
+        w = rand_mod(np.random.default_rng(rows), (rows, 1 << 9, 128), q)
+        wants[rows] = (w, oracle.commit_ck(p, 5, w))
+
+    def work(rows):
+        w, want = wants[rows]
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            dw, out = api.to_dev(w), api.dev_empty((12, rows, 128))
+            for _ in range(1000):
+                rc = lib().salsaa_commit(ctx.h, api._p(dw), rows, 1 << 9, api._p(out), ctypes.c_void_p(s.cuda_stream))
+                if rc:
+                    errors.append((rows, rc))
+                    return
+            if not np.array_equal(api.to_host(out), want):
+                errors.append((rows, "wrong"))
+
+    threads = [threading.Thread(target=work, args=(r,)) for r in (1, 9) * 4]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
