@@ -204,10 +204,10 @@ int salsaa_set_error(int code, const char* msg);
 // Stream-ordered scratch of one call, from the library's own memory pool (see
 // prover.cu); freed on the same stream.
 cudaError_t salsaa_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
-// Gives the pool's unused memory on the current device back to the system.
+// Gives the unused memory of every device's pool back to the system.
 void salsaa_scratch_trim();
 // A context or dense key came (+1) or went (-1); after the last one went the
-// pool's unused memory goes back.
+// pools' unused memory goes back.
 void salsaa_scratch_users(int delta);
 // Counts kernel launches issued by this library (reported by the benchmark).
 void salsaa_count_launch();

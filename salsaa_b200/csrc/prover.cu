@@ -11,6 +11,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/salsaa_gpu.h"
@@ -1845,21 +1846,79 @@ extern "C" void salsaa_ctx_destroy(salsaa_ctx* c) {
 // synchronisation as before, and all of it when the last context or dense key
 // is destroyed or one of the library's own allocations fails.
 static constexpr uint64_t SCRATCH_KEEP = 1ULL << 30;
-static std::mutex g_pool_mu;
-static cudaMemPool_t g_pool[64];
-static bool g_pool_tried[64];
 
-static cudaMemPool_t scratch_pool(cudaStream_t st) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (g_pool_tried[dev]) return g_pool[dev];
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return nullptr;  // not created inside a capture: the default pool serves this call
+namespace {
+// A pool lives as long as its context, whose handle may come again after a
+// device reset; the driver's id of a context never does.
+struct DriverFns {
+  int (*get_current)(void**) = nullptr;
+  int (*get_id)(void*, unsigned long long*) = nullptr;
+  int (*primary_state)(int, unsigned*, int*) = nullptr;
+  int (*primary_retain)(void**, int) = nullptr;
+  int (*primary_release)(int) = nullptr;
+  DriverFns() {
+    auto get = [](auto& fn, const char* name) {
+      void* p = nullptr;
+      cudaDriverEntryPointQueryResult res;
+      if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &res) == cudaSuccess && res == cudaDriverEntryPointSuccess)
+        fn = (std::remove_reference_t<decltype(fn)>)p;
+    };
+    get(get_current, "cuCtxGetCurrent");
+    get(get_id, "cuCtxGetId");
+    get(primary_state, "cuDevicePrimaryCtxGetState");
+    get(primary_retain, "cuDevicePrimaryCtxRetain");
+    get(primary_release, "cuDevicePrimaryCtxRelease");
   }
-  g_pool_tried[dev] = true;
+  bool ok() const { return get_current && get_id && primary_state && primary_retain && primary_release; }
+};
+const DriverFns& driver() {
+  static const DriverFns f;
+  return f;
+}
+// Id of the calling thread's context, 0 if it has none alive.
+u64 context_id() {
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  return driver().ok() && driver().get_current(&ctx) == 0 && ctx && driver().get_id(ctx, &id) == 0 ? id : 0;
+}
+// The same of a device's primary context.
+u64 primary_id(int dev) {
+  unsigned flags = 0;
+  int active = 0;
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  if (!driver().ok() || driver().primary_state(dev, &flags, &active) != 0 || !active ||
+      driver().primary_retain(&ctx, dev) != 0)
+    return 0;
+  if (driver().get_id(ctx, &id) != 0) id = 0;
+  driver().primary_release(dev);
+  return id;
+}
+
+struct ScratchPool {
+  u64 ctx;
+  int dev;
+  cudaMemPool_t pool;  // null: could not be created
+};
+std::mutex g_pool_mu;
+std::vector<ScratchPool> g_pools;  // those of contexts that are gone are not touched again
+
+cudaMemPool_t scratch_pool(cudaStream_t st) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool capturing = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  if (capturing) cudaGetLastError();
+  u64 id = context_id();
+  if (!id && !capturing) {  // the first call of this thread, or since a reset
+    cudaFree(nullptr);
+    id = context_id();
+  }
+  if (!id) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  for (const ScratchPool& p : g_pools)
+    if (p.ctx == id && p.dev == dev) return p.pool;
+  if (capturing) return nullptr;  // not created inside a capture: the default pool serves this call
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -1867,13 +1926,15 @@ static cudaMemPool_t scratch_pool(cudaStream_t st) {
   cudaMemPool_t pool = nullptr;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    pool = nullptr;
+  } else {
+    uint64_t keep = SCRATCH_KEEP;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
-  uint64_t keep = SCRATCH_KEEP;
-  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  g_pool[dev] = pool;
+  g_pools.push_back({id, dev, pool});
   return pool;
 }
+}  // namespace
 
 cudaError_t salsaa_scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
   cudaMemPool_t pool = scratch_pool(st);
@@ -1881,10 +1942,10 @@ cudaError_t salsaa_scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
 }
 
 void salsaa_scratch_trim() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+  const u64 here = g_pools.empty() ? 0 : context_id();
+  for (const ScratchPool& p : g_pools)
+    if (p.pool && (p.ctx == here || p.ctx == primary_id(p.dev))) cudaMemPoolTrimTo(p.pool, 0);
 }
 
 static std::atomic<int> g_scratch_users{0};
