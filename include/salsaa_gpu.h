@@ -125,6 +125,13 @@ uint64_t salsaa_kernel_launches(void);
  * has, in which case the results of that launch are invalid.  Call it after
  * the launches in question have finished (after synchronizing their stream). */
 int salsaa_device_status(void);
+/* The entry points that need temporary device memory take it, on the given
+ * stream, from a memory pool of the library (one per device), which keeps up
+ * to 1 GiB that is not in use for later calls.  This gives what is not in use
+ * back to the system, on every device; so does destroying the last context or
+ * dense key.  Memory of calls still running on a stream stays until a later
+ * call of this.  Returns 0. */
+int salsaa_scratch_release(void);
 /* Device-time trace for measurement (off by default): enable/reset, then read
  * the summed device time (CUDA events on the launching stream), summed
  * algorithmic work and launch count of a traced kernel by name.  Traced:

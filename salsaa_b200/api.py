@@ -59,6 +59,12 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def scratch_release():
+    """Gives the device memory that the library keeps for the scratch of later
+    calls (at most 1 GiB per device) back to the system."""
+    _check(lib().salsaa_scratch_release(), "scratch_release")
+
+
 # ---- parameter sets -----------------------------------------------------------
 def params_preset(name):
     p = SalsaaParams()

@@ -1844,7 +1844,8 @@ extern "C" void salsaa_ctx_destroy(salsaa_ctx* c) {
 // workspace of a call over an A0-sized witness (2^26 coefficients, 512 MiB)
 // with room for a second stream.  What exceeds it goes back at the next
 // synchronisation as before, and all of it when the last context or dense key
-// is destroyed or one of the library's own allocations fails.
+// is destroyed, salsaa_scratch_release is called or an allocation for one of
+// the library's objects fails.
 static constexpr uint64_t SCRATCH_KEEP = 1ULL << 30;
 
 namespace {
@@ -1946,6 +1947,11 @@ void salsaa_scratch_trim() {
   const u64 here = g_pools.empty() ? 0 : context_id();
   for (const ScratchPool& p : g_pools)
     if (p.pool && (p.ctx == here || p.ctx == primary_id(p.dev))) cudaMemPoolTrimTo(p.pool, 0);
+}
+
+extern "C" int salsaa_scratch_release(void) {
+  salsaa_scratch_trim();
+  return 0;
 }
 
 static std::atomic<int> g_scratch_users{0};

@@ -42,3 +42,19 @@ def test_scratch_after_device_reset(gpu_lib):
     """A pool ends with its context; calls after a reset get one of their own."""
     r = subprocess.run([sys.executable, "-c", AFTER_RESET], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_scratch_release(gpu_lib, cuda):
+    """Without a context or dense key nothing else gives the memory back."""
+    from salsaa_b200 import api, params as P
+    w = cuda.ones((8, 1 << 15, 128), dtype=cuda.int64, device="cuda")
+    c = cuda.ones((8, 128), dtype=cuda.int64, device="cuda")
+    api.fold(w, P.Q0, c)
+    cuda.cuda.synchronize()
+    kept = cuda.cuda.mem_get_info()[0]
+    api.scratch_release()
+    free = cuda.cuda.mem_get_info()[0]
+    assert free - kept >= w.numel() * 8  # the rows' slot form alone is that large
+    cuda.cuda.synchronize()
+    assert cuda.equal(api.fold(w, P.Q0, c), api.fold(w, P.Q0, c))
+    api.scratch_release()
