@@ -2,8 +2,6 @@
 // products, and a self-test of the int8 tensor-core building block.
 #include <cuda_runtime.h>
 
-#include <atomic>
-
 #include "../../include/salsaa_gpu.h"
 #include "kernels.cuh"
 #include "ntt.cuh"
@@ -944,16 +942,11 @@ int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScR
   return e == cudaSuccess ? 0 : salsaa_set_cuda_error(e, "sc_umma launch");
 }
 
+// Looked up on each call: the address belongs to the current context, and a
+// device reset or another context of the device has another.
 u32* tc_error_word() {
-  static std::atomic<u32*> word[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  u32* p = word[dev].load(std::memory_order_acquire);
-  if (p) return p;
   void* v = nullptr;
-  if (cudaGetSymbolAddress(&v, g_tc_error) != cudaSuccess) return nullptr;
-  word[dev].store((u32*)v, std::memory_order_release);
-  return (u32*)v;
+  return cudaGetSymbolAddress(&v, g_tc_error) == cudaSuccess ? (u32*)v : nullptr;
 }
 
 int tc_error_check() {

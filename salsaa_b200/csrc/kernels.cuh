@@ -131,7 +131,7 @@ int launch_sc_umma(const RowSet& wc, u32 rows, u32 d, u32 Bw, u32 nhi, const ScR
                    cudaStream_t st);
 // Nonzero (and the last error set) when a tensor-core kernel's bounded wait gave up.
 int tc_error_check();
-// The current device's error word of the tensor-core kernels (null if unavailable).
+// The current context's error word of the tensor-core kernels (null if unavailable).
 u32* tc_error_word();
 int launch_gen_witness(u64* w, u32 rows, u64 width, u32 d, u64 q, const DevState* ds, cudaStream_t st);
 int launch_expand_i8(const int8_t* in, u64 n, u64 q, u64* out, cudaStream_t st);
