@@ -842,13 +842,29 @@ int launch_sumcheck_fq2_batch(const u64* const* vecs, const u64* lens, u32 count
   return check_launch("sumcheck_fq2 claims");
 }
 
+// The plan of a batch (per level the instances still longer than SC_TAIL, the
+// tail's behind them, then each instance's first polynomial) goes to the device
+// as a kernel's arguments: a copy from host memory would be read again by every
+// replay of a captured graph, long after that memory is gone.
+constexpr u32 SB_MAX_LEV = 4;  // 2^30 / 16^4 = SC_TAIL
+struct SbPlan {
+  SbInst inst[(SB_MAX_LEV + 1) * SB_MAX_INST];
+  u64 offs[SB_MAX_INST];
+};
+static_assert(sizeof(SbPlan) % 8 == 0 && sizeof(SbPlan) < 32000, "a kernel's arguments");
+__global__ void __launch_bounds__(256) sb_plan_kernel(const __grid_constant__ SbPlan p, u64* out) {
+  pdl_wait();
+  const u32 t = blockIdx.x * 256 + threadIdx.x;
+  if (t < sizeof(SbPlan) / 8) out[t] = ((const u64*)&p)[t];
+}
+
 int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, const ModQ& M, u64 seed, u32 round,
                           u64* claims, u64* polys, cudaStream_t st) {
   if (count == 0) return 0;
   if (count > SB_MAX_INST) return salsaa_set_error(-2, "sumcheck_batch: at most 64 instances");
   u32 nrmax = 0;
   std::vector<u32> nrs(count);
-  std::vector<u64> offs(count);
+  SbPlan plan{};
   u64 tot_a = 0, tot_b = 0, off = 0, max_tiles = 0;
   for (u32 i = 0; i < count; i++) {
     const u64 L = lens[i];
@@ -856,7 +872,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       return salsaa_set_error(-2, "sumcheck_batch: lengths must be powers of two in 2..2^30");
     nrs[i] = 63u - (u32)__builtin_clzll(L);
     nrmax = nrs[i] > nrmax ? nrs[i] : nrmax;
-    offs[i] = off;
+    plan.offs[i] = off;
     off += nrs[i];
     if (L > SC_TAIL) {
       tot_a += L / 16;
@@ -867,9 +883,6 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   }
   const bool lazy = M.q < (1ULL << 50);
   const bool plain = lazy && max_tiles < (1ULL << 13);
-  // device scratch: sums, two ping-pong areas, descriptors, nrs / offs
-  const u32 maxlev = 8;  // 16^8 > 2^30
-  const u64 desc_bytes = (u64)(maxlev + 1) * SB_MAX_INST * sizeof(SbInst);
   int rc = 0;
   struct Guard {
     void* p;
@@ -878,7 +891,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       if (p) cudaFreeAsync(p, s);
     }
   } guard{nullptr, st};
-  // one allocation: sums | descriptors | nrs | offs | the two areas
+  // one allocation: sums | plan | the two areas
   auto up = [](u64 b) { return (b + 255) / 256 * 256; };
   // levels on the tensor cores where the modulus allows (their vectors, longer
   // than SC_TAIL, are whole tiles); their Gram matrices lie behind the sums
@@ -891,9 +904,9 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       glev = n > glev ? n : glev;
     }
   const u64 gram_b = up(glev * SB_MAX_INST * 256 * 8);
-  const u64 sum_b = up((u64)count * nrmax * 3 * 8) + gram_b, desc_b = up(desc_bytes), off_b = up(count * 8);
+  const u64 sum_b = up((u64)count * nrmax * 3 * 8) + gram_b, plan_b = up(sizeof(SbPlan));
   {
-    cudaError_t ea = salsaa_scratch_alloc(&guard.p, sum_b + desc_b + off_b + up(tot_a * 8) + tot_b * 8 + 256, st);
+    cudaError_t ea = salsaa_scratch_alloc(&guard.p, sum_b + plan_b + up(tot_a * 8) + tot_b * 8 + 256, st);
     if (ea != cudaSuccess) {
       guard.p = nullptr;
       return salsaa_set_cuda_error(ea, "sumcheck_batch: workspace");
@@ -901,15 +914,13 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
   }
   char* base = (char*)guard.p;
   u64* sums = (u64*)base;
-  SbInst* ddesc = (SbInst*)(base + sum_b);
-  u64* doffs = (u64*)(base + sum_b + desc_b);
-  u64* bufa = (u64*)(base + sum_b + desc_b + off_b);
+  const SbPlan* dplan = (const SbPlan*)(base + sum_b);
+  const SbInst* ddesc = dplan->inst;
+  u64* bufa = (u64*)(base + sum_b + plan_b);
   u64* bufb = (u64*)((char*)bufa + up(tot_a * 8));
   u64* gram = (u64*)(base + sum_b - gram_b);
   cudaError_t e = cudaMemsetAsync(sums, 0, sum_b, st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: memset");
-  // host plan: per level, the instances still longer than SC_TAIL, then the tail
-  std::vector<SbInst> plan((maxlev + 1) * SB_MAX_INST);
   std::vector<u32> lev_n;
   std::vector<u64> lev_tiles;
   std::vector<const u64*> cur_in(vecs, vecs + count);
@@ -927,7 +938,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       }
     }
   }
-  for (u32 lev = 0; lev < maxlev; lev++) {
+  for (u32 lev = 0; lev < SB_MAX_LEV; lev++) {
     u64 tiles = 0;
     u32 n = 0;
     for (u32 i = 0; i < count; i++) {
@@ -939,7 +950,7 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
       I.tile0 = tiles;
       I.j = cur_j[i];
       I.id = i;
-      plan[lev * SB_MAX_INST + n++] = I;
+      plan.inst[lev * SB_MAX_INST + n++] = I;
       tiles += cur_L[i] / 16 / SB_TILE_GROUPS;
       cur_in[i] = I.out;
       cur_L[i] /= 16;
@@ -957,13 +968,11 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     I.L = cur_L[i];
     I.j = cur_j[i];
     I.id = i;
-    plan[maxlev * SB_MAX_INST + i] = I;
+    plan.inst[SB_MAX_LEV * SB_MAX_INST + i] = I;
     tail_max = cur_L[i] > tail_max ? cur_L[i] : tail_max;
   }
-  e = cudaMemcpyAsync(ddesc, plan.data(), desc_bytes, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(doffs, offs.data(), count * 8, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: plan");
-  // (from pageable memory the copies are staged before cudaMemcpyAsync returns)
+  pdl(sb_plan_kernel, (unsigned)((sizeof(SbPlan) / 8 + 255) / 256), 256, 0, st)(plan, (u64*)dplan);
+  if ((rc = check_launch("sb_plan"))) return rc;
   for (u32 lev = 0; lev < nlev; lev++) {
     const u64 grid = lev_tiles[lev] < 296 ? lev_tiles[lev] : 296;
     if (tc) {
@@ -986,8 +995,8 @@ int launch_sumcheck_batch(const u64* const* vecs, const u64* lens, u32 count, co
     e = smem_limit(tail, SC_TAIL * sizeof(u64));
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck_batch: tail smem");
   }
-  pdl(tail, count, TAIL_THREADS, smem, st)(ddesc + maxlev * SB_MAX_INST, M, seed, round, sums, nrmax, glev ? gram : nullptr, doffs,
-                                   claims, polys);
+  pdl(tail, count, TAIL_THREADS, smem, st)(ddesc + SB_MAX_LEV * SB_MAX_INST, M, seed, round, sums, nrmax,
+                                           glev ? gram : nullptr, dplan->offs, claims, polys);
   return check_launch("sb_tail");
 }
 

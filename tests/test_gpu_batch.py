@@ -188,3 +188,23 @@ def test_sumcheck_fq2_bench_instances(api, oracle, cuda):
         claim, want, _ = oracle.sumcheck_fq2(v, q, shift, cs)
         assert int(claims[i]) == claim
         assert np.array_equal(api.to_host(polys[i]), want)
+
+
+@pytest.mark.parametrize("q", [P.Q0, P.Q62])
+def test_sumcheck_batch_captured(api, oracle, cuda, q):
+    """Replays of a captured batch, on the captured buffers' new contents."""
+    rng = np.random.default_rng(5)
+    vecs = [cuda.zeros(1 << k, dtype=cuda.int64, device="cuda") for k in (4, 15, 18, 19)]
+    api.sum_check_batch(vecs, q, 12, 3)
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph):
+        claims, polys = api.sum_check_batch(vecs, q, 12, 3)
+    for _ in range(2):
+        host = [rand_mod(rng, v.numel(), q) for v in vecs]
+        for v, h in zip(vecs, host):
+            v.copy_(api.to_dev(h))
+        graph.replay()
+        got = api.to_host(claims)
+        for i, h in enumerate(host):
+            claim, want, _ = oracle.sumcheck(h, q, nc_challenges(12, 3, i, h.size.bit_length() - 1, q))
+            assert int(got[i]) == claim and np.array_equal(api.to_host(polys[i]), want), i
