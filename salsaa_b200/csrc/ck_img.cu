@@ -378,7 +378,8 @@ int launch_ck_img(const CkImgArgs& a, const CkImage& im, const ModQ& M, const u6
   const u32 nkp = ck_tk8_nkp(a.nck), V = im.R * im.G;
   u32 nkc = 32;  // TMEM columns between accumulators
   while (nkc < nkp) nkc *= 2;
-  if (!im.p || !a.tk8 || V == 0 || V > CKI_MAX_V || a.nck == 0 || a.nck > CKU_MAX_KEYS || im.width > (u64)a.ck_bt * a.ck_nhi)
+  if (!im.p || !a.tk8 || V == 0 || V > CKI_MAX_V || a.nck == 0 || a.nck > CKU_MAX_KEYS ||
+      im.width > (u64)a.ck_bt * a.ck_nhi)
     return salsaa_set_error(-2, "ck_img: shape outside the image path");
   CkImgTiles t = cki_tiles(im, a.nck, nkp, nkc);
   const size_t epi = (size_t)V * 14 * (2 * a.nck + 1) * 16;

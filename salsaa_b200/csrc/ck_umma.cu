@@ -757,163 +757,161 @@ __global__ void __launch_bounds__(512, 1)
   const u32 idesc = umma::idesc_u8(128, SU_POS) | (1u << 10);
   bool ok = true;
   // work items: positions pb, element block hb (one s_hi factor), its part sub
-  // of split, witness row k; g0 counts the steps of earlier items
-  // and group of scalar rows
+  // of split, witness row k and group grp of scalar rows; g0 counts the steps
+  // of earlier items
   const u32 npb = d / SU_POS, per = npb * nhi * split * rows, items = per * rg.groups();
   u32 g0 = 0;
   for (u32 item = blockIdx.x; item < items; item += gridDim.x) {
-  const u32 pb = item % npb, hs = item / npb % (nhi * split), k = item / (npb * nhi * split) % rows;
-  const u32 grp = item / per, nrow = rg.rows(grp), j0 = rg.first(grp);
-  const u32 hb = hs / split, sub = hs % split;
-  if (!gates.open(k)) continue;
-  const u32 c0 = sub * nsteps;
-  const bool nar = (wc.narrow >> k) & 1;
-  const u64* src0 = row_advance(wc.p[k], nar, ((u64)hb * Bw + (u64)c0 * SU_KS) * d + (u64)pb * SU_POS);
-  const uint8_t* img = img0 + (u64)grp * Bw * 128 + (u64)c0 * SU_A;
-  bool bad = false;
-  // task of this thread: 16 consecutive elements x 2 neighbouring positions,
-  // one 16-byte load per element for word rows (two u64 values) and one
-  // 8-byte load for narrow rows (two int32 values, kept in wv[e].x); one
-  // 16-byte store per limb plane and position
-  ulonglong2 wv[16];
-  const u32 nkq = tid >> 6, np2 = tid & 63;
-  auto load = [&](u32 c) {
-    if (nar) {
-      const int* src = (const int*)src0 + (u64)c * SU_KS * d;
+    const u32 pb = item % npb, hs = item / npb % (nhi * split), k = item / (npb * nhi * split) % rows;
+    const u32 grp = item / per, nrow = rg.rows(grp), j0 = rg.first(grp);
+    const u32 hb = hs / split, sub = hs % split;
+    if (!gates.open(k)) continue;
+    const u32 c0 = sub * nsteps;
+    const bool nar = (wc.narrow >> k) & 1;
+    const u64* src0 = row_advance(wc.p[k], nar, ((u64)hb * Bw + (u64)c0 * SU_KS) * d + (u64)pb * SU_POS);
+    const uint8_t* img = img0 + (u64)grp * Bw * 128 + (u64)c0 * SU_A;
+    bool bad = false;
+    // task of this thread: 16 consecutive elements x 2 neighbouring positions,
+    // one 16-byte load per element for word rows (two u64 values) and one
+    // 8-byte load for narrow rows (two int32 values, kept in wv[e].x); one
+    // 16-byte store per limb plane and position
+    ulonglong2 wv[16];
+    const u32 nkq = tid >> 6, np2 = tid & 63;
+    auto load = [&](u32 c) {
+      if (nar) {
+        const int* src = (const int*)src0 + (u64)c * SU_KS * d;
 #pragma unroll
-      for (u32 e = 0; e < 16; e++)
-        wv[e].x = (u64)__ldg((const long long*)(src + (u64)(16 * nkq + e) * d + 2 * np2));
-    } else {
-      const u64* src = src0 + (u64)c * SU_KS * d;
+        for (u32 e = 0; e < 16; e++)
+          wv[e].x = (u64)__ldg((const long long*)(src + (u64)(16 * nkq + e) * d + 2 * np2));
+      } else {
+        const u64* src = src0 + (u64)c * SU_KS * d;
 #pragma unroll
-      for (u32 e = 0; e < 16; e++) wv[e] = __ldg((const ulonglong2*)(src + (u64)(16 * nkq + e) * d + 2 * np2));
-    }
-  };
-  load(0);
-  for (u32 c = 0; c < nsteps; c++) {
-    const u32 g = g0 + c, st = g & 1;
-    uint8_t* stage = smem + st * SU_STAGE;
-    if (g >= 2) ok &= umma::mbar_wait(&done_bar[st], ((g - 2) >> 1) & 1, err, 1);
-    if (tid == 0) {
-      umma::mbar_expect_tx(&full_bar[st], SU_A);
-      umma::bulk_g2s(stage, img + (u64)c * SU_A, SU_A, &full_bar[st]);
-    }
-#pragma unroll
-    for (u32 p = 0; p < 2; p++) {
-      u32 l0[4], l1[4], l2[4];
-#pragma unroll
-      for (u32 g = 0; g < 4; g++) {
-        u32 wq[4];
-#pragma unroll
-        for (u32 e = 0; e < 4; e++) {
-          const ulonglong2 v2 = wv[4 * g + e];
-          // centred value + 0x808080: its bytes are the signed limbs + 128 when
-          // the value lies in [-0x808080, 0x7f7f7f] (three balanced base-256 digits)
-          if (nar) {
-            const int v = (int)(u32)(p ? (v2.x >> 32) : v2.x);
-            bad |= (v > 0x7f7f7f) | (v < -0x808080);  // the value needs a fourth limb
-            wq[e] = ((u32)v + 0x808080u) ^ 0x808080u;
-          } else {
-            const u64 v = p ? v2.y : v2.x;
-            const u64 tb = v + 0x808080ULL - (v > half_q ? q : 0);
-            bad |= (tb >> 24) != 0;
-            wq[e] = (u32)tb ^ 0x808080u;
-          }
-        }
-        // limb planes of the four values: byte l of wq[0..3]
-        const u32 lo01 = __byte_perm(wq[0], wq[1], 0x5140), lo23 = __byte_perm(wq[2], wq[3], 0x5140);
-        const u32 hi01 = __byte_perm(wq[0], wq[1], 0x0062), hi23 = __byte_perm(wq[2], wq[3], 0x0062);
-        l0[g] = __byte_perm(lo01, lo23, 0x5410);
-        l1[g] = __byte_perm(lo01, lo23, 0x7632);
-        l2[g] = __byte_perm(hi01, hi23, 0x5410);
+        for (u32 e = 0; e < 16; e++) wv[e] = __ldg((const ulonglong2*)(src + (u64)(16 * nkq + e) * d + 2 * np2));
       }
-      const u32 off = SU_A + nkq * (SU_POS * 16) + (2 * np2 + p) * 16;
-      *(uint4*)(stage + off) = make_uint4(l0[0], l0[1], l0[2], l0[3]);
-      *(uint4*)(stage + off + SU_B) = make_uint4(l1[0], l1[1], l1[2], l1[3]);
-      *(uint4*)(stage + off + 2 * SU_B) = make_uint4(l2[0], l2[1], l2[2], l2[3]);
+    };
+    load(0);
+    for (u32 c = 0; c < nsteps; c++) {
+      const u32 g = g0 + c, st = g & 1;
+      uint8_t* stage = smem + st * SU_STAGE;
+      if (g >= 2) ok &= umma::mbar_wait(&done_bar[st], ((g - 2) >> 1) & 1, err, 1);
+      if (tid == 0) {
+        umma::mbar_expect_tx(&full_bar[st], SU_A);
+        umma::bulk_g2s(stage, img + (u64)c * SU_A, SU_A, &full_bar[st]);
+      }
+#pragma unroll
+      for (u32 p = 0; p < 2; p++) {
+        u32 l0[4], l1[4], l2[4];
+#pragma unroll
+        for (u32 g = 0; g < 4; g++) {
+          u32 wq[4];
+#pragma unroll
+          for (u32 e = 0; e < 4; e++) {
+            const ulonglong2 v2 = wv[4 * g + e];
+            // centred value + 0x808080: its bytes are the signed limbs + 128 when
+            // the value lies in [-0x808080, 0x7f7f7f] (three balanced base-256 digits)
+            if (nar) {
+              const int v = (int)(u32)(p ? (v2.x >> 32) : v2.x);
+              bad |= (v > 0x7f7f7f) | (v < -0x808080);  // the value needs a fourth limb
+              wq[e] = ((u32)v + 0x808080u) ^ 0x808080u;
+            } else {
+              const u64 v = p ? v2.y : v2.x;
+              const u64 tb = v + 0x808080ULL - (v > half_q ? q : 0);
+              bad |= (tb >> 24) != 0;
+              wq[e] = (u32)tb ^ 0x808080u;
+            }
+          }
+          // limb planes of the four values: byte l of wq[0..3]
+          const u32 lo01 = __byte_perm(wq[0], wq[1], 0x5140), lo23 = __byte_perm(wq[2], wq[3], 0x5140);
+          const u32 hi01 = __byte_perm(wq[0], wq[1], 0x0062), hi23 = __byte_perm(wq[2], wq[3], 0x0062);
+          l0[g] = __byte_perm(lo01, lo23, 0x5410);
+          l1[g] = __byte_perm(lo01, lo23, 0x7632);
+          l2[g] = __byte_perm(hi01, hi23, 0x5410);
+        }
+        const u32 off = SU_A + nkq * (SU_POS * 16) + (2 * np2 + p) * 16;
+        *(uint4*)(stage + off) = make_uint4(l0[0], l0[1], l0[2], l0[3]);
+        *(uint4*)(stage + off + SU_B) = make_uint4(l1[0], l1[1], l1[2], l1[3]);
+        *(uint4*)(stage + off + 2 * SU_B) = make_uint4(l2[0], l2[1], l2[2], l2[3]);
+      }
+      if (c + 1 < nsteps) load(c + 1);
+      umma::fence_proxy_async();
+      umma::fence_before_sync();
+      __syncthreads();
+      if (tid == 0) {
+        umma::fence_after_sync();
+        ok &= umma::mbar_wait(&full_bar[st], (g >> 1) & 1, err, 2);
+#pragma unroll
+        for (u32 l = 0; l < SU_LIMBS; l++)
+#pragma unroll
+          for (u32 ks = 0; ks < SU_KS / 32; ks++) {
+            const uint64_t ad = umma::desc_kmajor(umma::smem_u32(stage + ks * 2 * 128 * 16), 128 * 16, 128);
+            const uint64_t bd =
+                umma::desc_kmajor(umma::smem_u32(stage + SU_A + l * SU_B + ks * 2 * SU_POS * 16), SU_POS * 16, 128);
+            umma::mma_i8(tmem + l * 128, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
+          }
+        umma::commit(&done_bar[st]);
+      }
     }
-    if (c + 1 < nsteps) load(c + 1);
+    const u32 gl = g0 + nsteps - 1;
+    ok &= umma::mbar_wait(&done_bar[gl & 1], (gl >> 1) & 1, err, 3);
+    ok = __syncthreads_and(ok);
+    bad = __syncthreads_or(bad);
+    umma::fence_after_sync();
+    g0 += nsteps;
+    if (ok && !bad) {
+      // per TMEM lane (row (r, x)), per position: sum_l 2^(8l) D_l, reduced, times 2^(8x)
+      u64* Pm = (u64*)smem;  // 128 rows x 128 positions
+      const u32 row = (warp & 3) * 32 + lane, quarter = warp >> 2;  // four groups of 32 positions
+      const u32 x = row % 8;  // column 7 of a row's eight is zero
+      const u64 pw = ((u64)1 << (8 * x)) % q;
+      const u64 cpos = ((((u64)1 << 62) / q) + 1) * q;
+      for (u32 cb = quarter * 32; cb < quarter * 32 + 32; cb += 16) {
+        uint32_t r0[16], r1[16], r2[16];
+        const u32 base = tmem + (((warp & 3) * 32) << 16) + cb;
+        umma::tmem_ld16(base, r0);
+        umma::tmem_ld16(base + 128, r1);
+        umma::tmem_ld16(base + 256, r2);
+        umma::tmem_wait_ld();
+#pragma unroll
+        for (u32 e = 0; e < 16; e++) {
+          const long long v = (long long)(int)r0[e] + ((long long)(int)r1[e] << 8) + ((long long)(int)r2[e] << 16);
+          const u64 red = reduce64(M, v < 0 ? (u64)(v + (long long)cpos) : (u64)v);
+          Pm[(u64)row * 128 + cb + e] = mul_mod(M, red, pw);
+        }
+      }
+    }
+    __syncthreads();
+    if (ok && !bad) {
+      const u64* Pm = (const u64*)smem;
+      for (u32 t = tid; t < nrow * SU_POS; t += 512) {
+        const u32 r = t / SU_POS, pos = t % SU_POS;
+        u64 v = 0;
+#pragma unroll
+        for (u32 x = 0; x < 7; x++) v = salsaa::add_mod(v, Pm[(u64)(r * 8 + x) * 128 + pos], q);
+        const u32 j = j0 + r;
+        v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
+        atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
+      }
+    }
+    if (ok && bad) {  // exact CUDA-core sums of this item
+      for (u32 t = tid; t < nrow * SU_POS; t += 512) {
+        const u32 r = t / SU_POS, pos = t % SU_POS, j = j0 + r;
+        u64 v = 0;
+        for (u32 i = 0; i < nsteps * SU_KS; i++)
+          v = salsaa::add_mod(v, mul_mod(M, s_lo[(u64)j * Bw + c0 * SU_KS + i], wres(src0, nar, (u64)i * d + pos, q)), q);
+        v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
+        atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
+      }
+    }
+    // the next item's copies and MMAs reuse the stages and TMEM read above
     umma::fence_proxy_async();
     umma::fence_before_sync();
     __syncthreads();
-    if (tid == 0) {
-      umma::fence_after_sync();
-      ok &= umma::mbar_wait(&full_bar[st], (g >> 1) & 1, err, 2);
-#pragma unroll
-      for (u32 l = 0; l < SU_LIMBS; l++)
-#pragma unroll
-        for (u32 ks = 0; ks < SU_KS / 32; ks++) {
-          const uint64_t ad = umma::desc_kmajor(umma::smem_u32(stage + ks * 2 * 128 * 16), 128 * 16, 128);
-          const uint64_t bd =
-              umma::desc_kmajor(umma::smem_u32(stage + SU_A + l * SU_B + ks * 2 * SU_POS * 16), SU_POS * 16, 128);
-          umma::mma_i8(tmem + l * 128, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
-        }
-      umma::commit(&done_bar[st]);
-    }
-  }
-  const u32 gl = g0 + nsteps - 1;
-  ok &= umma::mbar_wait(&done_bar[gl & 1], (gl >> 1) & 1, err, 3);
-  ok = __syncthreads_and(ok);
-  bad = __syncthreads_or(bad);
-  umma::fence_after_sync();
-  g0 += nsteps;
-  if (ok && !bad) {
-    // per TMEM lane (row (r, x)), per position: sum_l 2^(8l) D_l, reduced, times 2^(8x)
-    u64* Pm = (u64*)smem;  // 128 rows x 128 positions
-    const u32 row = (warp & 3) * 32 + lane, quarter = warp >> 2;  // four groups of 32 positions
-    const u32 x = row % 8;  // column 7 of a row's eight is zero
-    const u64 pw = ((u64)1 << (8 * x)) % q;
-    const u64 cpos = ((((u64)1 << 62) / q) + 1) * q;
-    for (u32 cb = quarter * 32; cb < quarter * 32 + 32; cb += 16) {
-      uint32_t r0[16], r1[16], r2[16];
-      const u32 base = tmem + (((warp & 3) * 32) << 16) + cb;
-      umma::tmem_ld16(base, r0);
-      umma::tmem_ld16(base + 128, r1);
-      umma::tmem_ld16(base + 256, r2);
-      umma::tmem_wait_ld();
-#pragma unroll
-      for (u32 e = 0; e < 16; e++) {
-        const long long v = (long long)(int)r0[e] + ((long long)(int)r1[e] << 8) + ((long long)(int)r2[e] << 16);
-        const u64 red = reduce64(M, v < 0 ? (u64)(v + (long long)cpos) : (u64)v);
-        Pm[(u64)row * 128 + cb + e] = mul_mod(M, red, pw);
-      }
-    }
-  }
-  __syncthreads();
-  if (ok && !bad) {
-    const u64* Pm = (const u64*)smem;
-    for (u32 t = tid; t < nrow * SU_POS; t += 512) {
-      const u32 r = t / SU_POS, pos = t % SU_POS;
-      u64 v = 0;
-#pragma unroll
-      for (u32 x = 0; x < 7; x++) v = salsaa::add_mod(v, Pm[(u64)(r * 8 + x) * 128 + pos], q);
-      const u32 j = j0 + r;
-      v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
-      atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
-    }
-  }
-  if (ok && bad) {  // exact CUDA-core sums of this item
-    for (u32 t = tid; t < nrow * SU_POS; t += 512) {
-      const u32 r = t / SU_POS, pos = t % SU_POS, j = j0 + r;
-      u64 v = 0;
-      for (u32 i = 0; i < nsteps * SU_KS; i++)
-        v = salsaa::add_mod(v, mul_mod(M, s_lo[(u64)j * Bw + c0 * SU_KS + i], wres(src0, nar, (u64)i * d + pos, q)), q);
-      v = mul_mod(M, v, s_hi[(u64)j * nhi + hb]);
-      atomic_add_mod(acc + ((u64)j * rows + k) * d + (u64)pb * SU_POS + pos, v, q, plain);
-    }
-  }
-  // the next item's copies and MMAs reuse the stages and TMEM read above
-  umma::fence_proxy_async();
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  if (!ok) break;
+    umma::fence_after_sync();
+    if (!ok) break;
   }
   __syncthreads();
   if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
-
-
 
 int launch_sc_img(const u64* s_lo, u32 Bw, const ScRange& rg, uint8_t* img, cudaStream_t st) {
   const u64 g = ((u64)Bw * 128 * rg.groups() + 255) / 256;

@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2) gram_words_kernel(const __grid_
   uint8_t* btab = smem + GW_IMG;
   const u32 tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const u64 q = M.q;
-  const u32 t0 = (u32)((u64)blockIdx.x * a.ntiles / gridDim.x), t1 = (u32)((u64)(blockIdx.x + 1) * a.ntiles / gridDim.x);
+  const u32 t0 = (u32)((u64)blockIdx.x * a.ntiles / gridDim.x);
+  const u32 t1 = (u32)((u64)(blockIdx.x + 1) * a.ntiles / gridDim.x);
   if (MODE == GW_BATCH)
     for (u32 i = tid; i <= a.ninst; i += GR_THREADS) t0s[i] = i < a.ninst ? (u32)a.inst[i].tile0 * SB_GPT : a.ntiles;
   if (tid == 0) {
@@ -286,7 +287,7 @@ int gw_launch(GwArgs& a, const ModQ& M, cudaStream_t st) {
   const u32 grid = a.ntiles < 296 ? a.ntiles : 296;
   // adds to one Gram entry: one per segment
   a.plain = M.q < (1ULL << 50) && a.ntiles / GW_SEG + grid + SB_MAX_INST < (1u << 13);
-  cudaError_t e = cudaFuncSetAttribute(gram_words_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GW_SMEM);
+  cudaError_t e = smem_limit(gram_words_kernel<MODE>, GW_SMEM);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "gram_words smem attribute");
   pdl(gram_words_kernel<MODE>, grid, GR_THREADS, GW_SMEM, st)(a, M, tc_error_word());
   salsaa_count_launch();

@@ -579,7 +579,8 @@ __global__ void __launch_bounds__(TAIL_THREADS) sc_tail_kernel(const u64* in, u6
   // every round of this (rep, row) is summed: its claims and polynomials
   __syncthreads();
   for (u32 t = threadIdx.x; t < nr; t += TAIL_THREADS)
-    sc_poly(sums_of(t), M, (rep ? polys1 : polys0) + ((u64)t * rows + k) * 3, rep == 0 && t == 0 ? claims + k : nullptr);
+    sc_poly(sums_of(t), M, (rep ? polys1 : polys0) + ((u64)t * rows + k) * 3,
+            rep == 0 && t == 0 ? claims + k : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1103,12 +1104,8 @@ int launch_sumcheck(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, const De
   const u64 used = 2ULL * nr * rows * 3, full = used + gram_words(rows);
   cudaError_t e = cudaMemsetAsync(B.sums, 0, (full < B.sums_words ? full : B.sums_words) * sizeof(u64), st);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "sumcheck memset");
-  int rc = lazy ? sumcheck_passes<true>(w, rows, nlen, d, M, ds, round, B, nr, plain, st, w8, wide, proof_claims, proof_rep0,
-                                      proof_rep1)
-                : sumcheck_passes<false>(w, rows, nlen, d, M, ds, round, B, nr, plain, st, w8, wide, proof_claims, proof_rep0,
-                                      proof_rep1);
-  if (rc) return rc;
-  return 0;
+  auto passes = lazy ? sumcheck_passes<true> : sumcheck_passes<false>;
+  return passes(w, rows, nlen, d, M, ds, round, B, nr, plain, st, w8, wide, proof_claims, proof_rep0, proof_rep1);
 }
 
 // ---------------------------------------------------------------------------

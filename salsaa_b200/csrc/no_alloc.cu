@@ -46,7 +46,9 @@ typedef int (*CtxGetCurrentFn)(void**);
 CtxGetCurrentFn g_ctx_get_current = nullptr;
 
 __global__ void noalloc_seed_kernel(DevState* ds, u64 seed) {
-  pdl_wait(); ds->seed = seed; }
+  pdl_wait();
+  ds->seed = seed;
+}
 
 // The current driver context, through the runtime's driver entry-point lookup
 // (no link-time dependency on the driver library).

@@ -81,8 +81,8 @@ struct TcRed {
 //
 // SHORT (n = 64, one limb): for y > 0 column k = 0 of the matrix is zero (its
 // entry is 1), so |d_y| <= 63 x 255 x 128, and byte 6 is at most 3: pairs
-// combine in 32 bits and |hi + (lo >> 32)| < 2^31 - 2^24.  With hb = 2^31 - (less than 2^18), x lies in [0, 2^32), and
-// c = floor(x k / 2^49) is at most x 2^32 / q and less than 1 + 2^-17 below it.
+// combine in 32 bits and |hi + (lo >> 32)| < 2^31 - 2^24.  With hb = 2^31 - (less than
+// 2^18), x lies in [0, 2^32), and c = floor(x k / 2^49) is at most x 2^32 / q and less than 1 + 2^-17 below it.
 // Else |hi + (lo >> 32)| < 2^41, hb about 2^41, x < 2^42, and
 // c = floor(floor(x / 2^10) k / 2^39) is less than 1 + 2^-7 + 2^-7 below.
 template <bool SHORT>
@@ -154,7 +154,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) ntt_tc_kernel(TcArgs a, CkImage
                                                                u64 q, TcRed red, u32* err) {
   pdl_wait();
   using Geo = TcGeom<LOGN, MODE>;
-  constexpr u32 N = Geo::N, D = Geo::D, SEL = Geo::SEL, SELLOG = Geo::SELLOG, SUB = Geo::SUB, WPT = Geo::WPT, JG = Geo::JG, US = Geo::IU;
+  constexpr u32 N = Geo::N, D = Geo::D, SEL = Geo::SEL, SELLOG = Geo::SELLOG, SUB = Geo::SUB, WPT = Geo::WPT;
+  constexpr u32 JG = Geo::JG, US = Geo::IU;
   constexpr u32 EPI = MODE == TC_LIMBS ? 128 : 256;  // threads per unit
   // a barrier pair per set of threads that shares units, so each set sees
   // every phase of its own (a parity wait cannot skip one)

@@ -302,7 +302,7 @@ static Shapes walk(const salsaa_params* p) {
   // the sumcheck's former full-length buffers took; a set for which that is
   // not enough (no rounds, one folded row) keeps the slot-form path, so no
   // slot needs more memory than it did.
-  const u64 room = (S.max_fp_width + S.max_nc_rows_width * 7 / 8 + S.max_nc_rows_width / 2 - S.max_nc_rows_width / 128) * d;
+  const u64 nc = S.max_nc_rows_width, room = (S.max_fp_width + nc * 7 / 8 + nc / 2 - nc / 128) * d;
   S.use_short = S.use_img && (d == 128 || d == 256) && q > (1ULL << 49) && (u32)q >= (1u << 16) &&
                 S.max_img / 8 + short_words(S.max_d_rows_width, S.max_fp_width, d) <= room;
   S.use_img = S.use_img && S.max_img / 8 <= room;

@@ -15,8 +15,10 @@ __host__ __device__ constexpr u32 idesc_s8(u32 M, u32 N) { return IDESC_S8 | ((N
 // ---------------------------------------------------------------------------
 // Fold (src/subroutines/fold.rs:22-27) in coefficient form: with ternary
 // challenges c_k and byte rows w_k, out = sum_k c_k w_k mod X^d + 1 is an
-// exact integer product of negacyclic Toeplitz matrices (entries -1, 0, 1)
-// with the rows, |out| <= 8 x 256 x 128 < 2^19: no transforms at all.  Per
+// exact integer product of negacyclic Toeplitz matrices with the rows, no
+// transforms at all: |out| <= 8 x 256 x 128 <= 2^18 for the proof's ternary
+// challenges and, since launch_fold_words_tz takes coefficients up to 127,
+// <= 8 x 256 x 127 x 128 < 2^25 for given ones, either way within the s32 sums.  Per
 // (row, 64 elements): M = 128 output positions, N = 64 elements, K = d
 // positions, accumulated over the rows in TMEM.
 //
@@ -211,9 +213,10 @@ __global__ void fold_chal_tz_kernel(const DevState* ds, u32 round, u32 rows, u32
 // (byte row, positions) changes, then adds them to the accumulators.  Where
 // sc_umma_kernel turns every value into three byte limbs, here both operands
 // are bulk copies.  Bound by the copies' latency and L2 traffic: 16 KB per 64
-// elements with 16 rows; a launch takes two groups of 16 rows.  Together with the products that the proof no longer
-// recomputes (<projected_lhs, folded> is a combination of <projected_lhs, w_k>):
-// 1222 -> 374 us of an 8-round proof over 2^19 elements, d = 128.
+// elements with 16 rows; a launch takes two groups of 16 rows.  Together with
+// the products that the proof no longer recomputes (<projected_lhs, folded> is
+// a combination of <projected_lhs, w_k>): 1222 -> 374 us of an 8-round proof
+// over 2^19 elements, d = 128.
 // ---------------------------------------------------------------------------
 constexpr u32 ST_EPI = 256, ST_THREADS = ST_EPI + 64, ST_STAGES = 8;
 constexpr u32 ST_A = 64 * 128, ST_STAGE = ST_A + 64 * 128;
@@ -288,7 +291,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
     for (u32 item = i0; ok && item < i1; item++) {
       if (!open(item)) continue;
       const u32 nb = ui & 1;
-      const u32 idesc = (2u << 4) | (1u << 7) | (1u << 15) | ((ncol(group(item / per)) >> 3) << 17) | ((128u >> 4) << 24);
+      const u32 np = ncol(group(item / per));
+      const u32 idesc = (2u << 4) | (1u << 7) | (1u << 15) | ((np >> 3) << 17) | ((128u >> 4) << 24);
       if (ui >= 2 && !(ok = umma::mbar_wait(&acc_empty[nb], ((ui >> 1) - 1) & 1, err, 53))) break;
       umma::fence_after_sync();
       for (u32 c = 0; c < steps; c++, it++) {
@@ -298,7 +302,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
         if (umma::elect_one()) {
 #pragma unroll
           for (u32 ks = 0; ks < 2; ks++)
-            umma::mma_i8_u(tmem + nb * 128, ad0 + so + ks * 32, bd0 + so + ks * 256, idesc, (c > 0 || ks > 0) ? 1u : 0u);
+            umma::mma_i8_u(tmem + nb * 128, ad0 + so + ks * 32, bd0 + so + ks * 256, idesc,
+                           (c > 0 || ks > 0) ? 1u : 0u);
           umma::commit(&empty_bar[st]);
           if (c + 1 == steps) umma::commit(&acc_full[nb]);
         }
@@ -368,7 +373,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1)
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
-// The same blocks from words.
+// fold_chal_tz_kernel's Toeplitz blocks of given challenges c (rows x d words).
 __global__ void fold_words_tz_kernel(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* wide) {
   pdl_wait();
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -392,7 +397,8 @@ __global__ void fold_words_tz_kernel(const u64* c, u32 rows, u32 d, u64 q, int8_
 // 16-byte unit is one store and the warp's 256 bytes are one run.  Bound by
 // HBM: nine bytes a value.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u64 wpad, u32 d, u64 q, int8_t* c8, u32* wide) {
+__global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u64 wpad, u32 d, u64 q, int8_t* c8,
+                                                          u32* wide) {
   pdl_wait();
   const u32 lane = threadIdx.x & 31, k = blockIdx.y, npg = d / 16;
   const u64 tasks = wpad / 16 * npg, half_q = q >> 1;
@@ -591,7 +597,8 @@ int launch_fold_words_tz(const u64* c, u32 rows, u32 d, u64 q, int8_t* tz, u32* 
 
 int launch_fold_tc(const C8Rows& w, u32 d, u64 q, const int8_t* tz, u64 nout, u64* out, u64* mag_or, const u32* flag,
                    cudaStream_t st) {
-  if (!fold_tc_ok(w, d) || !flag || nout > w.width) return salsaa_set_error(-2, "fold_tc: rows outside the byte-tile path");
+  if (!fold_tc_ok(w, d) || !flag || nout > w.width)
+    return salsaa_set_error(-2, "fold_tc: rows outside the byte-tile path");
   const size_t ring = d == 128 ? (size_t)FtGeom<128>::STAGES * FtGeom<128>::TILE
                                : (size_t)FtGeom<256>::STAGES * FtGeom<256>::TILE;
   const size_t smem = (size_t)w.rows * 32 * d + ring;
