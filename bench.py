@@ -411,7 +411,10 @@ def run_ours(args):
     serial = plain_run(False, True)
     traced = None
     if args.plain_proofs > 1:
-        traced = {k: trace_read("ck_umma_kernel" + k) for k in ("", ":int8", ":mac")}
+        # shapes outside the byte image take the kernel over slot-form words
+        name = next((n for n in ("ck_img_kernel", "ck_umma_kernel") if trace_read(n)["launches"]), "ck_img_kernel")
+        traced = {k: trace_read(name + k) for k in ("", ":int8", ":mac")}
+        traced["name"] = name
     lib().salsaa_trace_enable(0)
     # then latency mode: each round's projection and each commitment's
     # statement rows run on a second stream beside the main chain
@@ -914,14 +917,14 @@ CK_TRAFFIC_CMD = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu_
 
 def roofline_ck(traced, elapsed_ms, a0):
     """Dominant kernel of the prove: the commitment-key rows on the tensor
-    cores.  Its bound is HBM: the algorithmic bytes are the slot-form witness
-    read once and the accumulators written once, against the measured copy
-    bandwidth.  Beside it, the tensor-pipe fraction (int8 operations the
-    tensor cores execute, against NVIDIA's dense int8 rate, which is twice
-    the dense bf16 rate; the bf16 rate is measured here) and the exact mod-q
-    multiply-accumulates per second.  elapsed_ms: summed device time of the
-    traced plain proofs; a0: the default A0 workload, the one the traffic
-    capture covers."""
+    cores.  The algorithmic bytes are the witness' byte image (7 of every 8
+    bytes of its words) and the key tiles read once and the accumulators
+    written once, against the measured copy bandwidth.  Beside it, the
+    tensor-pipe fraction (int8 operations the tensor cores execute, against
+    NVIDIA's dense int8 rate, which is twice the dense bf16 rate; the bf16
+    rate is measured here) and the exact mod-q multiply-accumulates per
+    second.  elapsed_ms: summed device time of the traced plain proofs; a0:
+    the default A0 workload, the one the traffic capture covers."""
     if not traced or not traced[""]["launches"]:
         return None
     t, t8, tm = traced[""], traced[":int8"], traced[":mac"]
@@ -934,7 +937,7 @@ def roofline_ck(traced, elapsed_ms, a0):
     ops = t8["work"] / t8["launches"]
     tops = ops / (per_ms * 1e-3) / 1e12
     macs = tm["work"] / tm["launches"]
-    return {"kernel": "ck_img_kernel (exact int8 limb-split commitment, tcgen05.mma kind::i8, TMEM; traced as ck_umma_kernel)",
+    return {"kernel": "%s (exact int8 limb-split commitment, tcgen05.mma kind::i8, TMEM)" % traced["name"],
             "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "peak_kind": hbm_kind + " copy bandwidth",
             "traffic": CK_TRAFFIC_A0 if a0 else None,

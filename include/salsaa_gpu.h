@@ -135,14 +135,18 @@ int salsaa_scratch_release(void);
 /* Device-time trace for measurement (off by default): enable/reset, then read
  * the summed device time (CUDA events on the launching stream), summed
  * algorithmic work and launch count of a traced kernel by name.  Traced:
- * "ck_umma_kernel" (work = algorithmic HBM bytes: the slot-form witness read
- * once and the accumulators written once), "ck_umma_kernel:int8" (the same
- * launches; work = int8 operations the tensor cores execute, 2 per byte-limb
- * product), "ck_umma_kernel:mac" (the same launches; work = exact mod-q
- * multiply-accumulates of the ring products), "ck_mma_kernel" (int8
- * operations), "nc_gram_kernel" (bytes), "ntt_kernel" (16 bytes per
- * coefficient) and "ntt_mul_kernel" (24 bytes per coefficient).  Reading
- * waits for the traced launches. */
+ * "ck_img_kernel" (work = the bytes it cannot do without: the witness' byte
+ * image and the key tiles read once, the accumulators written once),
+ * "ck_img_kernel:int8" (the same launches; work = int8 operations the tensor
+ * cores execute, 2 per byte-limb product), "ck_img_kernel:mac" (the same
+ * launches; work = exact mod-q multiply-accumulates of the ring products),
+ * "ck_umma_kernel", "ck_umma_kernel:int8", "ck_umma_kernel:mac" (the same of
+ * the key-row product over slot-form words, which are then what it reads),
+ * "ck_mma_kernel" (int8 operations), "gram_first" (a sumcheck's first pass:
+ * values read once, folded vectors written once), "ntt_kernel" (16 bytes per
+ * coefficient; transforms to the byte image what they read and write),
+ * "ntt_digits_kernel" (bytes) and "ntt_mul_kernel" (24 bytes per
+ * coefficient).  Reading waits for the traced launches. */
 void salsaa_trace_enable(int on);
 int salsaa_trace_read(const char* name, double* total_ms, double* total_work, uint64_t* launches);
 /* Fill *out with preset "A0".."C2", "F0".."F2" (src/protocol.rs:28-123). */

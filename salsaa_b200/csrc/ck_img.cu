@@ -20,9 +20,10 @@ namespace {
 // chunks into a ring of stages, warp 9 issues the MMAs, warps 0 .. 7 turn
 // finished accumulators into residues.  What bounds it is the L2 -> shared
 // memory traffic of the chunks (19 KB per chunk and accumulator at 9 witness
-// and 12 key rows, 10 .. 11 TB/s measured) and, for short witnesses, reading
-// the key table once (92 MB at 12 key rows); the MMAs take 176 of the about
-// 490 clocks of a chunk.  With 2 E nkp <= 512 columns the accumulators are
+// and 12 key rows: 12.6 TB/s, and 6.2 from DRAM, at 9 rows x 2^16; 7.5 and 4.7
+// at 3 rows x 2^17, whose accumulators share key tiles) and, for short
+// witnesses, reading the key table once (92 MB at 12 key rows); the tensor
+// pipe is busy 41 .. 42% of the time.  With 2 E nkp <= 512 columns the accumulators are
 // double-buffered, so the epilogue runs beside the next tile's MMAs.
 //
 // Epilogue: a thread folds the 7 key bytes x of its TMEM lane's sums into a
@@ -33,8 +34,8 @@ namespace {
 // for the MMAs: a dependent global load takes microseconds under the copies.
 //
 // One A0 proof's eight launches (B200, summed): 1932 us in ck_umma_kernel,
-// which split words into bytes itself.  Round 0 (3 rows x 2^18): 439 -> 167
-// us, round 1 (9 x 2^17): 593 -> 197 us.
+// which split words into bytes itself, 590 here.  Round 0 (3 rows x 2^18): 439
+// -> 167 us, round 1 (9 x 2^17): 593 -> 197 us.
 //
 // Every wait is bounded; a role that gives up stops, and the others then
 // give up on the arrivals it no longer makes.
@@ -395,11 +396,11 @@ int launch_ck_img(const CkImgArgs& a, const CkImage& im, const ModQ& M, const u6
   cudaError_t e = smem_limit(kern, most);
   if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ck_img smem attribute");
   const bool plain = M.q < (1ULL << 50) && im.width / t.Bw < (1ULL << 13);
-  const double wit_bytes = 8.0 * im.R * (double)im.width * 2 * im.n;
-  const double out_bytes = 8.0 * a.nck * im.R * 2 * im.n;
-  const int tr = salsaa_trace_begin("ck_umma_kernel", st, wit_bytes + out_bytes);
-  salsaa_trace_alias(tr, "ck_umma_kernel:int8", 2.0 * 196.0 * a.nck * im.R * (double)im.width * im.n);
-  salsaa_trace_alias(tr, "ck_umma_kernel:mac", (double)a.nck * im.R * (double)im.width * 2 * im.n);
+  // the image and the key table's tiles once, the sums once
+  const double bytes = (double)cki_bytes(im) + (double)((u64)im.n * nkp << im.btlog) + 8.0 * a.nck * im.R * 2 * im.n;
+  const int tr = salsaa_trace_begin("ck_img_kernel", st, bytes);
+  salsaa_trace_alias(tr, "ck_img_kernel:int8", 2.0 * 196.0 * a.nck * im.R * (double)im.width * im.n);
+  salsaa_trace_alias(tr, "ck_img_kernel:mac", (double)a.nck * im.R * (double)im.width * 2 * im.n);
   const u32 grid = t.ntiles < 148 ? t.ntiles : 148;
   pdl(kern, grid, CKI_THREADS, smem, st)(a.tk8, im, t, a.nck, nkp, nkc, a.thi, a.ck_nhi, M, zeta, a.acc,
                                                  plain, tc_error_word());

@@ -1045,7 +1045,8 @@ static int sumcheck_passes(RowSet w, u32 rows, u64 nlen, u32 d, const ModQ& M, c
     if (gram_room(rows) && gram_words_ok(L, M.q)) {
       u64* g = gram_take(rows, 1);
       const bool c8 = w8 && wide && sumcheck_reads_bytes(*w8, L, d, M.q);
-      const int tr = salsaa_trace_begin("nc_gram_kernel", st, (double)rows * L * 8.0 * (1.0 + 2.0 / 16.0));
+      // a value read (a byte of the tiles, else a word) and both repetitions' folded sixteenths written
+      const int tr = salsaa_trace_begin("gram_first", st, (double)rows * L * ((c8 ? 1.0 : 8.0) + 2.0 * 8.0 / 16.0));
       if (c8 && (rc = launch_gram_c8(*w8, d, M, ds, round, B.a, sa, g, wide, st))) return rc;
       if ((rc = launch_gram_first(w, rows, L, M, ds, round, B.a, sa, g, c8 ? wide : nullptr, st))) return rc;
       salsaa_trace_end(tr, st);

@@ -253,8 +253,8 @@ int img_go(const ImgDigits& a, const CkImage& im, const NttDev& T, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo::SMEM);
     if (e != cudaSuccess) return salsaa_set_cuda_error(e, "ntt_img smem attribute");
   }
-  // 16 bytes per coefficient read and written as words would be; the image is 7
-  const double coeffs = (double)a.rows.rows * a.rows.width * Geo::D;
+  // words in, words out or 7 image bytes; nothing behind a gate, which is nearly always closed
+  const double coeffs = a.rows.gate ? 0.0 : (double)a.rows.rows * a.rows.width * Geo::D;
   const int tr = salsaa_trace_begin(DIG ? "ntt_digits_kernel" : "ntt_kernel", st,
                                     coeffs * (DIG ? 8 + 2 * (7 + 4 + (a.rows.slots ? 8 : 0))
                                                   : 15 + (a.rows.slots ? 8 : 0)));

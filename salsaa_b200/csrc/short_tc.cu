@@ -394,8 +394,8 @@ __global__ void fold_words_tz_kernel(const u64* c, u32 rows, u32 d, u64 q, int8_
 // Words to byte tiles.  A warp takes 16 elements x 16 positions: eight lanes
 // read the 128 bytes of an element's 16 words, and after each lane has put
 // its bytes together (two a word pair, then eight lanes' by shuffles) every
-// 16-byte unit is one store and the warp's 256 bytes are one run.  Bound by
-// HBM: nine bytes a value.
+// 16-byte unit is one store and the warp's 256 bytes are one run.  Nine
+// bytes a value at 4.8 .. 5.1 TB/s of DRAM and 58% of the issue slots.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) words_to_c8_kernel(RowSet src, u64 width, u64 wpad, u32 d, u64 q, int8_t* c8,
                                                           u32* wide) {
